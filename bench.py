@@ -236,9 +236,9 @@ def algorithmic_bytes(kernel, w, nvol, nang, planes, batch=1, npk=0, energies=No
             "k_fft_rows": 2 * 8 * npk * V,
             "k_fft_cols<y>": 2 * 8 * npk * V,
             "k_fft_cols<z>": 8 * npk * V * (zload + zstore),
-            "k_fft_pass<x>": 2 * 8 * npk * V,
-            "k_fft_pass<y>": 2 * 8 * npk * V,
-            "k_fft_pass<z>": 2 * 8 * npk * V,
+            "k_mix_fft<x>": 2 * 8 * npk * V,
+            "k_mix_fft<y>": 2 * 8 * npk * V,
+            "k_mix_fft<z>": 2 * 8 * npk * V,
             # two planes of Z_j(k) and Z_j(-k) per pixel and energy, Gram maps out
             "k_ewald_fields": batch * (4 * 8 * npk * P + nq * P),
             "k_rotate_gram": batch * (nq * P + 4 * P),
@@ -258,9 +258,9 @@ def algorithmic_bytes(kernel, w, nvol, nang, planes, batch=1, npk=0, energies=No
         "k_build": (16 * M + 8 * nvol) * V,
         "k_build_fft_z": 16 * M * V + 8 * nvol * planes * P,
         "k_moments": 16 * M * V,
-        "k_fft_pass<x>": 2 * 8 * nvol * planes * P,
-        "k_fft_pass<y>": 2 * 8 * nvol * planes * P,
-        "k_fft_pass<z>": 2 * 8 * nvol * V,
+        "k_mix_fft<x>": 2 * 8 * nvol * planes * P,
+        "k_mix_fft<y>": 2 * 8 * nvol * planes * P,
+        "k_mix_fft<z>": 2 * 8 * nvol * V,
         "k_rotate_average": 4 * nang * P + 4 * P,
         "k_fill": 4 * P,
         "k_warp": 8 * P,

@@ -13,7 +13,7 @@
 //   MATERIAL frame: p = R^T Nt R x depends on the angle non-linearly; the
 //   engine runs the reference's per-angle schedule (3 volumes per angle).
 //
-//   k_build -> k_fft_pass<x,y,z> -> k_dc -> per k: k_ewald_angles ->
+//   k_build -> 3D FFT -> k_dc -> per k: k_ewald_angles ->
 //   k_rotate_average -> k_fill + k_warp (detector) -> projection[e][k]
 //
 // FIELDS strategy (fields.cuh): the spectra of the 7 M + 1 energy independent
@@ -54,6 +54,7 @@
 #include "../../include/cyrsoxs.h"
 #include "geometry.h"
 #include "kernels.cuh"
+#include "mixfft.cuh"
 #include "fields.cuh"
 #include "fp64.cuh"
 
@@ -118,10 +119,9 @@ bool smooth7(uint32_t n) {
   return factorize(n, r);
 }
 
-// Lengths with a prime factor above 7 run as Bluestein transforms over a
-// padded length M >= 2N - 1, itself limited to one block's FFT: the next power
-// of two while that is at most 1024 (the warp FFT's lengths), else the
-// smallest 7-smooth M.
+// The FP64 pipeline's padded length M >= 2N - 1 for lengths with a prime
+// factor above 7: the next power of two while that is at most 1024, else the
+// smallest 7-smooth M.  It also bounds the lengths both precisions accept.
 constexpr uint32_t kMaxBluesteinPad = 4096;
 uint32_t bluestein_length(uint32_t n) {
   uint32_t p2 = 128;
@@ -148,6 +148,122 @@ bool fft_length_ok(uint32_t n, const char **why) {
     return false;
   }
   return true;
+}
+
+// ---------------------------------------------------------------------------
+// Mixed-radix plans (mixfft.cuh)
+// ---------------------------------------------------------------------------
+// Radices of M with the least work: instructions per point of each radix's
+// butterfly plus a fixed cost per stage (its shared-memory round trip,
+// twiddles and barrier), so few stages of large radices; 0 when M has a prime
+// factor above 13.
+uint32_t mix_radices(uint32_t M, uint32_t most, std::vector<uint32_t> &radix) {
+  static constexpr uint8_t kPoint[kMixMaxRadix + 1] = {0, 0, 3, 6, 5, 9, 8, 13, 8, 12, 12, 21, 11, 25, 16, 15, 11};
+  constexpr uint32_t kStage = 6;
+  radix.clear();
+  if (M == 1) return 0;
+  uint32_t best = 0;
+  for (uint32_t r = std::min<uint32_t>(most, M); r >= 2; --r) {
+    if (M % r) continue;
+    std::vector<uint32_t> rest;
+    const uint32_t c = M == r ? 0 : mix_radices(M / r, r, rest);
+    if (M != r && rest.empty()) continue;
+    const uint32_t cost = c + kStage + kPoint[r];
+    if (best == 0 || cost < best) {
+      best = cost;
+      radix = rest;
+      radix.insert(radix.begin(), r);
+    }
+  }
+  return best;
+}
+
+// The radices of a transform of n points, with a penalty on unequal ones:
+// the threads that hold the butterflies of the small radix idle in the stage
+// of the large one.
+bool mix_best(uint32_t n, std::vector<uint32_t> &best) {
+  best.clear();
+  double least = 0;
+  std::vector<uint32_t> r;
+  for (uint32_t most = 2; most <= uint32_t(kMixMaxRadix); ++most) {
+    const uint32_t c = mix_radices(n, most, r);
+    if (c == 0 || r.size() > size_t(kMixMaxStages)) continue;
+    const double cost = c + 3.0 * r.front() / r.back();
+    if (best.empty() || cost < least) best = r, least = cost;
+  }
+  return !best.empty();
+}
+
+bool mix_length(uint32_t n) {
+  std::vector<uint32_t> r;
+  return mix_best(n, r);
+}
+
+// Padded length of a Bluestein transform of n points: the 7-smooth M >= 2n - 1 with the least work.
+uint32_t mix_bluestein_length(uint32_t n) {
+  const uint32_t lo = 2 * n - 1;
+  uint32_t best = 0;
+  uint64_t least = 0;
+  std::vector<uint32_t> r;
+  for (uint32_t m = lo; m <= std::min(2 * lo, kMaxBluesteinPad); ++m) {
+    if (!smooth7(m)) continue;
+    const uint64_t c = uint64_t(m) * mix_radices(m, kMixMaxRadix, r);
+    if (best == 0 || c < least) best = m, least = c;
+  }
+  return best;
+}
+
+// The stages of a transform of M points; row: with the row form's padding.
+struct MixPlan {
+  uint32_t M = 0, ns = 0, line_slots = 0, pad = 0, rs = 1, tw_len = 0, most_nb = 0;
+  MixStage st[kMixMaxStages];
+  std::vector<uint32_t> first;
+};
+
+uint32_t mix_magic(uint32_t d) { return d < 2 ? 0u : uint32_t(((uint64_t(1) << 32) + d - 1) / d); }
+
+int mix_plan(uint32_t M, bool row, MixPlan &pl) {
+  std::vector<uint32_t> r;
+  if (!mix_best(M, r))
+    return fail(CYR_ERR_UNSUPPORTED, "FFT length %u has a prime factor above 13", M);
+  // an odd radix last, when there is one: the row form's last stage then needs no padding
+  std::sort(r.begin(), r.end(), std::greater<uint32_t>());
+  auto odd = std::find_if(r.begin(), r.end(), [](uint32_t v) { return v & 1u; });
+  if (odd != r.end()) {
+    const uint32_t v = *odd;
+    r.erase(odd);
+    r.push_back(v);
+  }
+  pl.M = M;
+  pl.ns = uint32_t(r.size());
+  pl.rs = r.back();
+  pl.pad = row && pl.ns > 1 && pl.rs % 2 == 0 ? 1 : 0;
+  pl.tw_len = pl.most_nb = 0;
+  uint32_t L = M;
+  for (uint32_t s = 0; s < pl.ns; ++s) {
+    MixStage &st = pl.st[s];
+    st.radix = r[s];
+    st.nb = M / r[s];
+    st.nb_magic = mix_magic(st.nb);
+    st.m = L / r[s];
+    st.m_magic = mix_magic(st.m);
+    st.block = L / pl.rs * (pl.rs + pl.pad);
+    st.span = s + 1 < pl.ns ? st.m / pl.rs * (pl.rs + pl.pad) : 1;
+    st.tw = pl.tw_len;
+    if (s + 1 < pl.ns) pl.tw_len += st.m * ((r[s] + 1) & ~1u);
+    pl.most_nb = std::max(pl.most_nb, st.nb);
+    L = st.m;
+  }
+  // three stages, rows: blocks of the second stage an odd number of slots apart, as the last stage's lanes walk them
+  if (row && pl.ns == 3 && pl.st[0].span % 2 == 0) ++pl.st[0].span;
+  if (pl.ns == 3) pl.st[1].block = pl.st[0].span;
+  pl.line_slots = pl.ns > 1 ? r[0] * pl.st[0].span : 0;
+  pl.first.assign(M / pl.rs, 0);
+  for (uint32_t fb = 0; fb < M / pl.rs; ++fb) {
+    uint32_t f = fb;
+    for (uint32_t s = 0; s + 1 < pl.ns; ++s) pl.first[fb] += f % r[s] * pl.st[s].span, f /= r[s];
+  }
+  return CYR_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -197,7 +313,7 @@ enum Stage {
   kFieldMeans, kBuildFields, kEwaldFields, kRotateGram, kFftRows, kFftColsY, kFftColsZ, kBluestein, kBuildFieldsRows,
   kZMask, kNumStages
 };
-const char *const kStageNames[kNumStages] = {"k_build", "k_fft_pass<x>", "k_fft_pass<y>", "k_fft_pass<z>", "k_dc",
+const char *const kStageNames[kNumStages] = {"k_build", "k_mix_fft<x>", "k_mix_fft<y>", "k_mix_fft<z>", "k_dc",
                                              "k_ewald_angles", "k_rotate_average", "k_fill", "k_warp",
                                              "k_moments", "k_entry_means", "k_build_fft_z",
                                              "k_field_means", "k_build_fields", "k_ewald_fields", "k_rotate_gram",
@@ -249,7 +365,6 @@ struct ZTune {
 // share the device context's; every serving slot owns one.
 struct Scratch {
   DeviceBuffer spec, images, avg, params, dc, moments, means, errors, conv, flags, fmean;
-  DeviceBuffer blue;               // padded lines of the Bluestein transforms
   DeviceBuffer zmask;              // store mask of the FIELDS z pass (k_zmask)
   cudaEvent_t last_use = nullptr;  // completion of the last request that used it
   uint64_t generation = 0;         // bumped by every (re)allocation of a buffer above
@@ -259,11 +374,11 @@ struct Scratch {
   }
   // serving slots: stream-ordered allocations on `st`
   void bind(cudaStream_t st) {
-    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &moments, &means, &errors, &conv, &flags, &fmean, &blue, &zmask})
+    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &moments, &means, &errors, &conv, &flags, &fmean, &zmask})
       b->stream = st, b->generation = &generation;
   }
   void release() {
-    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &moments, &means, &errors, &conv, &flags, &fmean, &blue, &zmask})
+    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &moments, &means, &errors, &conv, &flags, &fmean, &zmask})
       b->release();
   }
 };
@@ -301,11 +416,18 @@ struct DeviceContext {
   bool attrs_done = false;
   bool attrs64 = false;                    // the FP64 FFT kernels' shared-memory attribute is set
   std::map<uint32_t, float2 *> twiddles;
-  struct BlueTables {
+  struct ConvTables {                   // a line length transformed as a convolution (get_conv)
     uint32_t m = 0;
-    float2 *chirp = nullptr, *bhat = nullptr;
+    void *chirp = nullptr, *bhat = nullptr;       // Bluestein: chirp set
+    uint32_t *in = nullptr, *out = nullptr;       // Rader: both set
   };
-  std::map<uint32_t, BlueTables> blue;  // per Bluestein line length
+  std::map<std::array<uint32_t, 2>, ConvTables> conv;  // key: length, bytes per real
+  struct MixTables {                    // one transform length and form of k_mix_fft
+    MixPlan plan;
+    void *tw = nullptr;
+    uint32_t *first = nullptr;
+  };
+  std::map<std::array<uint32_t, 3>, MixTables> mix;  // key: length, row form, bytes per real
   std::map<uint32_t, double2 *> tw64;   // FP64 twiddles W_n^m per length
   struct BlueTables64 {
     uint32_t m = 0;
@@ -363,9 +485,11 @@ int setup_attrs(DeviceContext &ctx) {
   std::lock_guard<std::mutex> lk(ctx.tables_mu);
   if (ctx.attrs_done) return CYR_OK;
   const int smem = int(kFftSmemBudget);
-  CYR_CUDA(cudaFuncSetAttribute(k_fft_pass<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CYR_CUDA(cudaFuncSetAttribute(k_fft_pass<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CYR_CUDA(cudaFuncSetAttribute(k_fft_pass<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+#define CYR_MIX_ATTR(T, C, B) \
+  CYR_CUDA(cudaFuncSetAttribute(k_mix_fft<T, C, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  CYR_MIX_ATTR(float2, false, kMixPlain) CYR_MIX_ATTR(float2, false, kMixBluestein) CYR_MIX_ATTR(float2, false, kMixRader)
+  CYR_MIX_ATTR(float2, true, kMixPlain) CYR_MIX_ATTR(float2, true, kMixBluestein) CYR_MIX_ATTR(float2, true, kMixRader)
+#undef CYR_MIX_ATTR
 #define CYR_COLS_ATTR(V, T) \
   CYR_CUDA(cudaFuncSetAttribute(k_fft_cols<V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   CYR_COLS_ATTR(32, 8)
@@ -644,110 +768,185 @@ int thread_fft_pass(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, 
   return CYR_OK;
 }
 
-// Chirp c_j = exp(-i pi j^2 / n) and bhat = FFT_m(b) / m, b_j = conj(c_j) at j
-// and m - j: in double (j^2 mod 2n in integers, a direct DFT with exact index
-// arithmetic), rounded to float, once per length and device.
-int get_blue(DeviceContext &ctx, uint32_t n, DeviceContext::BlueTables &out) {
+// Tables of an n-point transform as a convolution (mixfft.cuh): Rader's when
+// n is prime and n - 1 has radices up to 16 (half Bluestein's length or less),
+// else Bluestein's chirp.  In double (a direct DFT with exact index
+// arithmetic), rounded to T, once per length and device.
+template <class T>
+int get_conv(DeviceContext &ctx, uint32_t n, const DeviceContext::ConvTables **out) {
   std::lock_guard<std::mutex> lk(ctx.tables_mu);
-  auto it = ctx.blue.find(n);
-  if (it != ctx.blue.end()) {
-    out = it->second;
+  const std::array<uint32_t, 2> key{n, uint32_t(sizeof(T) / 2)};
+  auto it = ctx.conv.find(key);
+  if (it != ctx.conv.end()) {
+    *out = &it->second;
     return CYR_OK;
   }
-  const uint32_t m = bluestein_length(n);
-  std::vector<std::complex<double>> c(n), b(m, 0.0), w(m);
-  for (uint32_t j = 0; j < n; ++j) {
-    const uint64_t q = (uint64_t(j) * j) % (2 * uint64_t(n));
-    c[j] = std::polar(1.0, -kPi * double(q) / double(n));
-  }
-  for (uint32_t j = 0; j < n; ++j) {
-    b[j] = std::conj(c[j]);
-    if (j) b[m - j] = std::conj(c[j]);
+  DeviceContext::ConvTables t;
+  bool prime = true;
+  for (uint32_t d = 2; d * d <= n; ++d) prime = prime && n % d != 0;
+  const bool rader = prime && n - 1 > uint32_t(kMixMaxRadix) && mix_length(n - 1);  // two stages at least
+  t.m = rader ? n - 1 : mix_bluestein_length(n);
+  const uint32_t m = t.m;
+  std::vector<std::complex<double>> b(m, 0.0), w(m);
+  std::vector<T> hc;
+  std::vector<uint32_t> in, inv;
+  if (rader) {
+    uint32_t g = 2;  // a generator: its powers meet every residue
+    for (;; ++g) {
+      in.clear();
+      uint32_t v = 1;
+      do in.push_back(v), v = uint32_t(uint64_t(v) * g % n);
+      while (v != 1);
+      if (in.size() == n - 1) break;
+    }
+    inv.resize(m);
+    for (uint32_t q = 0; q < m; ++q) inv[q] = in[(m - q) % m];
+    for (uint32_t q = 0; q < m; ++q) b[q] = std::polar(1.0, -2.0 * kPi * double(inv[q]) / double(n));
+  } else {
+    hc.resize(n);
+    for (uint32_t j = 0; j < n; ++j) {
+      const uint64_t q = (uint64_t(j) * j) % (2 * uint64_t(n));
+      const std::complex<double> c = std::polar(1.0, -kPi * double(q) / double(n));
+      hc[j] = T{Real<T>(c.real()), Real<T>(c.imag())};
+      b[j] = std::conj(c);
+      if (j) b[m - j] = std::conj(c);
+    }
   }
   for (uint32_t j = 0; j < m; ++j) w[j] = std::polar(1.0, -2.0 * kPi * double(j) / double(m));
-  std::vector<float2> hc(n), hb(m);
-  for (uint32_t j = 0; j < n; ++j) hc[j] = make_float2(float(c[j].real()), float(c[j].imag()));
+  std::vector<T> hb(m);
   for (uint32_t k = 0; k < m; ++k) {
     std::complex<double> acc(0.0, 0.0);
-    uint64_t idx = 0;  // (j k) mod m
-    for (uint32_t j = 0; j < m; ++j, idx += k) {
-      if (idx >= m) idx %= m;
+    uint32_t idx = 0;  // (j k) mod m
+    for (uint32_t j = 0; j < m; ++j) {
       acc += b[j] * w[idx];
+      idx += k;
+      if (idx >= m) idx -= m;
     }
     acc /= double(m);
-    hb[k] = make_float2(float(acc.real()), float(acc.imag()));
+    hb[k] = T{Real<T>(acc.real()), Real<T>(acc.imag())};
   }
-  DeviceContext::BlueTables t;
-  t.m = m;
-  CYR_CUDA(cudaMalloc(&t.chirp, sizeof(float2) * n));
-  CYR_CUDA(cudaMalloc(&t.bhat, sizeof(float2) * m));
-  CYR_CUDA(cudaMemcpy(t.chirp, hc.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
-  CYR_CUDA(cudaMemcpy(t.bhat, hb.data(), sizeof(float2) * m, cudaMemcpyHostToDevice));
-  ctx.blue[n] = t;
-  out = t;
+  auto upload = [](auto **dst, const auto &src) -> int {
+    CYR_CUDA(cudaMalloc(dst, src.size() * sizeof(src[0])));
+    CYR_CUDA(cudaMemcpy(*dst, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice));
+    return CYR_OK;
+  };
+  CYR_TRY(upload(&t.bhat, hb));
+  if (rader) {
+    CYR_TRY(upload(&t.in, in));
+    CYR_TRY(upload(&t.out, inv));
+  } else {
+    CYR_TRY(upload(&t.chirp, hc));
+  }
+  *out = &ctx.conv.emplace(key, t).first->second;  // map nodes do not move, and tables are never changed once made
   return CYR_OK;
 }
 
-int fft_axes(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, cudaStream_t st,
-             int first, int last, size_t vstride = 0, DeviceBuffer *work = nullptr, const uint32_t *forms = nullptr,
-             const uint32_t *zmask = nullptr);
-
-// One axis of length n (a prime factor above 7) as a Bluestein transform, in
-// chunks of padded lines of at most 256 MB held in `work`.
-int bluestein_pass(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, int axis,
-                   cudaStream_t st, size_t vstride, DeviceBuffer *work) {
-  const uint32_t n = axis == 0 ? nx : axis == 1 ? ny : nz;
-  DeviceContext::BlueTables bt;
-  CYR_TRY(get_blue(ctx, n, bt));
-  const uint32_t lpv = axis == 0 ? ny * nz : axis == 1 ? nx * nz : nx * ny;
-  const uint64_t total = uint64_t(lpv) * count;
-  // a multiple of 32 lines per chunk, so the column pass of y and z lines can use TMA tiles
-  const uint64_t cap = std::max<uint64_t>(32, (size_t(256) << 20) / (size_t(bt.m) * sizeof(float2)) / 32 * 32);
-  const uint32_t chunk = uint32_t(std::min<uint64_t>(total, cap));
-  CYR_TRY(work->ensure(size_t(chunk) * bt.m * sizeof(float2)));
-  int sms = 0;
-  CYR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
-  BlueParams p{};
-  p.data = data;
-  p.work = work->as<float2>();
-  p.chirp = bt.chirp;
-  p.bhat = bt.bhat;
-  p.nx = nx, p.ny = ny, p.nz = nz;
-  p.vstride = vstride;
-  p.n = n, p.m = bt.m;
-  p.lines_per_vol = lpv;
-  for (uint64_t l0 = 0; l0 < total; l0 += chunk) {
-    p.line0 = l0;
-    p.nlines = uint32_t(std::min<uint64_t>(chunk, total - l0));
-    const size_t elems = size_t(p.nlines) * bt.m;
-    const unsigned grid = unsigned(std::min<size_t>((elems + 255) / 256, size_t(sms) * 16));
-    int slot = ctx.prof.begin(kBluestein, st);
-    if (axis == 0) k_blue_gather<0><<<grid, 256, 0, st>>>(p);
-    if (axis == 1) k_blue_gather<1><<<grid, 256, 0, st>>>(p);
-    if (axis == 2) k_blue_gather<2><<<grid, 256, 0, st>>>(p);
-    ctx.prof.end(slot, st);
-    CYR_CUDA(cudaGetLastError());
-    // m is 7-smooth: rows of m (x lines) or columns of m (y and z lines)
-    auto padded_fft = [&]() -> int {
-      if (axis == 0) return fft_axes(ctx, p.work, bt.m, p.nlines, 1, 1, st, 0, 0);
-      return fft_axes(ctx, p.work, p.nlines, bt.m, 1, 1, st, 1, 1);
-    };
-    CYR_TRY(padded_fft());
-    slot = ctx.prof.begin(kBluestein, st);
-    if (axis == 0)
-      k_blue_mul<0><<<grid, 256, 0, st>>>(p);
-    else
-      k_blue_mul<1><<<grid, 256, 0, st>>>(p);
-    ctx.prof.end(slot, st);
-    CYR_CUDA(cudaGetLastError());
-    CYR_TRY(padded_fft());
-    slot = ctx.prof.begin(kBluestein, st);
-    if (axis == 0) k_blue_scatter<0><<<grid, 256, 0, st>>>(p);
-    if (axis == 1) k_blue_scatter<1><<<grid, 256, 0, st>>>(p);
-    if (axis == 2) k_blue_scatter<2><<<grid, 256, 0, st>>>(p);
-    ctx.prof.end(slot, st);
-    CYR_CUDA(cudaGetLastError());
+// Stage twiddles and block table of a k_mix_fft transform of M points.
+template <class T>
+int get_mix(DeviceContext &ctx, uint32_t M, bool row, const DeviceContext::MixTables **out) {
+  std::lock_guard<std::mutex> lk(ctx.tables_mu);
+  const std::array<uint32_t, 3> key{M, row ? 1u : 0u, uint32_t(sizeof(T) / 2)};
+  auto it = ctx.mix.find(key);
+  if (it == ctx.mix.end()) {
+    DeviceContext::MixTables t;
+    CYR_TRY(mix_plan(M, row, t.plan));
+    std::vector<T> h(std::max(1u, t.plan.tw_len));
+    for (uint32_t s = 0; s + 1 < t.plan.ns; ++s) {
+      const MixStage &st = t.plan.st[s];
+      const uint32_t L = st.m * st.radix, pitch = (st.radix + 1) & ~1u;
+      for (uint32_t j = 0; j < st.m; ++j)
+        for (uint32_t k = 0; k < pitch; ++k) {
+          const std::complex<double> w = std::polar(1.0, -2.0 * kPi * double(uint64_t(j) * k % L) / double(L));
+          h[st.tw + (row ? k * st.m + j : j * pitch + k)] = T{Real<T>(w.real()), Real<T>(w.imag())};
+        }
+    }
+    CYR_CUDA(cudaMalloc(&t.tw, h.size() * sizeof(T)));
+    CYR_CUDA(cudaMalloc(&t.first, t.plan.first.size() * sizeof(uint32_t)));
+    CYR_CUDA(cudaMemcpy(t.tw, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
+    CYR_CUDA(cudaMemcpy(t.first, t.plan.first.data(), t.plan.first.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    it = ctx.mix.emplace(key, std::move(t)).first;
   }
+  *out = &it->second;  // map nodes do not move, and tables are never changed once made
+  return CYR_OK;
+}
+
+constexpr size_t kMixSmem = 56 * 1024;       // four blocks per SM
+constexpr size_t kMixSmemMax = 200 * 1024;   // one (lengths above 1792 points in the narrowest tile)
+constexpr uint32_t kMixMinBlocks = 304;      // two blocks on each of the 152 SMs
+
+// One axis with k_mix_fft: lines of n points, as a convolution of length
+// tables->m when n has a prime factor above 13.
+// Columns per block (column form): as many as give 256 threads one butterfly
+// each, at least 32 so that a warp works on one butterfly index, fewer when
+// the tile would not leave room for four blocks per SM (240-point y lines on
+// 240 x 240 x 90, 11 volumes: 16 columns 153 us, 32 columns 170 us) or the
+// grid would not fill the SMs.  Rows: about 128 threads' worth per block
+// (450-point rows: 128 threads 704 us, 256 726, 512 815).
+template <class T>
+int mix_pass(DeviceContext &ctx, T *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, int axis,
+             cudaStream_t st, size_t vstride, const DeviceContext::ConvTables *conv = nullptr) {
+  const bool row = axis == 0;
+  const uint32_t n = axis == 0 ? nx : axis == 1 ? ny : nz, M = conv ? conv->m : n;
+  const DeviceContext::MixTables *t = nullptr;
+  CYR_TRY(get_mix<T>(ctx, M, row, &t));
+  const MixPlan &pl = t->plan;
+  MixParams<T> p{};
+  p.data = data;
+  p.nx = nx, p.ny = ny;
+  p.vstride = vstride;
+  p.n = n;
+  p.M = M;
+  p.ns = pl.ns;
+  p.line_slots = pl.line_slots;
+  p.pad = pl.pad, p.rs = pl.rs, p.rs_magic = mix_magic(pl.rs);
+  std::copy(pl.st, pl.st + pl.ns, p.st);
+  p.tw = static_cast<const T *>(t->tw);
+  p.first = t->first;
+  if (conv) {
+    p.chirp = static_cast<const T *>(conv->chirp), p.bhat = static_cast<const T *>(conv->bhat);
+    p.in = conv->in, p.out = conv->out;
+  }
+  constexpr uint32_t kMixT = uint32_t(kMixThreads);
+  size_t smem = 0;
+  uint32_t threads, blocks;
+  if (row) {
+    p.nlines = ny * nz;
+    const size_t line = size_t(pl.line_slots) * sizeof(T);
+    uint32_t rows = std::max(1u, 128 / pl.most_nb);
+    while (rows > 1 && rows * line > kMixSmem) rows = (rows + 1) / 2;
+    while (rows > 1 && uint64_t((p.nlines + rows - 1) / rows) * count < kMixMinBlocks) rows /= 2;
+    p.rows = rows;
+    blocks = (p.nlines + rows - 1) / rows;
+    threads = std::min(kMixT, (rows * pl.most_nb + 31) / 32 * 32);
+    smem = rows * line;
+  } else {
+    // the z pass sees one run of nx ny columns, the y pass nx columns per plane
+    p.nlines = axis == 1 ? nx : nx * ny;
+    const uint32_t others = axis == 1 ? nz : 1;
+    p.ostride = size_t(nx) * ny;
+    p.estride = axis == 1 ? nx : nx * ny;
+    uint32_t lg = 8;
+    auto tiles = [&] { return (p.nlines + (1u << lg) - 1) >> lg; };
+    while (lg > 5 && (pl.most_nb << lg) > kMixT) --lg;
+    while (lg > 2 && pl.ns > 1 && (size_t(M) << lg) * sizeof(T) > kMixSmem) --lg;
+    while (lg > 3 && (1u << (lg - 1)) >= p.nlines) --lg;
+    while (lg > 3 && uint64_t(tiles()) * others * count < kMixMinBlocks) --lg;
+    p.lg_tx = lg;
+    p.tiles = tiles();
+    blocks = p.tiles * others;
+    // the butterflies of a stage in equal rounds of at most kMixT threads
+    const uint32_t rounds = ((pl.most_nb << lg) + kMixT - 1) / kMixT;
+    threads = std::min(kMixT, ((((pl.most_nb + rounds - 1) / rounds) << lg) + 31) / 32 * 32);
+    smem = pl.ns > 1 ? (size_t(M) << lg) * sizeof(T) : 0;
+  }
+  if (smem > kMixSmemMax) return fail(CYR_ERR_UNSUPPORTED, "FFT length %u too large for one block", M);
+  auto kern = !conv       ? (row ? k_mix_fft<T, false, kMixPlain> : k_mix_fft<T, true, kMixPlain>)
+              : conv->in ? (row ? k_mix_fft<T, false, kMixRader> : k_mix_fft<T, true, kMixRader>)
+                         : (row ? k_mix_fft<T, false, kMixBluestein> : k_mix_fft<T, true, kMixBluestein>);
+  const int slot = ctx.prof.begin(conv ? int(kBluestein) : kFftX + axis, st);
+  kern<<<dim3(blocks, count), threads, smem, st>>>(p);
+  ctx.prof.end(slot, st);
+  CYR_CUDA(cudaGetLastError());
   return CYR_OK;
 }
 
@@ -755,57 +954,35 @@ int bluestein_pass(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, u
 // (0 x, 1 y, 2 z).  vstride (elements between volumes) defaults to the volume
 // size; a larger one runs the x and y passes on nz planes of larger volumes
 // (data pointing at the first plane), as the slab pipeline does.
-// Lengths with a prime factor above 7 use `work` (default: the device's main
-// scratch, for callers holding the context lock).
+// Axis lengths: 128-1024 powers of two run the warp FFT, 8-64 along y and z
+// one thread per line, every other length k_mix_fft.
 int fft_axes(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, cudaStream_t st,
-             int first, int last, size_t vstride, DeviceBuffer *work, const uint32_t *forms, const uint32_t *zmask) {
+             int first, int last, size_t vstride = 0, const uint32_t *forms = nullptr,
+             const uint32_t *zmask = nullptr) {
   const size_t nvox = vstride ? vstride : size_t(nx) * ny * nz;
   const uint32_t dims[3] = {nx, ny, nz};
   for (int axis = first; axis <= last; ++axis) {
     const uint32_t n = dims[axis];
     if (n == 1) continue;
-    if (!smooth7(n)) {
-      CYR_TRY(bluestein_pass(ctx, data, nx, ny, nz, count, axis, st, nvox, work ? work : &ctx.main.blue));
-      continue;
-    }
     if (n == 128 || n == 256 || n == 512 || n == 1024) {
       CYR_TRY(warp_fft_pass(ctx, data, nx, ny, nz, count, axis, st, nvox, forms ? forms[axis] : kFormAuto,
                             axis == 2 ? zmask : nullptr));
-      continue;
-    }
-    if (axis > 0 && (n == 8 || n == 16 || n == 32 || n == 64) && count <= 65535) {
+    } else if (axis > 0 && (n == 8 || n == 16 || n == 32 || n == 64) && count <= 65535) {
       CYR_TRY(thread_fft_pass(ctx, data, nx, ny, nz, count, axis, st, nvox));
-      continue;
-    }
-    FftPassParams p{};
-    p.data = data;
-    p.nx = nx, p.ny = ny, p.nz = nz;
-    p.nvox = nvox;
-    CYR_TRY(make_axis(ctx, n, p.ax));
-    p.tx = fft_lines_per_block(n);
-    const size_t smem = (size_t(2) * n * (p.tx + 1) + n) * sizeof(float2);
-    if (smem > kFftSmemBudget) return fail(CYR_ERR_UNSUPPORTED, "FFT length %u too large for one block", n);
-    uint32_t tiles;
-    if (axis == 0) {
-      tiles = (ny * nz + p.tx - 1) / p.tx;
+    } else if (mix_length(n)) {
+      CYR_TRY(mix_pass<float2>(ctx, data, nx, ny, nz, count, axis, st, nvox));
     } else {
-      const uint32_t nxt = (nx + p.tx - 1) / p.tx;
-      tiles = nxt * (axis == 1 ? nz : ny);
+      const DeviceContext::ConvTables *conv = nullptr;
+      CYR_TRY(get_conv<float2>(ctx, n, &conv));
+      CYR_TRY(mix_pass<float2>(ctx, data, nx, ny, nz, count, axis, st, nvox, conv));
     }
-    const dim3 grid(tiles, count);
-    const int slot = ctx.prof.begin(kFftX + axis, st);
-    if (axis == 0) k_fft_pass<0><<<grid, kFftThreads, smem, st>>>(p);
-    if (axis == 1) k_fft_pass<1><<<grid, kFftThreads, smem, st>>>(p);
-    if (axis == 2) k_fft_pass<2><<<grid, kFftThreads, smem, st>>>(p);
-    ctx.prof.end(slot, st);
-    CYR_CUDA(cudaGetLastError());
   }
   return CYR_OK;
 }
 
 int fft3d(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, cudaStream_t st,
-          bool skip_z = false, DeviceBuffer *work = nullptr) {
-  return fft_axes(ctx, data, nx, ny, nz, count, st, 0, skip_z ? 1 : 2, 0, work);
+          bool skip_z = false) {
+  return fft_axes(ctx, data, nx, ny, nz, count, st, 0, skip_z ? 1 : 2);
 }
 
 // ---------------------------------------------------------------------------
@@ -1427,7 +1604,7 @@ int build_fields_x(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const 
     k_build_fields<1><<<blocks, 256, 0, st>>>(fp);
   ctx.prof.end(slot, st);
   CYR_CUDA(cudaGetLastError());
-  return fft_axes(ctx, spec + fp.i0, pl.nx, pl.ny, z1 - z0, npk, st, 0, 0, pl.nvox, &sc.blue);
+  return fft_axes(ctx, spec + fp.i0, pl.nx, pl.ny, z1 - z0, npk, st, 0, 0, pl.nvox);
 }
 
 // Autotuning of the FIELDS transform for one shape (the first device-resident
@@ -1594,11 +1771,11 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
       CYR_CUDA(cudaStreamWaitEvent(st, up->events[sl], 0));
     }
     CYR_TRY(build_fields_x(ctx, sc, o, pl, fp, z0, z1, fused, twx, st));
-    CYR_TRY(fft_axes(ctx, spec + size_t(z0) * pl.npix, pl.nx, pl.ny, z1 - z0, npk, st, 1, 1, pl.nvox, &sc.blue,
+    CYR_TRY(fft_axes(ctx, spec + size_t(z0) * pl.npix, pl.nx, pl.ny, z1 - z0, npk, st, 1, 1, pl.nvox,
                      ft.form));
     if (up) CYR_TRY(const_cast<SlabUpload *>(up)->issue(sl + 1));  // the next slab's copy, behind this slab's kernels
   }
-  CYR_TRY(fft_axes(ctx, spec, pl.nx, pl.ny, pl.nz, npk, st, 2, 2, 0, &sc.blue, ft.form, zmask));
+  CYR_TRY(fft_axes(ctx, spec, pl.nx, pl.ny, pl.nz, npk, st, 2, 2, 0, ft.form, zmask));
   // bin 0 of each packed volume replaced by the mean of its neighbours
   CYR_TRY(sc.dc.ensure(size_t(kMaxPacked) * sizeof(float2)));
   int slot = ctx.prof.begin(kDc, st);
@@ -1962,7 +2139,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
         ctx.prof.end(slot, st);
       }
       CYR_CUDA(cudaGetLastError());
-      CYR_TRY(fft3d(ctx, spec, pl.nx, pl.ny, pl.kz, bp.nvol, st, true, &sc.blue));
+      CYR_TRY(fft3d(ctx, spec, pl.nx, pl.ny, pl.kz, bp.nvol, st, true));
     } else {
       slot = ctx.prof.begin(kBuild, st, o->morphology_type == 0 ? 2 : 1);
       if (o->morphology_type == 0) {
@@ -1973,7 +2150,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
       }
       ctx.prof.end(slot, st);
       CYR_CUDA(cudaGetLastError());
-      CYR_TRY(fft3d(ctx, spec, pl.nx, pl.ny, pl.nz, bp.nvol, st, false, &sc.blue));
+      CYR_TRY(fft3d(ctx, spec, pl.nx, pl.ny, pl.nz, bp.nvol, st, false));
     }
     slot = ctx.prof.begin(kDc, st);
     k_dc<<<1, 32, 0, st>>>(spec, bp.nvol, pl.vstride, pl.nx, pl.ny, pl.nz, pl.p0, pl.p1, pl.pn, dc);
@@ -2696,14 +2873,14 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
       k_build_fields<1><<<dim3(blocks, G), 256, 0, st>>>(fp);
     ctx.prof.end(slot, st);
     CYR_CUDA(cudaGetLastError());
-    CYR_TRY(fft_axes(ctx, spec, p0.nx, p0.ny, p0.nz, npk * G, st, 0, 0, 0, &sc.blue, ft.form));
+    CYR_TRY(fft_axes(ctx, spec, p0.nx, p0.ny, p0.nz, npk * G, st, 0, 0, 0, ft.form));
   }
   // the planes the Ewald projection reads for any of the G E virtual energies
   const EwaldGeom geom = field_geometry(o, p0);
   const uint32_t *zmask = nullptr;
   CYR_TRY(field_zmask(ctx, sc, geom, reinterpret_cast<const float *>(dp + off_k), G * E,
                       reinterpret_cast<const float *>(dp + off_kv), 1, st, &zmask));
-  CYR_TRY(fft_axes(ctx, spec, p0.nx, p0.ny, p0.nz, npk * G, st, 1, 2, 0, &sc.blue, ft.form, zmask));
+  CYR_TRY(fft_axes(ctx, spec, p0.nx, p0.ny, p0.nz, npk * G, st, 1, 2, 0, ft.form, zmask));
   {
     const int slot = ctx.prof.begin(kDc, st);
     k_dc<<<1, (npk * G + 31) / 32 * 32, 0, st>>>(spec, npk * G, nvox, p0.nx, p0.ny, p0.nz, 0, 1 % p0.nz, p0.nz - 1,
