@@ -194,9 +194,11 @@ bool mix_best(uint32_t n, std::vector<uint32_t> &best) {
   return !best.empty();
 }
 
+// Lengths that k_mix_fft transforms directly (on every call's path, so no search: the prime factors decide).
 bool mix_length(uint32_t n) {
-  std::vector<uint32_t> r;
-  return mix_best(n, r);
+  for (uint32_t p : {2u, 3u, 5u, 7u, 11u, 13u})
+    while (n % p == 0) n /= p;
+  return n == 1;
 }
 
 // Padded length of a Bluestein transform of n points: the 7-smooth M >= 2n - 1 with the least work.
@@ -414,7 +416,6 @@ struct DeviceContext {
   bool sparse_ewald = true;                // CYRSOXS_GB300_SPARSE_EWALD=0 forms every combination term
   bool zmask = true;                       // CYRSOXS_GB300_ZMASK=0: the FIELDS z pass stores every plane
   bool attrs_done = false;
-  bool attrs64 = false;                    // the FP64 FFT kernels' shared-memory attribute is set
   std::map<uint32_t, float2 *> twiddles;
   struct ConvTables {                   // a line length transformed as a convolution (get_conv)
     uint32_t m = 0;
@@ -428,14 +429,8 @@ struct DeviceContext {
     uint32_t *first = nullptr;
   };
   std::map<std::array<uint32_t, 3>, MixTables> mix;  // key: length, row form, bytes per real
-  std::map<uint32_t, double2 *> tw64;   // FP64 twiddles W_n^m per length
-  struct BlueTables64 {
-    uint32_t m = 0;
-    double2 *chirp = nullptr, *bhat = nullptr;
-  };
-  std::map<uint32_t, BlueTables64> blue64;  // the FP64 pipeline's Bluestein tables per line length
   struct Fp64Scratch {
-    DeviceBuffer spec, images, avg, params, params64, vox, out, blue;
+    DeviceBuffer spec, images, avg, params, params64, vox, out;
   } f64;                                // the FP64 pipeline's buffers (plain entry points)
   Scratch main;
   DeviceBuffer vox_in, out_in;  // host-buffer entry points: morphology and projections
@@ -485,11 +480,8 @@ int setup_attrs(DeviceContext &ctx) {
   std::lock_guard<std::mutex> lk(ctx.tables_mu);
   if (ctx.attrs_done) return CYR_OK;
   const int smem = int(kFftSmemBudget);
-#define CYR_MIX_ATTR(T, C, B) \
-  CYR_CUDA(cudaFuncSetAttribute(k_mix_fft<T, C, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CYR_MIX_ATTR(float2, false, kMixPlain) CYR_MIX_ATTR(float2, false, kMixBluestein) CYR_MIX_ATTR(float2, false, kMixRader)
-  CYR_MIX_ATTR(float2, true, kMixPlain) CYR_MIX_ATTR(float2, true, kMixBluestein) CYR_MIX_ATTR(float2, true, kMixRader)
-#undef CYR_MIX_ATTR
+  CYR_CUDA(mix_attributes<float2>(smem));
+  CYR_CUDA(mix_attributes<double2>(smem));
 #define CYR_COLS_ATTR(V, T) \
   CYR_CUDA(cudaFuncSetAttribute(k_fft_cols<V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   CYR_COLS_ATTR(32, 8)
@@ -929,6 +921,7 @@ int mix_pass(DeviceContext &ctx, T *data, uint32_t nx, uint32_t ny, uint32_t nz,
     auto tiles = [&] { return (p.nlines + (1u << lg) - 1) >> lg; };
     while (lg > 5 && (pl.most_nb << lg) > kMixT) --lg;
     while (lg > 2 && pl.ns > 1 && (size_t(M) << lg) * sizeof(T) > kMixSmem) --lg;
+    while (lg > 0 && pl.ns > 1 && (size_t(M) << lg) * sizeof(T) > kMixSmemMax) --lg;  // the longest FP64 lines
     while (lg > 3 && (1u << (lg - 1)) >= p.nlines) --lg;
     while (lg > 3 && uint64_t(tiles()) * others * count < kMixMinBlocks) --lg;
     p.lg_tx = lg;
@@ -940,13 +933,10 @@ int mix_pass(DeviceContext &ctx, T *data, uint32_t nx, uint32_t ny, uint32_t nz,
     smem = pl.ns > 1 ? (size_t(M) << lg) * sizeof(T) : 0;
   }
   if (smem > kMixSmemMax) return fail(CYR_ERR_UNSUPPORTED, "FFT length %u too large for one block", M);
-  auto kern = !conv       ? (row ? k_mix_fft<T, false, kMixPlain> : k_mix_fft<T, true, kMixPlain>)
-              : conv->in ? (row ? k_mix_fft<T, false, kMixRader> : k_mix_fft<T, true, kMixRader>)
-                         : (row ? k_mix_fft<T, false, kMixBluestein> : k_mix_fft<T, true, kMixBluestein>);
+  const MixForm form = !conv ? kMixPlain : conv->in ? kMixRader : kMixBluestein;
   const int slot = ctx.prof.begin(conv ? int(kBluestein) : kFftX + axis, st);
-  kern<<<dim3(blocks, count), threads, smem, st>>>(p);
+  CYR_CUDA(mix_launch<T>(form, row, dim3(blocks, count), threads, smem, st, p));
   ctx.prof.end(slot, st);
-  CYR_CUDA(cudaGetLastError());
   return CYR_OK;
 }
 
@@ -2264,175 +2254,19 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
 // FP64 pipeline (fp64.cuh): geometry from the FP32 planner (float decisions),
 // amplitudes in double.
 // ---------------------------------------------------------------------------
-int get_tw64(DeviceContext &ctx, uint32_t n, const double2 **tw) {
-  std::lock_guard<std::mutex> lk(ctx.tables_mu);
-  auto it = ctx.tw64.find(n);
-  if (it != ctx.tw64.end()) {
-    *tw = it->second;
-    return CYR_OK;
-  }
-  std::vector<double2> h(n);
-  for (uint32_t m = 0; m < n; ++m) {
-    const std::complex<double> w = std::polar(1.0, -2.0 * kPi * double(m) / double(n));
-    h[m] = make_double2(w.real(), w.imag());
-  }
-  double2 *d = nullptr;
-  CYR_CUDA(cudaMalloc(&d, sizeof(double2) * n));
-  CYR_CUDA(cudaMemcpy(d, h.data(), sizeof(double2) * n, cudaMemcpyHostToDevice));
-  ctx.tw64[n] = d;
-  *tw = d;
-  return CYR_OK;
-}
+constexpr uint32_t kMax64Length = 6144;  // points per axis
 
-constexpr size_t kFft64Smem = 192 * 1024;
-
-// One axis of the in-place forward FFT of `count` double volumes, vstride
-// elements apart (7-smooth length).
-int fft64_axis(DeviceContext &ctx, double2 *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, int axis,
-               cudaStream_t st, size_t vstride) {
-  if (!ctx.attrs64) {  // once per device (the attribute belongs to the current device)
-    CYR_CUDA(cudaFuncSetAttribute(k64_fft<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFft64Smem)));
-    CYR_CUDA(cudaFuncSetAttribute(k64_fft<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFft64Smem)));
-    CYR_CUDA(cudaFuncSetAttribute(k64_fft<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFft64Smem)));
-    ctx.attrs64 = true;
-  }
-  const uint32_t dims[3] = {nx, ny, nz};
-  {
-    const uint32_t n = dims[axis];
-    if (n == 1) return CYR_OK;
-    std::vector<uint32_t> r;
-    if (!factorize(n, r)) return fail(CYR_ERR_UNSUPPORTED, "FP64 path: length %u has a prime factor above 7", n);
-    Fft64Params p{};
-    p.data = data;
-    p.nx = nx, p.ny = ny, p.nz = nz;
-    p.vstride = vstride;
-    p.n = n;
-    p.nstages = uint32_t(r.size());
-    for (size_t i = 0; i < r.size(); ++i) p.radix_code |= uint64_t(r[i]) << (4 * i);
-    CYR_TRY(get_tw64(ctx, n, &p.tw));
-    uint32_t tx = 16;
-    while (tx > 1 && size_t(2) * n * tx * sizeof(double2) > 96 * 1024) tx /= 2;
-    p.tx = tx;
-    const size_t smem = size_t(2) * n * tx * sizeof(double2);
-    if (smem > kFft64Smem) return fail(CYR_ERR_UNSUPPORTED, "FP64 path: length %u too large for one block", n);
-    const uint32_t tiles = axis == 0 ? (ny * nz + tx - 1) / tx : ((nx + tx - 1) / tx) * (axis == 1 ? nz : ny);
-    const dim3 grid(tiles, count);
-    if (axis == 0) k64_fft<0><<<grid, 256, smem, st>>>(p);
-    if (axis == 1) k64_fft<1><<<grid, 256, smem, st>>>(p);
-    if (axis == 2) k64_fft<2><<<grid, 256, smem, st>>>(p);
-    CYR_CUDA(cudaGetLastError());
-  }
-  return CYR_OK;
-}
-
-// The FP64 pipeline's Bluestein tables: the chirp and FFT_m(b) / m, formed
-// on the host as for the FP32 engine (get_blue) and kept in double.
-int get_blue64(DeviceContext &ctx, uint32_t n, DeviceContext::BlueTables64 &out) {
-  std::lock_guard<std::mutex> lk(ctx.tables_mu);
-  auto it = ctx.blue64.find(n);
-  if (it != ctx.blue64.end()) {
-    out = it->second;
-    return CYR_OK;
-  }
-  const uint32_t m = bluestein_length(n);
-  std::vector<std::complex<double>> c(n), b(m, 0.0), w(m);
-  for (uint32_t j = 0; j < n; ++j) {
-    const uint64_t q = (uint64_t(j) * j) % (2 * uint64_t(n));
-    c[j] = std::polar(1.0, -kPi * double(q) / double(n));
-  }
-  for (uint32_t j = 0; j < n; ++j) {
-    b[j] = std::conj(c[j]);
-    if (j) b[m - j] = std::conj(c[j]);
-  }
-  for (uint32_t j = 0; j < m; ++j) w[j] = std::polar(1.0, -2.0 * kPi * double(j) / double(m));
-  std::vector<double2> hc(n), hb(m);
-  for (uint32_t j = 0; j < n; ++j) hc[j] = make_double2(c[j].real(), c[j].imag());
-  for (uint32_t k = 0; k < m; ++k) {
-    std::complex<double> acc(0.0, 0.0);
-    uint64_t idx = 0;  // (j k) mod m
-    for (uint32_t j = 0; j < m; ++j, idx += k) {
-      if (idx >= m) idx %= m;
-      acc += b[j] * w[idx];
-    }
-    acc /= double(m);
-    hb[k] = make_double2(acc.real(), acc.imag());
-  }
-  DeviceContext::BlueTables64 t;
-  t.m = m;
-  CYR_CUDA(cudaMalloc(&t.chirp, sizeof(double2) * n));
-  CYR_CUDA(cudaMalloc(&t.bhat, sizeof(double2) * m));
-  CYR_CUDA(cudaMemcpy(t.chirp, hc.data(), sizeof(double2) * n, cudaMemcpyHostToDevice));
-  CYR_CUDA(cudaMemcpy(t.bhat, hb.data(), sizeof(double2) * m, cudaMemcpyHostToDevice));
-  ctx.blue64[n] = t;
-  out = t;
-  return CYR_OK;
-}
-
-// One axis of length n (a prime factor above 7) of the FP64 FFT as a
-// Bluestein transform: the FP32 engine's steps (bluestein_pass) in double,
-// the padded length-m transforms by fft64_axis, in chunks of padded lines of
-// at most 256 MB held in `work`.
-int bluestein64(DeviceContext &ctx, double2 *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, int axis,
-                cudaStream_t st, size_t vstride, DeviceBuffer *work) {
-  const uint32_t n = axis == 0 ? nx : axis == 1 ? ny : nz;
-  DeviceContext::BlueTables64 bt;
-  CYR_TRY(get_blue64(ctx, n, bt));
-  const uint32_t lpv = axis == 0 ? ny * nz : axis == 1 ? nx * nz : nx * ny;
-  const uint64_t total = uint64_t(lpv) * count;
-  const uint64_t cap = std::max<uint64_t>(1, (size_t(256) << 20) / (size_t(bt.m) * sizeof(double2)));
-  const uint32_t chunk = uint32_t(std::min<uint64_t>(total, cap));
-  CYR_TRY(work->ensure(size_t(chunk) * bt.m * sizeof(double2)));
-  int sms = 0;
-  CYR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
-  BlueParamsT<double2> p{};
-  p.data = data;
-  p.work = work->as<double2>();
-  p.chirp = bt.chirp;
-  p.bhat = bt.bhat;
-  p.nx = nx, p.ny = ny, p.nz = nz;
-  p.vstride = vstride;
-  p.n = n, p.m = bt.m;
-  p.lines_per_vol = lpv;
-  for (uint64_t l0 = 0; l0 < total; l0 += chunk) {
-    p.line0 = l0;
-    p.nlines = uint32_t(std::min<uint64_t>(chunk, total - l0));
-    const size_t elems = size_t(p.nlines) * bt.m;
-    const unsigned grid = unsigned(std::min<size_t>((elems + 255) / 256, size_t(sms) * 16));
-    if (axis == 0) k_blue_gather<0, double2><<<grid, 256, 0, st>>>(p);
-    if (axis == 1) k_blue_gather<1, double2><<<grid, 256, 0, st>>>(p);
-    if (axis == 2) k_blue_gather<2, double2><<<grid, 256, 0, st>>>(p);
-    CYR_CUDA(cudaGetLastError());
-    // rows of m (x lines) or columns of m (y and z lines, stored lines fastest)
-    auto padded_fft = [&]() -> int {
-      if (axis == 0) return fft64_axis(ctx, p.work, bt.m, p.nlines, 1, 1, 0, st, elems);
-      return fft64_axis(ctx, p.work, p.nlines, bt.m, 1, 1, 1, st, elems);
-    };
-    CYR_TRY(padded_fft());
-    if (axis == 0)
-      k_blue_mul<0, double2><<<grid, 256, 0, st>>>(p);
-    else
-      k_blue_mul<1, double2><<<grid, 256, 0, st>>>(p);
-    CYR_CUDA(cudaGetLastError());
-    CYR_TRY(padded_fft());
-    if (axis == 0) k_blue_scatter<0, double2><<<grid, 256, 0, st>>>(p);
-    if (axis == 1) k_blue_scatter<1, double2><<<grid, 256, 0, st>>>(p);
-    if (axis == 2) k_blue_scatter<2, double2><<<grid, 256, 0, st>>>(p);
-    CYR_CUDA(cudaGetLastError());
-  }
-  return CYR_OK;
-}
-
-// In-place forward FFT of `count` double volumes: 7-smooth axes by fft64_axis,
-// the others as Bluestein transforms.
+// In-place forward FFT of `count` double volumes (k_mix_fft in double).
 int fft64(DeviceContext &ctx, double2 *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, cudaStream_t st) {
   const uint32_t dims[3] = {nx, ny, nz};
   const size_t vstride = size_t(nx) * ny * nz;
   for (int axis = 0; axis < 3; ++axis) {
-    if (dims[axis] == 1) continue;
-    if (smooth7(dims[axis]))
-      CYR_TRY(fft64_axis(ctx, data, nx, ny, nz, count, axis, st, vstride));
-    else
-      CYR_TRY(bluestein64(ctx, data, nx, ny, nz, count, axis, st, vstride, &ctx.f64.blue));
+    const uint32_t n = dims[axis];
+    if (n == 1) continue;
+    if (n > kMax64Length) return fail(CYR_ERR_UNSUPPORTED, "FP64 path: length %u too large for one block", n);
+    const DeviceContext::ConvTables *conv = nullptr;
+    if (!mix_length(n)) CYR_TRY(get_conv<double2>(ctx, n, &conv));
+    CYR_TRY(mix_pass<double2>(ctx, data, nx, ny, nz, count, axis, st, vstride, conv));
   }
   return CYR_OK;
 }
@@ -2441,6 +2275,7 @@ int fft64(DeviceContext &ctx, double2 *data, uint32_t nx, uint32_t ny, uint32_t 
 // refractive indices per energy, Hanning tables and the E basis coefficients.
 struct Plan64 {
   std::vector<unsigned char> arena;
+  size_t off_con = 0, off_map = 0, off_kmag = 0;  // contrasts and wave numbers per energy, MATERIAL-frame maps per (k, angle)
   size_t off_mat = 0, off_hx = 0, off_hy = 0, off_hz = 0, off_e = 0;
 };
 
@@ -2466,6 +2301,40 @@ int make_plan64(const cyr_options *o, const double *optical, bool window, Plan &
   }
   p64.arena.clear();
   p64.off_mat = arena_put(p64.arena, mats.data(), mats.size());
+  // the same constants as contrasts n^2 - 1 = (n - 1)(n + 1), over 4 pi (k64_ewald_fields)
+  std::vector<Contrast64> cons(pl.ne);
+  for (uint32_t e = 0; e < pl.ne; ++e) {
+    std::memset(&cons[e], 0, sizeof(Contrast64));
+    for (uint32_t m = 0; m < pl.nmat; ++m) {
+      const double *op = optical + (size_t(e) * pl.nmat + m) * 4;
+      const std::complex<double> par(-op[0], op[1]), per(-op[2], op[3]), mean = (par + 2.0 * per) / 3.0;
+      const double s = 1.0 / (4.0 * kPi);
+      const std::complex<double> A = s * par * (par + 2.0), B = s * per * (per + 2.0), C = s * mean * (mean + 2.0);
+      const std::complex<double> D = s * (par - per) * (par + per + 2.0);
+      cons[e].A[m] = make_double2(A.real(), A.imag());
+      cons[e].B[m] = make_double2(B.real(), B.imag());
+      cons[e].C[m] = make_double2(C.real(), C.imag());
+      cons[e].D[m] = make_double2(D.real(), D.imag());
+    }
+  }
+  p64.off_con = arena_put(p64.arena, cons.data(), cons.size());
+  std::vector<float> km(pl.ne);
+  for (uint32_t e = 0; e < pl.ne; ++e) {
+    const float wavelength = static_cast<float>(1239.84197 / o->energies[e]);  // src/cudaMain.cu:607-608
+    km[e] = static_cast<float>(2 * kPi / wavelength);
+  }
+  p64.off_kmag = arena_put(p64.arena, km.data(), km.size());
+  if (pl.material_frame) {
+    // p = R^T Nt E as a real map of the six entries (include/uniaxial.h:163-165)
+    const uint32_t sym[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+    std::vector<double> map(size_t(pl.nk) * pl.nang * 18, 0.0);
+    for (size_t ka = 0; ka < size_t(pl.nk) * pl.nang; ++ka)
+      for (int c = 0; c < 3; ++c)
+        for (int b = 0; b < 3; ++b)
+          for (int i = 0; i < 3; ++i)
+            map[ka * 18 + c * 6 + sym[i][b]] += double(pl.rmats[ka].m[i * 3 + c]) * double(pl.evec[ka * 3 + b]);
+    p64.off_map = arena_put(p64.arena, map.data(), map.size());
+  }
   auto hann = [&](uint32_t n, bool unit) {
     std::vector<double> w(n);
     for (uint32_t j = 0; j < n; ++j) w[j] = unit || !window ? 1.0 : 0.5 * (1 - std::cos(2 * kPi * j / n));
@@ -2489,11 +2358,28 @@ int run_fp64(DeviceContext &ctx, const cyr_options *o, const double *optical, co
   Plan pl;
   Plan64 p64;
   CYR_TRY(make_plan64(o, optical, o->algorithm == 0 && o->windowing == 1, pl, p64));
+  CYR_TRY(setup_attrs(ctx));
   auto &f = ctx.f64;
   const uint32_t nvol = pl.material_frame ? 3u : pl.nvol;
-  CYR_TRY(f.spec.ensure(size_t(nvol) * pl.nvox * sizeof(double2)));
-  CYR_TRY(f.images.ensure(size_t(pl.nang) * pl.npix * sizeof(double)));
-  CYR_TRY(f.avg.ensure(pl.npix * sizeof(double)));
+  // Field spectra (one transform of the 7 M packed fields for every energy and
+  // angle) when they are fewer volumes than the per-energy spectra and fit;
+  // the transforms dominate both (256 x 256 x 32, 2 materials, 3 energies:
+  // 7 volumes against 15).
+  const uint32_t npk = fields64_packed(pl.nmat);
+  const double per_energy = double(pl.ne) * (pl.material_frame ? 3.0 * pl.nk * pl.nang : double(nvol));
+  bool fields = o->strategy == CYR_STRATEGY_FIELDS || (o->strategy == CYR_STRATEGY_AUTO && npk < per_energy);
+  if (fields && o->strategy == CYR_STRATEGY_AUTO) {
+    size_t free_b = 0, total_b = 0;
+    CYR_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if (size_t(npk) * pl.nvox * sizeof(double2) + (size_t(1) << 30) > free_b + f.spec.bytes) fields = false;
+  }
+  // energies per Ewald, rotation and warp launch: up to 512 MB of per-angle images
+  const size_t image = size_t(pl.nang) * pl.npix * sizeof(double);
+  const uint32_t batch =
+      fields ? uint32_t(std::max<size_t>(1, std::min<size_t>(std::min(pl.ne, 65535u), (size_t(512) << 20) / image))) : 1u;
+  CYR_TRY(f.spec.ensure(size_t(fields ? npk : nvol) * pl.nvox * sizeof(double2)));
+  CYR_TRY(f.images.ensure(batch * image));
+  CYR_TRY(f.avg.ensure(batch * pl.npix * sizeof(double)));
   CYR_TRY(f.params.ensure(pl.arena.size()));
   CYR_TRY(f.params64.ensure(p64.arena.size()));
   CYR_CUDA(cudaMemcpyAsync(f.params.ptr, pl.arena.data(), pl.arena.size(), cudaMemcpyHostToDevice, st));
@@ -2522,6 +2408,72 @@ int run_fp64(DeviceContext &ctx, const cyr_options *o, const double *optical, co
   const double *dE = reinterpret_cast<const double *>(dq + p64.off_e);
   const Mat64 *dmat = reinterpret_cast<const Mat64 *>(dq + p64.off_mat);
   const double prefill = o->rot_mask ? 0.0 : std::numeric_limits<double>::quiet_NaN();
+  auto geometry = [&] {
+    EwaldGeom g{};
+    g.start = -static_cast<float>(kPi / o->phys_size);
+    g.dx = static_cast<float>((2.0 * kPi / o->phys_size) / ((pl.nx - 1) * 1.0));
+    g.dy = static_cast<float>((2.0 * kPi / o->phys_size) / ((pl.ny - 1) * 1.0));
+    g.dz = pl.twod ? 0.f : static_cast<float>((2.0 * kPi / o->phys_size) / ((pl.nz - 1) * 1.0));
+    g.nx = pl.nx, g.ny = pl.ny, g.nz = pl.nz;
+    g.interp = o->ewald_interpolation;
+    g.twod = pl.twod ? 1u : 0u;
+    return g;
+  };
+  // rotation, mean and detector warp of nb energies' images from energy e on
+  auto finish = [&](uint32_t e, uint32_t nb, uint32_t k) -> int {
+    Rotate64Params rp{};
+    rp.images = images;
+    rp.coef = dwarp + size_t(k) * pl.nang;
+    rp.W = W, rp.H = H;
+    rp.nangles = pl.nang;
+    rp.rot_mask = o->rot_mask;
+    rp.avg = avg;
+    k64_rotate_average<<<dim3(pgrid, nb), 256, 0, st>>>(rp);
+    k64_warp<<<dim3(pgrid, nb), 256, 0, st>>>(avg, d_out + (size_t(e) * pl.nk + k) * pl.npix, W, H, pl.detector_warp[k],
+                                              prefill, size_t(pl.nk) * pl.npix);
+    CYR_CUDA(cudaGetLastError());
+    return CYR_OK;
+  };
+  if (fields) {
+    bp.out = spec;
+    k64_build_fields<<<bgrid, 256, 0, st>>>(bp);
+    CYR_CUDA(cudaGetLastError());
+    CYR_TRY(fft64(ctx, spec, pl.nx, pl.ny, pl.nz, npk, st));
+    k64_dc<<<1, (npk + 31) / 32 * 32, 0, st>>>(spec, npk, pl.nvox, pl.nx, pl.ny, pl.nz);
+    CYR_CUDA(cudaGetLastError());
+    FieldEwald64Params fe{};
+    fe.spec = spec;
+    fe.npk = npk, fe.nmat = pl.nmat;
+    fe.vstride = pl.nvox;
+    fe.con = reinterpret_cast<const Contrast64 *>(dq + p64.off_con);
+    fe.kmag = reinterpret_cast<const float *>(dq + p64.off_kmag);
+    fe.g = geometry();
+    fe.qx = reinterpret_cast<const float *>(dp + pl.off_qx);
+    fe.qy = reinterpret_cast<const float *>(dp + pl.off_qy);
+    fe.qz = reinterpret_cast<const float *>(dp + pl.off_qz);
+    fe.nangles = pl.nang;
+    fe.images = images;
+    for (uint32_t k = 0; k < pl.nk; ++k) {
+      const KFrame &fr = pl.frames[k];
+      fe.kvx = fr.k.x, fe.kvy = fr.k.y, fe.kvz = fr.k.z;
+      fe.E = dE + size_t(k) * pl.nang * pl.nbasis;
+      fe.map = reinterpret_cast<const double *>(dq + p64.off_map) + size_t(k) * pl.nang * 18;
+      for (uint32_t e = 0; e < pl.ne; e += batch) {
+        const uint32_t nb = std::min(batch, pl.ne - e);
+        fe.e0 = e;
+        const dim3 grid(unsigned((pl.npix + 127) / 128), nb);
+        if (pl.material_frame)
+          k64_ewald_fields<0><<<grid, 128, 0, st>>>(fe);
+        else if (pl.nbasis == 2)
+          k64_ewald_fields<2><<<grid, 128, 0, st>>>(fe);
+        else
+          k64_ewald_fields<3><<<grid, 128, 0, st>>>(fe);
+        CYR_CUDA(cudaGetLastError());
+        CYR_TRY(finish(e, nb, k));
+      }
+    }
+    return CYR_OK;
+  }
   for (uint32_t e = 0; e < pl.ne; ++e) {
     const float wavelength = static_cast<float>(1239.84197 / o->energies[e]);  // src/cudaMain.cu:607-608
     const float kmag = static_cast<float>(2 * kPi / wavelength);
@@ -2544,15 +2496,9 @@ int run_fp64(DeviceContext &ctx, const cyr_options *o, const double *optical, co
       Ewald64Params ep{};
       ep.spec = spec;
       ep.vstride = pl.nvox;
-      ep.g.start = -static_cast<float>(kPi / o->phys_size);
-      ep.g.dx = static_cast<float>((2.0 * kPi / o->phys_size) / ((pl.nx - 1) * 1.0));
-      ep.g.dy = static_cast<float>((2.0 * kPi / o->phys_size) / ((pl.ny - 1) * 1.0));
-      ep.g.dz = pl.twod ? 0.f : static_cast<float>((2.0 * kPi / o->phys_size) / ((pl.nz - 1) * 1.0));
+      ep.g = geometry();
       ep.g.kmag = kmag;
       ep.g.kx = kmag * fr.k.x, ep.g.ky = kmag * fr.k.y, ep.g.kz = kmag * fr.k.z;
-      ep.g.nx = pl.nx, ep.g.ny = pl.ny, ep.g.nz = pl.nz;
-      ep.g.interp = o->ewald_interpolation;
-      ep.g.twod = pl.twod ? 1u : 0u;
       ep.qx = reinterpret_cast<const float *>(dp + pl.off_qx);
       ep.qy = reinterpret_cast<const float *>(dp + pl.off_qy);
       ep.qz = reinterpret_cast<const float *>(dp + pl.off_qz);
@@ -2583,17 +2529,7 @@ int run_fp64(DeviceContext &ctx, const cyr_options *o, const double *optical, co
           CYR_CUDA(cudaGetLastError());
         }
       }
-      Rotate64Params rp{};
-      rp.images = images;
-      rp.coef = dwarp + size_t(k) * pl.nang;
-      rp.W = W, rp.H = H;
-      rp.nangles = pl.nang;
-      rp.rot_mask = o->rot_mask;
-      rp.avg = avg;
-      k64_rotate_average<<<pgrid, 256, 0, st>>>(rp);
-      k64_warp<<<pgrid, 256, 0, st>>>(avg, d_out + (size_t(e) * pl.nk + k) * pl.npix, W, H, pl.detector_warp[k],
-                                      prefill);
-      CYR_CUDA(cudaGetLastError());
+      CYR_TRY(finish(e, 1, k));
     }
   }
   return CYR_OK;

@@ -12,10 +12,19 @@
 // (include/cudaUtils.h:268-296), the plane interpolation, the bilinear blend of
 // the rotation and detector warps, and the angle sum and mean (:877-909).
 //
-// Schedule, per energy: LAB frame - the 5 (6 with a tilted k) distinct
-// entries of Nt are transformed once and every E angle's p = Nt E / 4pi is
-// formed at the Ewald sample points (exact by linearity); MATERIAL frame -
-// p = R^T Nt R x per angle, 3 transforms per angle, as the reference does.
+// Schedules.  Field spectra (k64_build_fields, k64_ewald_fields): the 7 M
+// energy independent real fields of the morphology are transformed once, in
+// pairs, and every energy and E angle is formed from them at the Ewald sample
+// points, exact by linearity as in fields.cuh; GB300's FP64 rate is 1/64 of
+// its FP32 rate, so the transforms' operations are what counts, and 3.5 M
+// volumes per request replace 5 per energy (256 x 256 x 32, 2 materials, 3
+// energies x 12 angles: 18.6 -> 2.57 ms, with the mixed-radix transforms of
+// mixfft.cuh in the place of direct radix-8 sums; bound by the FP64 pipe).
+// Per energy: LAB frame - the 5
+// (6 with a tilted k) distinct entries of Nt are transformed once per energy
+// and every E angle's p = Nt E / 4pi is formed at the sample points; MATERIAL
+// frame - p = R^T Nt R x per angle, 3 transforms per angle, as the reference
+// does.
 #pragma once
 
 #include "kernels.cuh"
@@ -129,114 +138,6 @@ __global__ void __launch_bounds__(256) k64_build(Build64Params p, const Mat64 *_
   }
 }
 
-// ---------------------------------------------------------------------------
-// FP64 FFT: shared-memory Stockham autosort, any 7-smooth length up to 4096,
-// radices 8/4/2/3/5/7 with a direct DFT per radix from a double twiddle
-// table W_n^m.  tx lines per block: rows along x, or tx adjacent columns for
-// lines along y and z.
-// ---------------------------------------------------------------------------
-struct Fft64Params {
-  double2 *data;
-  uint32_t nx, ny, nz;
-  size_t vstride;           // elements between volumes (blockIdx.y)
-  uint32_t n, tx, nstages;
-  uint64_t radix_code;      // radix of stage s in bits [4s, 4s+4)
-  const double2 *tw;        // W_n^m
-};
-
-// One Stockham stage of radix R over tx lines of n: group j of line l reads
-// x_q = src[j + q m] (m = n / R), twiddles x_q by W^(q k n / (ns R)) with
-// k = j mod ns, takes its R-point DFT and writes element o to
-// dst[(j / ns) ns R + k + o ns].
-template <uint32_t R>
-__device__ __forceinline__ void stage64(const double2 *__restrict__ src, double2 *__restrict__ dst, uint32_t n,
-                                        uint32_t tx, uint32_t ns, const double2 *__restrict__ tw) {
-  const uint32_t m = n / R, tstep = n / (ns * R);
-  for (uint32_t g = threadIdx.x; g < tx * m; g += blockDim.x) {
-    const uint32_t l = g / m, j = g % m, k = j % ns;
-    const double2 *sl = src + size_t(l) * n;
-    double2 x[R];
-#pragma unroll
-    for (uint32_t q = 0; q < R; ++q) {
-      x[q] = sl[j + q * m];
-      if (q && k) x[q] = zmul(x[q], tw[q * k * tstep]);
-    }
-    double2 *dl = dst + size_t(l) * n + (j / ns) * ns * R + k;
-#pragma unroll
-    for (uint32_t o = 0; o < R; ++o) {
-      double2 acc = x[0];
-#pragma unroll
-      for (uint32_t q = 1; q < R; ++q) acc = zadd(acc, zmul(x[q], tw[((o * q) % R) * m]));
-      dl[o * ns] = acc;
-    }
-  }
-}
-
-template <int AXIS>
-__global__ void __launch_bounds__(256) k64_fft(Fft64Params p) {
-  extern __shared__ double2 zsm[];
-  const uint32_t n = p.n, TX = p.tx;
-  double2 *bufa = zsm, *bufb = zsm + size_t(n) * TX;
-  size_t base;
-  uint32_t valid, lstep, estep;
-  if (AXIS == 0) {
-    const uint32_t rows = p.ny * p.nz, r0 = blockIdx.x * TX;
-    base = size_t(r0) * p.nx;
-    valid = min(TX, rows - r0);
-    lstep = p.nx, estep = 1;
-  } else {
-    const uint32_t nxt = (p.nx + TX - 1) / TX;
-    const uint32_t x0 = (blockIdx.x % nxt) * TX, other = blockIdx.x / nxt;
-    valid = min(TX, p.nx - x0);
-    lstep = 1;
-    if (AXIS == 1) {
-      base = size_t(other) * p.nx * p.ny + x0;
-      estep = p.nx;
-    } else {
-      base = size_t(other) * p.nx + x0;
-      estep = p.nx * p.ny;
-    }
-  }
-  double2 *tile = p.data + size_t(blockIdx.y) * p.vstride + base;
-  const uint32_t total = n * TX;
-  for (uint32_t t = threadIdx.x; t < total; t += blockDim.x) {
-    uint32_t l, i;
-    if (AXIS == 0) {
-      l = t / n, i = t % n;
-    } else {
-      l = t % TX, i = t / TX;
-    }
-    bufa[size_t(l) * n + i] = l < valid ? tile[size_t(l) * lstep + size_t(i) * estep] : make_double2(0.0, 0.0);
-  }
-  __syncthreads();
-  double2 *src = bufa, *dst = bufb;
-  uint32_t ns = 1;
-  for (uint32_t s = 0; s < p.nstages; ++s) {
-    const uint32_t R = uint32_t((p.radix_code >> (4 * s)) & 15u);
-    switch (R) {
-      case 2: stage64<2>(src, dst, n, TX, ns, p.tw); break;
-      case 3: stage64<3>(src, dst, n, TX, ns, p.tw); break;
-      case 4: stage64<4>(src, dst, n, TX, ns, p.tw); break;
-      case 5: stage64<5>(src, dst, n, TX, ns, p.tw); break;
-      case 7: stage64<7>(src, dst, n, TX, ns, p.tw); break;
-      default: stage64<8>(src, dst, n, TX, ns, p.tw); break;
-    }
-    __syncthreads();
-    double2 *t = src;
-    src = dst, dst = t;
-    ns *= R;
-  }
-  for (uint32_t t = threadIdx.x; t < total; t += blockDim.x) {
-    uint32_t l, i;
-    if (AXIS == 0) {
-      l = t / n, i = t % n;
-    } else {
-      l = t % TX, i = t / TX;
-    }
-    if (l < valid) tile[size_t(l) * lstep + size_t(i) * estep] = src[size_t(l) * n + i];
-  }
-}
-
 // Bin 0 of each volume <- mean of its 6 (4 in 2D) periodic neighbours (src/cudaMain.cu:123-176).
 __global__ void k64_dc(double2 *spec, uint32_t nvol, size_t vstride, uint32_t nx, uint32_t ny, uint32_t nz) {
   const uint32_t v = threadIdx.x;
@@ -250,6 +151,16 @@ __global__ void k64_dc(double2 *spec, uint32_t nvol, size_t vstride, uint32_t nx
     cnt = 6.0;
   }
   V[0] = zscale(s, 1.0 / cnt);
+}
+
+// Weight of the second Ewald plane in double from the float plane position, as the reference's FP64 interpolation.
+__device__ __forceinline__ double ewald_weight64(const EwaldGeom &g, uint32_t X, uint32_t Y, uint32_t Z0) {
+  const float posx = __fadd_rn(g.start, __fmul_rn(float(X), g.dx));
+  const float posy = __fadd_rn(g.start, __fmul_rn(float(Y), g.dy));
+  const float ax = __fadd_rn(g.kx, posx), ay = __fadd_rn(g.ky, posy);
+  const float val = __fsub_rn(__fsub_rn(__fmul_rn(g.kmag, g.kmag), __fmul_rn(ax, ax)), __fmul_rn(ay, ay));
+  const float posz = __fadd_rn(-g.kz, __fsqrt_rn(val));
+  return (double(posz) - (double(g.start) + double(__fmul_rn(float(Z0), g.dz)))) / double(g.dz);
 }
 
 // Ewald projection in double for every E angle: per detector pixel, the float
@@ -283,16 +194,7 @@ __global__ void __launch_bounds__(256) k64_ewald(Ewald64Params p) {
     for (uint32_t a = 0; a < p.nangles; ++a) p.images[size_t(a) * npix + t] = nan;
     return;
   }
-  // plane weight in double from the float plane position, as the reference's FP64 interpolation
-  double w1 = 0.0;
-  if (nplanes == 2) {
-    const float posx = __fadd_rn(g.start, __fmul_rn(float(X), g.dx));
-    const float posy = __fadd_rn(g.start, __fmul_rn(float(Y), g.dy));
-    const float ax = __fadd_rn(g.kx, posx), ay = __fadd_rn(g.ky, posy);
-    const float val = __fsub_rn(__fsub_rn(__fmul_rn(g.kmag, g.kmag), __fmul_rn(ax, ax)), __fmul_rn(ay, ay));
-    const float posz = __fadd_rn(-g.kz, __fsqrt_rn(val));
-    w1 = (double(posz) - (double(g.start) + double(__fmul_rn(float(zs[0]), g.dz)))) / double(g.dz);
-  }
+  const double w1 = nplanes == 2 ? ewald_weight64(g, X, Y, zs[0]) : 0.0;
   const uint32_t ux = igor(X, g.nx), uy = igor(Y, g.ny);
   double2 P[2][3][3];
   double Q[2][3];
@@ -328,6 +230,208 @@ __global__ void __launch_bounds__(256) k64_ewald(Ewald64Params p) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// Field spectra in double.  Field 7 m + f of material m is w u_x^2, w u_y^2,
+// w u_z^2, w u_x u_y, w u_x u_z, w u_y u_z, w phi_ui (f = 0..6; u = sqrt(phi_a) s,
+// w the window), and with n^2 - 1 in the place of n^2 (the identity
+// phi_a |s|^2 + phi_ui = phi)
+//   Nt_ii = sum_m A u_i^2 + B (|u|^2 - u_i^2) + C phi_ui,  Nt_ij = sum_m D u_i u_j.
+// Volume j holds fields 2 j and 2 j + 1 as real and imaginary part.
+// ---------------------------------------------------------------------------
+__host__ __device__ constexpr uint32_t fields64_packed(uint32_t nmat) { return (7 * nmat + 1) / 2; }
+
+// Contrasts over 4 pi of one energy: A = n_par^2 - 1, B = n_perp^2 - 1, C = ((n_par + 2 n_perp) / 3)^2 - 1, D = A - B.
+struct Contrast64 {
+  double2 A[kMaxMaterials], B[kMaxMaterials], C[kMaxMaterials], D[kMaxMaterials];
+};
+
+__global__ void __launch_bounds__(256) k64_build_fields(Build64Params p) {
+  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < p.nvox; i += size_t(gridDim.x) * blockDim.x) {
+    double w = 1.0;
+    if (p.hann_x) {
+      const uint32_t X = uint32_t(i % p.nx), Y = uint32_t((i / p.nx) % p.ny), Z = uint32_t(i / (size_t(p.nx) * p.ny));
+      w = p.hann_x[X] * p.hann_y[Y] * p.hann_z[Z];
+    }
+    double pend = 0.0;
+    double2 *o = p.out + i;
+    uint32_t g = 0;
+    auto emit = [&](double v) {
+      if (g & 1u)
+        o[size_t(g >> 1) * p.nvox] = make_double2(pend, v);
+      else
+        pend = v;
+      ++g;
+    };
+    for (uint32_t m = 0; m < p.nmat; ++m) {
+      double s[4];
+      load_s64(p, m, i, s);
+      double sx, sy, sz, wa, wu;
+      if (p.morphology == 0) {  // Euler: (S, theta, psi, Vfrac)
+        double st, ct, sp, cp;
+        sincos(s[1], &st, &ct);
+        sincos(s[2], &sp, &cp);
+        sx = cp * st, sy = sp * st, sz = ct;
+        const double phi_a = s[3] * s[0];
+        wa = w * phi_a;
+        wu = w * (s[3] - phi_a);
+      } else {  // vector: (sx, sy, sz, phi_unaligned)
+        sx = s[0], sy = s[1], sz = s[2];
+        wa = w;
+        wu = w * s[3];
+      }
+      const double ax = wa * sx, ay = wa * sy;
+      emit(ax * sx);
+      emit(ay * sy);
+      emit(wa * sz * sz);
+      emit(ax * sy);
+      emit(ax * sz);
+      emit(ay * sz);
+      emit(wu);
+    }
+    if (g & 1u) o[size_t(g >> 1) * p.nvox] = make_double2(pend, 0.0);
+  }
+}
+
+struct FieldEwald64Params {
+  const double2 *spec;      // [npk][V]
+  uint32_t npk, nmat;
+  size_t vstride;
+  const Contrast64 *con;    // [ne]
+  const float *kmag;        // [ne] wave numbers (float, as ewald_geometry takes them)
+  uint32_t e0;              // the launch's first energy (blockIdx.y = energy - e0)
+  float kvx, kvy, kvz;
+  EwaldGeom g;              // kmag, kx, ky, kz filled per energy
+  const float *qx, *qy, *qz;
+  uint32_t nangles;
+  const double *E;          // NB > 0: [nangles][NB]
+  const double *map;        // NB = 0: [nangles][3][6]
+  double *images;           // [batch][nangles][P]
+};
+
+// Ewald projection from the field spectra, for a batch of energies and every
+// E angle.  NB = 2 or 3 (LAB frame): per plane the Gram matrix of the scattered
+// basis fields, from which each angle takes NB (NB + 1) / 2 multiply-adds;
+// NB = 0 (MATERIAL frame): p = map Nt per angle.
+template <int NB>
+__global__ void __launch_bounds__(128) k64_ewald_fields(FieldEwald64Params p) {
+  const uint32_t e = p.e0 + blockIdx.y;
+  EwaldGeom g = p.g;
+  g.kmag = p.kmag[e];
+  g.kx = __fmul_rn(g.kmag, p.kvx), g.ky = __fmul_rn(g.kmag, p.kvy), g.kz = __fmul_rn(g.kmag, p.kvz);
+  const size_t npix = size_t(g.nx) * g.ny;
+  const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t >= npix) return;
+  const uint32_t Y = uint32_t(t / g.nx), X = uint32_t(t % g.nx);
+  double *img = p.images + size_t(blockIdx.y) * p.nangles * npix + t;
+  uint32_t zs[2];
+  float w1f;
+  int nplanes;
+  if (!ewald_geometry(g, X, Y, zs[0], zs[1], w1f, nplanes)) {
+    for (uint32_t a = 0; a < p.nangles; ++a) img[size_t(a) * npix] = __longlong_as_double(0x7ff8000000000000ll);
+    return;
+  }
+  const double w1 = nplanes == 2 ? ewald_weight64(g, X, Y, zs[0]) : 0.0;
+  const uint32_t ux = igor(X, g.nx), uy = igor(Y, g.ny);
+  const uint32_t mx = ux ? g.nx - ux : 0u, my = uy ? g.ny - uy : 0u;
+  const Contrast64 &c = p.con[e];
+  const double d = double(g.kmag) * double(g.kmag);
+  constexpr int NG = NB * (NB + 1) / 2;
+  double G[NG > 0 ? NG : 1] = {};
+  double2 nt2[2][6];
+  double Q2[2][3];
+  for (int pl = 0; pl < nplanes; ++pl) {
+    double2(&nt)[6] = nt2[NB == 0 ? pl : 0];
+    double(&Q)[3] = Q2[NB == 0 ? pl : 0];
+    const uint32_t uz = g.twod ? 0u : igor(zs[pl], g.nz), mz = uz ? g.nz - uz : 0u;
+    const double2 *za = p.spec + (size_t(uz) * g.ny + uy) * g.nx + ux;
+    const double2 *zb = p.spec + (size_t(mz) * g.ny + my) * g.nx + mx;
+#pragma unroll
+    for (int v = 0; v < 6; ++v) nt[v] = make_double2(0.0, 0.0);
+    uint32_t m = 0, f = 0;  // the same in every thread
+    auto mac = [](double2 &acc, double2 a, double2 b) {
+      acc.x += a.x * b.x - a.y * b.y;
+      acc.y += a.x * b.y + a.y * b.x;
+    };
+    auto add = [&](double2 F) {
+      if (m >= p.nmat) return;
+      if (f < 3 || f == 6) {
+        mac(nt[0], f == 6 ? c.C[m] : f == 0 ? c.A[m] : c.B[m], F);
+        mac(nt[3], f == 6 ? c.C[m] : f == 1 ? c.A[m] : c.B[m], F);
+        if (NB != 2) mac(nt[5], f == 6 ? c.C[m] : f == 2 ? c.A[m] : c.B[m], F);
+      } else if (f == 3) {
+        mac(nt[1], c.D[m], F);
+      } else if (f == 4) {
+        mac(nt[2], c.D[m], F);
+      } else {
+        mac(nt[4], c.D[m], F);
+      }
+      if (++f == 7) f = 0, ++m;
+    };
+    for (uint32_t j = 0; j < p.npk; ++j) {
+      const double2 a = __ldg(&za[size_t(j) * p.vstride]), b = __ldg(&zb[size_t(j) * p.vstride]);
+      // F_2j = (Z(k) + conj Z(-k)) / 2, F_2j+1 = (Z(k) - conj Z(-k)) / 2i
+      add(make_double2(0.5 * (a.x + b.x), 0.5 * (a.y - b.y)));
+      add(make_double2(0.5 * (a.y + b.y), 0.5 * (b.x - a.x)));
+    }
+    Q[0] = double(g.kx) + double(p.qx[X]);
+    Q[1] = double(g.ky) + double(p.qy[Y]);
+    Q[2] = double(g.kz) + (g.twod ? 0.0 : double(p.qz[zs[pl]]));
+    if constexpr (NB > 0) {
+      const double w = nplanes == 2 ? (pl == 0 ? 1.0 - w1 : w1) : 1.0;
+      double2 tt[NB][3];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        const double2 p0 = nt[b], p1 = nt[b == 0 ? 1 : b == 1 ? 3 : 4], p2 = nt[b == 0 ? 2 : b == 1 ? 4 : 5];
+        const double2 qp = zadd(zadd(zscale(p0, Q[0]), zscale(p1, Q[1])), zscale(p2, Q[2]));
+        tt[b][0] = zsub(zscale(p0, d), zscale(qp, Q[0]));
+        tt[b][1] = zsub(zscale(p1, d), zscale(qp, Q[1]));
+        tt[b][2] = zsub(zscale(p2, d), zscale(qp, Q[2]));
+      }
+      int q = 0;
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int b2 = b; b2 < NB; ++b2) {
+          double r = 0.0;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) r += tt[b][i].x * tt[b2][i].x + tt[b][i].y * tt[b2][i].y;
+          G[q++] += (b == b2 ? w : 2.0 * w) * r;
+        }
+    }
+  }
+  for (uint32_t a = 0; a < p.nangles; ++a) {
+    double I = 0.0;
+    if constexpr (NB > 0) {
+      const double *E = p.E + size_t(a) * NB;
+      int q = 0;
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int b2 = b; b2 < NB; ++b2) I += __ldg(&E[b]) * __ldg(&E[b2]) * G[q++];
+    } else {
+      const double *M = p.map + size_t(a) * 18;
+      for (int pl = 0; pl < nplanes; ++pl) {
+        double2 pc[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          pc[i] = make_double2(0.0, 0.0);
+#pragma unroll
+          for (int v = 0; v < 6; ++v) pc[i] = zadd(pc[i], zscale(nt2[pl][v], __ldg(&M[i * 6 + v])));
+        }
+        const double2 qp = zadd(zadd(zscale(pc[0], Q2[pl][0]), zscale(pc[1], Q2[pl][1])), zscale(pc[2], Q2[pl][2]));
+        double r = 0.0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const double2 s = zsub(zscale(pc[i], d), zscale(qp, Q2[pl][i]));
+          r += s.x * s.x + s.y * s.y;
+        }
+        I += (nplanes == 2 ? (pl == 0 ? 1.0 - w1 : w1) : 1.0) * r;
+      }
+    }
+    img[size_t(a) * npix] = I;
+  }
+}
+
 // Bilinear blend in double at NPP's float sample position.
 __device__ __forceinline__ bool warp_sample64(const double *__restrict__ src, int W, int H, const WarpCoef &c, int xd,
                                               int yd, double &out) {
@@ -343,11 +447,11 @@ __device__ __forceinline__ bool warp_sample64(const double *__restrict__ src, in
 // Rotation of every angle's image (NaN prefill), mask, sum and mean in double
 // (src/cudaMain.cu:830-909, include/uniaxial.h:958-992).
 struct Rotate64Params {
-  const double *images;     // [nangles][P]
+  const double *images;     // [batch = blockIdx.y][nangles][P]
   const WarpCoef *coef;     // [nangles]
   int W, H;
   uint32_t nangles, rot_mask;
-  double *avg;              // [P]
+  double *avg;              // [batch][P]
 };
 
 __global__ void __launch_bounds__(256) k64_rotate_average(Rotate64Params p) {
@@ -360,23 +464,24 @@ __global__ void __launch_bounds__(256) k64_rotate_average(Rotate64Params p) {
   uint32_t count = 0;
   for (uint32_t a = 0; a < p.nangles; ++a) {
     double v = nan;
-    warp_sample64(p.images + size_t(a) * npix, p.W, p.H, p.coef[a], xd, yd, v);
+    warp_sample64(p.images + (size_t(blockIdx.y) * p.nangles + a) * npix, p.W, p.H, p.coef[a], xd, yd, v);
     if (p.rot_mask) {
       if (isnan(v)) continue;
       ++count;
     }
     sum += v;
   }
-  p.avg[t] = p.rot_mask ? (count == 0 ? 0.0 : sum / double(count)) : sum / double(p.nangles);
+  p.avg[size_t(blockIdx.y) * npix + t] = p.rot_mask ? (count == 0 ? 0.0 : sum / double(count)) : sum / double(p.nangles);
 }
 
 // Detector warp (src/cudaMain.cu:916-960): dst holds the prefill; written where the source falls inside.
 __global__ void k64_warp(const double *__restrict__ src, double *__restrict__ dst, int W, int H, WarpCoef c,
-                         double prefill) {
-  const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= size_t(W) * H) return;
+                         double prefill, size_t dst_stride) {
+  const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x, npix = size_t(W) * H;
+  if (t >= npix) return;
   double v;
-  dst[t] = warp_sample64(src, W, H, c, int(t % W), int(t / W), v) ? v : prefill;
+  if (!warp_sample64(src + blockIdx.y * npix, W, H, c, int(t % W), int(t / W), v)) v = prefill;
+  dst[blockIdx.y * dst_stride + t] = v;
 }
 
 }  // namespace cyr

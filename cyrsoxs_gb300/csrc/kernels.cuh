@@ -15,42 +15,12 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "complex.cuh"
+
 namespace cyr {
 
 constexpr int kMaxMaterials = 32;
 constexpr int kMaxAngles = 4096;
-
-// Complex add and subtract as packed FP32 pairs (add/sub.rn.f32x2, sm_100
-// and later): one instruction performs both IEEE round-to-nearest operations,
-// so each component is bit-identical to the scalar form, at half the
-// instructions in the FFT butterflies.
-__device__ __forceinline__ unsigned long long f2_pack(float2 v) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v.x), "f"(v.y));
-  return r;
-}
-__device__ __forceinline__ float2 f2_unpack(unsigned long long r) {
-  float2 v;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
-  return v;
-}
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_pack(a)), "l"(f2_pack(b)));
-  return f2_unpack(r);
-}
-__device__ __forceinline__ float2 csub(float2 a, float2 b) {
-  unsigned long long r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_pack(a)), "l"(f2_pack(b)));
-  return f2_unpack(r);
-}
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
-__device__ __forceinline__ float2 cfma(float s, float2 a, float2 acc) {
-  return make_float2(fmaf(s, a.x, acc.x), fmaf(s, a.y, acc.y));
-}
 
 // ---------------------------------------------------------------------------
 // 1. Dielectric tensor build.
@@ -580,115 +550,6 @@ __global__ void __launch_bounds__(kFftThreads, 3) k_fft_pass(FftPassParams p) {
       l = t % TX, i = t / TX;
     }
     if (l < valid) tile[l * lstep + i * estep] = res[i * S + l];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Bluestein (chirp-z) transform, for line lengths N with a prime factor above 7
-// (cuFFT's cufftPlan3d accepts every size, src/cudaMain.cu:479-482).
-//
-// With c_j = exp(-i pi j^2 / N), jk = (j^2 + k^2 - (k - j)^2) / 2 gives
-//   X_k = c_k sum_j (x_j c_j) conj(c_{k-j}),
-// a circular convolution of length M >= 2N - 1 (M 7-smooth), evaluated as
-// FFT_M -> product with the table bhat = FFT_M(b) / M, where b holds
-// conj(c_m) at m and M - m -> a second FFT_M of the conjugate, since the
-// inverse transform is conj(FFT(conj(y))) / M.  Chirp and table are formed in
-// double on the host (j^2 reduced mod 2N in integers) and rounded to float.
-// The lines of a pass are processed in chunks of `nlines` padded lines held
-// in `work`: [nlines][M] for x lines (the padded FFT is a row pass), [M][nlines]
-// for y and z lines (a column pass), so every gather, product and scatter
-// reads and writes contiguous memory.
-// ---------------------------------------------------------------------------
-// T = float2 for the FP32 engine, double2 for the FP64 pipeline (its tables in double).
-template <class T>
-struct BlueParamsT {
-  T *data;                // the volumes being transformed
-  T *work;                // x lines: [nlines][m]; y and z lines: [m][nlines] (lines fastest)
-  const T *chirp;         // c_j, j < n
-  const T *bhat;          // FFT_m(b) / m
-  uint32_t nx, ny, nz;    // volume dimensions (nz: the planes this call covers)
-  size_t vstride;         // elements between volumes
-  uint32_t n, m;          // line length, padded length
-  uint64_t line0;         // first line of this chunk
-  uint32_t nlines;        // lines in this chunk
-  uint32_t lines_per_vol; // x pass: ny nz; y pass: nx nz; z pass: nx ny
-};
-using BlueParams = BlueParamsT<float2>;
-
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-
-// Offset of line `line` and the stride between its elements.
-template <int AXIS, class P>
-__device__ __forceinline__ size_t blue_line(const P &p, uint64_t line, size_t &estep) {
-  const uint64_t v = line / p.lines_per_vol;
-  const uint32_t r = uint32_t(line % p.lines_per_vol);
-  size_t base = v * p.vstride;
-  if (AXIS == 0) {
-    base += size_t(r) * p.nx;
-    estep = 1;
-  } else if (AXIS == 1) {
-    base += size_t(r / p.nx) * p.nx * p.ny + r % p.nx;
-    estep = p.nx;
-  } else {
-    base += size_t(r / p.nx) * p.nx + r % p.nx;
-    estep = size_t(p.nx) * p.ny;
-  }
-  return base;
-}
-
-// work = x_j c_j (j < n), 0 (n <= j < m).  Thread t takes element t of the
-// work buffer, so its stores are contiguous; for y and z lines consecutive
-// lines are consecutive x, so the volume reads are contiguous too.
-template <int AXIS, class T = float2>
-__global__ void k_blue_gather(BlueParamsT<T> p) {
-  const size_t total = size_t(p.nlines) * p.m;
-  for (size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x; t < total; t += size_t(gridDim.x) * blockDim.x) {
-    uint32_t l, j;
-    if (AXIS == 0) {
-      l = uint32_t(t / p.m), j = uint32_t(t % p.m);
-    } else {
-      l = uint32_t(t % p.nlines), j = uint32_t(t / p.nlines);
-    }
-    T v{};
-    if (j < p.n) {
-      size_t es;
-      const size_t b = blue_line<AXIS>(p, p.line0 + l, es);
-      v = cmul(p.data[b + j * es], p.chirp[j]);
-    }
-    p.work[t] = v;
-  }
-}
-
-// work = conj(work * bhat): the product of the transforms, conjugated for the inverse
-template <int AXIS, class T = float2>
-__global__ void k_blue_mul(BlueParamsT<T> p) {
-  const size_t total = size_t(p.nlines) * p.m;
-  for (size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x; t < total; t += size_t(gridDim.x) * blockDim.x) {
-    const T w = cmul(p.work[t], p.bhat[AXIS == 0 ? t % p.m : t / p.nlines]);
-    p.work[t] = T{w.x, -w.y};
-  }
-}
-
-// x_k = c_k conj(work element k of line l), k < n
-template <int AXIS, class T = float2>
-__global__ void k_blue_scatter(BlueParamsT<T> p) {
-  const size_t total = size_t(p.nlines) * p.n;
-  for (size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x; t < total; t += size_t(gridDim.x) * blockDim.x) {
-    uint32_t l, k;
-    size_t wi;
-    if (AXIS == 0) {
-      l = uint32_t(t / p.n), k = uint32_t(t % p.n);
-      wi = size_t(l) * p.m + k;
-    } else {
-      l = uint32_t(t % p.nlines), k = uint32_t(t / p.nlines);
-      wi = t;  // element k of line l at k nlines + l
-    }
-    const T w = p.work[wi];
-    size_t es;
-    const size_t b = blue_line<AXIS>(p, p.line0 + l, es);
-    p.data[b + k * es] = cmul(p.chirp[k], T{w.x, -w.y});
   }
 }
 

@@ -49,15 +49,10 @@
 #include <type_traits>
 #include <utility>
 
-#include "kernels.cuh"
+#include "complex.cuh"
 
 namespace cyr {
 
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 cfma(double s, double2 a, double2 acc) {
-  return make_double2(fma(s, a.x, acc.x), fma(s, a.y, acc.y));
-}
 template <class T>
 using Real = decltype(T::x);
 
@@ -352,7 +347,7 @@ struct MixTile {
 };
 
 template <class T, bool COL, int FORM>
-__global__ void __launch_bounds__(kMixThreads, sizeof(T) == 8 ? 4 : 1) k_mix_fft(const __grid_constant__ MixParams<T> p) {
+__global__ void __launch_bounds__(kMixThreads, sizeof(T) == 8 ? 4 : 2) k_mix_fft(const __grid_constant__ MixParams<T> p) {
   extern __shared__ unsigned char mix_smem[];
   MixTile<T, COL> tile{p, reinterpret_cast<T *>(mix_smem), nullptr, 0, 0};
   T *vol = p.data + size_t(blockIdx.y) * p.vstride;
@@ -484,5 +479,13 @@ __global__ void __launch_bounds__(kMixThreads, sizeof(T) == 8 ? 4 : 1) k_mix_fft
     });
   }
 }
+
+// The kernel instances live in translation units of their own (mixfft_f32.cu, mixfft_f64.cu).
+template <class T>
+cudaError_t mix_launch(MixForm form, bool row, dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                       const MixParams<T> &p);
+// Sets the instances' shared-memory limit on the current device.
+template <class T>
+cudaError_t mix_attributes(int smem);
 
 }  // namespace cyr
