@@ -14,14 +14,14 @@
 //   engine runs the reference's per-angle schedule (3 volumes per angle).
 //
 //   k_build -> 3D FFT -> k_dc -> per k: k_ewald_angles ->
-//   k_rotate_average -> k_fill + k_warp (detector) -> projection[e][k]
+//   k_rotate_gram -> k_warp_out (detector) -> projection[e][k]
 //
 // FIELDS strategy (fields.cuh): the spectra of the 7 M + 1 energy independent
 // morphology fields are formed once per request; every energy and angle is
 // combined from them inside the Ewald kernel, batched over energies:
 //
 //   k_moments -> k_build_fields -> 3D FFT -> per k and
-//   energy batch: k_ewald_fields -> k_rotate_average -> k_fill + k_warp
+//   energy batch: k_ewald_fields -> k_rotate_gram -> k_warp_out (detector)
 //
 // All per-request constants (optical constants of every energy, angle
 // coefficients, warp coefficients, q-grid and window tables) are computed on
@@ -366,21 +366,33 @@ struct ZTune {
 // Device scratch of one request in flight (grow-only).  The plain entry points
 // share the device context's; every serving slot owns one.
 struct Scratch {
-  DeviceBuffer spec, images, avg, params, dc, moments, means, errors, conv, flags, fmean;
+  DeviceBuffer spec, images, avg, params, dc, means, conv;
+  // words that a request starts at zero, cleared by one memset: the error count, the negative-fraction flag and,
+  // from kMomentsAt on, the moment sums
+  DeviceBuffer errors;
   DeviceBuffer zmask;              // store mask of the FIELDS z pass (k_zmask)
   cudaEvent_t last_use = nullptr;  // completion of the last request that used it
   uint64_t generation = 0;         // bumped by every (re)allocation of a buffer above
+  static constexpr size_t kMomentsAt = 256;
+  unsigned *flag() const { return errors.as<unsigned>() + 1; }
+  double *moments() const { return reinterpret_cast<double *>(errors.as<unsigned char>() + kMomentsAt); }
+  int clear(size_t nmoments, cudaStream_t st) {
+    const size_t bytes = kMomentsAt + nmoments * sizeof(double);
+    CYR_TRY(errors.ensure(bytes));
+    CYR_CUDA(cudaMemsetAsync(errors.ptr, 0, bytes, st));
+    return CYR_OK;
+  }
   int init() {
     if (!last_use) CYR_CUDA(cudaEventCreateWithFlags(&last_use, cudaEventDisableTiming));
     return CYR_OK;
   }
   // serving slots: stream-ordered allocations on `st`
   void bind(cudaStream_t st) {
-    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &moments, &means, &errors, &conv, &flags, &fmean, &zmask})
+    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &means, &errors, &conv, &zmask})
       b->stream = st, b->generation = &generation;
   }
   void release() {
-    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &moments, &means, &errors, &conv, &flags, &fmean, &zmask})
+    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &means, &errors, &conv, &zmask})
       b->release();
   }
 };
@@ -1008,7 +1020,7 @@ struct Plan {
   uint32_t ebatch = 1;                  // energies per Ewald / rotation launch
   bool ewald_sparse = false;            // the combination coefficients keep their structural zeros
   size_t off_fcoef = 0, off_kmag = 0, off_mat = 0, off_kvec = 0;
-  uint32_t mom_zstep = 1;               // z planes between the moment samples (FIELDS)
+  uint32_t mom_zstep = 1, mom_ystep = 1;  // z planes and rows between the moment samples
   // LAB frame, square detector: conservative per-row column ranges of the
   // Ewald output, [k][energy][row] (ewald_rows)
   bool has_rows = false;
@@ -1341,11 +1353,19 @@ int make_plan(const cyr_options *o, const float *optical, Plan &pl) {
   // FIELDS strategy: choose it, then its tables
   pl.npk = num_packed(pl.nmat);
   if (o->strategy == CYR_STRATEGY_AUTO) {
-    // plane-volumes moved per request (read + write of the FFT passes, morphology reads)
+    // plane-volumes moved per request (read + write of the FFT passes, morphology
+    // reads), and its launches: one costs about 2 us, in which the device moves
+    // 0.84 M points (16 bytes each).  Small volumes are bound by their launches, of
+    // which the per-energy spectra need more from the second energy on.
+    const double launch = 0.84e6 / double(pl.npix);
     const double planes = pl.pruned ? pl.kz : pl.nz;
     const double spectra = pl.material_frame ? double(pl.nk) * pl.nang * 3.0 : double(pl.nvol);
-    const double per_energy = double(pl.ne) * (spectra * planes + 2.0 * pl.nmat * pl.nz);
-    const double once = (1.5 * pl.npk + 2.0 * pl.nmat) * pl.nz;
+    const double builds = double(pl.ne) * (pl.material_frame ? double(pl.nk) * pl.nang : 1.0);
+    // the build fused with the z transform is bound by issue: 1.2 times its traffic's time with the warp FFT,
+    // 1.8 with other z lengths, relative to the field passes (256 x 256 x 128 and x 90, 4 materials, 1 to 4 energies)
+    const double per_energy = double(pl.ne) * (spectra * planes + 2.0 * pl.nmat * pl.nz) * (pl.zwarp ? 1.2 : 1.8) +
+                              launch * (1.0 + builds * (pl.material_frame ? 5.0 : 4.0) + 3.0 * pl.ne * pl.nk);
+    const double once = (1.5 * pl.npk + 2.0 * pl.nmat) * pl.nz + launch * (5.0 + 3.0 * pl.nk);
     pl.fields = once < per_energy;
   } else {
     pl.fields = o->strategy == CYR_STRATEGY_FIELDS;
@@ -1362,8 +1382,9 @@ int make_plan(const cyr_options *o, const float *optical, Plan &pl) {
     const uint32_t eb = (pl.ne + nbatches - 1) / nbatches;
     pl.ebatch = nbatches == 1 ? pl.ne : std::min(pl.ne, (eb + nep - 1) / nep * nep);
   }
+  pl.mom_zstep = std::max(1u, pl.nz / 16);  // 16 sampled planes, 256 K points in all (at least 16 rows of a plane)
+  pl.mom_ystep = std::max<uint32_t>(1, std::min<uint32_t>(pl.ny / 16, uint32_t(pl.npix * std::min(pl.nz, 16u) >> 18)));
   if (pl.fields) {
-    pl.mom_zstep = std::max(1u, pl.nz / 16);  // 16 sampled planes
     // coef[e][v][j] = (alpha, beta): Nt_v(k) = sum_j alpha Z_j(k) + beta conj Z_j(-k), where
     // Z_j = F_2j + i F_2j+1 and field g = 7 m + f (f: u_x^2 u_y^2 u_z^2 u_xu_y u_xu_z u_yu_z phi_ui), T last
     const uint32_t nf = num_fields(pl.nmat), npk = pl.npk;
@@ -1715,7 +1736,7 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
   fp.vox = d_vox;
   fp.nx = pl.nx, fp.ny = pl.ny, fp.nz = pl.nz, fp.nmat = pl.nmat;
   fp.nvox = pl.nvox;
-  fp.mom = sc.moments.as<double>();  // each block forms the field means from the moments
+  fp.mom = sc.moments();  // each block forms the field means from the moments
   fp.nsamp = nsamp;
   if (pl.hanning) {
     fp.hann_x = reinterpret_cast<const float *>(dp + pl.off_hx);
@@ -1855,12 +1876,9 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
         k_rotate_gram<3, packed_energies<3>()><<<rgrid, kRotTile * kRotTile, rsm, st>>>(rg);
       ctx.prof.end(slot, st);
       float *dst = d_out + (size_t(e0) * pl.nk + k) * pl.npix;
-      slot = ctx.prof.begin(kFill, st);
-      k_fill<<<dim3(pix_blocks, nb), 256, 0, st>>>(dst, pl.npix, fillv, ostride);
-      ctx.prof.end(slot, st);
       slot = ctx.prof.begin(kWarp, st);
-      k_warp<<<dim3(pix_blocks, nb), 256, 0, st>>>(sc.avg.as<float>(), dst, W, H, pl.detector_warp[k], pl.npix,
-                                                   ostride);
+      k_warp_out<<<dim3(pix_blocks, nb), 256, 0, st>>>(sc.avg.as<float>(), dst, W, H, pl.detector_warp[k], fillv,
+                                                       ostride);
       ctx.prof.end(slot, st);
       CYR_CUDA(cudaGetLastError());
     }
@@ -1886,6 +1904,11 @@ struct RunMode {
 };
 
 
+// Builds from which the conversion pass (a read and a write of the morphology,
+// 217 us on 256 x 256 x 128 with 4 materials) repays the trigonometry that each
+// build of the unconverted form repeats.
+constexpr size_t kConvertBuilds = 4;
+
 int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const float *optical, const float4 *d_vox,
                 float *d_out, cudaStream_t st, const RunMode &mode = RunMode()) {
   Plan local;
@@ -1902,8 +1925,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
   }
   // scratch (grow-only); wait for the previous user of the scratch
   if (!mode.capturing) CYR_CUDA(cudaStreamWaitEvent(st, sc.last_use, 0));
-  CYR_TRY(sc.errors.ensure(sizeof(unsigned)));
-  CYR_CUDA(cudaMemsetAsync(sc.errors.ptr, 0, sizeof(unsigned), st));
+  CYR_TRY(sc.clear(size_t(pl.nmat) * kMoments, st));
   if (!pl.fields) {
     CYR_TRY(sc.spec.ensure(pl.nvol * pl.vstride * sizeof(float2)));
     CYR_TRY(sc.images.ensure(image_bytes(pl)));
@@ -1944,13 +1966,11 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
   }
   const bool slabs = mode.host_vox && pl.fields;
   // volume moments of the morphology -> mean of every tensor entry, per energy
-  CYR_TRY(sc.moments.ensure(size_t(pl.nmat) * kMoments * sizeof(double)));
   CYR_TRY(sc.means.ensure(size_t(pl.ne) * 6 * sizeof(float2)));
-  CYR_CUDA(cudaMemsetAsync(sc.moments.ptr, 0, size_t(pl.nmat) * kMoments * sizeof(double), st));
-  // Euler morphologies are converted once per request to the trigonometry-free vector form
-  const bool convert = o->morphology_type == 0 && !pl.fields;
-  CYR_TRY(sc.flags.ensure(sizeof(unsigned)));
-  CYR_CUDA(cudaMemsetAsync(sc.flags.ptr, 0, sizeof(unsigned), st));
+  // Per-energy spectra of Euler morphologies: converted to the trigonometry-free
+  // vector form once per request when enough builds follow to repay the pass
+  const size_t builds = pl.material_frame ? size_t(pl.ne) * pl.nk * pl.nang : pl.ne;
+  const bool convert = o->morphology_type == 0 && !pl.fields && builds >= kConvertBuilds;
   if (convert) CYR_TRY(sc.conv.ensure(pl.nvox * pl.nmat * sizeof(float4)));
   {
     MomentParams mp{};
@@ -1962,21 +1982,22 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
       mp.hann_y = reinterpret_cast<const float *>(dp + pl.off_hy);
       mp.hann_z = reinterpret_cast<const float *>(dp + pl.off_hz);
     }
-    mp.out = sc.moments.as<double>();
+    mp.out = sc.moments();
     mp.conv = convert ? sc.conv.as<float4>() : nullptr;
     // the conversion needs every voxel; the means alone need only a subsample of planes
     // (with a slab upload: the planes copied first for that purpose)
     mp.zstep = convert ? 1u : pl.mom_zstep;
+    mp.ystep = convert ? 1u : pl.mom_ystep;
     if (slabs) {
       mp.zstep = upload.sample_zstep;
       CYR_CUDA(cudaStreamWaitEvent(st, upload.sample, 0));
     }
-    mp.neg = sc.flags.as<unsigned>();
+    mp.neg = sc.flag();
     int nsm = 0;
     CYR_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx.device));
     // about 8 samples per thread: small volumes get few blocks (each block ends in
     // kMoments double atomics on the same addresses), large ones 4 per SM
-    const size_t nsamp = pl.npix * ((pl.nz + mp.zstep - 1) / mp.zstep);
+    const size_t nsamp = size_t(pl.nx) * ((pl.ny + mp.ystep - 1) / mp.ystep) * ((pl.nz + mp.zstep - 1) / mp.zstep);
     const dim3 grid(uint32_t(std::max<size_t>(1, std::min<size_t>((nsamp + 2047) / 2048, size_t(nsm) * 4))), pl.nmat);
     int slot = ctx.prof.begin(kMom, st);
     if (o->morphology_type == 0)
@@ -1986,14 +2007,13 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
     ctx.prof.end(slot, st);
     CYR_CUDA(cudaGetLastError());
     if (pl.fields) {
-      const size_t nsamp = pl.npix * ((mp.nz + mp.zstep - 1) / mp.zstep);
       CYR_TRY(run_fields(ctx, sc, o, pl, dp, d_vox, d_out, st, nsamp, slabs ? &upload : nullptr, mode.capturing));
       // an event recorded inside a capture cannot be waited on outside it (slots keep order by their stream)
       if (!mode.capturing) CYR_CUDA(cudaEventRecord(sc.last_use, st));
       return CYR_OK;
     }
     slot = ctx.prof.begin(kMeans, st);
-    k_entry_means<<<1, 64, 0, st>>>(sc.moments.as<double>(), pl.nmat, pl.nvox,
+    k_entry_means<<<(pl.ne * 12 + 127) / 128, 128, 0, st>>>(sc.moments(), pl.nmat, nsamp,
                                     reinterpret_cast<const MaterialConsts *>(dp + pl.off_mc), pl.ne,
                                     sc.means.as<float2>());
     ctx.prof.end(slot, st);
@@ -2012,7 +2032,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
   bp.morphology = o->morphology_type;
   bp.out = spec;
   bp.conv = convert ? sc.conv.as<float4>() : nullptr;
-  bp.neg = sc.flags.as<unsigned>();
+  bp.neg = sc.flag();
   if (pl.hanning) {
     bp.hann_x = reinterpret_cast<const float *>(dp + pl.off_hx);
     bp.hann_y = reinterpret_cast<const float *>(dp + pl.off_hy);
@@ -2045,7 +2065,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
           const size_t smem = zwarp_smem(pl.nz, bp.nvol, cfg.tx, pl.nmat, cfg.stage);
 #define CYR_LAUNCH_WARP_ZT(V, T)                                                   \
   if (o->morphology_type == 0) {                                                   \
-    k_build_fft_z_warp<0, true, V, T><<<g, 256, smem, st>>>(zp, mce);              \
+    if (convert) k_build_fft_z_warp<0, true, V, T><<<g, 256, smem, st>>>(zp, mce); \
     k_build_fft_z_warp<0, false, V, T><<<g, 256, smem, st>>>(zp, mce);             \
   } else {                                                                         \
     k_build_fft_z_warp<1, false, V, T><<<g, 256, smem, st>>>(zp, mce);             \
@@ -2112,16 +2132,16 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
             cfg.stage = pl.zstage;
             cfg.tx = pl.ztx;
           }
-          slot = ctx.prof.begin(kBuildZ, st, o->morphology_type == 0 ? 2 : 1);
+          slot = ctx.prof.begin(kBuildZ, st, convert ? 2 : 1);
           launch_warp(cfg);
           ctx.prof.end(slot, st);
         }
       } else {
         const dim3 grid((pl.nx + pl.ztx - 1) / pl.ztx * pl.ny);
-        slot = ctx.prof.begin(kBuildZ, st, o->morphology_type == 0 ? 2 : 1);
+        slot = ctx.prof.begin(kBuildZ, st, convert ? 2 : 1);
         const size_t smem = (size_t(2) * bp.nvol * pl.nz * (pl.ztx + 1) + pl.nz) * sizeof(float2);
         if (o->morphology_type == 0) {
-          k_build_fft_z<0, true><<<grid, kFftThreads, smem, st>>>(zp, mce);
+          if (convert) k_build_fft_z<0, true><<<grid, kFftThreads, smem, st>>>(zp, mce);
           k_build_fft_z<0, false><<<grid, kFftThreads, smem, st>>>(zp, mce);
         } else {
           k_build_fft_z<1, false><<<grid, kFftThreads, smem, st>>>(zp, mce);
@@ -2131,9 +2151,9 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
       CYR_CUDA(cudaGetLastError());
       CYR_TRY(fft3d(ctx, spec, pl.nx, pl.ny, pl.kz, bp.nvol, st, true));
     } else {
-      slot = ctx.prof.begin(kBuild, st, o->morphology_type == 0 ? 2 : 1);
+      slot = ctx.prof.begin(kBuild, st, convert ? 2 : 1);
       if (o->morphology_type == 0) {
-        k_build<0, true><<<build_blocks, 256, 0, st>>>(bp, mce);
+        if (convert) k_build<0, true><<<build_blocks, 256, 0, st>>>(bp, mce);
         k_build<0, false><<<build_blocks, 256, 0, st>>>(bp, mce);
       } else {
         k_build<1, false><<<build_blocks, 256, 0, st>>>(bp, mce);
@@ -2236,11 +2256,9 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
       ctx.prof.end(slot, st);
       CYR_CUDA(cudaGetLastError());
       float *dst = d_out + (size_t(e) * pl.nk + k) * pl.npix;
-      slot = ctx.prof.begin(kFill, st);
-      k_fill<<<pix_blocks, 256, 0, st>>>(dst, pl.npix, o->rot_mask ? 0.f : std::numeric_limits<float>::quiet_NaN());
-      ctx.prof.end(slot, st);
       slot = ctx.prof.begin(kWarp, st);
-      k_warp<<<pix_blocks, 256, 0, st>>>(avg, dst, W, H, pl.detector_warp[k]);
+      k_warp_out<<<pix_blocks, 256, 0, st>>>(avg, dst, W, H, pl.detector_warp[k],
+                                             o->rot_mask ? 0.f : std::numeric_limits<float>::quiet_NaN(), 0);
       ctx.prof.end(slot, st);
       CYR_CUDA(cudaGetLastError());
     }
@@ -2725,11 +2743,8 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   CYR_TRY(sc.spec.ensure(size_t(G) * npk * nvox * sizeof(float2)));
   CYR_TRY(sc.images.ensure(image_bytes(p0, vb)));
   CYR_TRY(sc.avg.ensure(size_t(vb) * npix * sizeof(float)));
-  CYR_TRY(sc.moments.ensure(size_t(G) * nmat * kMoments * sizeof(double)));
   CYR_TRY(sc.dc.ensure(size_t(G) * npk * sizeof(float2)));
-  CYR_TRY(sc.errors.ensure(sizeof(unsigned)));
-  CYR_CUDA(cudaMemsetAsync(sc.errors.ptr, 0, sizeof(unsigned), st));
-  CYR_CUDA(cudaMemsetAsync(sc.moments.ptr, 0, size_t(G) * nmat * kMoments * sizeof(double), st));
+  CYR_TRY(sc.clear(size_t(G) * nmat * kMoments, st));
   float2 *spec = sc.spec.as<float2>();
   int sms = 0;
   CYR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
@@ -2744,9 +2759,9 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     mp.hann_y = reinterpret_cast<const float *>(dp + p0.off_hy);
     mp.hann_z = reinterpret_cast<const float *>(dp + p0.off_hz);
   }
-  mp.out = sc.moments.as<double>();
-  mp.zstep = p0.mom_zstep;
-  const size_t nsamp = npix * ((p0.nz + mp.zstep - 1) / mp.zstep);
+  mp.out = sc.moments();
+  mp.zstep = p0.mom_zstep, mp.ystep = p0.mom_ystep;
+  const size_t nsamp = size_t(p0.nx) * ((p0.ny + mp.ystep - 1) / mp.ystep) * ((p0.nz + mp.zstep - 1) / mp.zstep);
   {
     const dim3 grid(uint32_t(std::max<size_t>(1, std::min<size_t>((nsamp + 2047) / 2048, size_t(sms) * 4))), nmat, G);
     const int slot = ctx.prof.begin(kMom, st);
@@ -2762,7 +2777,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   fp.vox_g = vox_g;
   fp.nx = p0.nx, fp.ny = p0.ny, fp.nz = p0.nz, fp.nmat = nmat;
   fp.nvox = nvox;
-  fp.mom = sc.moments.as<double>();
+  fp.mom = sc.moments();
   fp.mom_stride = size_t(nmat) * kMoments;
   fp.nsamp = nsamp;
   fp.out = spec;

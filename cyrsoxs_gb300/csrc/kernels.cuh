@@ -131,7 +131,7 @@ __device__ __forceinline__ void nt_entries(const BuildParams &p, const MaterialC
 // the path always replaces by the mean of its neighbours (src/cudaMain.cu:
 // 123-176); removing it keeps the FP32 FFT's rounding floor proportional to
 // the fluctuations instead of to the (~5x larger) mean.
-constexpr int kMoments = 7;
+constexpr int kMoments = 7;  // at most 8 (k_moments)
 struct MomentParams {
   const float4 *vox;
   const float4 *const *vox_g;  // request group (blockIdx.z = request): its morphologies, or null
@@ -141,7 +141,9 @@ struct MomentParams {
   double *out;      // [nmat][kMoments], accumulated
   float4 *conv;     // Euler only: (sqrt(phi_a) s, phi_ui) per material and voxel, or null
   unsigned *neg;    // set when some phi_a < 0
-  uint32_t zstep;   // sample every zstep-th z plane (1: all; must be 1 with conv)
+  // sample every ystep-th row of every zstep-th z plane (1: all; must be 1 with conv).  The sums only have to give
+  // a constant near the mean: 16 planes of about 16 K points each leave a residual far below the strongest bins
+  uint32_t ystep, zstep;
 };
 
 template <int MORPH>
@@ -157,18 +159,20 @@ __global__ void __launch_bounds__(256) k_moments(MomentParams p) {
   float acc[kMoments];
 #pragma unroll
   for (int q = 0; q < kMoments; ++q) acc[q] = 0.f;
-  // samples: every pixel of the planes z = 0, zstep, 2 zstep, ...; the
-  // thread's (sampled plane, pixel) position advances by the grid stride
-  // without an index division per sample
-  const size_t plane = size_t(p.nx) * p.ny, stride = size_t(gridDim.x) * blockDim.x;
-  const uint32_t nzs = (p.nz + p.zstep - 1) / p.zstep;
-  const size_t s0 = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  uint32_t zi = uint32_t(s0 / plane);
-  size_t pix = s0 - size_t(zi) * plane;
-  for (; zi < nzs; pix += stride) {
-    while (pix >= plane) pix -= plane, ++zi;
-    if (zi >= nzs) break;
-    const size_t i = size_t(zi) * p.zstep * plane + pix;
+  // samples: the rows y = 0, ystep, 2 ystep, ... of the planes z = 0, zstep,
+  // 2 zstep, ..., whole rows, so that a warp's loads stay contiguous; the
+  // thread's (row, x) position advances by the grid stride
+  const uint32_t stride = gridDim.x * blockDim.x, srow = stride / p.nx, sx0 = stride % p.nx;
+  const uint32_t nys = (p.ny + p.ystep - 1) / p.ystep, rows = nys * ((p.nz + p.zstep - 1) / p.zstep);
+  const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t row = first / p.nx, x = first % p.nx;
+  for (; row < rows; row += srow, x += sx0) {
+    if (x >= p.nx) {
+      x -= p.nx;
+      if (++row >= rows) break;
+    }
+    const uint32_t zi = row / nys, y = (row - zi * nys) * p.ystep, z = zi * p.zstep;
+    const size_t i = (size_t(z) * p.ny + y) * p.nx + x;
     float sx, sy, sz, pa, pui;
     director<MORPH>(__ldg(&p.vox[m * p.nvox + i]), sx, sy, sz, pa, pui);
     if (MORPH == 0 && p.conv) {
@@ -177,10 +181,7 @@ __global__ void __launch_bounds__(256) k_moments(MomentParams p) {
       p.conv[m * p.nvox + i] = make_float4(r * sx, r * sy, r * sz, pui);
     }
     float w = 1.f;
-    if (p.hann_x) {
-      const uint32_t x = uint32_t(pix) % p.nx, y = uint32_t(pix) / p.nx, z = zi * p.zstep;
-      w = p.hann_x[x] * p.hann_y[y] * p.hann_z[z];
-    }
+    if (p.hann_x) w = p.hann_x[x] * p.hann_y[y] * p.hann_z[z];
     const float wa = w * pa;
     acc[0] += wa * sx * sx;
     acc[1] += wa * sy * sy;
@@ -190,41 +191,56 @@ __global__ void __launch_bounds__(256) k_moments(MomentParams p) {
     acc[5] += wa * sy * sz;
     acc[6] += w * pui;
   }
+  // Warp sums of the eight slots (seven moments and a zero), by halving: at
+  // each of the first three exchanges a lane keeps half of its slots and gives
+  // the other half away, so 4 + 2 + 1 + 1 + 1 double additions do the work of
+  // 7 x 5; the FP64 pipe (1/64 of the FP32 rate) is what this reduction waits
+  // for (37 -> 12 us on 256 x 256 x 32, 2 materials, with the rest of the kernel).
+  const uint32_t lane = threadIdx.x & 31u;
+  double v[8];
 #pragma unroll
-  for (int q = 0; q < kMoments; ++q) {
-    double v = double(acc[q]);
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][q] = v;
+  for (int q = 0; q < 8; ++q) v[q] = q < kMoments ? double(acc[q < kMoments ? q : 0]) : 0.0;
+#pragma unroll
+  for (int h = 4; h >= 1; h >>= 1) {
+    const bool up = (lane & uint32_t(4 * h)) != 0;  // lanes 16, 8, 4 apart for h = 4, 2, 1
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const double give = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * h);
+    }
   }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  // lane 4 q of the warp holds slot q: bit 4 of the lane selects slots 4-7, bit 3 the upper pair, bit 2 the odd one
+  if ((lane & 3u) == 0 && (lane >> 2) < uint32_t(kMoments)) red[threadIdx.x >> 5][lane >> 2] = v[0];
   __syncthreads();
   if (threadIdx.x < kMoments) {
-    double v = 0.0;
-    for (int wi = 0; wi < int(blockDim.x >> 5); ++wi) v += red[wi][threadIdx.x];
-    atomicAdd(&p.out[m * kMoments + threadIdx.x], v);
+    double r = 0.0;
+    for (int wi = 0; wi < int(blockDim.x >> 5); ++wi) r += red[wi][threadIdx.x];
+    atomicAdd(&p.out[m * kMoments + threadIdx.x], r);
   }
 }
 
 // Mean of each windowed tensor entry for every energy: out[e][6] (xx xy xz yy yz zz).
-__global__ void k_entry_means(const double *__restrict__ mom, uint32_t nmat, size_t nvox,
+// One thread per (energy, entry, real or imaginary part): a thread per energy ran 150 dependent FP64 operations
+// (11 us for one energy of 4 materials).
+__global__ void k_entry_means(const double *__restrict__ mom, uint32_t nmat, size_t nsamp,
                               const MaterialConsts *__restrict__ mcs, uint32_t ne, float2 *__restrict__ out) {
-  for (uint32_t e = threadIdx.x; e < ne; e += blockDim.x) {
-    double r[6][2] = {};
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ne * 12; t += gridDim.x * blockDim.x) {
+    const uint32_t e = t / 12, q = t % 12 / 2, part = t % 2;
+    const MaterialConsts &c = mcs[e];
+    auto comp = [&](float2 v) { return double(part ? v.y : v.x); };
+    double r = 0.0;
     for (uint32_t m = 0; m < nmat; ++m) {
       const double *M = mom + m * kMoments;
-      const MaterialConsts &c = mcs[e];
-      const double A[2] = {c.A[m].x, c.A[m].y}, B[2] = {c.B[m].x, c.B[m].y};
-      const double C[2] = {c.C[m].x, c.C[m].y}, D[2] = {c.D[m].x, c.D[m].y};
-      for (int k = 0; k < 2; ++k) {
-        r[0][k] += A[k] * M[0] + B[k] * (M[1] + M[2]) + C[k] * M[6];
-        r[3][k] += A[k] * M[1] + B[k] * (M[0] + M[2]) + C[k] * M[6];
-        r[5][k] += A[k] * M[2] + B[k] * (M[0] + M[1]) + C[k] * M[6];
-        r[1][k] += D[k] * M[3];
-        r[2][k] += D[k] * M[4];
-        r[4][k] += D[k] * M[5];
-      }
+      if (q == 0) r += comp(c.A[m]) * M[0] + comp(c.B[m]) * (M[1] + M[2]) + comp(c.C[m]) * M[6];
+      if (q == 3) r += comp(c.A[m]) * M[1] + comp(c.B[m]) * (M[0] + M[2]) + comp(c.C[m]) * M[6];
+      if (q == 5) r += comp(c.A[m]) * M[2] + comp(c.B[m]) * (M[0] + M[1]) + comp(c.C[m]) * M[6];
+      if (q == 1) r += comp(c.D[m]) * M[3];
+      if (q == 2) r += comp(c.D[m]) * M[4];
+      if (q == 4) r += comp(c.D[m]) * M[5];
     }
-    for (int q = 0; q < 6; ++q)
-      out[e * 6 + q] = make_float2(float(r[q][0] / double(nvox)), float(r[q][1] / double(nvox)));
+    (part ? out[e * 6 + q].y : out[e * 6 + q].x) = float(r / double(nsamp));
   }
 }
 
@@ -1865,13 +1881,10 @@ __device__ __forceinline__ bool warp_sample(const float *__restrict__ src, int W
   return true;
 }
 
-// blockIdx.y selects image src + y * src_stride -> dst + y * dst_stride.
-__global__ void k_warp(const float *__restrict__ src, float *__restrict__ dst, int W, int H, WarpCoef c,
-                       size_t src_stride = 0, size_t dst_stride = 0) {
+// dst keeps its value where the source point lies outside the image.
+__global__ void k_warp(const float *__restrict__ src, float *__restrict__ dst, int W, int H, WarpCoef c) {
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= size_t(W) * H) return;
-  src += blockIdx.y * src_stride;
-  dst += blockIdx.y * dst_stride;
   float v;
   if (warp_sample(src, W, H, c, int(t % W), int(t / W), v)) dst[t] = v;
 }
@@ -2069,8 +2082,8 @@ __global__ void __launch_bounds__(kRotTile * kRotTile, 3) k_rotate_gram(RotateGr
 }
 
 // Detector warp of a request group's angle averages (one image per virtual
-// energy ve = ve0 + blockIdx.y, request ve / e_per_req): the fill and the warp of
-// k_fill + k_warp in one pass, written to that request's own projection.
+// energy ve = ve0 + blockIdx.y, request ve / e_per_req), as k_warp_out, written to
+// that request's own projection.
 __global__ void k_warp_group(const float *__restrict__ src, float *const *__restrict__ out_g, uint32_t e_per_req,
                              uint32_t ve0, int W, int H, WarpCoef c, float prefill) {
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -2082,9 +2095,17 @@ __global__ void k_warp_group(const float *__restrict__ src, float *const *__rest
   out_g[ve / e_per_req][size_t(ve % e_per_req) * npix + t] = v;
 }
 
-__global__ void k_fill(float *dst, size_t n, float v, size_t stride = 0) {
+// Detector warp of a batch of angle averages (blockIdx.y): every pixel of dst
+// is written, the prefill where the source point falls outside, so no fill
+// pass runs before it (src/cudaMain.cu:916-960).
+__global__ void k_warp_out(const float *__restrict__ src, float *__restrict__ dst, int W, int H, WarpCoef c,
+                           float prefill, size_t dst_stride) {
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t < n) dst[blockIdx.y * stride + t] = v;
+  const size_t npix = size_t(W) * H;
+  if (t >= npix) return;
+  float v;
+  if (!warp_sample(src + blockIdx.y * npix, W, H, c, int(t % W), int(t / W), v)) v = prefill;
+  dst[blockIdx.y * dst_stride + t] = v;
 }
 
 }  // namespace cyr
