@@ -1021,10 +1021,6 @@ struct Plan {
   bool ewald_sparse = false;            // the combination coefficients keep their structural zeros
   size_t off_fcoef = 0, off_kmag = 0, off_mat = 0, off_kvec = 0;
   uint32_t mom_zstep = 1, mom_ystep = 1;  // z planes and rows between the moment samples
-  // LAB frame, square detector: conservative per-row column ranges of the
-  // Ewald output, [k][energy][row] (ewald_rows)
-  bool has_rows = false;
-  size_t off_rows = 0;
 };
 
 // Energies per Gram record: the FIELDS strategy packs 12 floats per pixel (4
@@ -1038,7 +1034,7 @@ size_t image_bytes(const Plan &pl, uint32_t nb = 1) {
   if (pl.material_frame) return size_t(nb) * pl.nang * pl.npix * sizeof(float);
   const uint32_t nep = gram_nep(pl), ng = pl.nbasis * (pl.nbasis + 1) / 2;
   const size_t rq = (size_t(nep) * ng + 3) / 4;
-  return size_t((nb + nep - 1) / nep) * gram_plane_size(int(pl.ny), int(pl.nx)) * rq * sizeof(float4);
+  return size_t((nb + nep - 1) / nep) * pl.npix * rq * sizeof(float4);
 }
 
 // Device bytes of the FIELDS strategy: packed field spectra, per-batch images and averages.
@@ -1113,42 +1109,6 @@ size_t arena_put(std::vector<unsigned char> &a, const T *src, size_t count) {
   a.resize(off + sizeof(T) * count);
   if (count) std::memcpy(a.data() + off, src, sizeof(T) * count);
   return off;
-}
-
-// Column ranges of the Ewald output that can hold a number, per k, energy and
-// detector row (LAB frame, square detector, where the rotation's image row y
-// is detector row Y).  ewald_geometry marks a pixel NaN unless
-// val = k^2 - (kx + qx)^2 - (ky + qy)^2 >= 0, so outside the disc
-// |kx + qx| <= sqrt(k^2 - (ky + qy)^2) the pixel is NaN.  The bound takes val
-// down to -1e-5 k^2 and adds two columns on each side, far beyond the float
-// rounding of the device's test; a row with no such column stores [W, -1].
-void ewald_rows(const cyr_options *o, Plan &pl) {
-  pl.has_rows = !pl.material_frame && pl.nx == pl.ny && size_t(pl.nx) * sizeof(int2) <= 48 * 1024;
-  if (!pl.has_rows) return;
-  const int W = int(pl.ny), H = int(pl.nx);
-  const float start = -static_cast<float>(kPi / o->phys_size);
-  const float dy = static_cast<float>((2.0 * kPi / o->phys_size) / ((pl.ny - 1) * 1.0));
-  const float dx = static_cast<float>((2.0 * kPi / o->phys_size) / ((pl.nx - 1) * 1.0));
-  std::vector<int2> rows(size_t(pl.nk) * pl.ne * H);
-  for (uint32_t k = 0; k < pl.nk; ++k)
-    for (uint32_t e = 0; e < pl.ne; ++e) {
-      const float kmag = static_cast<float>(2 * kPi / static_cast<float>(1239.84197 / o->energies[e]));
-      const double kx = double(kmag * pl.frames[k].k.x), ky = double(kmag * pl.frames[k].k.y);
-      for (int Y = 0; Y < H; ++Y) {
-        int lo = W, hi = -1;
-        const double ay = ky + double(start + float(Y) * dy);
-        const double r2 = double(kmag) * kmag * (1.0 + 1e-5) - ay * ay;
-        if (r2 >= 0) {
-          const double r = std::sqrt(r2);
-          const double xl = (-kx - r - double(start)) / double(dx), xh = (-kx + r - double(start)) / double(dx);
-          lo = int(std::max(0.0, std::floor(xl) - 2.0));
-          hi = int(std::min(double(W - 1), std::ceil(xh) + 2.0));
-          if (hi < lo) lo = W, hi = -1;
-        }
-        rows[(size_t(k) * pl.ne + e) * H + Y] = int2{lo, hi};
-      }
-    }
-  pl.off_rows = arena_put(pl.arena, rows.data(), rows.size());
 }
 
 // make_kframe scans 100 000 candidate base angles (as the reference does per
@@ -1458,7 +1418,6 @@ int make_plan(const cyr_options *o, const float *optical, Plan &pl) {
     }
     pl.off_mat = arena_put(pl.arena, mat.data(), mat.size());
   }
-  ewald_rows(o, pl);
   pl.arena.resize((pl.arena.size() + 255) & ~size_t(255));
   return CYR_OK;
 }
@@ -1722,6 +1681,26 @@ int tune_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Pla
   return rc;
 }
 
+// Rotation and angle average of rg.nenergies energies' Gram records, in tiles of
+// 32 x 32 pixels (1.2 source pixels in a tile's rotated square per destination
+// pixel; 16 x 16: 1.4) where that leaves six blocks per SM, else of 16 x 16
+// (240 x 240, 6 record groups: 384 tiles of 32 143 us, 1350 of 16 99 us).
+// Below four 16 x 16 tiles per SM the tile kernel waits for load latency, and
+// k_rotate_direct runs (256 x 256, one energy, 36 angles: 49 -> 37 us).
+constexpr size_t kRotateBlocks = 912, kRotateDirect = 608;
+
+template <int NB, int NEP>
+void launch_rotate(const RotateGramParams &rg, bool mask, cudaStream_t st) {
+  const unsigned groups = (rg.nenergies + NEP - 1) / NEP;
+  auto tiles = [&](int t) { return unsigned(((rg.W + t - 1) / t) * ((rg.H + t - 1) / t)); };
+  const bool large = size_t(tiles(32)) * groups >= kRotateBlocks;
+  const bool direct = size_t(tiles(16)) * groups < kRotateDirect;
+  auto kern = large    ? (mask ? k_rotate_gram<NB, NEP, 32, true> : k_rotate_gram<NB, NEP, 32, false>)
+              : direct ? (mask ? k_rotate_direct<NB, NEP, true> : k_rotate_direct<NB, NEP, false>)
+                       : (mask ? k_rotate_gram<NB, NEP, 16, true> : k_rotate_gram<NB, NEP, 16, false>);
+  kern<<<dim3(tiles(large ? 32 : 16), groups), kRotThreads, 0, st>>>(rg);
+}
+
 // FIELDS strategy after the moments: field means, packed field spectra, then
 // every energy (in batches) and k from them.
 int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan &pl, const unsigned char *dp,
@@ -1809,12 +1788,10 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
   fe.nangles = pl.nang;
   fe.images = sc.images.as<float>();
   fe.gram = sc.images.as<float4>();
-  fe.gplane = gram_plane_size(int(pl.ny), int(pl.nx));
   const size_t fsmem = size_t(kEwaldEnergies) * 6 * npk * sizeof(float4);
   const unsigned pix_blocks = unsigned((pl.npix + 255) / 256);
   const unsigned fpix_blocks = unsigned((pl.npix + 31) / 32);  // k_ewald_fields: 32 pixels per block
   const int W = int(pl.ny), H = int(pl.nx);  // the reference hands NPP width = Ny, height = Nx
-  const unsigned rot_tiles = unsigned(((W + kRotTile - 1) / kRotTile) * ((H + kRotTile - 1) / kRotTile));
   const WarpCoef *dwarp = reinterpret_cast<const WarpCoef *>(dp + pl.off_warp);
   const float *dmat = reinterpret_cast<const float *>(dp + pl.off_mat);
   const float fillv = o->rot_mask ? 0.f : std::numeric_limits<float>::quiet_NaN();
@@ -1833,22 +1810,17 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
     rp.avg = sc.avg.as<float>();
     RotateGramParams rg{};
     rg.gram = sc.images.as<float4>();
-    rg.plane = fe.gplane;
     rg.coef = rp.coef;
     rg.ecoef = fe.ecoef;
     rg.W = W, rg.H = H;
     rg.nangles = pl.nang;
-    rg.rot_mask = o->rot_mask;
     rg.avg = rp.avg;
     const uint32_t nep = gram_nep(pl);
-    const size_t rsm = pl.has_rows ? size_t(H) * sizeof(int2) : 0;
     for (uint32_t e0 = 0; e0 < pl.ne; e0 += pl.ebatch) {
       const uint32_t nb = std::min(pl.ebatch, pl.ne - e0);
       fe.e0 = e0;
       fe.nbatch = nb;
       rg.nenergies = nb;
-      rg.rows = pl.has_rows ? reinterpret_cast<const int2 *>(dp + pl.off_rows) + (size_t(k) * pl.ne + e0) * H : nullptr;
-      const dim3 rgrid(rot_tiles, (nb + nep - 1) / nep);
       slot = ctx.prof.begin(kEwaldFields, st);
       const unsigned fgrid = fpix_blocks * ((nb + kEwaldEnergies - 1) / kEwaldEnergies);
       const bool sparse = pl.ewald_sparse && ctx.sparse_ewald;
@@ -1871,9 +1843,9 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
       if (pl.material_frame)
         k_rotate_average<<<dim3(pix_blocks, nb), 256, 0, st>>>(rp);
       else if (pl.nbasis == 2)
-        k_rotate_gram<2, packed_energies<2>()><<<rgrid, kRotTile * kRotTile, rsm, st>>>(rg);
+        launch_rotate<2, packed_energies<2>()>(rg, o->rot_mask != 0, st);
       else
-        k_rotate_gram<3, packed_energies<3>()><<<rgrid, kRotTile * kRotTile, rsm, st>>>(rg);
+        launch_rotate<3, packed_energies<3>()>(rg, o->rot_mask != 0, st);
       ctx.prof.end(slot, st);
       float *dst = d_out + (size_t(e0) * pl.nk + k) * pl.npix;
       slot = ctx.prof.begin(kWarp, st);
@@ -2170,7 +2142,6 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
   };
   const unsigned pix_blocks = unsigned((pl.npix + 255) / 256);
   const int W = int(pl.ny), H = int(pl.nx);  // the reference hands NPP width = Ny, height = Nx
-  const unsigned rot_tiles = unsigned(((W + kRotTile - 1) / kRotTile) * ((H + kRotTile - 1) / kRotTile));
   const WarpCoef *dwarp = reinterpret_cast<const WarpCoef *>(dp + pl.off_warp);
   const float *dcoef = reinterpret_cast<const float *>(dp + pl.off_coef);
 
@@ -2196,7 +2167,6 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
         ep.coef = dcoef + size_t(k) * pl.nang * pl.nbasis;
         ep.images = images;
         ep.gram = reinterpret_cast<float4 *>(images);
-        ep.gplane = gram_plane_size(int(pl.ny), int(pl.nx));
         const int slot = ctx.prof.begin(kEwald, st);
         if (pl.nbasis == 2)
           k_ewald_angles<2><<<pix_blocks, 256, 0, st>>>(ep);
@@ -2238,20 +2208,16 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
       } else {
         RotateGramParams rg{};
         rg.gram = reinterpret_cast<const float4 *>(images);
-        rg.plane = gram_plane_size(int(pl.ny), int(pl.nx));
         rg.coef = dwarp + size_t(k) * pl.nang;
         rg.ecoef = dcoef + size_t(k) * pl.nang * pl.nbasis;
         rg.W = W, rg.H = H;
         rg.nangles = pl.nang;
         rg.nenergies = 1;
-        rg.rot_mask = o->rot_mask;
         rg.avg = avg;
-        rg.rows = pl.has_rows ? reinterpret_cast<const int2 *>(dp + pl.off_rows) + (size_t(k) * pl.ne + e) * H : nullptr;
-        const size_t rsm = pl.has_rows ? size_t(H) * sizeof(int2) : 0;
         if (pl.nbasis == 2)
-          k_rotate_gram<2, 1><<<rot_tiles, kRotTile * kRotTile, rsm, st>>>(rg);
+          launch_rotate<2, 1>(rg, o->rot_mask != 0, st);
         else
-          k_rotate_gram<3, 1><<<rot_tiles, kRotTile * kRotTile, rsm, st>>>(rg);
+          launch_rotate<3, 1>(rg, o->rot_mask != 0, st);
       }
       ctx.prof.end(slot, st);
       CYR_CUDA(cudaGetLastError());
@@ -2655,10 +2621,10 @@ int plan_request(ServerRequest &r, bool staged) {
   r.group_key.clear();
   if (pl.fields && !pl.material_frame && r.opt.case_type == 0 && pl.nk == 1 && pl.nbasis == 2 && r.d_vox) {
     char g[256];
-    std::snprintf(g, sizeof g, "%u,%u,%u,%u,%u,%a,%a,%a,%a,%u,%u,%u,%u,%u", r.opt.nx, r.opt.ny, r.opt.nz,
+    std::snprintf(g, sizeof g, "%u,%u,%u,%u,%u,%a,%a,%a,%a,%u,%u,%u,%u", r.opt.nx, r.opt.ny, r.opt.nz,
                   r.opt.num_material, r.opt.num_energies, double(r.opt.start_angle), double(r.opt.end_angle),
                   double(r.opt.increment_angle), double(r.opt.phys_size), r.opt.morphology_type,
-                  r.opt.ewald_interpolation, pl.hanning ? 1u : 0u, r.opt.rot_mask, pl.has_rows ? 1u : 0u);
+                  r.opt.ewald_interpolation, pl.hanning ? 1u : 0u, r.opt.rot_mask);
     r.group_key = g;
   }
   return CYR_OK;
@@ -2703,7 +2669,6 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   std::vector<unsigned char> arena = p0.arena;
   std::vector<float4> fc;
   std::vector<float> km;
-  std::vector<int2> rows;
   std::vector<const float4 *> vp;
   std::vector<float *> op;
   bool sparse = nmat <= 4 && ctx.sparse_ewald;  // every member's coefficients keep the structural zeros
@@ -2714,10 +2679,6 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     fc.insert(fc.end(), c, c + size_t(E) * 6 * npk);
     const float *k = reinterpret_cast<const float *>(pl.arena.data() + pl.off_kmag);
     km.insert(km.end(), k, k + E);
-    if (p0.has_rows) {
-      const int2 *rw = reinterpret_cast<const int2 *>(pl.arena.data() + pl.off_rows);
-      rows.insert(rows.end(), rw, rw + size_t(E) * H);
-    }
     vp.push_back(r->d_vox);
     op.push_back(r->d_out);
   }
@@ -2725,7 +2686,6 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   const size_t off_k = arena_put(arena, km.data(), km.size());
   const float kv0[3] = {p0.frames[0].k.x, p0.frames[0].k.y, p0.frames[0].k.z};
   const size_t off_kv = arena_put(arena, kv0, 3);
-  const size_t off_r = p0.has_rows ? arena_put(arena, rows.data(), rows.size()) : 0;
   const size_t off_v = arena_put(arena, vp.data(), vp.size());
   const size_t off_o = arena_put(arena, op.data(), op.size());
   arena.resize((arena.size() + 255) & ~size_t(255));
@@ -2855,24 +2815,19 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   fe.nangles = p0.nang;
   fe.images = sc.images.as<float>();
   fe.gram = sc.images.as<float4>();
-  fe.gplane = gram_plane_size(int(p0.ny), int(p0.nx));
   const KFrame &f = p0.frames[0];
   fe.kvx = f.k.x, fe.kvy = f.k.y, fe.kvz = f.k.z;
   fe.mat = reinterpret_cast<const float *>(dp + p0.off_mat);
   fe.ecoef = reinterpret_cast<const float *>(dp + p0.off_coef);
   RotateGramParams rg{};
   rg.gram = sc.images.as<float4>();
-  rg.plane = fe.gplane;
   rg.coef = reinterpret_cast<const WarpCoef *>(dp + p0.off_warp);
   rg.ecoef = fe.ecoef;
   rg.W = W, rg.H = H;
   rg.nangles = p0.nang;
-  rg.rot_mask = o->rot_mask;
   rg.avg = sc.avg.as<float>();
   const size_t fsmem = size_t(kEwaldEnergies) * 6 * npk * sizeof(float4);
   const unsigned fpix_blocks = unsigned((npix + 31) / 32), pix_blocks = unsigned((npix + 255) / 256);
-  const unsigned rot_tiles = unsigned(((W + kRotTile - 1) / kRotTile) * ((H + kRotTile - 1) / kRotTile));
-  const size_t rsm = p0.has_rows ? size_t(H) * sizeof(int2) : 0;
   const float fillv = o->rot_mask ? 0.f : std::numeric_limits<float>::quiet_NaN();
   float *const *out_g = reinterpret_cast<float *const *>(dp + off_o);
   for (uint32_t e0 = 0; e0 < total; e0 += vb) {
@@ -2880,7 +2835,6 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     fe.e0 = e0;
     fe.nbatch = nb;
     rg.nenergies = nb;
-    rg.rows = p0.has_rows ? reinterpret_cast<const int2 *>(dp + off_r) + size_t(e0) * H : nullptr;
     int slot = ctx.prof.begin(kEwaldFields, st);
     const unsigned fgrid = fpix_blocks * ((nb + kEwaldEnergies - 1) / kEwaldEnergies);
     if (sparse && nmat == 1)
@@ -2895,7 +2849,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
       k_ewald_fields<2, true><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
     ctx.prof.end(slot, st);
     slot = ctx.prof.begin(kRotateGram, st);
-    k_rotate_gram<2, packed_energies<2>()><<<dim3(rot_tiles, (nb + nep - 1) / nep), kRotTile * kRotTile, rsm, st>>>(rg);
+    launch_rotate<2, packed_energies<2>()>(rg, o->rot_mask != 0, st);
     ctx.prof.end(slot, st);
     slot = ctx.prof.begin(kWarp, st);
     k_warp_group<<<dim3(pix_blocks, nb), 256, 0, st>>>(sc.avg.as<float>(), out_g, E, e0, W, H, p0.detector_warp[0],

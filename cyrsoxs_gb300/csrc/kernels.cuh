@@ -1613,8 +1613,7 @@ struct EwaldParams {
   uint32_t zlo, nplanes;
   unsigned int *errors;   // incremented when a needed plane is not stored
   uint32_t nbasis;        // 1..3
-  float4 *gram;           // when set: Gram maps [NQ][gplane] (gram_at) instead of per-angle images
-  size_t gplane;          // float4 per Gram plane (gram_plane_size(ny, nx))
+  float4 *gram;           // when set: Gram maps [NQ][npix] instead of per-angle images
   uint32_t vol[3][3];     // vol[c][b]: volume holding component c of basis b
   uint32_t nangles;
   const float *coef;      // [nangles][nbasis]
@@ -1676,16 +1675,6 @@ __device__ __forceinline__ float gram_intensity(const float (&G)[NB * (NB + 1) /
 #pragma unroll
     for (int b2 = b; b2 < NB; ++b2) I += (b == b2 ? 1.f : 2.f) * e[b] * e[b2] * G[q++];
   return I;
-}
-
-// Gram planes hold the pixels of the rotation's source image (x < W, y < H,
-// row-major index y W + x) in 4 x 2 blocks, one 128-byte line per block: the
-// rotated bilinear taps of an 8 x 4 warp tile touch about 8 lines per load,
-// where row order touches about 14.
-__host__ __device__ inline size_t gram_plane_size(int W, int H) { return size_t((H + 1) / 2) * ((W + 3) / 4) * 8; }
-__device__ __forceinline__ uint32_t gram_at(int x, int y, int W) {
-  return ((uint32_t(y) >> 1) * ((uint32_t(W) + 3) >> 2) + (uint32_t(x) >> 2)) * 8 + ((uint32_t(y) & 1) << 2) +
-         (uint32_t(x) & 3);
 }
 
 // Gram maps: NB = 1 or 2 -> one float4 plane (G00 [G01 G11]), NB = 3 -> two
@@ -1777,11 +1766,10 @@ __global__ void __launch_bounds__(256) k_ewald_angles(EwaldParams p) {
   const bool isnan_px = !ewald_geometry(g, X, Y, zs[0], zs[1], w1, nplanes);
   const float nanv = __int_as_float(0x7fc00000);
   float *img = p.images + t;
-  // the rotation's image: width ny, so pixel t is (x, y) = (t % ny, t / ny)
-  float4 *gm = p.gram ? p.gram + gram_at(int(t % p.ny), int(t / p.ny), int(p.ny)) : nullptr;
+  float4 *gm = p.gram ? p.gram + t : nullptr;
   if (isnan_px) {
     if (gm) {
-      gram_store_nan<NB>(gm, p.gplane);
+      gram_store_nan<NB>(gm, npix);
       return;
     }
     for (uint32_t a = 0; a < p.nangles; ++a) img[size_t(a) * npix] = nanv;
@@ -1799,7 +1787,7 @@ __global__ void __launch_bounds__(256) k_ewald_angles(EwaldParams p) {
       if (zs[pl] < p.zlo || pz >= p.nplanes) {  // the host's plane range missed this pixel
         atomicAdd(p.errors, 1u);
         if (gm) {
-          gram_store_nan<NB>(gm, p.gplane);
+          gram_store_nan<NB>(gm, npix);
           return;
         }
         for (uint32_t a = 0; a < p.nangles; ++a) img[size_t(a) * npix] = nanv;
@@ -1820,7 +1808,7 @@ __global__ void __launch_bounds__(256) k_ewald_angles(EwaldParams p) {
     gram_add<NB>(Q, d, P, nplanes == 2 ? (pl == 0 ? 1.f - w1 : w1) : 1.f, G);
   }
   if (gm) {
-    gram_store<NB>(gm, p.gplane, G);
+    gram_store<NB>(gm, npix, G);
     return;
   }
   for (uint32_t a = 0; a < p.nangles; ++a) img[size_t(a) * npix] = gram_intensity<NB>(G, p.coef + size_t(a) * NB);
@@ -1945,10 +1933,10 @@ __global__ void __launch_bounds__(256) k_rotate_average(RotateParams p) {
   p.avg[size_t(blockIdx.y) * npix + t] = angle_mean(sum, count, p.nangles, p.rot_mask);
 }
 
-// Gram records: the Gram matrices of NEP energies of one pixel, energy s at
-// float s * NG, padded to whole float4s and stored as RQ planes of float4
-// ([group][RQ][plane], pixels placed by gram_at), so each of a warp's loads
-// reads whole 16-byte pixels of one plane.  NEP = 1 is the per-energy layout (GramLayout); the
+// Gram records: the Gram matrices of NEP energies of one pixel, entry g of
+// energy s at float g * NEP + s, padded to whole float4s and stored as RQ planes of float4
+// ([group][RQ][npix]), so each of a warp's loads reads whole 16-byte pixels of
+// one plane.  NEP = 1 is the per-energy layout (GramLayout); the
 // field-spectrum path packs 12 floats per record (4 energies at NB = 2, 2 at
 // NB = 3), so no load fetches padding.
 template <int NB, int NEP>
@@ -1962,123 +1950,297 @@ __host__ __device__ constexpr int packed_energies() {
   return 12 / (NB * (NB + 1) / 2);
 }
 
-// Rotation and angle average from Gram maps (LAB frame): per angle a the
-// corners' Gram matrices are blended as NPP blends intensities, then
-// I(a) = sum_{b,b'} E_b(a) E_b'(a) G_bb' (the blend is linear, so this equals
-// blending the per-angle intensities).  One thread forms one destination
-// pixel for the NEP energies of its record group, so the tap arithmetic and
-// each corner load serve all of them.  A NaN at any corner makes the blend
-// NaN, so a tap with a corner outside its row's possibly-valid column range
-// (the union over the group's energies of rows[e][y] = [x, y], conservative:
-// every pixel outside is NaN) is a NaN sample without a load.
+// Rotation and angle average from Gram maps (LAB frame).  Per angle a block
+// forms the intensities I(a) = sum_{b,b'} E_b(a) E_b'(a) G_bb' of the source
+// pixels that its destination tile samples, for the NEP energies of the record
+// group, into shared memory, and each destination pixel blends its four corners
+// there and adds to its angle sum.
+//
+// What bounds it: the load/store pipe and issue, about evenly.  A Gram entry is
+// read once per tile and angle, in rows (3 loads of 16 bytes a source pixel,
+// 1.2 source pixels a destination pixel), where blending the Gram matrices at
+// every destination pixel took 12 rotated loads and three times the blend
+// arithmetic (256 x 512 x 512, 50 energies x 36 angles: 1.67 -> 1.04 ms; 1024 x
+// 1024, 20 x 36: 2.63 -> 1.55 ms).  Blends and sums run on packed FP32 pairs of
+// energies.  Four blocks per SM, although 32 x 32 tiles then spill some sums:
+// 1.13 ms with three or five.  The shared rows are a multiple of 8 plus 4 pixels apart and the
+// lanes of a quarter-warp take 4 x 2 pixels, which over all rotations costs the
+// fewest bank conflicts (6.9 wavefronts per load; rows of 8: 8.1).
+//
+// The coordinates, the pixels written and the corners are NPP's (warp_tap).
 struct RotateGramParams {
-  const float4 *gram;       // [group = blockIdx.y][RQ][plane] (gram_at)
-  size_t plane;             // float4 per plane (gram_plane_size(W, H))
-  const WarpCoef *coef;     // [nangles]
+  const float4 *gram;       // [group = blockIdx.y][RQ][npix], row-major W x H
+  const WarpCoef *coef;     // [nangles], rotations
   const float *ecoef;       // [nangles][NB]
-  const int2 *rows;         // [energy][H] from the launch's first energy, or null: no bound known
   int W, H;
   uint32_t nangles;
   uint32_t nenergies;       // energies of this launch (the last group may be partial)
-  uint32_t rot_mask;
-  float *avg;               // [energy][P]
+  float *avg;               // [energy][npix]
 };
 
-// Blocks own 16 x 16 destination tiles (a warp: 8 x 4), so the rotated
-// source taps of a warp stay within a few cache lines.
-constexpr int kRotTile = 16;
+constexpr int kRotThreads = 256;
 
+// A tile's source pixels: the rotated tile spans at most (TILE - 1)(|cos| + |sin|) pixels each way,
+// a pixel of margin below, two above.
+template <int TILE>
+struct RotBox {
+  static constexpr int SIDE = TILE == 32 ? 48 : 26;
+  static constexpr int PITCH = TILE == 32 ? 52 : 28;
+  WarpCoef c;
+  float fx0, fx1, fy0, fy1;  // the tile
+  int bx, by, bw, bh;        // its source box (the map is affine: the extremes lie at the tile's corners)
+  __device__ __forceinline__ RotBox(const WarpCoef &coef, int X0, int Y0, int W, int H)
+      : c(coef), fx0(float(X0)), fx1(float(X0 + TILE - 1)), fy0(float(Y0)), fy1(float(Y0 + TILE - 1)) {
+    const float xl = c.a02 + fminf(c.a00 * fx0, c.a00 * fx1) + fminf(c.a01 * fy0, c.a01 * fy1);
+    const float xh = c.a02 + fmaxf(c.a00 * fx0, c.a00 * fx1) + fmaxf(c.a01 * fy0, c.a01 * fy1);
+    const float yl = c.a12 + fminf(c.a10 * fx0, c.a10 * fx1) + fminf(c.a11 * fy0, c.a11 * fy1);
+    const float yh = c.a12 + fmaxf(c.a10 * fx0, c.a10 * fx1) + fmaxf(c.a11 * fy0, c.a11 * fy1);
+    bx = max(0, int(floorf(xl)) - 1), by = max(0, int(floorf(yl)) - 1);
+    bw = min(SIDE, min(W - 1, int(floorf(xh)) + 2) - bx + 1);
+    bh = min(SIDE, min(H - 1, int(floorf(yh)) + 2) - by + 1);
+  }
+};
+
+// Margin around the destination tile, in pixels, within which a source pixel can be a corner of one of its samples
+// (a corner lies less than sqrt(2) from the sample point).
+constexpr float kRotMargin = 1.6f;
+
+// Angle sums of one destination pixel for the NEP energies of a record, in float-float arithmetic (AngleSum) on packed
+// pairs of energies.
+template <int NEP, bool MASK>
+struct RotSum {
+  static constexpr int NP = NEP / 2, NP1 = NP > 0 ? NP : 1;
+  float2 hi[NP1], lo[NP1];
+  uint32_t count[NP1];  // MASK: samples that are numbers, 16 bits an energy
+  __device__ __forceinline__ RotSum() {
+#pragma unroll
+    for (int e = 0; e < NP1; ++e) hi[e] = lo[e] = make_float2(0.f, 0.f), count[e] = 0;
+  }
+  // NPP's bilinear blend of the corners' intensities (warp_blend), added
+  __device__ __forceinline__ void add(const WarpTap &tp, const float2 (&A)[NP1], const float2 (&B)[NP1],
+                                      const float2 (&C)[NP1], const float2 (&D)[NP1]) {
+    const float gx = __fsub_rn(1.f, tp.fx), gy = __fsub_rn(1.f, tp.fy);
+    const float2 fx2 = make_float2(tp.fx, tp.fx), gx2 = make_float2(gx, gx);
+    const float2 fy2 = make_float2(tp.fy, tp.fy), gy2 = make_float2(gy, gy);
+#pragma unroll
+    for (int e = 0; e < NP1; ++e) {
+      const float2 t0 = pfma(gx2, A[e], pmul(fx2, B[e])), t1 = pfma(gx2, C[e], pmul(fx2, D[e]));
+      float2 v = pfma(gy2, t0, pmul(fy2, t1));
+      if (MASK) {
+        const bool nx = isnan(v.x), ny = isnan(v.y);
+        count[e] += (nx ? 0u : 1u) + (ny ? 0u : 0x10000u);
+        v = make_float2(nx ? 0.f : v.x, ny ? 0.f : v.y);
+      }
+      const float2 s = cadd(hi[e], v), bp = csub(s, hi[e]);
+      const float2 er = cadd(csub(hi[e], csub(s, bp)), csub(v, bp));
+      hi[e] = s;
+      lo[e] = cadd(lo[e], er);
+    }
+  }
+  // a sample outside the image: NaN, which the mask skips
+  __device__ __forceinline__ void outside() {
+    if (MASK) return;
+    const float n = __int_as_float(0x7fc00000);
+#pragma unroll
+    for (int e = 0; e < NP1; ++e) hi[e] = make_float2(n, n);
+  }
+  // some sum is still a number
+  __device__ __forceinline__ bool alive() const {
+    bool r = false;
+#pragma unroll
+    for (int e = 0; e < NP1; ++e) r = r || !isnan(hi[e].x) || (NEP > 1 && !isnan(hi[e].y));
+    return r;
+  }
+  __device__ __forceinline__ void store(float *o, size_t npix, int ne, uint32_t nangles) const {
+#pragma unroll
+    for (int e = 0; e < NEP; ++e) {
+      if (e >= ne) break;
+      AngleSum s;
+      s.hi = e % 2 ? hi[e / 2].y : hi[e / 2].x;
+      s.lo = e % 2 ? lo[e / 2].y : lo[e / 2].x;
+      o[size_t(e) * npix] =
+          angle_mean(s, e % 2 ? count[e / 2] >> 16 : count[e / 2] & 0xffffu, nangles, MASK ? 1u : 0u);
+    }
+  }
+};
+
+// Weights of the Gram entries at one angle: E_b E_b' (x2 off the diagonal).
+template <int NB>
+__device__ __forceinline__ void gram_weights(const float *__restrict__ ecoef, float (&wq)[NB * (NB + 1) / 2]) {
+  float e[NB];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) e[b] = __ldg(&ecoef[b]);
+  int q = 0;
+#pragma unroll
+  for (int b = 0; b < NB; ++b)
+#pragma unroll
+    for (int b2 = b; b2 < NB; ++b2) wq[q++] = (b == b2 ? 1.f : 2.f) * e[b] * e[b2];
+}
+
+// Intensities of a record's energies, in pairs (NEP = 1: in .x), from its float4s.
 template <int NB, int NEP>
-__global__ void __launch_bounds__(kRotTile * kRotTile, 3) k_rotate_gram(RotateGramParams p) {
-  constexpr int NG = GramRec<NB, NEP>::NG, RQ = GramRec<NB, NEP>::RQ;
-  constexpr int U = RQ == 1 ? 4 : RQ == 2 ? 2 : 1;  // angles whose loads are issued together
-  extern __shared__ int2 rows[];                    // [H] when p.rows is set
+__device__ __forceinline__ void gram_intensities(const float4 (&q)[GramRec<NB, NEP>::RQ],
+                                                 const float (&wq)[NB * (NB + 1) / 2], float2 (&I)[NEP > 1 ? NEP / 2 : 1]) {
+  constexpr int NG = NB * (NB + 1) / 2;
+  const float *f = reinterpret_cast<const float *>(q);
+  if constexpr (NEP == 1) {
+    float v = wq[0] * f[0];
+#pragma unroll
+    for (int k = 1; k < NG; ++k) v = fmaf(wq[k], f[k], v);
+    I[0] = make_float2(v, 0.f);
+  } else {
+#pragma unroll
+    for (int e = 0; e < NEP / 2; ++e) {
+      I[e] = pmul(make_float2(wq[0], wq[0]), make_float2(f[2 * e], f[2 * e + 1]));
+#pragma unroll
+      for (int k = 1; k < NG; ++k)
+        I[e] = pfma(make_float2(wq[k], wq[k]), make_float2(f[k * NEP + 2 * e], f[k * NEP + 2 * e + 1]), I[e]);
+    }
+  }
+}
+
+// Position of thread t's pixel in a 16-pixel-wide tile, warps of 8 x 4 and quarter-warps of 4 x 2 pixels.
+__device__ __forceinline__ int2 rot_pixel(int sub, int per_row, int lane) {
+  return make_int2((sub % per_row) * 8 + ((lane >> 3) & 1) * 4 + (lane & 3),
+                   (sub / per_row) * 4 + (lane >> 4) * 2 + ((lane >> 2) & 1));
+}
+
+template <int NB, int NEP, int TILE, bool MASK>
+__global__ void __launch_bounds__(kRotThreads, 4) k_rotate_gram(RotateGramParams p) {
+  constexpr int NG = GramRec<NB, NEP>::NG, RQ = GramRec<NB, NEP>::RQ, NT = kRotThreads;
+  using Box = RotBox<TILE>;
+  using Sum = RotSum<NEP, MASK>;
+  constexpr int PX = TILE * TILE / NT, SIDE = Box::SIDE, PITCH = Box::PITCH, NP1 = Sum::NP1;
+  __shared__ __align__(16) float sm[SIDE * PITCH * NEP];
   const uint32_t group = blockIdx.y;
   const int ne = int(min(uint32_t(NEP), p.nenergies - group * NEP));
-  if (p.rows)
-    for (int y = int(threadIdx.x); y < p.H; y += int(blockDim.x)) {
-      int2 r = p.rows[size_t(group) * NEP * p.H + y];
-      for (int s = 1; s < ne; ++s) {
-        const int2 q = p.rows[(size_t(group) * NEP + s) * p.H + y];
-        r.x = min(r.x, q.x), r.y = max(r.y, q.y);
-      }
-      rows[y] = r;
-    }
-  __syncthreads();
   const size_t npix = size_t(p.W) * p.H;
-  const int tiles_x = (p.W + kRotTile - 1) / kRotTile;
+  const int tiles_x = (p.W + TILE - 1) / TILE;
+  const int X0 = int(blockIdx.x % tiles_x) * TILE, Y0 = int(blockIdx.x / tiles_x) * TILE;
   const int warp = int(threadIdx.x >> 5), lane = int(threadIdx.x & 31);
-  const int xd = int(blockIdx.x % tiles_x) * kRotTile + (warp & 1) * 8 + (lane & 7);
-  const int yd = int(blockIdx.x / tiles_x) * kRotTile + (warp >> 1) * 4 + (lane >> 3);
-  if (xd >= p.W || yd >= p.H) return;
-  const float4 *gm = p.gram + size_t(group) * p.plane * RQ;
-  AngleSum sum[NEP];
-  uint32_t count[NEP];
+  // this thread's pixels: sub-tiles warp + i NT / 32
+  auto pixel = [&](int i) {
+    const int2 o = rot_pixel(warp + NT / 32 * i, TILE / 8, lane);
+    return make_int2(X0 + o.x, Y0 + o.y);
+  };
+  const float4 *gm = p.gram + size_t(group) * npix * RQ;
+  Sum sum[PX];
+  for (uint32_t a = 0; a < p.nangles; ++a) {
+    const Box bo(p.coef[a], X0, Y0, p.W, p.H);
+    float wq[NG];
+    gram_weights<NB>(p.ecoef + size_t(a) * NB, wq);
+    const uint32_t total = bo.bw > 0 && bo.bh > 0 ? uint32_t(bo.bw * bo.bh) : 0u;
+    const uint32_t magic = bo.bw > 1 ? 0xffffffffu / uint32_t(bo.bw) + 1u : 0u;
+    for (uint32_t t = threadIdx.x; t < total; t += NT) {
+      const uint32_t r = bo.bw > 1 ? __umulhi(t, magic) : t;
+      const int ix = int(t - r * uint32_t(bo.bw)), x = bo.bx + ix, y = bo.by + int(r);
+      // destination of this source pixel (the rotation's transpose): pixels no sample of the tile touches are skipped
+      const float dx = float(x) - bo.c.a02, dy = float(y) - bo.c.a12;
+      const float u = bo.c.a00 * dx + bo.c.a10 * dy, v = bo.c.a01 * dx + bo.c.a11 * dy;
+      if (u < bo.fx0 - kRotMargin || u > bo.fx1 + kRotMargin || v < bo.fy0 - kRotMargin || v > bo.fy1 + kRotMargin)
+        continue;
+      float4 q[RQ];
 #pragma unroll
-  for (int s = 0; s < NEP; ++s) count[s] = 0;
+      for (int k = 0; k < RQ; ++k) q[k] = __ldg(&gm[k * npix + size_t(y) * p.W + x]);
+      float2 I[NP1];
+      gram_intensities<NB, NEP>(q, wq, I);
+      float *s = sm + (int(r) * PITCH + ix) * NEP;
+      if constexpr (NEP == 4)
+        *reinterpret_cast<float4 *>(s) = make_float4(I[0].x, I[0].y, I[NP1 - 1].x, I[NP1 - 1].y);
+      else if constexpr (NEP == 2)
+        *reinterpret_cast<float2 *>(s) = I[0];
+      else
+        s[0] = I[0].x;
+    }
+    __syncthreads();
+    bool alive = false;
+#pragma unroll
+    for (int i = 0; i < PX; ++i) {
+      const int2 d = pixel(i);
+      WarpTap tp;
+      const bool here = d.x < p.W && d.y < p.H;
+      if (here && warp_tap(p.W, p.H, bo.c, d.x, d.y, tp)) {
+        const float *s00 = sm + ((tp.y0 - bo.by) * PITCH + (tp.x0 - bo.bx)) * NEP;
+        const int ox = (tp.x1 - tp.x0) * NEP, oy = (tp.y1 - tp.y0) * PITCH * NEP;
+        auto corner = [&](const float *s, float2 (&o)[NP1]) {
+          if constexpr (NEP == 4) {
+            const float4 t = *reinterpret_cast<const float4 *>(s);
+            o[0] = make_float2(t.x, t.y), o[NP1 - 1] = make_float2(t.z, t.w);
+          } else if constexpr (NEP == 2) {
+            o[0] = *reinterpret_cast<const float2 *>(s);
+          } else {
+            o[0] = make_float2(s[0], 0.f);
+          }
+        };
+        float2 A[NP1], B[NP1], C[NP1], D[NP1];
+        corner(s00, A), corner(s00 + ox, B), corner(s00 + oy, C), corner(s00 + oy + ox, D);
+        sum[i].add(tp, A, B, C, D);
+      } else {
+        sum[i].outside();
+      }
+      if (!MASK && here) alive = alive || sum[i].alive();
+    }
+    if (MASK)
+      __syncthreads();
+    else if (!__syncthreads_or(alive))
+      break;  // every mean of the tile is NaN already
+  }
+#pragma unroll
+  for (int i = 0; i < PX; ++i) {
+    const int2 d = pixel(i);
+    if (d.x < p.W && d.y < p.H)
+      sum[i].store(p.avg + size_t(group) * NEP * npix + size_t(d.y) * p.W + d.x, npix, ne, p.nangles);
+  }
+}
+
+// The same means with each corner read from the Gram planes and weighted where it is blended: no shared memory, no
+// barriers, several angles' loads in flight, for launches whose few blocks wait for load latency.  One pixel a thread.
+template <int NB, int NEP, bool MASK>
+__global__ void __launch_bounds__(kRotThreads, 2) k_rotate_direct(RotateGramParams p) {
+  constexpr int NG = GramRec<NB, NEP>::NG, RQ = GramRec<NB, NEP>::RQ;
+  constexpr int U = RQ == 1 ? 4 : RQ == 2 ? 2 : 1;  // angles whose loads are issued together
+  using Sum = RotSum<NEP, MASK>;
+  const uint32_t group = blockIdx.y;
+  const size_t npix = size_t(p.W) * p.H;
+  const int tiles_x = (p.W + 15) / 16;
+  const int2 o = rot_pixel(int(threadIdx.x >> 5), 2, int(threadIdx.x & 31));
+  const int xd = int(blockIdx.x % tiles_x) * 16 + o.x, yd = int(blockIdx.x / tiles_x) * 16 + o.y;
+  if (xd >= p.W || yd >= p.H) return;
+  const float4 *gm = p.gram + size_t(group) * npix * RQ;
+  Sum sum;
   for (uint32_t a0 = 0; a0 < p.nangles; a0 += U) {
     WarpTap tp[U];
     bool in[U];
     float4 cv[U][4][RQ];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const uint32_t a = a0 + u;
-      in[u] = a < p.nangles && warp_tap(p.W, p.H, p.coef[a < p.nangles ? a : 0], xd, yd, tp[u]);
-      if (in[u] && p.rows) {
-        const int2 r0 = rows[tp[u].y0], r1 = rows[tp[u].y1];
-        in[u] = tp[u].x0 >= r0.x && tp[u].x1 <= r0.y && tp[u].x0 >= r1.x && tp[u].x1 <= r1.y;
-      }
+      in[u] = a0 + u < p.nangles && warp_tap(p.W, p.H, p.coef[min(a0 + u, p.nangles - 1)], xd, yd, tp[u]);
       if (in[u]) {
-        const uint32_t idx[4] = {gram_at(tp[u].x0, tp[u].y0, p.W), gram_at(tp[u].x1, tp[u].y0, p.W),
-                                 gram_at(tp[u].x0, tp[u].y1, p.W), gram_at(tp[u].x1, tp[u].y1, p.W)};
+        const size_t i0 = size_t(tp[u].y0) * p.W, i1 = size_t(tp[u].y1) * p.W;
+        const size_t idx[4] = {i0 + tp[u].x0, i0 + tp[u].x1, i1 + tp[u].x0, i1 + tp[u].x1};
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
-          for (int q = 0; q < RQ; ++q) cv[u][c][q] = __ldg(&gm[q * p.plane + idx[c]]);
+          for (int k = 0; k < RQ; ++k) cv[u][c][k] = __ldg(&gm[k * npix + idx[c]]);
       }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const uint32_t a = a0 + u;
-      if (a >= p.nangles) break;
-      // per-angle weights of the Gram entries: E_b E_b' (x2 off the diagonal)
+      if (a0 + u >= p.nangles) break;
+      if (!in[u]) {
+        sum.outside();
+        continue;
+      }
       float wq[NG];
-      {
-        float e[NB];
+      gram_weights<NB>(p.ecoef + size_t(a0 + u) * NB, wq);
+      float2 I[4][Sum::NP1];
 #pragma unroll
-        for (int b = 0; b < NB; ++b) e[b] = __ldg(&p.ecoef[size_t(a) * NB + b]);
-        int q = 0;
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-          for (int b2 = b; b2 < NB; ++b2) wq[q++] = (b == b2 ? 1.f : 2.f) * e[b] * e[b2];
-      }
-#pragma unroll
-      for (int s = 0; s < NEP; ++s) {
-        if (s >= ne) break;
-        float v = __int_as_float(0x7fc00000);
-        if (in[u]) {
-          v = 0.f;
-#pragma unroll
-          for (int g = 0; g < NG; ++g) {
-            const int f = s * NG + g, q = f / 4, r = f % 4;
-            auto comp = [&](const float4 &x) { return r == 0 ? x.x : r == 1 ? x.y : r == 2 ? x.z : x.w; };
-            const float G = warp_blend(tp[u].fx, tp[u].fy, comp(cv[u][0][q]), comp(cv[u][1][q]),
-                                       comp(cv[u][2][q]), comp(cv[u][3][q]));
-            v += wq[g] * G;
-          }
-        }
-        if (p.rot_mask) {
-          if (isnan(v)) continue;
-          ++count[s];
-        }
-        sum[s].add(v);
-      }
+      for (int c = 0; c < 4; ++c) gram_intensities<NB, NEP>(cv[u][c], wq, I[c]);
+      sum.add(tp[u], I[0], I[1], I[2], I[3]);
     }
   }
-#pragma unroll
-  for (int s = 0; s < NEP; ++s)
-    if (s < ne) p.avg[(size_t(group) * NEP + s) * npix + size_t(yd) * p.W + xd] = angle_mean(sum[s], count[s], p.nangles, p.rot_mask);
+  sum.store(p.avg + size_t(group) * NEP * npix + size_t(yd) * p.W + xd, npix, int(min(uint32_t(NEP), p.nenergies - group * NEP)),
+            p.nangles);
 }
 
 // Detector warp of a request group's angle averages (one image per virtual
