@@ -1701,6 +1701,25 @@ void launch_rotate(const RotateGramParams &rg, bool mask, cudaStream_t st) {
   kern<<<dim3(tiles(large ? 32 : 16), groups), kRotThreads, 0, st>>>(rg);
 }
 
+// k_ewald_fields for a basis of nb vectors (0: MATERIAL frame) and nmat materials with sparse coefficients (0: any).
+void launch_ewald_fields(const FieldEwaldParams &fe, uint32_t nb, uint32_t nmat, unsigned grid, size_t smem,
+                         cudaStream_t st) {
+  auto run = [&](auto two, auto one) {
+    (fe.g.interp && !fe.g.twod ? two : one)<<<grid, kFieldEwaldThreads, smem, st>>>(fe);
+  };
+  auto basis = [&](auto nbc) {
+    constexpr int NB = decltype(nbc)::value;
+    if (nmat == 1) return run(k_ewald_fields<NB, 2, 1>, k_ewald_fields<NB, 1, 1>);
+    if (nmat == 2) return run(k_ewald_fields<NB, 2, 2>, k_ewald_fields<NB, 1, 2>);
+    if (nmat == 3) return run(k_ewald_fields<NB, 2, 3>, k_ewald_fields<NB, 1, 3>);
+    if (nmat == 4) return run(k_ewald_fields<NB, 2, 4>, k_ewald_fields<NB, 1, 4>);
+    run(k_ewald_fields<NB, 2>, k_ewald_fields<NB, 1>);
+  };
+  if (nb == 0) return basis(std::integral_constant<int, 0>{});
+  if (nb == 3) return basis(std::integral_constant<int, 3>{});
+  basis(std::integral_constant<int, 2>{});
+}
+
 // FIELDS strategy after the moments: field means, packed field spectra, then
 // every energy (in batches) and k from them.
 int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan &pl, const unsigned char *dp,
@@ -1788,7 +1807,7 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
   fe.nangles = pl.nang;
   fe.images = sc.images.as<float>();
   fe.gram = sc.images.as<float4>();
-  const size_t fsmem = size_t(kEwaldEnergies) * 6 * npk * sizeof(float4);
+  const size_t fsmem = size_t(kEwaldEnergies) * 6 * npk * sizeof(FieldCoef);
   const unsigned pix_blocks = unsigned((pl.npix + 255) / 256);
   const unsigned fpix_blocks = unsigned((pl.npix + 31) / 32);  // k_ewald_fields: 32 pixels per block
   const int W = int(pl.ny), H = int(pl.nx);  // the reference hands NPP width = Ny, height = Nx
@@ -1824,20 +1843,7 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
       slot = ctx.prof.begin(kEwaldFields, st);
       const unsigned fgrid = fpix_blocks * ((nb + kEwaldEnergies - 1) / kEwaldEnergies);
       const bool sparse = pl.ewald_sparse && ctx.sparse_ewald;
-      if (pl.material_frame)
-        k_ewald_fields<0><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
-      else if (pl.nbasis == 2 && sparse && pl.nmat == 1)
-        k_ewald_fields<2, false, 1><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
-      else if (pl.nbasis == 2 && sparse && pl.nmat == 2)
-        k_ewald_fields<2, false, 2><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
-      else if (pl.nbasis == 2 && sparse && pl.nmat == 3)
-        k_ewald_fields<2, false, 3><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
-      else if (pl.nbasis == 2 && sparse && pl.nmat == 4)
-        k_ewald_fields<2, false, 4><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
-      else if (pl.nbasis == 2)
-        k_ewald_fields<2><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
-      else
-        k_ewald_fields<3><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
+      launch_ewald_fields(fe, pl.material_frame ? 0u : pl.nbasis, sparse ? pl.nmat : 0u, fgrid, fsmem, st);
       ctx.prof.end(slot, st);
       slot = ctx.prof.begin(pl.material_frame ? kRotate : kRotateGram, st);
       if (pl.material_frame)
@@ -2826,7 +2832,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   rg.W = W, rg.H = H;
   rg.nangles = p0.nang;
   rg.avg = sc.avg.as<float>();
-  const size_t fsmem = size_t(kEwaldEnergies) * 6 * npk * sizeof(float4);
+  const size_t fsmem = size_t(kEwaldEnergies) * 6 * npk * sizeof(FieldCoef);
   const unsigned fpix_blocks = unsigned((npix + 31) / 32), pix_blocks = unsigned((npix + 255) / 256);
   const float fillv = o->rot_mask ? 0.f : std::numeric_limits<float>::quiet_NaN();
   float *const *out_g = reinterpret_cast<float *const *>(dp + off_o);
@@ -2837,16 +2843,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     rg.nenergies = nb;
     int slot = ctx.prof.begin(kEwaldFields, st);
     const unsigned fgrid = fpix_blocks * ((nb + kEwaldEnergies - 1) / kEwaldEnergies);
-    if (sparse && nmat == 1)
-      k_ewald_fields<2, true, 1><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
-    else if (sparse && nmat == 2)
-      k_ewald_fields<2, true, 2><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
-    else if (sparse && nmat == 3)
-      k_ewald_fields<2, true, 3><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
-    else if (sparse && nmat == 4)
-      k_ewald_fields<2, true, 4><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
-    else
-      k_ewald_fields<2, true><<<fgrid, kFieldEwaldThreads, fsmem, st>>>(fe);
+    launch_ewald_fields(fe, 2, sparse ? nmat : 0u, fgrid, fsmem, st);
     ctx.prof.end(slot, st);
     slot = ctx.prof.begin(kRotateGram, st);
     launch_rotate<2, packed_energies<2>()>(rg, o->rot_mask != 0, st);

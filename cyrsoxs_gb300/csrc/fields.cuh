@@ -246,8 +246,8 @@ struct FieldEwaldParams {
   float *images;         // NB = 0: [batch][nangles][npix]
   float4 *gram;          // NB > 0: Gram records [batch / NEP][RQ][npix] (GramRec<NB, packed_energies<NB>()>)
   uint32_t nbatch;       // energies of this launch
-  // request group (k_ewald_fields<NB, true>): energy e belongs to request e / e_per_req, whose
-  // packed volumes start at zspec + request * npk * nvox (DC at zdc + request * npk)
+  // request group (0: none): energy e belongs to request e / e_per_req, whose packed
+  // volumes start at zspec + request * npk * nvox (DC at zdc + request * npk)
   uint32_t e_per_req;
 };
 
@@ -273,39 +273,54 @@ constexpr int kEwaldEnergies = 4;  // energies (warps) per block
 constexpr int kFieldEwaldThreads = 32 * kEwaldEnergies;
 constexpr int kFieldGather = 4;  // packed volumes whose loads are issued together
 
+// Coefficients of one (entry, volume) as the packed multiply-adds take them:
+//   N += (ax, ax) Z + (-ay, ay) swap(Z) + (bx, -bx) Z' + (by, by) swap(Z'),
+// Z = Z_j(k), Z' = Z_j(-k): alpha Z + beta conj Z'.
+struct FieldCoef {
+  float4 a, b;
+};
+
 // NB = 2 or 3: LAB frame, Gram maps over the E basis (p(a) = sum_b E_b(a) Nt e_b),
 // rotated and averaged by k_rotate_gram.  NB = 0: any frame, p(a) = M(a) Nt per
 // angle, per-angle images.  The energy is the fastest block index, so the
 // blocks gathering one pixel tile for neighbouring energies (nearly the same
 // Ewald sphere) run together and share the gathered sectors in L2.
+// NPL: Ewald planes per pixel, 2 for the linear interpolation in 3D, else 1
+// (the plane count is the same for every pixel that is a number).
 // MT > 0: the morphology has MT materials and its coefficients keep the
 // structural zeros (coef_used), so the volumes and entries are walked at
 // compile time and the zero terms are never formed; MT = 0: any material
 // count, every term formed.
-template <int NB, bool GROUP = false, int MT = 0>
-__global__ void __launch_bounds__(kFieldEwaldThreads) k_ewald_fields(FieldEwaldParams p) {
+// What bounds it: the gathers (issued kFieldGather volumes at a time) in 3D,
+// the multiply-adds with one plane.  A coefficient's four packed FP32
+// multiply-adds serve both components (eight scalar ones before).
+template <int NB, int NPL, int MT = 0>
+__global__ void __launch_bounds__(kFieldEwaldThreads, NPL == 1 ? 8 : NB == 2 ? 5 : 6) k_ewald_fields(FieldEwaldParams p) {
   // a block: 32 pixels x kEwaldEnergies neighbouring energies, one warp per
   // energy, so the warps of an SM gather nearly the same sectors (their Ewald
   // spheres almost coincide) and share them in L1
-  extern __shared__ float4 fcoef_all[];  // [kEwaldEnergies][6][npk]
+  extern __shared__ FieldCoef fcoef_all[];  // [kEwaldEnergies][6][npk]
   const uint32_t ngrp = (p.nbatch + kEwaldEnergies - 1) / kEwaldEnergies;
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t eb = (blockIdx.x % ngrp) * kEwaldEnergies + warp, e = p.e0 + eb;
   const uint32_t nx = p.g.nx, ny = p.g.ny, nz = p.g.nz;
   for (uint32_t i = threadIdx.x; i < kEwaldEnergies * 6 * p.npk; i += blockDim.x) {
     const uint32_t w = i / (6 * p.npk), eg = (blockIdx.x % ngrp) * kEwaldEnergies + w;
-    if (eg < p.nbatch) fcoef_all[i] = p.coef[size_t(p.e0 + eg) * 6 * p.npk + i % (6 * p.npk)];
+    if (eg < p.nbatch) {
+      const float4 c = p.coef[size_t(p.e0 + eg) * 6 * p.npk + i % (6 * p.npk)];
+      fcoef_all[i] = FieldCoef{make_float4(c.x, c.x, -c.y, c.y), make_float4(c.z, -c.z, c.w, c.w)};
+    }
   }
   __syncthreads();
   if (eb >= p.nbatch) return;
   constexpr uint32_t NPKC = MT > 0 ? num_packed(uint32_t(MT)) : 0u;
   const uint32_t npk = MT > 0 ? NPKC : p.npk;
-  const float4 *fcoef = fcoef_all + warp * 6 * npk;
+  const FieldCoef *fcoef = fcoef_all + warp * 6 * npk;
   const size_t npix = size_t(nx) * ny;
   const size_t t = size_t(blockIdx.x / ngrp) * 32 + (threadIdx.x & 31);
   if (t >= npix) return;
   const uint32_t Y = uint32_t(t / nx), X = uint32_t(t % nx);
-  if (GROUP) {  // a request group (e_per_req > 0): this energy's request's packed volumes and DC
+  if (p.e_per_req) {  // a request group: this energy's request's packed volumes and DC
     const uint32_t rq = e / p.e_per_req;
     p.zspec += size_t(rq) * p.npk * p.nvox;
     p.zdc += size_t(rq) * p.npk;
@@ -336,33 +351,32 @@ __global__ void __launch_bounds__(kFieldEwaldThreads) k_ewald_fields(FieldEwaldP
   const uint32_t ux = igor(X, nx), uy = igor(Y, ny);
   const uint32_t mx = ux ? nx - ux : 0u, my = uy ? ny - uy : 0u;
   const float d = g.kmag * g.kmag;
-  // Z_j(k) and Z_j(-k) at both planes: the loads of kFieldGather volumes of
-  // both planes are issued together, and each coefficient serves both planes
-  size_t i0[2], i1[2];
-  bool is_dc[2];
+  // Z_j(k) and Z_j(-k) at the planes: the loads of kFieldGather volumes of
+  // all planes are issued together, and each coefficient serves every plane
+  size_t i0[NPL], i1[NPL];
+  bool is_dc[NPL];
 #pragma unroll
-  for (int pl = 0; pl < 2; ++pl) {
-    const uint32_t uz = (g.twod || pl >= nplanes) ? 0u : igor(zs[pl], nz);
+  for (int pl = 0; pl < NPL; ++pl) {
+    const uint32_t uz = g.twod ? 0u : igor(zs[pl], nz);
     const uint32_t mz = uz ? nz - uz : 0u;
     is_dc[pl] = ux == 0 && uy == 0 && uz == 0;
     i0[pl] = size_t(ux) + size_t(uy) * nx + size_t(uz) * npix;
     i1[pl] = size_t(mx) + size_t(my) * nx + size_t(mz) * npix;
   }
-  const bool two = nplanes == 2;
-  float2 N[2][6];
+  float2 N[NPL][6];
 #pragma unroll
-  for (int pl = 0; pl < 2; ++pl)
+  for (int pl = 0; pl < NPL; ++pl)
 #pragma unroll
     for (int v = 0; v < 6; ++v) N[pl][v] = make_float2(0.f, 0.f);
   auto chunk = [&](uint32_t j0) {
-    float2 za[2][kFieldGather], zb[2][kFieldGather];
+    float2 za[NPL][kFieldGather], zb[NPL][kFieldGather];
 #pragma unroll
     for (int q = 0; q < kFieldGather; ++q) {
       const uint32_t j = j0 + q;
 #pragma unroll
-      for (int pl = 0; pl < 2; ++pl) {
+      for (int pl = 0; pl < NPL; ++pl) {
         za[pl][q] = zb[pl][q] = make_float2(0.f, 0.f);
-        if (j < npk && (pl == 0 || two)) {
+        if (j < npk) {
           if (is_dc[pl]) {
             za[pl][q] = zb[pl][q] = p.zdc[j];
           } else {
@@ -380,12 +394,14 @@ __global__ void __launch_bounds__(kFieldEwaldThreads) k_ewald_fields(FieldEwaldP
 #pragma unroll
       for (int v = 0; v < 6; ++v) {
         if (MT > 0 && !coef_used(uint32_t(MT), v, j)) continue;
-        const float4 c = fcoef[v * npk + j];
+        const FieldCoef c = fcoef[v * npk + j];
 #pragma unroll
-        for (int pl = 0; pl < 2; ++pl) {
-          const float2 a = za[pl][q], b = make_float2(zb[pl][q].x, -zb[pl][q].y);  // b = conj Z_j(-k)
-          N[pl][v].x += c.x * a.x - c.y * a.y + c.z * b.x - c.w * b.y;
-          N[pl][v].y += c.x * a.y + c.y * a.x + c.z * b.y + c.w * b.x;
+        for (int pl = 0; pl < NPL; ++pl) {
+          const float2 a = za[pl][q], b = zb[pl][q];
+          float2 n = pfma(make_float2(c.a.x, c.a.y), a, N[pl][v]);
+          n = pfma(make_float2(c.a.z, c.a.w), make_float2(a.y, a.x), n);
+          n = pfma(make_float2(c.b.x, c.b.y), b, n);
+          N[pl][v] = pfma(make_float2(c.b.z, c.b.w), make_float2(b.y, b.x), n);
         }
       }
     }
@@ -396,17 +412,18 @@ __global__ void __launch_bounds__(kFieldEwaldThreads) k_ewald_fields(FieldEwaldP
   } else {
     for (uint32_t j0 = 0; j0 < npk; j0 += kFieldGather) chunk(j0);
   }
-  float Q[2][3];
+  float Q[NPL][3];
 #pragma unroll
-  for (int pl = 0; pl < 2; ++pl) {
+  for (int pl = 0; pl < NPL; ++pl) {
     Q[pl][0] = g.kx + p.qx[X];
     Q[pl][1] = g.ky + p.qy[Y];
-    Q[pl][2] = g.kz + ((g.twod || pl >= nplanes) ? 0.f : p.qz[zs[pl]]);
+    Q[pl][2] = g.kz + (g.twod ? 0.f : p.qz[zs[pl]]);
   }
   if constexpr (NB > 0) {
     constexpr int NG = NB * (NB + 1) / 2;
     float G[NG] = {};
-    for (int pl = 0; pl < nplanes; ++pl) {
+#pragma unroll
+    for (int pl = 0; pl < NPL; ++pl) {
       // symmetric entry (c, b) of Nt: volumes xx xy xz yy yz zz
       float2 P[3][NB];
 #pragma unroll
@@ -415,7 +432,7 @@ __global__ void __launch_bounds__(kFieldEwaldThreads) k_ewald_fields(FieldEwaldP
         P[1][b] = N[pl][b == 0 ? 1 : b == 1 ? 3 : 4];
         P[2][b] = N[pl][b == 0 ? 2 : b == 1 ? 4 : 5];
       }
-      gram_add<NB>(Q[pl], d, P, two ? (pl == 0 ? 1.f - w1 : w1) : 1.f, G);
+      gram_add<NB>(Q[pl], d, P, NPL == 2 ? (pl == 0 ? 1.f - w1 : w1) : 1.f, G);
     }
 #pragma unroll
     for (int q = 0; q < NG; ++q) gput(q, G[q]);
@@ -423,8 +440,9 @@ __global__ void __launch_bounds__(kFieldEwaldThreads) k_ewald_fields(FieldEwaldP
     const float w0 = 1.f - w1;
     for (uint32_t a = 0; a < p.nangles; ++a) {
       const float *M = p.mat + size_t(a) * 18;
-      float I[2];
-      for (int pl = 0; pl < nplanes; ++pl) {
+      float I[NPL];
+#pragma unroll
+      for (int pl = 0; pl < NPL; ++pl) {
         float2 pc[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -435,7 +453,7 @@ __global__ void __launch_bounds__(kFieldEwaldThreads) k_ewald_fields(FieldEwaldP
         }
         I[pl] = intensity(Q[pl][0], Q[pl][1], Q[pl][2], d, pc[0], pc[1], pc[2]);
       }
-      img[size_t(a) * npix] = two ? w0 * I[0] + w1 * I[1] : I[0];
+      img[size_t(a) * npix] = NPL == 2 ? w0 * I[0] + w1 * I[NPL - 1] : I[0];
     }
   }
 }
