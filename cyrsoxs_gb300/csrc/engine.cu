@@ -16,7 +16,7 @@
 //   k_build -> 3D FFT -> k_dc -> per k: k_ewald_angles ->
 //   k_rotate_gram -> k_warp_out (detector) -> projection[e][k]
 //
-// FIELDS strategy (fields.cuh): the spectra of the 7 M + 1 energy independent
+// FIELDS strategy (fields.cuh): the spectra of the 7 M energy independent
 // morphology fields are formed once per request; every energy and angle is
 // combined from them inside the Ewald kernel, batched over energies:
 //
@@ -488,6 +488,33 @@ int get_context(DeviceContext **out) {
 // GB300 for each.
 constexpr uint32_t kColsTxY = 8, kColsTxZ = 16;
 
+// k_build_fields / k_build_fields_rows for a morphology type and material count (compile-time up to 4).
+template <class F>
+int with_materials(bool euler, uint32_t nmat, F &&f) {
+  auto morph = [&](auto mc) -> int {
+    switch (nmat) {
+      case 1: return f(mc, std::integral_constant<int, 1>{});
+      case 2: return f(mc, std::integral_constant<int, 2>{});
+      case 3: return f(mc, std::integral_constant<int, 3>{});
+      case 4: return f(mc, std::integral_constant<int, 4>{});
+      default: return f(mc, std::integral_constant<int, 0>{});
+    }
+  };
+  return euler ? morph(std::integral_constant<int, 0>{}) : morph(std::integral_constant<int, 1>{});
+}
+
+// f(kernel) for k_build_fields_rows with this row length (128, 256, 512 or 1024).
+template <class F>
+int with_rows_kernel(bool euler, uint32_t nmat, uint32_t nx, F &&f) {
+  return with_materials(euler, nmat, [&](auto mc, auto tc) -> int {
+    constexpr int M = decltype(mc)::value, T = decltype(tc)::value;
+    return nx == 128   ? f(k_build_fields_rows<M, 4, T>)
+           : nx == 256 ? f(k_build_fields_rows<M, 8, T>)
+           : nx == 512 ? f(k_build_fields_rows<M, 16, T>)
+                       : f(k_build_fields_rows<M, 32, T>);
+  });
+}
+
 int setup_attrs(DeviceContext &ctx) {
   std::lock_guard<std::mutex> lk(ctx.tables_mu);
   if (ctx.attrs_done) return CYR_OK;
@@ -528,11 +555,13 @@ int setup_attrs(DeviceContext &ctx) {
 #undef CYR_WS_ATTR
   CYR_CUDA(cudaFuncSetAttribute(k_fft_cols_tma64<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 int(cols_tma64_smem(1024))));
-#define CYR_ROWS_ATTR(M, V) \
-  CYR_CUDA(cudaFuncSetAttribute(k_build_fields_rows<M, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CYR_ROWS_ATTR(0, 4) CYR_ROWS_ATTR(0, 8) CYR_ROWS_ATTR(0, 16) CYR_ROWS_ATTR(0, 32)
-  CYR_ROWS_ATTR(1, 4) CYR_ROWS_ATTR(1, 8) CYR_ROWS_ATTR(1, 16) CYR_ROWS_ATTR(1, 32)
-#undef CYR_ROWS_ATTR
+  for (bool euler : {true, false})
+    for (uint32_t nmat = 0; nmat <= 4; ++nmat)
+      for (uint32_t nx : {128u, 256u, 512u, 1024u})
+        CYR_TRY(with_rows_kernel(euler, nmat, nx, [&](auto kern) -> int {
+          CYR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+          return CYR_OK;
+        }));
   {
     cudaDriverEntryPointQueryResult q{};
     void *fn = nullptr;
@@ -1017,9 +1046,10 @@ struct Plan {
   // FIELDS strategy
   bool fields = false;
   uint32_t npk = 0;                     // packed field volumes
+  uint32_t first_mat = 0;               // the material whose fields come first (fields.cuh)
   uint32_t ebatch = 1;                  // energies per Ewald / rotation launch
   bool ewald_sparse = false;            // the combination coefficients keep their structural zeros
-  size_t off_fcoef = 0, off_kmag = 0, off_mat = 0, off_kvec = 0;
+  size_t off_fcoef = 0, off_kmag = 0, off_mat = 0, off_kvec = 0, off_first = 0;
   uint32_t mom_zstep = 1, mom_ystep = 1;  // z planes and rows between the moment samples
 };
 
@@ -1346,24 +1376,35 @@ int make_plan(const cyr_options *o, const float *optical, Plan &pl) {
   pl.mom_ystep = std::max<uint32_t>(1, std::min<uint32_t>(pl.ny / 16, uint32_t(pl.npix * std::min(pl.nz, 16u) >> 18)));
   if (pl.fields) {
     // coef[e][v][j] = (alpha, beta): Nt_v(k) = sum_j alpha Z_j(k) + beta conj Z_j(-k), where
-    // Z_j = F_2j + i F_2j+1 and field g = 7 m + f (f: u_x^2 u_y^2 u_z^2 u_xu_y u_xu_z u_yu_z phi_ui), T last
+    // Z_j = F_2j + i F_2j+1 and field g = 7 m + f of the m-th material walked (f: u_x^2 u_y^2 u_z^2 u_xu_y u_xu_z u_yu_z phi_ui), T in the place of
+    // the last phi_ui
     const uint32_t nf = num_fields(pl.nmat), npk = pl.npk;
     std::vector<float4> fc(size_t(pl.ne) * 6 * npk);
     std::vector<std::complex<double>> c(size_t(6) * 2 * npk);
+    // the material walked last gives the common part R = C: the one that leaves the smallest coefficients
+    double least = 0.0;
+    for (uint32_t l = 0; l < pl.nmat; ++l) {
+      double rest = 0.0;
+      for (uint32_t e = 0; e < pl.ne; ++e)
+        for (uint32_t m = 0; m < pl.nmat; ++m) {
+          const size_t em = size_t(e) * pl.nmat + m;
+          const std::complex<double> R = cC[size_t(e) * pl.nmat + l];
+          rest += std::norm(cB[em] - R) + std::norm(cC[em] - R);
+        }
+      if (l == 0 || rest < least) least = rest, pl.first_mat = (l + 1) % pl.nmat;
+    }
     for (uint32_t e = 0; e < pl.ne; ++e) {
       std::fill(c.begin(), c.end(), std::complex<double>(0.0, 0.0));
       auto at = [&](int v, uint32_t g) -> std::complex<double> & { return c[size_t(v) * 2 * npk + g]; };
-      std::complex<double> R(0.0, 0.0);  // common part of the diagonal coefficients
-      for (uint32_t m = 0; m < pl.nmat; ++m) R += cB[size_t(e) * pl.nmat + m] + cC[size_t(e) * pl.nmat + m];
-      R /= double(2 * pl.nmat);
+      const std::complex<double> R = cC[size_t(e) * pl.nmat + (pl.first_mat + pl.nmat - 1) % pl.nmat];  // common part of the diagonal coefficients
       for (uint32_t m = 0; m < pl.nmat; ++m) {
-        const size_t em = size_t(e) * pl.nmat + m;
+        const size_t em = size_t(e) * pl.nmat + (pl.first_mat + m) % pl.nmat;
         const uint32_t g = kFieldsPerMaterial * m;
         const std::complex<double> B = cB[em] - R, C = cC[em] - R, DB = cD[em] + cB[em] - R;
         const int diag[3] = {0, 3, 5};  // xx yy zz
         for (int i = 0; i < 3; ++i) {
           for (int f = 0; f < 3; ++f) at(diag[i], g + f) = f == i ? DB : B;
-          at(diag[i], g + 6) = C;
+          if (m + 1 < pl.nmat) at(diag[i], g + 6) = C;
         }
         at(1, g + 3) = cD[em];  // xy
         at(2, g + 4) = cD[em];  // xz
@@ -1389,6 +1430,7 @@ int make_plan(const cyr_options *o, const float *optical, Plan &pl) {
             pl.ewald_sparse = false;
         }
     pl.off_fcoef = arena_put(pl.arena, fc.data(), fc.size());
+    pl.off_first = arena_put(pl.arena, &pl.first_mat, 1);
     std::vector<float> km(pl.ne);
     for (uint32_t e = 0; e < pl.ne; ++e) {
       const float wavelength = static_cast<float>(1239.84197 / o->energies[e]);  // src/cudaMain.cu:607-608
@@ -1550,28 +1592,23 @@ int build_fields_x(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const 
     const size_t smem = fields_rows_smem(pl.nx, npk, pl.nmat);
     const uint32_t rows = (z1 - z0) * pl.ny;
     int per_sm = 1;
-    auto launch = [&](auto kern) -> int {
+    const int slot = ctx.prof.begin(kBuildFieldsRows, st);
+    CYR_TRY(with_rows_kernel(o->morphology_type == 0, pl.nmat, pl.nx, [&](auto kern) -> int {
       CYR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
       const unsigned grid = unsigned(std::min<size_t>(rows, size_t(std::max(1, per_sm)) * sms));
       kern<<<grid, 256, smem, st>>>(fp, twx, npk);
       return CYR_OK;
-    };
-    const int slot = ctx.prof.begin(kBuildFieldsRows, st);
-    const bool euler = o->morphology_type == 0;
-    if (pl.nx == 128) CYR_TRY(launch(euler ? k_build_fields_rows<0, 4> : k_build_fields_rows<1, 4>));
-    if (pl.nx == 256) CYR_TRY(launch(euler ? k_build_fields_rows<0, 8> : k_build_fields_rows<1, 8>));
-    if (pl.nx == 512) CYR_TRY(launch(euler ? k_build_fields_rows<0, 16> : k_build_fields_rows<1, 16>));
-    if (pl.nx == 1024) CYR_TRY(launch(euler ? k_build_fields_rows<0, 32> : k_build_fields_rows<1, 32>));
+    }));
     ctx.prof.end(slot, st);
     CYR_CUDA(cudaGetLastError());
     return CYR_OK;
   }
   const uint32_t blocks = uint32_t(std::min<size_t>((fp.i1 - fp.i0 + 255) / 256, size_t(sms) * 8));
   const int slot = ctx.prof.begin(kBuildFields, st);
-  if (o->morphology_type == 0)
-    k_build_fields<0><<<blocks, 256, 0, st>>>(fp);
-  else
-    k_build_fields<1><<<blocks, 256, 0, st>>>(fp);
+  CYR_TRY(with_materials(o->morphology_type == 0, pl.nmat, [&](auto mc, auto tc) -> int {
+    k_build_fields<decltype(mc)::value, decltype(tc)::value><<<blocks, 256, 0, st>>>(fp);
+    return CYR_OK;
+  }));
   ctx.prof.end(slot, st);
   CYR_CUDA(cudaGetLastError());
   return fft_axes(ctx, spec + fp.i0, pl.nx, pl.ny, z1 - z0, npk, st, 0, 0, pl.nvox);
@@ -1733,6 +1770,7 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
   FieldParams fp{};
   fp.vox = d_vox;
   fp.nx = pl.nx, fp.ny = pl.ny, fp.nz = pl.nz, fp.nmat = pl.nmat;
+  fp.first_g = reinterpret_cast<const uint32_t *>(dp + pl.off_first);
   fp.nvox = pl.nvox;
   fp.mom = sc.moments();  // each block forms the field means from the moments
   fp.nsamp = nsamp;
@@ -2677,6 +2715,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   std::vector<float> km;
   std::vector<const float4 *> vp;
   std::vector<float *> op;
+  std::vector<uint32_t> first;
   bool sparse = nmat <= 4 && ctx.sparse_ewald;  // every member's coefficients keep the structural zeros
   for (const auto &r : g) {
     const Plan &pl = r->plan;
@@ -2687,6 +2726,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     km.insert(km.end(), k, k + E);
     vp.push_back(r->d_vox);
     op.push_back(r->d_out);
+    first.push_back(pl.first_mat);
   }
   const size_t off_c = arena_put(arena, fc.data(), fc.size());
   const size_t off_k = arena_put(arena, km.data(), km.size());
@@ -2694,6 +2734,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   const size_t off_kv = arena_put(arena, kv0, 3);
   const size_t off_v = arena_put(arena, vp.data(), vp.size());
   const size_t off_o = arena_put(arena, op.data(), op.size());
+  const size_t off_f = arena_put(arena, first.data(), first.size());
   arena.resize((arena.size() + 255) & ~size_t(255));
   CYR_TRY(ensure_host_arena(sl, arena.size()));
   std::memcpy(sl.host_arena, arena.data(), arena.size());
@@ -2741,6 +2782,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   // field build + x pass (blockIdx.y = request), then y and z over all G npk volumes
   FieldParams fp{};
   fp.vox_g = vox_g;
+  fp.first_g = reinterpret_cast<const uint32_t *>(dp + off_f);
   fp.nx = p0.nx, fp.ny = p0.ny, fp.nz = p0.nz, fp.nmat = nmat;
   fp.nvox = nvox;
   fp.mom = sc.moments();
@@ -2766,28 +2808,23 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     const size_t smem = fields_rows_smem(p0.nx, npk, nmat);
     const uint32_t rws = p0.nz * p0.ny;
     int per_sm = 1;
-    auto launch = [&](auto kern) -> int {
+    const int slot = ctx.prof.begin(kBuildFieldsRows, st);
+    CYR_TRY(with_rows_kernel(o->morphology_type == 0, nmat, p0.nx, [&](auto kern) -> int {
       CYR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
       const size_t want = (size_t(std::max(1, per_sm)) * sms + G - 1) / G;
       kern<<<dim3(unsigned(std::min<size_t>(rws, want)), G), 256, smem, st>>>(fp, twx, npk);
       return CYR_OK;
-    };
-    const int slot = ctx.prof.begin(kBuildFieldsRows, st);
-    const bool euler = o->morphology_type == 0;
-    if (p0.nx == 128) CYR_TRY(launch(euler ? k_build_fields_rows<0, 4> : k_build_fields_rows<1, 4>));
-    if (p0.nx == 256) CYR_TRY(launch(euler ? k_build_fields_rows<0, 8> : k_build_fields_rows<1, 8>));
-    if (p0.nx == 512) CYR_TRY(launch(euler ? k_build_fields_rows<0, 16> : k_build_fields_rows<1, 16>));
-    if (p0.nx == 1024) CYR_TRY(launch(euler ? k_build_fields_rows<0, 32> : k_build_fields_rows<1, 32>));
+    }));
     ctx.prof.end(slot, st);
     CYR_CUDA(cudaGetLastError());
   } else {
     const uint32_t blocks =
         uint32_t(std::max<size_t>(1, std::min<size_t>((nvox + 255) / 256, (size_t(sms) * 8 + G - 1) / G)));
     const int slot = ctx.prof.begin(kBuildFields, st);
-    if (o->morphology_type == 0)
-      k_build_fields<0><<<dim3(blocks, G), 256, 0, st>>>(fp);
-    else
-      k_build_fields<1><<<dim3(blocks, G), 256, 0, st>>>(fp);
+    CYR_TRY(with_materials(o->morphology_type == 0, nmat, [&](auto mc, auto tc) -> int {
+      k_build_fields<decltype(mc)::value, decltype(tc)::value><<<dim3(blocks, G), 256, 0, st>>>(fp);
+      return CYR_OK;
+    }));
     ctx.prof.end(slot, st);
     CYR_CUDA(cudaGetLastError());
     CYR_TRY(fft_axes(ctx, spec, p0.nx, p0.ny, p0.nz, npk * G, st, 0, 0, 0, ft.form));

@@ -9,12 +9,18 @@
 // seven real fields u_x^2, u_y^2, u_z^2, u_x u_y, u_x u_z, u_y u_z, phi_ui,
 // with energy dependent complex coefficients.  The FFT is linear, hence
 //   FFT(Nt_v) = sum_g c_vg(E) FFT(F_g),
-// exactly.  The diagonal coefficients share a common part R(E) (the base
-// optical constants are the same for every material), which would cancel in
-// the sum and amplify the FP32 rounding of the field spectra; it is taken out
-// with one more field, T = sum_m (|u_m|^2 + phi_ui_m):
+// exactly.  The diagonal coefficients share a common part (the base optical
+// constants are alike for every material), which would cancel in the sum and
+// amplify the FP32 rounding of the field spectra; it is taken out with the
+// field T = sum_m (|u_m|^2 + phi_ui_m), constant where the volume fractions
+// sum to one:
 //   Nt_xx = sum_m [(D+B-R) u_x^2 + (B-R)(u_y^2 + u_z^2) + (C-R) phi_ui] + R T.
-// The 7 M + 1 real fields are packed in pairs into complex volumes
+// With R(E) = C of one material that material's phi_ui drops out, so T takes
+// its place and 7 M fields do (R as the mean of all B and C needs 7 M + 1: one
+// packed volume more for every even M).  The planner takes the material whose C
+// lies nearest to all B and C of the request; the materials are walked from the
+// one after it, so it comes last.
+// The 7 M real fields are packed in pairs into complex volumes
 // Z_j = F_2j + i F_2j+1 and transformed with the engine's complex 3D FFT; the
 // Ewald kernel unpacks them with
 //   F_2j(k) = (Z_j(k) + conj Z_j(-k)) / 2,  F_2j+1(k) = (Z_j(k) - conj Z_j(-k)) / 2i.
@@ -29,7 +35,8 @@ namespace cyr {
 
 constexpr int kFieldsPerMaterial = 7;
 
-__host__ __device__ constexpr uint32_t num_fields(uint32_t nmat) { return kFieldsPerMaterial * nmat + 1; }
+// field 7 m + f of the m-th material walked; the last one (phi_ui of the last material) is T
+__host__ __device__ constexpr uint32_t num_fields(uint32_t nmat) { return kFieldsPerMaterial * nmat; }
 __host__ __device__ constexpr uint32_t num_packed(uint32_t nmat) { return (num_fields(nmat) + 1) / 2; }
 
 constexpr uint32_t kMaxFields = num_fields(kMaxMaterials);
@@ -40,13 +47,17 @@ constexpr uint32_t kMaxPacked = num_packed(kMaxMaterials);
 // changes only bin 0, which is replaced, so the means need only be close (a
 // z-plane subsample suffices); they keep the FP32 rounding of the transform
 // proportional to the fluctuations.
-__device__ __forceinline__ void field_means(const double *__restrict__ mom, uint32_t nmat, size_t nsamp,
+__device__ __forceinline__ uint32_t walked_material(uint32_t m, uint32_t first, uint32_t nmat) {
+  return m + first < nmat ? m + first : m + first - nmat;
+}
+
+__device__ __forceinline__ void field_means(const double *__restrict__ mom, uint32_t first, uint32_t nmat, size_t nsamp,
                                             float *__restrict__ out) {
   const uint32_t nf = num_fields(nmat);
   for (uint32_t g = threadIdx.x; g < nf; g += blockDim.x) {
     double v = 0.0;
     if (g + 1 < nf) {
-      v = mom[(g / kFieldsPerMaterial) * kMoments + g % kFieldsPerMaterial];
+      v = mom[walked_material(g / kFieldsPerMaterial, first, nmat) * kMoments + g % kFieldsPerMaterial];
     } else {
       for (uint32_t m = 0; m < nmat; ++m) {
         const double *M = mom + m * kMoments;
@@ -64,6 +75,9 @@ struct FieldParams {
   const float4 *const *vox_g;
   size_t mom_stride, out_stride;
   uint32_t nx, ny, nz, nmat;
+  const uint32_t *first_g;  // [request] the material walked first: in the parameter arena, because it follows from the
+                            // optical constants, which a captured graph's replays change
+  uint32_t first;           // this request's (field_group)
   size_t nvox;
   const double *mom;     // [nmat][kMoments] moment sums over nsamp voxels
   size_t nsamp;
@@ -72,20 +86,70 @@ struct FieldParams {
   float2 *out;           // [num_packed][nvox]: field 2j in .x, field 2j+1 in .y
 };
 
-// Windowed, mean-free fields of every voxel, packed in pairs.
-// Selects request blockIdx.y of a request group.
+// Selects request blockIdx.y of a request group (0: the only one).
 __device__ __forceinline__ void field_group(FieldParams &p) {
+  p.first = __ldg(&p.first_g[blockIdx.y]);
   if (!p.vox_g) return;
   p.vox = p.vox_g[blockIdx.y];
   p.mom += size_t(blockIdx.y) * p.mom_stride;
   p.out += size_t(blockIdx.y) * p.out_stride;
 }
 
-template <int MORPH>
+// The packed fields of voxel i (window weight w), put(j, volume j's value) in order.  MT > 0: the material count is
+// known at compile time, so every field's place, mean and parity are too; MT = 0: any count, four materials at a time.
+template <int MORPH, int MT, class Put>
+__device__ __forceinline__ void voxel_fields(const FieldParams &p, size_t i, float w, const float *mean, Put &&put) {
+  float T = 0.f, pend = 0.f;
+  uint32_t g = 0;
+  // g is the same in every thread: the parity branches do not diverge
+  auto emit = [&](float v) {
+    v -= mean[g];
+    if (g & 1u)
+      put(g >> 1, make_float2(pend, v));
+    else
+      pend = v;
+    ++g;
+  };
+  auto material = [&](float4 sv, bool last) {
+    float sx, sy, sz, pa, pui;
+    director<MORPH>(sv, sx, sy, sz, pa, pui);
+    const float wa = w * pa;
+    const float f0 = wa * sx * sx, f1 = wa * sy * sy, f2 = wa * sz * sz, f6 = w * pui;
+    T += f0 + f1 + f2 + f6;
+    emit(f0);
+    emit(f1);
+    emit(f2);
+    emit(wa * sx * sy);
+    emit(wa * sx * sz);
+    emit(wa * sy * sz);
+    if (!last) emit(f6);
+  };
+  if constexpr (MT > 0) {
+    float4 sv[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) sv[m] = __ldg(&p.vox[walked_material(uint32_t(m), p.first, MT) * p.nvox + i]);
+#pragma unroll
+    for (int m = 0; m < MT; ++m) material(sv[m], m + 1 == MT);
+  } else {
+    for (uint32_t m0 = 0; m0 < p.nmat; m0 += 4) {
+      float4 sv[4];  // the loads of up to 4 materials are issued before any is used
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (m0 + u < p.nmat) sv[u] = __ldg(&p.vox[walked_material(m0 + u, p.first, p.nmat) * p.nvox + i]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (m0 + u < p.nmat) material(sv[u], m0 + u + 1 == p.nmat);
+    }
+  }
+  emit(T);
+  if (g & 1u) put(g >> 1, make_float2(pend, 0.f));
+}
+
+template <int MORPH, int MT>
 __global__ void __launch_bounds__(256) k_build_fields(FieldParams p) {
   __shared__ float mean[kMaxFields];  // volume mean of each windowed field
   field_group(p);
-  field_means(p.mom, p.nmat, p.nsamp, mean);
+  field_means(p.mom, p.first, p.nmat, p.nsamp, mean);
   __syncthreads();
   const size_t stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = p.i0 + size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < p.i1; i += stride) {
@@ -94,42 +158,8 @@ __global__ void __launch_bounds__(256) k_build_fields(FieldParams p) {
       const uint32_t x = uint32_t(i % p.nx), y = uint32_t((i / p.nx) % p.ny), z = uint32_t(i / (size_t(p.nx) * p.ny));
       w = p.hann_x[x] * p.hann_y[y] * p.hann_z[z];
     }
-    float T = 0.f, pend = 0.f;
-    uint32_t g = 0;
     float2 *o = p.out + i;
-    // g is the same in every thread: the parity branches do not diverge
-    auto emit = [&](float v) {
-      v -= mean[g];
-      if (g & 1u)
-        o[size_t(g >> 1) * p.nvox] = make_float2(pend, v);
-      else
-        pend = v;
-      ++g;
-    };
-    for (uint32_t m0 = 0; m0 < p.nmat; m0 += 4) {
-      float4 sv[4];  // the loads of up to 4 materials are issued before any is used
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (m0 + u < p.nmat) sv[u] = __ldg(&p.vox[(m0 + u) * p.nvox + i]);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (m0 + u >= p.nmat) break;
-        float sx, sy, sz, pa, pui;
-        director<MORPH>(sv[u], sx, sy, sz, pa, pui);
-        const float wa = w * pa;
-        const float f0 = wa * sx * sx, f1 = wa * sy * sy, f2 = wa * sz * sz, f6 = w * pui;
-        T += f0 + f1 + f2 + f6;
-        emit(f0);
-        emit(f1);
-        emit(f2);
-        emit(wa * sx * sy);
-        emit(wa * sx * sz);
-        emit(wa * sy * sz);
-        emit(f6);
-      }
-    }
-    emit(T);
-    if (g & 1u) o[size_t(g >> 1) * p.nvox] = make_float2(pend, 0.f);
+    voxel_fields<MORPH, MT>(p, i, w, mean, [&](uint32_t j, float2 v) { o[size_t(j) * p.nvox] = v; });
   }
 }
 
@@ -140,17 +170,22 @@ __global__ void __launch_bounds__(256) k_build_fields(FieldParams p) {
 // FFT with that line as its exchange buffer, and stores the transformed row.
 // The packed volumes leave the chip once, already x-transformed: the build's
 // write and the row pass's read-back of 8 npk bytes per voxel are gone.
-// Shared memory: (npk + 1) N float2 (lines and twiddles).  Three blocks per SM
+// Shared memory: (npk + 1) N float2 (lines and twiddles).  What bounds it:
+// issue (62% active) and the load and shared-memory latencies of 32% occupancy.
+// The material count at compile time took the field places, parities and index
+// products out of every voxel: 3.41 -> 2.76 ms on 256 x 512 x 512 with 4 materials (with 14
+// packed volumes for 15), 70 -> 58 us on 256 x 256 x 32 with 2.  Three blocks per SM
 // (80 registers) measured faster than two blocks that also stage the next
-// row's voxels in shared memory with cp.async.  (A hardware sine/cosine for
+// row's voxels in shared memory with cp.async; seven warps for 7 or 14 lines
+// were slower (2.90 ms).  (A hardware sine/cosine for
 // the Euler angles saved 0.17 ms of 3.6 on the 256 x 512 x 512 request but
 // doubled the full-size error against FP64, to 3.6e-5: not kept.)
 __host__ __device__ constexpr size_t fields_rows_smem(uint32_t n, uint32_t npk, uint32_t nmat) {
   return (void)nmat, size_t(npk + 1) * n * sizeof(float2);
 }
 
-template <int MORPH, int V>
-__global__ void __launch_bounds__(256, V <= 16 ? 3 : 1) k_build_fields_rows(FieldParams p, const float2 *__restrict__ tw_n,
+template <int MORPH, int V, int MT>
+__global__ void __launch_bounds__(256, V == 4 ? 5 : V == 8 ? 4 : V == 16 ? 3 : 1) k_build_fields_rows(FieldParams p, const float2 *__restrict__ tw_n,
                                                                             uint32_t npk) {
   constexpr uint32_t N = 32 * V;
   extern __shared__ float2 fsm[];
@@ -158,7 +193,7 @@ __global__ void __launch_bounds__(256, V <= 16 ? 3 : 1) k_build_fields_rows(Fiel
   float2 *lines = fsm + N;  // [npk][N]: element x of line j at lines[j N + swz(x)]
   __shared__ float mean[kMaxFields];
   field_group(p);
-  field_means(p.mom, p.nmat, p.nsamp, mean);
+  field_means(p.mom, p.first, p.nmat, p.nsamp, mean);
   warp_twiddles<V>(tws, tw_n);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const uint32_t nrows = uint32_t((p.i1 - p.i0) / N);
@@ -171,40 +206,7 @@ __global__ void __launch_bounds__(256, V <= 16 ? 3 : 1) k_build_fields_rows(Fiel
       const size_t i = rowbase + x;
       const float w = p.hann_x ? p.hann_x[x] * wyz : 1.f;
       float2 *o = lines + swz(x);
-      float T = 0.f, pend = 0.f;
-      uint32_t g = 0;
-      auto emit = [&](float v) {
-        v -= mean[g];
-        if (g & 1u)
-          o[(g >> 1) * N] = make_float2(pend, v);
-        else
-          pend = v;
-        ++g;
-      };
-      for (uint32_t m0 = 0; m0 < p.nmat; m0 += 4) {
-        float4 sv[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (m0 + u < p.nmat) sv[u] = __ldg(&p.vox[(m0 + u) * p.nvox + i]);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (m0 + u >= p.nmat) break;
-          float sx, sy, sz, pa, pui;
-          director<MORPH>(sv[u], sx, sy, sz, pa, pui);
-          const float wa = w * pa;
-          const float f0 = wa * sx * sx, f1 = wa * sy * sy, f2 = wa * sz * sz, f6 = w * pui;
-          T += f0 + f1 + f2 + f6;
-          emit(f0);
-          emit(f1);
-          emit(f2);
-          emit(wa * sx * sy);
-          emit(wa * sx * sz);
-          emit(wa * sy * sz);
-          emit(f6);
-        }
-      }
-      emit(T);
-      if (g & 1u) o[(g >> 1) * N] = make_float2(pend, 0.f);
+      voxel_fields<MORPH, MT>(p, i, w, mean, [&](uint32_t j, float2 v) { o[j * N] = v; });
     }
     __syncthreads();
     for (uint32_t j = warp; j < npk; j += nw) {
@@ -256,7 +258,7 @@ struct FieldEwaldParams {
 // diagonal, which also takes T), u_x u_y (xy), u_x u_z (xz) or u_y u_z (yz)
 // (include/uniaxial.h:94-151 in the contrast form above); coef[e][v][j] can
 // be non-zero only when field 2j or 2j+1 enters entry v.  With 4 materials
-// 34 of the 75 (entry, volume) pairs of the LAB frame's five entries are used.
+// 32 of the 70 (entry, volume) pairs of the LAB frame's five entries are used.
 __host__ __device__ constexpr bool field_enters(uint32_t nmat, int v, uint32_t g) {
   return g >= num_fields(nmat)        ? false                                    // T's zero partner
          : g + 1 == num_fields(nmat)  ? (v == 0 || v == 3 || v == 5)             // T
