@@ -441,6 +441,8 @@ struct DeviceContext {
     uint32_t *first = nullptr;
   };
   std::map<std::array<uint32_t, 3>, MixTables> mix;  // key: length, row form, bytes per real
+  int sms = 0;                                       // multiprocessors
+  std::map<std::pair<const void *, size_t>, int> occupancy;  // blocks per SM of a kernel at a shared-memory size
   struct Fp64Scratch {
     DeviceBuffer spec, images, avg, params, params64, vox, out;
   } f64;                                // the FP64 pipeline's buffers (plain entry points)
@@ -450,6 +452,7 @@ struct DeviceContext {
   // by every call (the calls hold `mu`)
   cudaStream_t main_stream = nullptr, copy_stream = nullptr;
   std::vector<cudaEvent_t> slab_events;
+  unsigned *host_errors = nullptr;  // pinned: the error count and the tile-copy word of the last cyr_cuda_main
   // TMA column passes: the driver's tensor-map encoder, and a word set when a
   // tile copy did not complete within the kernel's wait limit
   void *encode_tiled = nullptr;
@@ -470,8 +473,11 @@ int get_context(DeviceContext **out) {
   std::lock_guard<std::mutex> lk(g_ctx_mu);
   auto &slot = g_ctx[dev];
   if (!slot) {
+    int sms = 0;
+    CYR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     slot.reset(new DeviceContext);
     slot->device = dev;
+    slot->sms = sms;
     const char *env = std::getenv("CYRSOXS_GB300_AUTOTUNE");
     slot->autotune = !(env && std::strcmp(env, "0") == 0);
     env = std::getenv("CYRSOXS_GB300_ZMASK");
@@ -513,6 +519,21 @@ int with_rows_kernel(bool euler, uint32_t nmat, uint32_t nx, F &&f) {
            : nx == 512 ? f(k_build_fields_rows<M, 16, T>)
                        : f(k_build_fields_rows<M, 32, T>);
   });
+}
+
+// Resident blocks per SM of a kernel (a driver query of 1 to 2 us, made once per kernel and shared-memory size).
+template <class K>
+int blocks_per_sm(DeviceContext &ctx, K kern, int threads, size_t smem, int *out) {
+  std::lock_guard<std::mutex> lk(ctx.tables_mu);
+  const std::pair<const void *, size_t> key(reinterpret_cast<const void *>(kern), smem);
+  auto it = ctx.occupancy.find(key);
+  if (it == ctx.occupancy.end()) {
+    int n = 0;
+    CYR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem));
+    it = ctx.occupancy.emplace(key, n).first;
+  }
+  *out = it->second;
+  return CYR_OK;
 }
 
 int setup_attrs(DeviceContext &ctx) {
@@ -654,9 +675,9 @@ int warp_fft_pass_v(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, 
     tp.axis = uint32_t(axis);
     tp.tw = tw;
     tp.error = ctx.tma_error;
-    int sms = 0, per_sm = 0;
-    CYR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
-    CYR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fft_cols_tma64<32>, 9 * 32, cols_tma64_smem(N)));
+    const int sms = ctx.sms;
+    int per_sm = 0;
+    CYR_TRY(blocks_per_sm(ctx, k_fft_cols_tma64<32>, 9 * 32, cols_tma64_smem(N), &per_sm));
     const unsigned grid = unsigned(std::min<size_t>(tp.ntiles, size_t(std::max(1, per_sm)) * sms));
     k_fft_cols_tma64<32><<<grid, 9 * 32, cols_tma64_smem(N), st>>>(map, tp);
   } else if ((V == 4 || V == 8 || V == 16) && nx % kTmaCols == 0 && ctx.encode_tiled && ctx.tma_error &&
@@ -676,8 +697,8 @@ int warp_fft_pass_v(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, 
     tp.axis = uint32_t(axis);
     tp.tw = tw;
     tp.error = ctx.tma_error;
-    int sms = 0, per_sm = 0;
-    CYR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+    const int sms = ctx.sms;
+    int per_sm = 0;
     // 128-point lines: 32 columns in three stages (nx a multiple of 32) or 16 in two,
     // with a producer warp; 256-point lines: 32 columns with a producer warp in
     // three or two stages (nx a multiple of 32; 256-byte runs per line), else the
@@ -691,7 +712,7 @@ int warp_fft_pass_v(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, 
       // the masked form (z pass with a store mask) is its own instantiation, so
       // the unmasked passes keep the plain tile walk and its registers
       auto kern = tp.smask ? k_fft_cols_tma_ws<VV, HH, SS, true> : k_fft_cols_tma_ws<VV, HH, SS, false>;
-      CYR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (8 * HH + 1) * 32, smem));
+      CYR_TRY(blocks_per_sm(ctx, kern, (8 * HH + 1) * 32, smem, &per_sm));
       const unsigned grid = unsigned(std::min<size_t>(tp.ntiles, size_t(std::max(1, per_sm)) * sms));
       kern<<<grid, (8 * HH + 1) * 32, smem, st>>>(map, smap, tp);
       return CYR_OK;
@@ -714,7 +735,7 @@ int warp_fft_pass_v(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, 
         else
           CYR_TRY(launch_ws(I8{}, I2{}, I3{}));
       } else {
-        CYR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fft_cols_tma<8>, kTmaWarps * 32, cols_tma_smem(N)));
+        CYR_TRY(blocks_per_sm(ctx, k_fft_cols_tma<8>, kTmaWarps * 32, cols_tma_smem(N), &per_sm));
         const unsigned grid = unsigned(std::min<size_t>(tp.ntiles, size_t(std::max(1, per_sm)) * sms));
         k_fft_cols_tma<8><<<grid, kTmaWarps * 32, cols_tma_smem(N), st>>>(map, tp);
       }
@@ -1528,32 +1549,22 @@ struct SlabUpload {
     CYR_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
     return CYR_OK;
   }
-  // every sample_zstep-th plane, copied first for the means (a sample spread over the volume)
-  uint32_t sample_zstep = 1;
+  // the first plane of every slab, copied first for the means (a sample spread over the volume)
   cudaEvent_t sample = nullptr;
   const float *host = nullptr;
   float4 *dev = nullptr;
   uint32_t nmat = 0, nz = 0;
   size_t nvox = 0, npix = 0;
   cudaStream_t stream = nullptr;
+  // One copy per slab (the materials are the rows of a 2D copy): from pageable memory every copy call stages its
+  // data and waits, about 10 us beyond the transfer.  The first plane of a slab has come with the sample.
   int issue(uint32_t s) {  // queues the copies of slabs up to s
-    // planes the sample already brought (every sample_zstep-th, once it was issued) are not copied again
-    auto sampled = [&](uint32_t z) { return sample != nullptr && z % sample_zstep == 0; };
     for (; issued <= s && issued < count; ++issued) {
-      const uint32_t z0 = issued * planes, z1 = std::min(nz, z0 + planes);
-      for (uint32_t a = z0; a < z1;) {
-        if (sampled(a)) {
-          ++a;
-          continue;
-        }
-        uint32_t b = a + 1;
-        while (b < z1 && !sampled(b)) ++b;
-        for (uint32_t m = 0; m < nmat; ++m) {
-          const size_t off = size_t(m) * nvox + size_t(a) * npix;  // float4 elements
-          CYR_CUDA(cudaMemcpyAsync(dev + off, host + 4 * off, size_t(b - a) * npix * sizeof(float4),
-                                   cudaMemcpyHostToDevice, stream));
-        }
-        a = b;
+      const uint32_t z0 = issued * planes + (sample ? 1u : 0u), z1 = std::min(nz, (issued + 1) * planes);
+      if (z1 > z0) {
+        const size_t off = size_t(z0) * npix;  // float4 elements
+        CYR_CUDA(cudaMemcpy2DAsync(dev + off, nvox * sizeof(float4), host + 4 * off, nvox * sizeof(float4),
+                                   size_t(z1 - z0) * npix * sizeof(float4), nmat, cudaMemcpyHostToDevice, stream));
       }
       cudaEvent_t ev = nullptr;
       CYR_TRY(next_event(&ev));
@@ -1563,11 +1574,10 @@ struct SlabUpload {
     return CYR_OK;
   }
   int issue_sample() {
-    const size_t pitch = size_t(sample_zstep) * npix * sizeof(float4);
+    const size_t pitch = size_t(planes) * npix * sizeof(float4);
     for (uint32_t m = 0; m < nmat; ++m)
       CYR_CUDA(cudaMemcpy2DAsync(dev + size_t(m) * nvox, pitch, host + 4 * size_t(m) * nvox, pitch,
-                                 npix * sizeof(float4), (nz + sample_zstep - 1) / sample_zstep,
-                                 cudaMemcpyHostToDevice, stream));
+                                 npix * sizeof(float4), count, cudaMemcpyHostToDevice, stream));
     CYR_TRY(next_event(&sample));
     CYR_CUDA(cudaEventRecord(sample, stream));
     return CYR_OK;
@@ -1585,8 +1595,7 @@ int build_fields_x(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const 
                    uint32_t z1, bool fused, const float2 *twx, cudaStream_t st) {
   const uint32_t npk = pl.npk;
   float2 *spec = sc.spec.as<float2>();
-  int sms = 0;
-  CYR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+  const int sms = ctx.sms;
   fp.i0 = size_t(z0) * pl.npix, fp.i1 = size_t(z1) * pl.npix;
   if (fused) {
     const size_t smem = fields_rows_smem(pl.nx, npk, pl.nmat);
@@ -1594,7 +1603,7 @@ int build_fields_x(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const 
     int per_sm = 1;
     const int slot = ctx.prof.begin(kBuildFieldsRows, st);
     CYR_TRY(with_rows_kernel(o->morphology_type == 0, pl.nmat, pl.nx, [&](auto kern) -> int {
-      CYR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
+      CYR_TRY(blocks_per_sm(ctx, kern, 256, smem, &per_sm));
       const unsigned grid = unsigned(std::min<size_t>(rows, size_t(std::max(1, per_sm)) * sms));
       kern<<<grid, 256, smem, st>>>(fp, twx, npk);
       return CYR_OK;
@@ -1925,6 +1934,9 @@ struct RunMode {
 // build of the unconverted form repeats.
 constexpr size_t kConvertBuilds = 4;
 
+constexpr size_t kSlabBytes = size_t(24) << 20;
+constexpr uint32_t kSampleSlabs = 2;  // slabs from which the means come from the planes copied first
+
 int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const float *optical, const float4 *d_vox,
                 float *d_out, cudaStream_t st, const RunMode &mode = RunMode()) {
   Plan local;
@@ -1933,11 +1945,15 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
   CYR_TRY(setup_attrs(ctx));
   CYR_TRY(sc.init());
   if (!mode.plan && pl.fields && o->strategy == CYR_STRATEGY_AUTO && !mode.capturing) {
-    // AUTO falls back to the per-energy spectra when the field volumes do not fit
-    size_t free_b = 0, total_b = 0;
-    CYR_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const size_t reusable = sc.spec.bytes + sc.images.bytes + sc.avg.bytes;
-    if (field_bytes(pl) + (size_t(1) << 30) > free_b + reusable) pl.fields = false;
+    // AUTO falls back to the per-energy spectra when the field volumes do not fit (no query, 15 us, when every buffer
+    // has its place already)
+    if (sc.spec.bytes < size_t(pl.npk) * pl.nvox * sizeof(float2) || sc.images.bytes < image_bytes(pl, pl.ebatch) ||
+        sc.avg.bytes < size_t(pl.ebatch) * pl.npix * sizeof(float)) {
+      size_t free_b = 0, total_b = 0;
+      CYR_CUDA(cudaMemGetInfo(&free_b, &total_b));
+      const size_t reusable = sc.spec.bytes + sc.images.bytes + sc.avg.bytes;
+      if (field_bytes(pl) + (size_t(1) << 30) > free_b + reusable) pl.fields = false;
+    }
   }
   // scratch (grow-only); wait for the previous user of the scratch
   if (!mode.capturing) CYR_CUDA(cudaStreamWaitEvent(st, sc.last_use, 0));
@@ -1967,13 +1983,14 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
     upload.dev = const_cast<float4 *>(d_vox);
     upload.nmat = pl.nmat, upload.nz = pl.nz, upload.nvox = pl.nvox, upload.npix = pl.npix;
     // slabs: after the last one lands, its fields and x/y passes are still ahead
-    // of the z pass, so thinner slabs shorten that tail
-    upload.count = !pl.fields ? 1u : pl.nz >= 64 ? 16u : pl.nz >= 8 ? 8u : 1u;
+    // of the z pass, so thinner slabs shorten that tail, but each costs a copy
+    // call and launches of few blocks: at least kSlabBytes a slab, 16 at most
+    const size_t bytes = pl.nvox * pl.nmat * sizeof(float4);
+    upload.count = !pl.fields ? 1u : uint32_t(std::clamp<size_t>(bytes / kSlabBytes, 1, std::min(16u, std::max(1u, pl.nz / 2))));
     upload.planes = (pl.nz + upload.count - 1) / upload.count;
     upload.count = (pl.nz + upload.planes - 1) / upload.planes;
     if (pl.fields) {
-      upload.sample_zstep = std::max(1u, pl.nz / 8);
-      CYR_TRY(upload.issue_sample());
+      if (upload.count >= kSampleSlabs) CYR_TRY(upload.issue_sample());
       CYR_TRY(upload.issue(0));
     } else {
       CYR_TRY(upload.issue(upload.count - 1));
@@ -2004,13 +2021,15 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
     // (with a slab upload: the planes copied first for that purpose)
     mp.zstep = convert ? 1u : pl.mom_zstep;
     mp.ystep = convert ? 1u : pl.mom_ystep;
-    if (slabs) {
-      mp.zstep = upload.sample_zstep;
+    if (slabs && upload.sample) {
+      mp.zstep = upload.planes;
       CYR_CUDA(cudaStreamWaitEvent(st, upload.sample, 0));
+    } else if (slabs) {  // few slabs: the means wait for the whole volume, whose planes they sample as ever
+      CYR_TRY(upload.issue(upload.count - 1));
+      CYR_CUDA(cudaStreamWaitEvent(st, upload.events.back(), 0));
     }
     mp.neg = sc.flag();
-    int nsm = 0;
-    CYR_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx.device));
+    const int nsm = ctx.sms;
     // about 8 samples per thread: small volumes get few blocks (each block ends in
     // kMoments double atomics on the same addresses), large ones 4 per SM
     const size_t nsamp = size_t(pl.nx) * ((pl.ny + mp.ystep - 1) / mp.ystep) * ((pl.nz + mp.zstep - 1) / mp.zstep);
@@ -2054,8 +2073,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
     bp.hann_y = reinterpret_cast<const float *>(dp + pl.off_hy);
     bp.hann_z = reinterpret_cast<const float *>(dp + pl.off_hz);
   }
-  int sms = 0;
-  CYR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+  const int sms = ctx.sms;
   const uint32_t build_blocks = uint32_t(std::min<size_t>((pl.nvox + 255) / 256, size_t(sms) * 8));
   EwaldParams ep = ewald_params(pl, o, dp, spec, dc, images);
   ep.errors = sc.errors.as<unsigned>();
@@ -2396,15 +2414,19 @@ int run_fp64(DeviceContext &ctx, const cyr_options *o, const double *optical, co
   const uint32_t npk = fields64_packed(pl.nmat);
   const double per_energy = double(pl.ne) * (pl.material_frame ? 3.0 * pl.nk * pl.nang : double(nvol));
   bool fields = o->strategy == CYR_STRATEGY_FIELDS || (o->strategy == CYR_STRATEGY_AUTO && npk < per_energy);
-  if (fields && o->strategy == CYR_STRATEGY_AUTO) {
-    size_t free_b = 0, total_b = 0;
-    CYR_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    if (size_t(npk) * pl.nvox * sizeof(double2) + (size_t(1) << 30) > free_b + f.spec.bytes) fields = false;
-  }
   // energies per Ewald, rotation and warp launch: up to 512 MB of per-angle images
   const size_t image = size_t(pl.nang) * pl.npix * sizeof(double);
-  const uint32_t batch =
-      fields ? uint32_t(std::max<size_t>(1, std::min<size_t>(std::min(pl.ne, 65535u), (size_t(512) << 20) / image))) : 1u;
+  const uint32_t most =
+      uint32_t(std::max<size_t>(1, std::min<size_t>(std::min(pl.ne, 65535u), (size_t(512) << 20) / image)));
+  if (fields && o->strategy == CYR_STRATEGY_AUTO &&
+      (f.spec.bytes < size_t(npk) * pl.nvox * sizeof(double2) || f.images.bytes < most * image)) {
+    size_t free_b = 0, total_b = 0;
+    CYR_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if (size_t(npk) * pl.nvox * sizeof(double2) + most * image + (size_t(1) << 30) >
+        free_b + f.spec.bytes + f.images.bytes)
+      fields = false;
+  }
+  const uint32_t batch = fields ? most : 1u;
   CYR_TRY(f.spec.ensure(size_t(fields ? npk : nvol) * pl.nvox * sizeof(double2)));
   CYR_TRY(f.images.ensure(batch * image));
   CYR_TRY(f.avg.ensure(batch * pl.npix * sizeof(double)));
@@ -2415,8 +2437,7 @@ int run_fp64(DeviceContext &ctx, const cyr_options *o, const double *optical, co
   const unsigned char *dp = f.params.as<unsigned char>(), *dq = f.params64.as<unsigned char>();
   double2 *spec = f.spec.as<double2>();
   double *images = f.images.as<double>(), *avg = f.avg.as<double>();
-  int sms = 0;
-  CYR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+  const int sms = ctx.sms;
   Build64Params bp{};
   bp.vox = d_vox;
   bp.vox_fp64 = vox64 ? 1u : 0u;
@@ -2753,8 +2774,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   CYR_TRY(sc.dc.ensure(size_t(G) * npk * sizeof(float2)));
   CYR_TRY(sc.clear(size_t(G) * nmat * kMoments, st));
   float2 *spec = sc.spec.as<float2>();
-  int sms = 0;
-  CYR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+  const int sms = ctx.sms;
   const float4 *const *vox_g = reinterpret_cast<const float4 *const *>(dp + off_v);
   // moments of every request (blockIdx.z = request), over the z-plane subsample
   MomentParams mp{};
@@ -2810,7 +2830,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     int per_sm = 1;
     const int slot = ctx.prof.begin(kBuildFieldsRows, st);
     CYR_TRY(with_rows_kernel(o->morphology_type == 0, nmat, p0.nx, [&](auto kern) -> int {
-      CYR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
+      CYR_TRY(blocks_per_sm(ctx, kern, 256, smem, &per_sm));
       const size_t want = (size_t(std::max(1, per_sm)) * sms + G - 1) / G;
       kern<<<dim3(unsigned(std::min<size_t>(rws, want)), G), 256, smem, st>>>(fp, twx, npk);
       return CYR_OK;
@@ -3249,6 +3269,7 @@ static int cuda_main_impl(const cyr_options *opt, const float *optical, const fl
   CYR_TRY(ctx->out_in.ensure(out_bytes));
   if (!ctx->main_stream) CYR_CUDA(cudaStreamCreateWithFlags(&ctx->main_stream, cudaStreamNonBlocking));
   if (!ctx->copy_stream) CYR_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
+  if (!ctx->host_errors) CYR_CUDA(cudaMallocHost(&ctx->host_errors, 2 * sizeof(unsigned)));
   cudaStream_t st = ctx->main_stream, cs = ctx->copy_stream;
   int rc = CYR_OK;
   do {
@@ -3263,20 +3284,23 @@ static int cuda_main_impl(const cyr_options *opt, const float *optical, const fl
       rc = fail(CYR_ERR_CUDA, "projection download failed: %s", cudaGetErrorString(cudaGetLastError()));
       break;
     }
+    // the error words ride ahead of the one synchronisation
+    unsigned *errs = ctx->host_errors;
+    errs[0] = errs[1] = 0;
+    cudaMemcpyAsync(&errs[0], ctx->main.errors.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+    if (ctx->tma_error) cudaMemcpyAsync(&errs[1], ctx->tma_error, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
     const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
       rc = fail(CYR_ERR_CUDA, "simulation failed: %s", cudaGetErrorString(e));
       break;
     }
-    unsigned errs = 0;
-    if (cudaMemcpy(&errs, ctx->main.errors.ptr, sizeof errs, cudaMemcpyDeviceToHost) == cudaSuccess && errs != 0)
-      rc = fail(CYR_ERR_CUDA, "%u detector pixels needed z planes outside the kept range", errs);
-    if (ctx->tma_error && cudaMemcpy(&errs, ctx->tma_error, sizeof errs, cudaMemcpyDeviceToHost) == cudaSuccess &&
-        errs != 0)
-      rc = fail(CYR_ERR_CUDA, "an FFT tile copy did not complete within its wait limit");
+    if (errs[0] != 0) rc = fail(CYR_ERR_CUDA, "%u detector pixels needed z planes outside the kept range", errs[0]);
+    if (errs[1] != 0) rc = fail(CYR_ERR_CUDA, "an FFT tile copy did not complete within its wait limit");
   } while (false);
-  cudaStreamSynchronize(cs);
-  cudaStreamSynchronize(st);
+  if (rc != CYR_OK) {  // whatever was enqueued ends before the caller's buffers may go
+    cudaStreamSynchronize(cs);
+    cudaStreamSynchronize(st);
+  }
   return rc;
 }
 
