@@ -16,8 +16,8 @@ REPO = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(BUILD, "libcyrsoxs_gb300.so")
-SOURCES = ["engine.cu", "mixfft_f32.cu", "mixfft_f64.cu"]
-DEPS = SOURCES + ["complex.cuh", "kernels.cuh", "mixfft.cuh", "fields.cuh", "fp64.cuh", "geometry.h"]
+SOURCES = ["engine.cu", "mixfft_f32.cu", "mixfft_f64.cu", "mixbuild.cu"]
+DEPS = SOURCES + ["complex.cuh", "fieldbuild.cuh", "kernels.cuh", "mixfft.cuh", "fields.cuh", "fp64.cuh", "geometry.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

@@ -439,9 +439,11 @@ struct DeviceContext {
     MixPlan plan;
     void *tw = nullptr;
     uint32_t *first = nullptr;
+    uint32_t *slot = nullptr;  // row form: slot of each element (mixbuild.cu)
   };
   std::map<std::array<uint32_t, 3>, MixTables> mix;  // key: length, row form, bytes per real
   int sms = 0;                                       // multiprocessors
+  std::map<size_t, int> mix_build_occupancy;         // blocks per SM of k_build_fields_mix at a shared-memory size
   std::map<std::pair<const void *, size_t>, int> occupancy;  // blocks per SM of a kernel at a shared-memory size
   struct Fp64Scratch {
     DeviceBuffer spec, images, avg, params, params64, vox, out;
@@ -542,6 +544,7 @@ int setup_attrs(DeviceContext &ctx) {
   const int smem = int(kFftSmemBudget);
   CYR_CUDA(mix_attributes<float2>(smem));
   CYR_CUDA(mix_attributes<double2>(smem));
+  CYR_CUDA(mix_build_attributes(smem));
 #define CYR_COLS_ATTR(V, T) \
   CYR_CUDA(cudaFuncSetAttribute(k_fft_cols<V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   CYR_COLS_ATTR(32, 8)
@@ -918,10 +921,30 @@ int get_mix(DeviceContext &ctx, uint32_t M, bool row, const DeviceContext::MixTa
     CYR_CUDA(cudaMalloc(&t.first, t.plan.first.size() * sizeof(uint32_t)));
     CYR_CUDA(cudaMemcpy(t.tw, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
     CYR_CUDA(cudaMemcpy(t.first, t.plan.first.data(), t.plan.first.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    if (row && t.plan.ns > 1) {
+      const MixStage &st = t.plan.st[0];
+      std::vector<uint32_t> slot(M);
+      for (uint32_t x = 0; x < M; ++x)
+        slot[x] = x % st.m + (t.plan.pad ? x % st.m / t.plan.rs : 0) + x / st.m * st.span;
+      CYR_CUDA(cudaMalloc(&t.slot, M * sizeof(uint32_t)));
+      CYR_CUDA(cudaMemcpy(t.slot, slot.data(), M * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    }
     it = ctx.mix.emplace(key, std::move(t)).first;
   }
   *out = &it->second;  // map nodes do not move, and tables are never changed once made
   return CYR_OK;
+}
+
+// The plan's part of a launch's parameters.
+template <class T>
+void mix_tables(MixParams<T> &p, const DeviceContext::MixTables &t) {
+  const MixPlan &pl = t.plan;
+  p.ns = pl.ns;
+  p.line_slots = pl.line_slots;
+  p.pad = pl.pad, p.rs = pl.rs, p.rs_magic = mix_magic(pl.rs);
+  std::copy(pl.st, pl.st + pl.ns, p.st);
+  p.tw = static_cast<const T *>(t.tw);
+  p.first = t.first;
 }
 
 constexpr size_t kMixSmem = 56 * 1024;       // four blocks per SM
@@ -950,12 +973,7 @@ int mix_pass(DeviceContext &ctx, T *data, uint32_t nx, uint32_t ny, uint32_t nz,
   p.vstride = vstride;
   p.n = n;
   p.M = M;
-  p.ns = pl.ns;
-  p.line_slots = pl.line_slots;
-  p.pad = pl.pad, p.rs = pl.rs, p.rs_magic = mix_magic(pl.rs);
-  std::copy(pl.st, pl.st + pl.ns, p.st);
-  p.tw = static_cast<const T *>(t->tw);
-  p.first = t->first;
+  mix_tables(p, *t);
   if (conv) {
     p.chirp = static_cast<const T *>(conv->chirp), p.bhat = static_cast<const T *>(conv->bhat);
     p.in = conv->in, p.out = conv->out;
@@ -1589,29 +1607,81 @@ struct SlabUpload {
   }
 };
 
-// Fields of planes [z0, z1) and their x pass: fused (k_build_fields_rows) or
-// the separate build and row pass.
-int build_fields_x(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan &pl, FieldParams fp, uint32_t z0,
-                   uint32_t z1, bool fused, const float2 *twx, cudaStream_t st) {
-  const uint32_t npk = pl.npk;
-  float2 *spec = sc.spec.as<float2>();
-  const int sms = ctx.sms;
-  fp.i0 = size_t(z0) * pl.npix, fp.i1 = size_t(z1) * pl.npix;
-  if (fused) {
-    const size_t smem = fields_rows_smem(pl.nx, npk, pl.nmat);
-    const uint32_t rows = (z1 - z0) * pl.ny;
-    int per_sm = 1;
+// Whether the field build of nx-point rows with npk packed volumes can be fused with the x pass: warp-FFT lengths
+// (k_build_fields_rows) or mixed-radix lengths of two stages and more (k_build_fields_mix) whose lines fit.
+bool rows_length(uint32_t nx) { return nx == 128 || nx == 256 || nx == 512 || nx == 1024; }
+bool fused_build(uint32_t nx, uint32_t npk, uint32_t nmat) {
+  if (rows_length(nx)) return fields_rows_smem(nx, npk, nmat) <= kFftSmemBudget;
+  // the padded line is at most 17/16 of the row and a slot per block of the second stage
+  return nx > uint32_t(kMixMaxRadix) && mix_length(nx) && size_t(npk) * (nx + nx / 2 + 16) * sizeof(float2) <= kMixSmemMax;
+}
+
+// The fused build + x pass of `groups` requests' voxels [fp.i0, fp.i1) (blockIdx.y = request).
+int launch_fused_build(DeviceContext &ctx, const FieldParams &fp, uint32_t npk, bool euler, uint32_t groups,
+                       cudaStream_t st) {
+  const uint32_t rows = uint32_t((fp.i1 - fp.i0) / fp.nx);
+  int per_sm = 1;
+  auto grid = [&](uint32_t tiles) {
+    const size_t want = (size_t(std::max(1, per_sm)) * ctx.sms + groups - 1) / groups;
+    return dim3(unsigned(std::min<size_t>(tiles, want)), groups);
+  };
+  if (rows_length(fp.nx)) {
+    const float2 *tw = nullptr;
+    CYR_TRY(get_twiddles(ctx, fp.nx, &tw));
+    const size_t smem = fields_rows_smem(fp.nx, npk, fp.nmat);
     const int slot = ctx.prof.begin(kBuildFieldsRows, st);
-    CYR_TRY(with_rows_kernel(o->morphology_type == 0, pl.nmat, pl.nx, [&](auto kern) -> int {
+    CYR_TRY(with_rows_kernel(euler, fp.nmat, fp.nx, [&](auto kern) -> int {
       CYR_TRY(blocks_per_sm(ctx, kern, 256, smem, &per_sm));
-      const unsigned grid = unsigned(std::min<size_t>(rows, size_t(std::max(1, per_sm)) * sms));
-      kern<<<grid, 256, smem, st>>>(fp, twx, npk);
+      kern<<<grid(rows), 256, smem, st>>>(fp, tw, npk);
       return CYR_OK;
     }));
     ctx.prof.end(slot, st);
     CYR_CUDA(cudaGetLastError());
     return CYR_OK;
   }
+  const DeviceContext::MixTables *t = nullptr;
+  CYR_TRY(get_mix<float2>(ctx, fp.nx, true, &t));
+  MixBuildParams q{};
+  q.f = fp;
+  mix_tables(q.m, *t);
+  q.m.nx = fp.nx;
+  q.slot = t->slot;
+  q.npk = npk, q.npk_magic = mix_magic(npk);
+  q.form = (euler ? 0u : 5u) + (fp.nmat <= 4 ? fp.nmat : 0u);
+  // rows per block: the fewest rounds of 256 threads per row over the build (about 100 instructions a voxel and
+  // material) and the stages (about 20 a point), within three blocks per SM
+  const size_t row = size_t(npk) * t->plan.line_slots * sizeof(float2);
+  uint32_t rpb = 1;
+  double least = 0.0;
+  for (uint32_t r = 1; r <= 8 && (r == 1 || (r * row <= 72 * 1024 && size_t(rows / r) * groups >= 3 * size_t(ctx.sms))); ++r) {
+    auto rounds = [&](uint32_t work) { return double((work + kMixThreads - 1) / kMixThreads); };
+    double c = rounds(r * fp.nx) * 100.0 * fp.nmat;
+    for (uint32_t s = 0; s < t->plan.ns; ++s) c += rounds(r * npk * t->plan.st[s].nb) * 20.0 * t->plan.st[s].radix;
+    if (r == 1 || c / r < least) rpb = r, least = c / r;
+  }
+  q.m.rows = rpb;
+  const size_t smem = rpb * row;
+  if (smem > kMixSmemMax) return fail(CYR_ERR_UNSUPPORTED, "row length %u too large for the fused build", fp.nx);
+  {
+    std::lock_guard<std::mutex> lk(ctx.tables_mu);
+    auto it = ctx.mix_build_occupancy.find(smem);
+    if (it == ctx.mix_build_occupancy.end()) it = ctx.mix_build_occupancy.emplace(smem, mix_build_blocks(smem)).first;
+    per_sm = it->second;
+  }
+  const int slot = ctx.prof.begin(kBuildFieldsRows, st);
+  CYR_CUDA(mix_build_launch(grid((rows + rpb - 1) / rpb), smem, st, q));
+  ctx.prof.end(slot, st);
+  return CYR_OK;
+}
+
+// Fields of planes [z0, z1) and their x pass: fused or the separate build and row pass.
+int build_fields_x(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan &pl, FieldParams fp, uint32_t z0,
+                   uint32_t z1, bool fused, cudaStream_t st) {
+  const uint32_t npk = pl.npk;
+  float2 *spec = sc.spec.as<float2>();
+  const int sms = ctx.sms;
+  fp.i0 = size_t(z0) * pl.npix, fp.i1 = size_t(z1) * pl.npix;
+  if (fused) return launch_fused_build(ctx, fp, npk, o->morphology_type == 0, 1, st);
   const uint32_t blocks = uint32_t(std::min<size_t>((fp.i1 - fp.i0 + 255) / 256, size_t(sms) * 8));
   const int slot = ctx.prof.begin(kBuildFields, st);
   CYR_TRY(with_materials(o->morphology_type == 0, pl.nmat, [&](auto mc, auto tc) -> int {
@@ -1669,7 +1739,7 @@ int field_zmask(DeviceContext &ctx, Scratch &sc, const EwaldGeom &g, const float
 }
 
 int tune_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan &pl, const FieldParams &fp,
-                bool fused_ok, const float2 *twx, cudaStream_t st, DeviceContext::FieldTune &ft,
+                bool fused_ok, cudaStream_t st, DeviceContext::FieldTune &ft,
                 const uint32_t *zmask) {
   struct Cand {
     int kind;  // 0 build + x, 1 y pass, 2 z pass
@@ -1691,16 +1761,19 @@ int tune_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Pla
     CYR_CUDA(cudaEventCreate(&c.b));
   }
   int rc = CYR_OK;
-  for (Cand &c : cands) {
-    CYR_CUDA(cudaEventRecord(c.a, st));
-    if (c.kind == 0)
-      rc = build_fields_x(ctx, sc, o, pl, fp, 0, pl.nz, c.choice == 1, twx, st);
-    else
-      rc = warp_fft_pass(ctx, sc.spec.as<float2>(), pl.nx, pl.ny, pl.nz, pl.npk, c.kind, st, pl.nvox, c.choice,
-                         c.kind == 2 ? zmask : nullptr);
-    if (rc != CYR_OK) break;
-    CYR_CUDA(cudaEventRecord(c.b, st));
-  }
+  // each candidate runs twice and its second run is timed: a kernel's first launch in a process also loads its code,
+  // which made the fused build of small volumes look slower than the separate one in some processes
+  for (int pass = 0; pass < 2 && rc == CYR_OK; ++pass)
+    for (Cand &c : cands) {
+      if (pass) CYR_CUDA(cudaEventRecord(c.a, st));
+      if (c.kind == 0)
+        rc = build_fields_x(ctx, sc, o, pl, fp, 0, pl.nz, c.choice == 1, st);
+      else
+        rc = warp_fft_pass(ctx, sc.spec.as<float2>(), pl.nx, pl.ny, pl.nz, pl.npk, c.kind, st, pl.nvox, c.choice,
+                           c.kind == 2 ? zmask : nullptr);
+      if (rc != CYR_OK) break;
+      if (pass) CYR_CUDA(cudaEventRecord(c.b, st));
+    }
   if (rc == CYR_OK) {
     CYR_CUDA(cudaEventSynchronize(cands.back().b));
     float best[3] = {1e30f, 1e30f, 1e30f};
@@ -1794,11 +1867,7 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
   const uint32_t *zmask = nullptr;
   CYR_TRY(field_zmask(ctx, sc, geom, reinterpret_cast<const float *>(dp + pl.off_kmag), pl.ne,
                       reinterpret_cast<const float *>(dp + pl.off_kvec), pl.nk, st, &zmask));
-  // the field build fused with the x pass when x is a warp-FFT length and the row's lines fit
-  const bool fused_ok = (pl.nx == 128 || pl.nx == 256 || pl.nx == 512 || pl.nx == 1024) &&
-                        fields_rows_smem(pl.nx, npk, pl.nmat) <= kFftSmemBudget;
-  const float2 *twx = nullptr;
-  if (fused_ok) CYR_TRY(get_twiddles(ctx, pl.nx, &twx));
+  const bool fused_ok = fused_build(pl.nx, npk, pl.nmat);
   // tuned launch forms of this shape, tuned here on its first device-resident request
   char key[96];
   std::snprintf(key, sizeof key, "%u,%u,%u,%u", pl.nx, pl.ny, pl.nz, npk);
@@ -1812,7 +1881,7 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
   if (!have) {
     ft.fused = fused_ok;
     if (ctx.autotune && !up && !capturing && !ctx.prof.active) {
-      CYR_TRY(tune_fields(ctx, sc, o, pl, fp, fused_ok, twx, st, ft, zmask));
+      CYR_TRY(tune_fields(ctx, sc, o, pl, fp, fused_ok, st, ft, zmask));
       std::lock_guard<std::mutex> lk(ctx.tables_mu);
       ctx.ftune[key] = ft;
     }
@@ -1826,7 +1895,7 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
       CYR_TRY(const_cast<SlabUpload *>(up)->issue(sl));
       CYR_CUDA(cudaStreamWaitEvent(st, up->events[sl], 0));
     }
-    CYR_TRY(build_fields_x(ctx, sc, o, pl, fp, z0, z1, fused, twx, st));
+    CYR_TRY(build_fields_x(ctx, sc, o, pl, fp, z0, z1, fused, st));
     CYR_TRY(fft_axes(ctx, spec + size_t(z0) * pl.npix, pl.nx, pl.ny, z1 - z0, npk, st, 1, 1, pl.nvox,
                      ft.form));
     if (up) CYR_TRY(const_cast<SlabUpload *>(up)->issue(sl + 1));  // the next slab's copy, behind this slab's kernels
@@ -2812,8 +2881,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   fp.out_stride = size_t(npk) * nvox;
   fp.i0 = 0, fp.i1 = nvox;
   if (p0.hanning) fp.hann_x = mp.hann_x, fp.hann_y = mp.hann_y, fp.hann_z = mp.hann_z;
-  const bool fused_ok = (p0.nx == 128 || p0.nx == 256 || p0.nx == 512 || p0.nx == 1024) &&
-                        fields_rows_smem(p0.nx, npk, nmat) <= kFftSmemBudget;
+  const bool fused_ok = fused_build(p0.nx, npk, nmat);
   DeviceContext::FieldTune ft;
   {
     char key[96];
@@ -2823,20 +2891,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     if (it != ctx.ftune.end()) ft = it->second;
   }
   if (fused_ok && ft.fused) {
-    const float2 *twx = nullptr;
-    CYR_TRY(get_twiddles(ctx, p0.nx, &twx));
-    const size_t smem = fields_rows_smem(p0.nx, npk, nmat);
-    const uint32_t rws = p0.nz * p0.ny;
-    int per_sm = 1;
-    const int slot = ctx.prof.begin(kBuildFieldsRows, st);
-    CYR_TRY(with_rows_kernel(o->morphology_type == 0, nmat, p0.nx, [&](auto kern) -> int {
-      CYR_TRY(blocks_per_sm(ctx, kern, 256, smem, &per_sm));
-      const size_t want = (size_t(std::max(1, per_sm)) * sms + G - 1) / G;
-      kern<<<dim3(unsigned(std::min<size_t>(rws, want)), G), 256, smem, st>>>(fp, twx, npk);
-      return CYR_OK;
-    }));
-    ctx.prof.end(slot, st);
-    CYR_CUDA(cudaGetLastError());
+    CYR_TRY(launch_fused_build(ctx, fp, npk, o->morphology_type == 0, G, st));
   } else {
     const uint32_t blocks =
         uint32_t(std::max<size_t>(1, std::min<size_t>((nvox + 255) / 256, (size_t(sms) * 8 + G - 1) / G)));

@@ -16,10 +16,10 @@
 #include <stdint.h>
 
 #include "complex.cuh"
+#include "fieldbuild.cuh"
 
 namespace cyr {
 
-constexpr int kMaxMaterials = 32;
 constexpr int kMaxAngles = 4096;
 
 // ---------------------------------------------------------------------------
@@ -58,25 +58,6 @@ struct BuildParams {
   const float *hann_x, *hann_y, *hann_z;  // null when no windowing
   float2 *out;          // [nvol][V]
 };
-
-// Direction and fractions of one material at one voxel.
-template <int MORPH>
-__device__ __forceinline__ void director(float4 s, float &sx, float &sy, float &sz, float &pa, float &pui) {
-  if (MORPH == 0) {  // Euler: s1 = (S, theta, psi, Vfrac), uniaxial.h:82-92
-    float st, ct, sp, cp;
-    sincosf(s.y, &st, &ct);
-    sincosf(s.z, &sp, &cp);
-    sx = cp * st;
-    sy = sp * st;
-    sz = ct;
-    pa = s.w * s.x;
-    pui = s.w - pa;
-  } else {  // vector: s1 = (sx, sy, sz, phi_unaligned), uniaxial.h:207-216
-    sx = s.x, sy = s.y, sz = s.z;
-    pa = 1.f;
-    pui = s.w;
-  }
-}
 
 // Tensor entries of one voxel.  With CONV the morphology has been converted
 // to the vector form u = sqrt(phi_a) s, phi_ui (phi_a s_i s_j = u_i u_j),
@@ -131,7 +112,6 @@ __device__ __forceinline__ void nt_entries(const BuildParams &p, const MaterialC
 // the path always replaces by the mean of its neighbours (src/cudaMain.cu:
 // 123-176); removing it keeps the FP32 FFT's rounding floor proportional to
 // the fluctuations instead of to the (~5x larger) mean.
-constexpr int kMoments = 7;  // at most 8 (k_moments)
 struct MomentParams {
   const float4 *vox;
   const float4 *const *vox_g;  // request group (blockIdx.z = request): its morphologies, or null

@@ -50,6 +50,7 @@
 #include <utility>
 
 #include "complex.cuh"
+#include "fieldbuild.cuh"
 
 namespace cyr {
 
@@ -346,6 +347,26 @@ struct MixTile {
   }
 };
 
+// A stage between the first and the last; inverse: its transpose, for the second transform of a convolution.
+template <class T, bool COL, class Tile>
+__device__ __forceinline__ void mix_middle(const MixParams<T> &p, const Tile &tile, const MixStage &st, bool inverse) {
+  mix_radix(st.radix, [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+    tile.each(st, [&](T *, T *s, uint32_t b, bool) {
+      const uint32_t blk = mix_div(b, st.m, st.m_magic), j = b - blk * st.m;
+      T *e = s + tile.at(blk * st.block + tile.jslot(j));
+      T v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = e[tile.at(q * st.span)];
+      if (inverse) mix_twiddle<R, COL>(v, p.tw + st.tw, j, st.m);
+      dft_reg<R>(v);
+      if (!inverse) mix_twiddle<R, COL>(v, p.tw + st.tw, j, st.m);
+#pragma unroll
+      for (int k = 0; k < R; ++k) e[tile.at(k * st.span)] = v[k];
+    });
+  });
+}
+
 template <class T, bool COL, int FORM>
 __global__ void __launch_bounds__(kMixThreads, sizeof(T) == 8 ? 4 : 2) k_mix_fft(const __grid_constant__ MixParams<T> p) {
   extern __shared__ unsigned char mix_smem[];
@@ -393,27 +414,9 @@ __global__ void __launch_bounds__(kMixThreads, sizeof(T) == 8 ? 4 : 2) k_mix_fft
     });
   }
   if (FORM == kMixPlain && p.ns == 1) return;
-  // stages between the first and the last; inverse: the transposed stages of the Bluestein product's transform
-  auto middle = [&](const MixStage &st, bool inverse) {
-    mix_radix(st.radix, [&](auto rc) {
-      constexpr int R = decltype(rc)::value;
-      tile.each(st, [&](T *, T *s, uint32_t b, bool) {
-        const uint32_t blk = mix_div(b, st.m, st.m_magic), j = b - blk * st.m;
-        T *e = s + tile.at(blk * st.block + tile.jslot(j));
-        T v[R];
-#pragma unroll
-        for (int q = 0; q < R; ++q) v[q] = e[tile.at(q * st.span)];
-        if (inverse) mix_twiddle<R, COL>(v, p.tw + st.tw, j, st.m);
-        dft_reg<R>(v);
-        if (!inverse) mix_twiddle<R, COL>(v, p.tw + st.tw, j, st.m);
-#pragma unroll
-        for (int k = 0; k < R; ++k) e[tile.at(k * st.span)] = v[k];
-      });
-    });
-  };
   for (uint32_t s = 1; s + 1 < p.ns; ++s) {
     __syncthreads();
-    middle(p.st[s], false);
+    mix_middle<T, COL>(p, tile, p.st[s], false);
   }
   __syncthreads();
   // last stage: blocks of R consecutive points, frequencies fb + k M / R
@@ -453,7 +456,7 @@ __global__ void __launch_bounds__(kMixThreads, sizeof(T) == 8 ? 4 : 2) k_mix_fft
   if constexpr (FORM != kMixPlain) {
     for (uint32_t s = p.ns - 2; s >= 1; --s) {
       __syncthreads();
-      middle(p.st[s], true);
+      mix_middle<T, COL>(p, tile, p.st[s], true);
     }
     __syncthreads();
     const MixStage &st = p.st[0];
@@ -479,6 +482,19 @@ __global__ void __launch_bounds__(kMixThreads, sizeof(T) == 8 ? 4 : 2) k_mix_fft
     });
   }
 }
+
+// Field build fused with the x pass for the row lengths that k_mix_fft takes in two stages or more
+// (mixbuild.cu): the general form of k_build_fields_rows.
+struct MixBuildParams {
+  FieldParams f;
+  MixParams<float2> m;       // row form: tables and stages; rows = rows per block
+  const uint32_t *slot;      // [nx]: shared-memory slot of element x of a line
+  uint32_t npk, npk_magic;
+  uint32_t form;             // 5 (morphology) + material count up to 4 (0: any)
+};
+cudaError_t mix_build_launch(dim3 grid, size_t smem, cudaStream_t st, const MixBuildParams &p);
+cudaError_t mix_build_attributes(int smem);
+int mix_build_blocks(size_t smem);  // resident blocks per SM
 
 // The kernel instances live in translation units of their own (mixfft_f32.cu, mixfft_f64.cu).
 template <class T>
