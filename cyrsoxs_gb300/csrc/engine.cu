@@ -1999,10 +1999,10 @@ struct RunMode {
 
 
 // Builds from which the conversion pass (a read and a write of the morphology,
-// 217 us on 256 x 256 x 128 with 4 materials) repays the trigonometry that each
-// build of the unconverted form repeats.
-constexpr size_t kConvertBuilds = 4;
-
+// 235 us on 256 x 256 x 128 with 4 materials) repays the trigonometry that each
+// build of the unconverted form repeats: 4 us of 293 with the warp FFT (whose
+// exchanges hide it), 32 of 403 with other z lengths (x 90).
+constexpr size_t kConvertBuildsWarp = 64, kConvertBuilds = 6;
 constexpr size_t kSlabBytes = size_t(24) << 20;
 constexpr uint32_t kSampleSlabs = 2;  // slabs from which the means come from the planes copied first
 
@@ -2072,7 +2072,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
   // Per-energy spectra of Euler morphologies: converted to the trigonometry-free
   // vector form once per request when enough builds follow to repay the pass
   const size_t builds = pl.material_frame ? size_t(pl.ne) * pl.nk * pl.nang : pl.ne;
-  const bool convert = o->morphology_type == 0 && !pl.fields && builds >= kConvertBuilds;
+  const bool convert = o->morphology_type == 0 && !pl.fields && builds >= (pl.zwarp ? kConvertBuildsWarp : kConvertBuilds);
   if (convert) CYR_TRY(sc.conv.ensure(pl.nvox * pl.nmat * sizeof(float4)));
   {
     MomentParams mp{};
@@ -2203,15 +2203,15 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
           if (have_tuned) tuned = it->second;
         }
         if (!have_tuned && pl.zcands.size() > 1 && !ctx.prof.active && !mode.capturing) {
-          // autotune: time every candidate once on this energy; the last one's
-          // output stays in `spec` and is used
+          // autotune: time every candidate on this energy
           std::vector<cudaEvent_t> ev(2 * pl.zcands.size());
           for (auto &e : ev) CYR_CUDA(cudaEventCreate(&e));
-          for (size_t c = 0; c < pl.zcands.size(); ++c) {
-            CYR_CUDA(cudaEventRecord(ev[2 * c], st));
-            launch_warp(pl.zcands[c]);
-            CYR_CUDA(cudaEventRecord(ev[2 * c + 1], st));
-          }
+          for (int pass = 0; pass < 2; ++pass)  // the second run is timed: the first also loads the code
+            for (size_t c = 0; c < pl.zcands.size(); ++c) {
+              if (pass) CYR_CUDA(cudaEventRecord(ev[2 * c], st));
+              launch_warp(pl.zcands[c]);
+              if (pass) CYR_CUDA(cudaEventRecord(ev[2 * c + 1], st));
+            }
           CYR_CUDA(cudaGetLastError());
           CYR_CUDA(cudaEventSynchronize(ev.back()));
           ZTune best = pl.zcands[0];

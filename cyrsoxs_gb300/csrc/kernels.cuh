@@ -64,11 +64,16 @@ struct BuildParams {
 // which needs no trigonometry per energy.
 // `base` points at material 0 of the voxel, material m at base + m * mstride
 // (global memory, or a tile staged in shared memory).
+// The diagonal's A s_i^2 + B (|s|^2 - s_i^2) is taken as D s_i^2 + B |s|^2, D = A - B formed in double: the part that
+// the three entries share is added once, and every term is one packed multiply-add (256 x 256 x 128, 4 materials, one
+// energy: 318 -> 291 us for the fused build + z pass).
 template <int MORPH, bool CONV>
 __device__ __forceinline__ void nt_entries_at(const BuildParams &p, const MaterialConsts &mc, const float4 *base,
                                               size_t mstride, float2 nt[6]) {
 #pragma unroll
   for (int q = 0; q < 6; ++q) nt[q] = make_float2(0.f, 0.f);
+  float2 shared = make_float2(0.f, 0.f);
+  auto mac = [](float2 &acc, float s, float2 c) { acc = pfma(make_float2(s, s), c, acc); };
   for (uint32_t m0 = 0; m0 < p.nmat; m0 += 4) {
     float4 sv[4];
 #pragma unroll
@@ -80,23 +85,19 @@ __device__ __forceinline__ void nt_entries_at(const BuildParams &p, const Materi
       const uint32_t m = m0 + u;
       float sx, sy, sz, pa, pui;
       director<CONV ? 1 : MORPH>(sv[u], sx, sy, sz, pa, pui);
-      const float xx = sx * sx, yy = sy * sy, zz = sz * sz;
-      const float2 A = mc.A[m], B = mc.B[m], C = mc.C[m], D = mc.D[m];
-      // diagonal: phi_a (A s_i^2 + B (|s|^2 - s_i^2)) + phi_ui C, with |s|^2 - s_i^2 as the reference sums it
-      const float ax = pa * xx, ay = pa * yy, az = pa * zz;
-      const float bx = pa * (yy + zz), by = pa * (xx + zz), bz = pa * (xx + yy);
-      nt[0].x += ax * A.x + bx * B.x + pui * C.x;
-      nt[0].y += ax * A.y + bx * B.y + pui * C.y;
-      nt[3].x += ay * A.x + by * B.x + pui * C.x;
-      nt[3].y += ay * A.y + by * B.y + pui * C.y;
-      nt[5].x += az * A.x + bz * B.x + pui * C.x;
-      nt[5].y += az * A.y + bz * B.y + pui * C.y;
-      const float pxy = pa * sx * sy, pxz = pa * sx * sz, pyz = pa * sy * sz;
-      nt[1] = cfma(pxy, D, nt[1]);
-      nt[2] = cfma(pxz, D, nt[2]);
-      nt[4] = cfma(pyz, D, nt[4]);
+      const float2 B = mc.B[m], C = mc.C[m], D = mc.D[m];
+      const float ax = pa * sx, ay = pa * sy, xx = ax * sx, yy = ay * sy, zz = pa * sz * sz;
+      mac(shared, xx + yy + zz, B);
+      mac(shared, pui, C);
+      mac(nt[0], xx, D);
+      mac(nt[3], yy, D);
+      mac(nt[5], zz, D);
+      mac(nt[1], ax * sy, D);
+      mac(nt[2], ax * sz, D);
+      mac(nt[4], ay * sz, D);
     }
   }
+  nt[0] = cadd(nt[0], shared), nt[3] = cadd(nt[3], shared), nt[5] = cadd(nt[5], shared);
 }
 
 template <int MORPH, bool CONV>
