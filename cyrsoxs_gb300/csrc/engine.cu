@@ -1088,7 +1088,7 @@ struct Plan {
   uint32_t first_mat = 0;               // the material whose fields come first (fields.cuh)
   uint32_t ebatch = 1;                  // energies per Ewald / rotation launch
   bool ewald_sparse = false;            // the combination coefficients keep their structural zeros
-  size_t off_fcoef = 0, off_kmag = 0, off_mat = 0, off_kvec = 0, off_first = 0;
+  size_t off_fcoef = 0, off_kmag = 0, off_mat = 0, off_kvec = 0, off_first = 0, off_ptrs = 0;
   uint32_t mom_zstep = 1, mom_ystep = 1;  // z planes and rows between the moment samples
 };
 
@@ -1470,6 +1470,8 @@ int make_plan(const cyr_options *o, const float *optical, Plan &pl) {
         }
     pl.off_fcoef = arena_put(pl.arena, fc.data(), fc.size());
     pl.off_first = arena_put(pl.arena, &pl.first_mat, 1);
+    const void *none[2] = {nullptr, nullptr};
+    pl.off_ptrs = arena_put(pl.arena, none, 2);  // the morphology's and the projection's address (RunMode::indirect)
     std::vector<float> km(pl.ne);
     for (uint32_t e = 0; e < pl.ne; ++e) {
       const float wavelength = static_cast<float>(1239.84197 / o->energies[e]);  // src/cudaMain.cu:607-608
@@ -1843,14 +1845,19 @@ void launch_ewald_fields(const FieldEwaldParams &fe, uint32_t nb, uint32_t nmat,
 // every energy (in batches) and k from them.
 int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan &pl, const unsigned char *dp,
                const float4 *d_vox, float *d_out, cudaStream_t st, size_t nsamp, const SlabUpload *up,
-               bool capturing) {
+               bool capturing, bool indirect) {
   const uint32_t npk = pl.npk;
+  // indirect: the morphology's and the projection's addresses are read from the arena
+  const float4 *const *vox_g = indirect ? reinterpret_cast<const float4 *const *>(dp + pl.off_ptrs) : nullptr;
+  float *const *out_g = indirect ? reinterpret_cast<float *const *>(dp + pl.off_ptrs + sizeof(void *)) : nullptr;
+  if (indirect) d_out = nullptr;
   CYR_TRY(sc.spec.ensure(size_t(npk) * pl.nvox * sizeof(float2)));
   CYR_TRY(sc.images.ensure(image_bytes(pl, pl.ebatch)));
   CYR_TRY(sc.avg.ensure(size_t(pl.ebatch) * pl.npix * sizeof(float)));
   float2 *spec = sc.spec.as<float2>();
   FieldParams fp{};
   fp.vox = d_vox;
+  fp.vox_g = vox_g;
   fp.nx = pl.nx, fp.ny = pl.ny, fp.nz = pl.nz, fp.nmat = pl.nmat;
   fp.first_g = reinterpret_cast<const uint32_t *>(dp + pl.off_first);
   fp.nvox = pl.nvox;
@@ -1969,10 +1976,10 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
       else
         launch_rotate<3, packed_energies<3>()>(rg, o->rot_mask != 0, st);
       ctx.prof.end(slot, st);
-      float *dst = d_out + (size_t(e0) * pl.nk + k) * pl.npix;
       slot = ctx.prof.begin(kWarp, st);
-      k_warp_out<<<dim3(pix_blocks, nb), 256, 0, st>>>(sc.avg.as<float>(), dst, W, H, pl.detector_warp[k], fillv,
-                                                       ostride);
+      k_warp_out<<<dim3(pix_blocks, nb), 256, 0, st>>>(sc.avg.as<float>(), d_out, out_g,
+                                                       (size_t(e0) * pl.nk + k) * pl.npix, W, H, pl.detector_warp[k],
+                                                       fillv, ostride);
       ctx.prof.end(slot, st);
       CYR_CUDA(cudaGetLastError());
     }
@@ -1995,6 +2002,9 @@ struct RunMode {
   const float *host_vox = nullptr;
   cudaStream_t copy_stream = nullptr;
   std::vector<cudaEvent_t> *event_pool = nullptr;  // reused slab events, or null: made per call
+  // FIELDS requests on device buffers whose addresses the arena holds (Plan::off_ptrs): a captured graph then serves
+  // every morphology and projection of its signature without staging copies
+  bool indirect = false;
 };
 
 
@@ -2077,6 +2087,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
   {
     MomentParams mp{};
     mp.vox = d_vox;
+    if (mode.indirect) mp.vox_g = reinterpret_cast<const float4 *const *>(dp + pl.off_ptrs);
     mp.nx = pl.nx, mp.ny = pl.ny, mp.nz = pl.nz, mp.nmat = pl.nmat;
     mp.nvox = pl.nvox;
     if (pl.hanning) {
@@ -2111,7 +2122,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
     ctx.prof.end(slot, st);
     CYR_CUDA(cudaGetLastError());
     if (pl.fields) {
-      CYR_TRY(run_fields(ctx, sc, o, pl, dp, d_vox, d_out, st, nsamp, slabs ? &upload : nullptr, mode.capturing));
+      CYR_TRY(run_fields(ctx, sc, o, pl, dp, d_vox, d_out, st, nsamp, slabs ? &upload : nullptr, mode.capturing, mode.indirect));
       // an event recorded inside a capture cannot be waited on outside it (slots keep order by their stream)
       if (!mode.capturing) CYR_CUDA(cudaEventRecord(sc.last_use, st));
       return CYR_OK;
@@ -2352,9 +2363,9 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
       }
       ctx.prof.end(slot, st);
       CYR_CUDA(cudaGetLastError());
-      float *dst = d_out + (size_t(e) * pl.nk + k) * pl.npix;
       slot = ctx.prof.begin(kWarp, st);
-      k_warp_out<<<pix_blocks, 256, 0, st>>>(avg, dst, W, H, pl.detector_warp[k],
+      k_warp_out<<<pix_blocks, 256, 0, st>>>(avg, d_out, nullptr, (size_t(e) * pl.nk + k) * pl.npix, W, H,
+                                             pl.detector_warp[k],
                                              o->rot_mask ? 0.f : std::numeric_limits<float>::quiet_NaN(), 0);
       ctx.prof.end(slot, st);
       CYR_CUDA(cudaGetLastError());
@@ -2677,6 +2688,8 @@ struct ServerRequest {
   const float4 *d_vox = nullptr;  // or device buffers
   float *d_out = nullptr;
   size_t vox_bytes = 0, out_bytes = 0, footprint = 0;
+  bool staged = false;    // runs on the slot's staging buffers
+  bool indirect = false;  // runs on the caller's device buffers through the arena (RunMode::indirect)
   std::string key;  // graph signature
   std::string group_key;  // requests with the same key may share launches (empty: never grouped)
   Plan plan;        // host plan (strategy resolved), made once at submit
@@ -2733,9 +2746,17 @@ constexpr double kSaturatingWork = 8.0e6;
 // two, concurrency only time-slices large requests and lengthens latency.
 constexpr double kMaxInflightWork = 2.0;
 
-int plan_request(ServerRequest &r, bool staged) {
+int plan_request(ServerRequest &r, bool graphs) {
   Plan &pl = r.plan;
   CYR_TRY(make_plan(&r.opt, r.optical.data(), pl));
+  // (a morphology that the kernels' 16-byte loads could not read in place is staged, as before)
+  r.indirect = graphs && r.d_vox && pl.fields && reinterpret_cast<uintptr_t>(r.d_vox) % sizeof(float4) == 0;
+  r.staged = r.h_vox != nullptr || (graphs && !r.indirect);
+  const bool staged = r.staged;
+  if (r.indirect) {
+    const void *ptrs[2] = {r.d_vox, r.d_out};
+    std::memcpy(pl.arena.data() + pl.off_ptrs, ptrs, sizeof ptrs);
+  }
   if (r.opt.strategy == CYR_STRATEGY_AUTO) r.opt.strategy = pl.fields ? CYR_STRATEGY_FIELDS : CYR_STRATEGY_PER_ENERGY;
   r.footprint = request_bytes(pl) + (staged ? r.vox_bytes + r.out_bytes : 0);
   r.work = std::min(1.0, double(pl.nvox) * pl.nmat / kSaturatingWork);
@@ -2745,8 +2766,9 @@ int plan_request(ServerRequest &r, bool staged) {
                 double(r.opt.end_angle), double(r.opt.increment_angle), double(r.opt.phys_size), r.opt.case_type,
                 r.opt.num_k, r.opt.morphology_type, r.opt.ewald_interpolation, r.opt.windowing,
                 r.opt.scatter_approach, r.opt.algorithm, r.opt.rot_mask, r.opt.reference_frame, r.opt.strategy,
-                staged ? 1u : 0u, double(r.opt.detector[0]), double(r.opt.detector[1]), double(r.opt.detector[2]),
-                staged ? nullptr : static_cast<const void *>(r.d_vox), staged ? nullptr : static_cast<void *>(r.d_out));
+                staged ? 1u : r.indirect ? 2u : 0u, double(r.opt.detector[0]), double(r.opt.detector[1]),
+                double(r.opt.detector[2]), staged || r.indirect ? nullptr : static_cast<const void *>(r.d_vox),
+                staged || r.indirect ? nullptr : static_cast<void *>(r.d_out));
   r.key = head;
   for (float e : r.energies) r.key += std::to_string(e) + ",";
   for (float k : r.kvecs) r.key += std::to_string(k) + ",";
@@ -2971,16 +2993,15 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
 }
 
 // Enqueues request r on slot sl (worker thread).
-// Host buffers always go through the slot's staging buffers; with graphs,
-// device buffers do too (device-to-device), so a signature does not depend on
-// the caller's pointers and one graph serves every morphology of a shape.
-bool staged_request(const Server &S, const ServerRequest &r) { return r.h_vox != nullptr || S.graphs; }
-
+// Host buffers go through the slot's staging buffers.  With graphs a signature
+// does not depend on the caller's pointers, so one graph serves every morphology
+// of a shape: FIELDS requests read their device buffers' addresses from the
+// arena; per-energy requests go through the staging buffers too (device-to-device).
 int start_request(Server &S, Slot &sl, ServerRequest &r) {
   cudaStream_t st = sl.stream;
   const float4 *d_vox = r.d_vox;
   float *d_out = r.d_out;
-  const bool staged = staged_request(S, r);
+  const bool staged = r.staged;
   if (staged) {
     CYR_TRY(sl.vox.ensure(r.vox_bytes));
     CYR_TRY(sl.out.ensure(r.out_bytes));
@@ -2995,6 +3016,7 @@ int start_request(Server &S, Slot &sl, ServerRequest &r) {
   mode.host_arena = sl.host_arena;
   mode.host_arena_bytes = sl.host_arena_bytes;
   mode.plan = &r.plan;
+  mode.indirect = r.indirect;
   auto git = S.graphs ? sl.graphs.find(r.key) : sl.graphs.end();
   if (git != sl.graphs.end() && git->second.generation == sl.generation()) {
     std::memcpy(sl.host_arena, pl.arena.data(), pl.arena.size());
@@ -3748,7 +3770,7 @@ int cyr_server_submit(cyr_server *s, const cyr_options *opt, const float *optica
     r->h_out = projection;
   }
   Server &S = *s->impl;
-  CYR_TRY(plan_request(*r, staged_request(S, *r)));
+  CYR_TRY(plan_request(*r, S.graphs));
   {
     std::lock_guard<std::mutex> lk(S.mu);
     r->id = S.next_id++;

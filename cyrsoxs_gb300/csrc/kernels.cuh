@@ -2240,15 +2240,16 @@ __global__ void k_warp_group(const float *__restrict__ src, float *const *__rest
 
 // Detector warp of a batch of angle averages (blockIdx.y): every pixel of dst
 // is written, the prefill where the source point falls outside, so no fill
-// pass runs before it (src/cudaMain.cu:916-960).
-__global__ void k_warp_out(const float *__restrict__ src, float *__restrict__ dst, int W, int H, WarpCoef c,
-                           float prefill, size_t dst_stride) {
+// pass runs before it (src/cudaMain.cu:916-960).  dst_g: where the projection's
+// pointer is read on the device (captured graphs), dst then being null.
+__global__ void k_warp_out(const float *__restrict__ src, float *__restrict__ dst, float *const *dst_g, size_t dst_off,
+                           int W, int H, WarpCoef c, float prefill, size_t dst_stride) {
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const size_t npix = size_t(W) * H;
   if (t >= npix) return;
   float v;
   if (!warp_sample(src + blockIdx.y * npix, W, H, c, int(t % W), int(t / W), v)) v = prefill;
-  dst[blockIdx.y * dst_stride + t] = v;
+  (dst_g ? *dst_g : dst)[dst_off + blockIdx.y * dst_stride + t] = v;
 }
 
 }  // namespace cyr
