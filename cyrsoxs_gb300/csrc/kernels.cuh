@@ -794,8 +794,8 @@ __global__ void __launch_bounds__(TX * 32, cols_min_blocks(V, TX)) k_fft_cols(Co
 // at chunk c ^ (r & 7)), so a warp reads its two columns 2w, 2w+1 as one
 // 16-byte chunk per line, eight lines per quarter-warp on eight distinct
 // chunks: no bank conflicts, and no load/store unit work for the tile copies
-// at all.  Each warp transforms its columns with the warp FFT through its own
-// exchange line.  Three forms:
+// at all.  Each warp transforms its columns with the warp FFT, exchanged in the
+// tile itself or through a line of its own.  Three forms:
 //  * k_fft_cols_tma: 8 warps, thread 0 issues the copies between tiles
 //    (256-point lines with nx a multiple of 16 but not of 32);
 //  * k_fft_cols_tma_ws<V, H, NST>: H 16-column halves per tile, NST tile
@@ -995,6 +995,79 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// The warp FFT of two columns of a swizzled TMA tile, exchanged in place.  The
+// warp's two columns are one 16-byte chunk of each 128-byte line, chunk
+// cw ^ (line & 7), and no other warp touches those chunks, so the tile itself is
+// the exchange buffer: an exchange moves both columns as one float4, and both
+// share each twiddle read.  Element p goes to line p ^ pair_mask(p >> 3): the
+// eight lanes of a quarter-warp then touch eight distinct chunks in every access
+// of the 128-, 256- and 512-point plans (identity lines would put stage 0's
+// stores, lines 4 or 8 apart, on one or two chunks).  pair_off, the byte offset
+// of element p, is linear over GF(2) in p.  Against a line of its own per warp
+// and one column after the other: 128-point lines 88 -> 84 us (128^3 x 14),
+// 256-point y lines 590 -> 585 us (256^3 x 14), masked z pass 1431 -> 1411 us.
+__host__ __device__ constexpr uint32_t pair_mask(uint32_t h) {  // h = p >> 3
+  return ((h & 1u) ? 1u : 0u) ^ ((h & 2u) ? 6u : 0u) ^ ((h & 4u) ? 4u : 0u);
+}
+__host__ __device__ constexpr uint32_t pair_off(uint32_t p) {
+  return (p << 7) ^ (pair_mask(p >> 3) << 7) ^ (((p & 7u) ^ pair_mask(p >> 3)) << 4);
+}
+
+template <int V, int R, int NS, bool LAST>
+__device__ __forceinline__ void pair_stage(float2 (&a)[V], float2 (&c)[V], unsigned char *tb, uint32_t cw,
+                                           const float2 *__restrict__ tw, uint32_t lane) {
+  constexpr int B = V / R;                                        // butterflies per lane
+  constexpr int TWOFF = NS > 1 ? NS - WarpPlan<V>::radix(0) : 0;  // this stage's table (warp_twiddles)
+#pragma unroll
+  for (int q = 0; q < B; ++q) {
+    const uint32_t j = lane + 32 * q;
+    const uint32_t k = j & (NS - 1);
+    float2 w[R], u[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) w[r] = a[q + r * B], u[r] = c[q + r * B];
+    if (NS > 1) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) {
+        const float2 t = tw[TWOFF + k * (R - 1) + r - 1];
+        w[r] = cmul(w[r], t), u[r] = cmul(u[r], t);
+      }
+    }
+    if (R == 2) dft2(w), dft2(u);
+    if (R == 4) dft4(w[0], w[1], w[2], w[3]), dft4(u[0], u[1], u[2], u[3]);
+    if (R == 8) dft8(w), dft8(u);
+    if (LAST) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) a[q + r * B] = w[r], c[q + r * B] = u[r];
+    } else {
+      const uint32_t base = pair_off((j / NS) * NS * R + k) ^ (cw << 4);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        *reinterpret_cast<float4 *>(tb + (base ^ pair_off(uint32_t(r) * NS))) = make_float4(w[r].x, w[r].y, u[r].x, u[r].y);
+    }
+  }
+  if (!LAST) {
+    __syncwarp();
+    const uint32_t base = pair_off(lane) ^ (cw << 4);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const float4 v = *reinterpret_cast<const float4 *>(tb + (base ^ pair_off(32u * i)));
+      a[i] = make_float2(v.x, v.y), c[i] = make_float2(v.z, v.w);
+    }
+    __syncwarp();
+  }
+}
+
+template <int V, int S, int NS>
+__device__ __forceinline__ void pair_fft_from(float2 (&a)[V], float2 (&c)[V], unsigned char *tb, uint32_t cw,
+                                              const float2 *tw, uint32_t lane) {
+  using P = WarpPlan<V>;
+  if constexpr (S < P::NSTAGES) {
+    constexpr int R = P::radix(S);
+    pair_stage<V, R, NS, S + 1 == P::NSTAGES>(a, c, tb, cw, tw, lane);
+    pair_fft_from<V, S + 1, NS * R>(a, c, tb, cw, tw, lane);
+  }
+}
+
 // Warp-specialised form: H halves of 16 columns per tile (each its own
 // swizzled N x 128-byte region), NST tile stages, 8 H compute warps (two
 // columns each) and a producer warp.  Per stage s: full[s] completes when a
@@ -1004,11 +1077,18 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 // compute warps never wait on the copies' shared-memory reads and never meet
 // at a block barrier.  With NST = 3 the loads run two tiles ahead of the
 // compute, which hides their latency when the stores are few (the masked z
-// pass).  Twiddles take N - R0 entries (warp_twiddles), so three stages of
+// pass).  That pass is bound by its stages' turn-round, of which issuing the
+// stores is the part the producer serialises: with the marked boxes issued by
+// one lane each instead of all by lane 0, it takes 1251 instead of 1411 us on
+// 512 x 512 x 256 x 14 (the boxes it moves take 1.05 ms at the copy rate).  Twiddles take N - R0 entries (warp_twiddles), so three stages of
 // 256-point, 32-column tiles fit the 227 KB a block may hold.
+// 512-point lines exchange through lines of their own: in the tile, with 64
+// registers of data, the y pass of 512 x 512 x 256 x 14 takes 2425 instead of 2388 us.
+__host__ __device__ constexpr bool cols_in_place(int v) { return v <= 8; }
+
 template <int V, int H, int NST>
 __host__ __device__ constexpr size_t cols_tma_ws_smem() {
-  return size_t(NST) * H * (32 * V) * kTmaCols * 8 + size_t(8 * H) * (32 * V) * 8 +
+  return size_t(NST) * H * (32 * V) * kTmaCols * 8 + (cols_in_place(V) ? 0 : size_t(8 * H) * (32 * V) * 8) +
          size_t(32 * V - WarpPlan<V>::radix(0)) * 8 + 16 * NST + 1024;
 }
 
@@ -1021,8 +1101,8 @@ __global__ void __launch_bounds__((8 * H + 1) * 32, 1) k_fft_cols_tma_ws(const _
   extern __shared__ unsigned char smem_raw[];
   unsigned char *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   float2 *tiles = reinterpret_cast<float2 *>(base);  // [NST][H][N][16], each half swizzled
-  float2 *lines = tiles + NST * TILE;                // [compute warps][N]
-  float2 *tws = lines + NW * N;                      // [N - R0]
+  float2 *lines = tiles + NST * TILE;                // [compute warps][N], unless cols_in_place
+  float2 *tws = lines + (cols_in_place(V) ? 0 : NW * N);  // [N - R0]
   uint64_t *full = reinterpret_cast<uint64_t *>(tws + (N - WarpPlan<V>::radix(0))), *empty = full + NST;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -1098,7 +1178,7 @@ __global__ void __launch_bounds__((8 * H + 1) * 32, 1) k_fft_cols_tma_ws(const _
       }
     }
   };
-  if (warp == NW) {  // producer: lane 0 issues the copies, the warp reads the mask words
+  if (warp == NW) {  // producer: lane 0 issues the loads and plain stores; masked stores are issued a box per lane
     auto store = [&](uint32_t t, uint32_t s, const uint32_t (&wm)[H][MW]) {
       if constexpr (!MASK) {
 #pragma unroll
@@ -1110,20 +1190,18 @@ __global__ void __launch_bounds__((8 * H + 1) * 32, 1) k_fft_cols_tma_ws(const _
             tma_store_4d(&tmap, c[0], c[1], c[2], c[3], region(s, h, b));
           }
       } else {
-        // the marked 8-plane boxes only: box g starts 8 g lines (g KB, a
-        // multiple of the swizzle's 1024-byte period) into the half
+        // the marked 8-plane boxes only, box 32 w + lane by each lane: box g
+        // starts 8 g lines (g KB, a multiple of the swizzle's 1024-byte period)
+        // into the half
 #pragma unroll
         for (uint32_t h = 0; h < H; ++h) {
           int c[4];
           coords(t, h, 0, c);
 #pragma unroll
           for (uint32_t w = 0; w < MW; ++w) {
-            uint32_t bits = wm[h][w];
-            while (bits) {
-              const uint32_t g = 32u * w + uint32_t(__ffs(int(bits)) - 1);
-              bits &= bits - 1u;
+            const uint32_t g = 32u * w + lane;
+            if ((wm[h][w] >> lane) & 1u)
               tma_store_4d(&smap, c[0], c[1], int(8 * g), c[3], region(s, h, 0) + g * 8 * kTmaCols);
-            }
           }
         }
       }
@@ -1139,23 +1217,25 @@ __global__ void __launch_bounds__((8 * H + 1) * 32, 1) k_fft_cols_tma_ws(const _
     for (int st = 0; st < NST; ++st) last[st] = -1, held[st] = 0;
     if (!MASK && lane != 0) return;  // without a mask lane 0 walks the tiles alone
     walk([&](uint32_t t, const uint32_t (&wt)[H][MW]) {
-        if (lane == 0) {
-          const uint32_t s = k % NST;
-          if (k >= NST) {  // the tile taken NST before occupies stage s: store it, let the store read it, then reload
-            ok = mbar_wait(&empty[s], (k / NST - 1) & 1u, limit);
-            if (ok) {
-              store(held[s], s, hwords[s]);
-              bulk_wait_read_all();
-            }
-          }
+        const uint32_t s = k % NST;
+        if (k >= NST) {  // the tile taken NST before occupies stage s: store it, let the store read it, then reload
+          ok = mbar_wait(&empty[s], (k / NST - 1) & 1u, limit);
+          if (MASK) ok = __all_sync(0xffffffffu, ok) != 0;
           if (ok) {
+            store(held[s], s, hwords[s]);
+            bulk_wait_read_all();
+          }
+          if (MASK) __syncwarp();  // every lane's boxes are read
+        }
+        if (ok) {
+          held[s] = t;
+#pragma unroll
+          for (uint32_t h = 0; h < H; ++h)
+#pragma unroll
+            for (uint32_t w = 0; w < MW; ++w) hwords[s][h][w] = wt[h][w];
+          last[s] = int(k);
+          if (lane == 0) {
             mbar_expect_tx(&full[s], TILE * 8 + p.extra_tx);
-            last[s] = int(k);
-            held[s] = t;
-#pragma unroll
-            for (uint32_t h = 0; h < H; ++h)
-#pragma unroll
-              for (uint32_t w = 0; w < MW; ++w) hwords[s][h][w] = wt[h][w];
 #pragma unroll
             for (uint32_t h = 0; h < H; ++h)
 #pragma unroll
@@ -1166,18 +1246,17 @@ __global__ void __launch_bounds__((8 * H + 1) * 32, 1) k_fft_cols_tma_ws(const _
               }
           }
         }
-        if (MASK) ok = __shfl_sync(0xffffffffu, ok, 0) != 0;
         ++k;
         return ok;
     });
-    if (lane != 0) return;
     // the last (up to) NST tiles
     for (uint32_t kk = k >= NST ? k - NST : 0u; ok && kk < k; ++kk) {
       const uint32_t s = kk % NST;
       ok = mbar_wait(&empty[s], (kk / NST) & 1u, limit);
+      if (MASK) ok = __all_sync(0xffffffffu, ok) != 0;
       if (ok) store(held[s], s, hwords[s]);
     }
-    if (!ok) {
+    if (!ok && lane == 0) {
       atomicOr(p.error, 1u);
       // the block must not release its shared memory under copies still landing
       for (int st = 0; st < NST; ++st)
@@ -1187,7 +1266,6 @@ __global__ void __launch_bounds__((8 * H + 1) * 32, 1) k_fft_cols_tma_ws(const _
     return;
   }
   // compute warps: warp w owns columns 2 (w % 8), 2 (w % 8) + 1 of half w / 8
-  float2 *line = lines + warp * N;
   const uint32_t cw = warp & 7u, hw = warp >> 3;
   const uint32_t limit = p.poll_limit ? p.poll_limit : kTmaWaitPolls;
   uint32_t k = 0;
@@ -1211,8 +1289,13 @@ __global__ void __launch_bounds__((8 * H + 1) * 32, 1) k_fft_cols_tma_ws(const _
         a[i] = make_float2(q.x, q.y);
         c2[i] = make_float2(q.z, q.w);
       }
-      warp_fft<V>(a, line, tws, lane);
-      warp_fft<V>(c2, line, tws, lane);
+      if constexpr (cols_in_place(V)) {
+        __syncwarp();  // every lane has read its lines before the exchanges write the tile
+        pair_fft_from<V, 0, 1>(a, c2, tb, cw, tws, lane);
+      } else {
+        warp_fft<V>(a, lines + warp * N, tws, lane);
+        warp_fft<V>(c2, lines + warp * N, tws, lane);
+      }
 #pragma unroll
       for (int i = 0; i < V; ++i) {
         const uint32_t r = lane + 32 * i;
