@@ -226,13 +226,16 @@ def algorithmic_bytes(kernel, w, nvol, nang, planes, batch=1, npk=0, energies=No
     pass moves the tiles and plane boxes of zmask_fractions (over `energies`, default the
     workload's)."""
     V, P, M = w.nvox, w.nx * w.ny, w.num_material
+    # the means' sample: every (nz / 16)-th plane, every row of it that 256 K points allow
+    ystep = max(1, min(w.ny // 16, (P * min(w.nz, 16)) >> 18))
+    moments = 16 * M * w.nx * math.ceil(w.ny / ystep) * math.ceil(w.nz / max(1, w.nz // 16))
     if npk:
         nq = 4 * (6 if nvol == 6 else 3)  # Gram bytes per pixel and energy (packed records)
         zload, zstore = zmask_fractions(w, w.energies if energies is None else energies)
         table = {
             "k_build_fields": (16 * M + 8 * npk) * V,
             "k_build_fields_rows": (16 * M + 8 * npk) * V,  # build fused with the x pass: one write
-            "k_moments": 16 * M * P * math.ceil(w.nz / max(1, w.nz // 16)),  # every (nz / 16)-th z plane
+            "k_moments": moments,
             "k_fft_rows": 2 * 8 * npk * V,
             "k_fft_cols<y>": 2 * 8 * npk * V,
             "k_fft_cols<z>": 8 * npk * V * (zload + zstore),
@@ -243,7 +246,6 @@ def algorithmic_bytes(kernel, w, nvol, nang, planes, batch=1, npk=0, energies=No
             "k_ewald_fields": batch * (4 * 8 * npk * P + nq * P),
             "k_rotate_gram": batch * (nq * P + 4 * P),
             "k_rotate_average": batch * (4 * nang * P + 4 * P),
-            "k_fill": batch * 4 * P,
             "k_warp": batch * 8 * P,
             "k_dc": 6 * 8 * npk,
         }
@@ -257,12 +259,11 @@ def algorithmic_bytes(kernel, w, nvol, nang, planes, batch=1, npk=0, energies=No
         "k_rotate_gram": nq * P + 4 * P,
         "k_build": (16 * M + 8 * nvol) * V,
         "k_build_fft_z": 16 * M * V + 8 * nvol * planes * P,
-        "k_moments": 16 * M * V,
+        "k_moments": moments,
         "k_mix_fft<x>": 2 * 8 * nvol * planes * P,
         "k_mix_fft<y>": 2 * 8 * nvol * planes * P,
         "k_mix_fft<z>": 2 * 8 * nvol * V,
         "k_rotate_average": 4 * nang * P + 4 * P,
-        "k_fill": 4 * P,
         "k_warp": 8 * P,
         "k_dc": 6 * 8 * nvol,
     }

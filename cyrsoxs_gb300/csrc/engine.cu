@@ -311,12 +311,12 @@ struct DeviceBuffer {
 // Optional per-launch timing: an event pair around every kernel launch,
 // read back after the caller has synchronised (cyr_profile_end).
 enum Stage {
-  kBuild = 0, kFftX, kFftY, kFftZ, kDc, kEwald, kRotate, kFill, kWarp, kMom, kMeans, kBuildZ,
+  kBuild = 0, kFftX, kFftY, kFftZ, kDc, kEwald, kRotate, kWarp, kMom, kMeans, kBuildZ,
   kFieldMeans, kBuildFields, kEwaldFields, kRotateGram, kFftRows, kFftColsY, kFftColsZ, kBluestein, kBuildFieldsRows,
   kZMask, kNumStages
 };
 const char *const kStageNames[kNumStages] = {"k_build", "k_mix_fft<x>", "k_mix_fft<y>", "k_mix_fft<z>", "k_dc",
-                                             "k_ewald_angles", "k_rotate_average", "k_fill", "k_warp",
+                                             "k_ewald_angles", "k_rotate_average", "k_warp",
                                              "k_moments", "k_entry_means", "k_build_fft_z",
                                              "k_field_means", "k_build_fields", "k_ewald_fields", "k_rotate_gram",
                                              "k_fft_rows", "k_fft_cols<y>", "k_fft_cols<z>", "k_bluestein",
@@ -1695,11 +1695,6 @@ int build_fields_x(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const 
   return fft_axes(ctx, spec + fp.i0, pl.nx, pl.ny, z1 - z0, npk, st, 0, 0, pl.nvox);
 }
 
-// Autotuning of the FIELDS transform for one shape (the first device-resident
-// request of it on this device): the fused or separate build + x pass and the
-// launch form of the y and z passes are each timed once on the packed-field
-// buffer, before the build overwrites every element of it, and the fastest
-// kept.  Every candidate computes the same numbers.
 // Ewald geometry of a FIELDS request (k_ewald_fields); kmag, kx, ky, kz are set per energy and k.
 EwaldGeom field_geometry(const cyr_options *o, const Plan &pl) {
   EwaldGeom g{};
@@ -1740,6 +1735,12 @@ int field_zmask(DeviceContext &ctx, Scratch &sc, const EwaldGeom &g, const float
   return CYR_OK;
 }
 
+// Autotuning of the FIELDS transform for one shape (the first device-resident
+// request of it on this device): the fused or separate build + x pass and the
+// launch form of the y and z passes each run twice on the packed-field buffer,
+// before the build overwrites every element of it.  The second runs are timed
+// (the first also loads the kernel's code) and the fastest kept.  Every
+// candidate computes the same numbers.
 int tune_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan &pl, const FieldParams &fp,
                 bool fused_ok, cudaStream_t st, DeviceContext::FieldTune &ft,
                 const uint32_t *zmask) {

@@ -1080,8 +1080,8 @@ __device__ __forceinline__ void pair_fft_from(float2 (&a)[V], float2 (&c)[V], un
 // pass).  That pass is bound by its stages' turn-round, of which issuing the
 // stores is the part the producer serialises: with the marked boxes issued by
 // one lane each instead of all by lane 0, it takes 1251 instead of 1411 us on
-// 512 x 512 x 256 x 14 (the boxes it moves take 1.05 ms at the copy rate).  Twiddles take N - R0 entries (warp_twiddles), so three stages of
-// 256-point, 32-column tiles fit the 227 KB a block may hold.
+// 512 x 512 x 256 x 14 (the boxes it moves take 1.05 ms at the copy rate).
+// Twiddles take N - R0 entries (warp_twiddles).
 // 512-point lines exchange through lines of their own: in the tile, with 64
 // registers of data, the y pass of 512 x 512 x 256 x 14 takes 2425 instead of 2388 us.
 __host__ __device__ constexpr bool cols_in_place(int v) { return v <= 8; }
