@@ -1824,8 +1824,8 @@ void launch_rotate(const RotateGramParams &rg, bool mask, cudaStream_t st) {
 }
 
 // k_ewald_fields for a basis of nb vectors (0: MATERIAL frame) and nmat materials with sparse coefficients (0: any).
-void launch_ewald_fields(const FieldEwaldParams &fe, uint32_t nb, uint32_t nmat, unsigned grid, size_t smem,
-                         cudaStream_t st) {
+void launch_ewald_fields(const FieldEwaldParams &fe, uint32_t nb, uint32_t nmat, unsigned grid, cudaStream_t st) {
+  const size_t smem = size_t(kEwaldEnergies) * 6 * fe.npk * (nmat > 0 ? sizeof(FieldCoef) : sizeof(float4));
   auto run = [&](auto two, auto one) {
     (fe.g.interp && !fe.g.twod ? two : one)<<<grid, kFieldEwaldThreads, smem, st>>>(fe);
   };
@@ -1931,7 +1931,6 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
   fe.nangles = pl.nang;
   fe.images = sc.images.as<float>();
   fe.gram = sc.images.as<float4>();
-  const size_t fsmem = size_t(kEwaldEnergies) * 6 * npk * sizeof(FieldCoef);
   const unsigned pix_blocks = unsigned((pl.npix + 255) / 256);
   const unsigned fpix_blocks = unsigned((pl.npix + 31) / 32);  // k_ewald_fields: 32 pixels per block
   const int W = int(pl.ny), H = int(pl.nx);  // the reference hands NPP width = Ny, height = Nx
@@ -1967,7 +1966,7 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
       slot = ctx.prof.begin(kEwaldFields, st);
       const unsigned fgrid = fpix_blocks * ((nb + kEwaldEnergies - 1) / kEwaldEnergies);
       const bool sparse = pl.ewald_sparse && ctx.sparse_ewald;
-      launch_ewald_fields(fe, pl.material_frame ? 0u : pl.nbasis, sparse ? pl.nmat : 0u, fgrid, fsmem, st);
+      launch_ewald_fields(fe, pl.material_frame ? 0u : pl.nbasis, sparse ? pl.nmat : 0u, fgrid, st);
       ctx.prof.end(slot, st);
       slot = ctx.prof.begin(pl.material_frame ? kRotate : kRotateGram, st);
       if (pl.material_frame)
@@ -2967,7 +2966,6 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   rg.W = W, rg.H = H;
   rg.nangles = p0.nang;
   rg.avg = sc.avg.as<float>();
-  const size_t fsmem = size_t(kEwaldEnergies) * 6 * npk * sizeof(FieldCoef);
   const unsigned fpix_blocks = unsigned((npix + 31) / 32), pix_blocks = unsigned((npix + 255) / 256);
   const float fillv = o->rot_mask ? 0.f : std::numeric_limits<float>::quiet_NaN();
   float *const *out_g = reinterpret_cast<float *const *>(dp + off_o);
@@ -2978,7 +2976,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     rg.nenergies = nb;
     int slot = ctx.prof.begin(kEwaldFields, st);
     const unsigned fgrid = fpix_blocks * ((nb + kEwaldEnergies - 1) / kEwaldEnergies);
-    launch_ewald_fields(fe, 2, sparse ? nmat : 0u, fgrid, fsmem, st);
+    launch_ewald_fields(fe, 2, sparse ? nmat : 0u, fgrid, st);
     ctx.prof.end(slot, st);
     slot = ctx.prof.begin(kRotateGram, st);
     launch_rotate<2, packed_energies<2>()>(rg, o->rot_mask != 0, st);

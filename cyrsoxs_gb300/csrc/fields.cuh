@@ -171,6 +171,21 @@ constexpr int kFieldGather = 4;  // packed volumes whose loads are issued togeth
 struct FieldCoef {
   float4 a, b;
 };
+__host__ __device__ __forceinline__ FieldCoef field_coef(float4 c) {  // c = (alpha, beta)
+  return FieldCoef{make_float4(c.x, c.x, -c.y, c.y), make_float4(c.z, -c.z, c.w, c.w)};
+}
+
+// A block's coefficients in shared memory: expanded for the material counts
+// walked at compile time (at most 12 KB), as (alpha, beta) for any other, up to
+// 42 KB with 32 materials, below the 48 KB that every launch may have.
+template <int MT>
+struct FieldStage {
+  using Coef = FieldCoef;
+};
+template <>
+struct FieldStage<0> {
+  using Coef = float4;
+};
 
 // NB = 2 or 3: LAB frame, Gram maps over the E basis (p(a) = sum_b E_b(a) Nt e_b),
 // rotated and averaged by k_rotate_gram.  NB = 0: any frame, p(a) = M(a) Nt per
@@ -191,7 +206,9 @@ __global__ void __launch_bounds__(kFieldEwaldThreads, NPL == 1 ? 8 : NB == 2 ? 5
   // a block: 32 pixels x kEwaldEnergies neighbouring energies, one warp per
   // energy, so the warps of an SM gather nearly the same sectors (their Ewald
   // spheres almost coincide) and share them in L1
-  extern __shared__ FieldCoef fcoef_all[];  // [kEwaldEnergies][6][npk]
+  using Coef = typename FieldStage<MT>::Coef;
+  extern __shared__ float4 fcoef_raw[];
+  Coef *fcoef_all = reinterpret_cast<Coef *>(fcoef_raw);  // [kEwaldEnergies][6][npk]
   const uint32_t ngrp = (p.nbatch + kEwaldEnergies - 1) / kEwaldEnergies;
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t eb = (blockIdx.x % ngrp) * kEwaldEnergies + warp, e = p.e0 + eb;
@@ -200,14 +217,17 @@ __global__ void __launch_bounds__(kFieldEwaldThreads, NPL == 1 ? 8 : NB == 2 ? 5
     const uint32_t w = i / (6 * p.npk), eg = (blockIdx.x % ngrp) * kEwaldEnergies + w;
     if (eg < p.nbatch) {
       const float4 c = p.coef[size_t(p.e0 + eg) * 6 * p.npk + i % (6 * p.npk)];
-      fcoef_all[i] = FieldCoef{make_float4(c.x, c.x, -c.y, c.y), make_float4(c.z, -c.z, c.w, c.w)};
+      if constexpr (MT > 0)
+        fcoef_all[i] = field_coef(c);
+      else
+        fcoef_all[i] = c;
     }
   }
   __syncthreads();
   if (eb >= p.nbatch) return;
   constexpr uint32_t NPKC = MT > 0 ? num_packed(uint32_t(MT)) : 0u;
   const uint32_t npk = MT > 0 ? NPKC : p.npk;
-  const FieldCoef *fcoef = fcoef_all + warp * 6 * npk;
+  const Coef *fcoef = fcoef_all + warp * 6 * npk;
   const size_t npix = size_t(nx) * ny;
   const size_t t = size_t(blockIdx.x / ngrp) * 32 + (threadIdx.x & 31);
   if (t >= npix) return;
@@ -286,7 +306,11 @@ __global__ void __launch_bounds__(kFieldEwaldThreads, NPL == 1 ? 8 : NB == 2 ? 5
 #pragma unroll
       for (int v = 0; v < 6; ++v) {
         if (MT > 0 && !coef_used(uint32_t(MT), v, j)) continue;
-        const FieldCoef c = fcoef[v * npk + j];
+        FieldCoef c;
+        if constexpr (MT > 0)
+          c = fcoef[v * npk + j];
+        else
+          c = field_coef(fcoef[v * npk + j]);
 #pragma unroll
         for (int pl = 0; pl < NPL; ++pl) {
           const float2 a = za[pl][q], b = zb[pl][q];
