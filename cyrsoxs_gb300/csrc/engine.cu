@@ -443,6 +443,7 @@ struct DeviceContext {
   };
   std::map<std::array<uint32_t, 3>, MixTables> mix;  // key: length, row form, bytes per real
   int sms = 0;                                       // multiprocessors
+  size_t max_pitch = 0;                              // bytes that the pitch of a 2D copy may have
   std::map<size_t, int> mix_build_occupancy;         // blocks per SM of k_build_fields_mix at a shared-memory size
   std::map<std::pair<const void *, size_t>, int> occupancy;  // blocks per SM of a kernel at a shared-memory size
   struct Fp64Scratch {
@@ -477,9 +478,12 @@ int get_context(DeviceContext **out) {
   if (!slot) {
     int sms = 0;
     CYR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int pitch = 0;
+    CYR_CUDA(cudaDeviceGetAttribute(&pitch, cudaDevAttrMaxPitch, dev));
     slot.reset(new DeviceContext);
     slot->device = dev;
     slot->sms = sms;
+    slot->max_pitch = size_t(pitch);
     const char *env = std::getenv("CYRSOXS_GB300_AUTOTUNE");
     slot->autotune = !(env && std::strcmp(env, "0") == 0);
     env = std::getenv("CYRSOXS_GB300_ZMASK");
@@ -1575,16 +1579,27 @@ struct SlabUpload {
   float4 *dev = nullptr;
   uint32_t nmat = 0, nz = 0;
   size_t nvox = 0, npix = 0;
+  size_t max_pitch = 0;  // of a 2D copy (2^31 - 1 bytes)
   cudaStream_t stream = nullptr;
-  // One copy per slab (the materials are the rows of a 2D copy): from pageable memory every copy call stages its
-  // data and waits, about 10 us beyond the transfer.  The first plane of a slab has come with the sample.
+  // `rows` runs of `width` bytes, `pitch` apart on both sides: one 2D copy where the pitch allows it, else a copy each
+  int copy(float4 *to, const float *from, size_t pitch, size_t width, size_t rows) {
+    if (rows == 1 || pitch > max_pitch) {
+      for (size_t r = 0; r < rows; ++r)
+        CYR_CUDA(cudaMemcpyAsync(reinterpret_cast<char *>(to) + r * pitch,
+                                 reinterpret_cast<const char *>(from) + r * pitch, width, cudaMemcpyHostToDevice, stream));
+      return CYR_OK;
+    }
+    CYR_CUDA(cudaMemcpy2DAsync(to, pitch, from, pitch, width, rows, cudaMemcpyHostToDevice, stream));
+    return CYR_OK;
+  }
+  // One copy per slab (the materials are the rows of a 2D copy, below 2^27 voxels): from pageable memory every copy
+  // call stages its data and waits, about 10 us beyond the transfer.  The first plane of a slab has come with the sample.
   int issue(uint32_t s) {  // queues the copies of slabs up to s
     for (; issued <= s && issued < count; ++issued) {
       const uint32_t z0 = issued * planes + (sample ? 1u : 0u), z1 = std::min(nz, (issued + 1) * planes);
       if (z1 > z0) {
         const size_t off = size_t(z0) * npix;  // float4 elements
-        CYR_CUDA(cudaMemcpy2DAsync(dev + off, nvox * sizeof(float4), host + 4 * off, nvox * sizeof(float4),
-                                   size_t(z1 - z0) * npix * sizeof(float4), nmat, cudaMemcpyHostToDevice, stream));
+        CYR_TRY(copy(dev + off, host + 4 * off, nvox * sizeof(float4), size_t(z1 - z0) * npix * sizeof(float4), nmat));
       }
       cudaEvent_t ev = nullptr;
       CYR_TRY(next_event(&ev));
@@ -1596,8 +1611,7 @@ struct SlabUpload {
   int issue_sample() {
     const size_t pitch = size_t(planes) * npix * sizeof(float4);
     for (uint32_t m = 0; m < nmat; ++m)
-      CYR_CUDA(cudaMemcpy2DAsync(dev + size_t(m) * nvox, pitch, host + 4 * size_t(m) * nvox, pitch,
-                                 npix * sizeof(float4), count, cudaMemcpyHostToDevice, stream));
+      CYR_TRY(copy(dev + size_t(m) * nvox, host + 4 * size_t(m) * nvox, pitch, npix * sizeof(float4), count));
     CYR_TRY(next_event(&sample));
     CYR_CUDA(cudaEventRecord(sample, stream));
     return CYR_OK;
@@ -2061,6 +2075,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
     upload.host = mode.host_vox;
     upload.dev = const_cast<float4 *>(d_vox);
     upload.nmat = pl.nmat, upload.nz = pl.nz, upload.nvox = pl.nvox, upload.npix = pl.npix;
+    upload.max_pitch = ctx.max_pitch;
     // slabs: after the last one lands, its fields and x/y passes are still ahead
     // of the z pass, so thinner slabs shorten that tail, but each costs a copy
     // call and launches of few blocks: at least kSlabBytes a slab, 16 at most
