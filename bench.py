@@ -226,9 +226,10 @@ def algorithmic_bytes(kernel, w, nvol, nang, planes, batch=1, npk=0, energies=No
     pass moves the tiles and plane boxes of zmask_fractions (over `energies`, default the
     workload's)."""
     V, P, M = w.nvox, w.nx * w.ny, w.num_material
-    # the means' sample: every (nz / 16)-th plane, every row of it that 256 K points allow
-    ystep = max(1, min(w.ny // 16, (P * min(w.nz, 16)) >> 18))
-    moments = 16 * M * w.nx * math.ceil(w.ny / ystep) * math.ceil(w.nz / max(1, w.nz // 16))
+    # the means' sample: whole rows, about 256 K points of each material
+    mean_rows = max(64, (1 << 18) // w.nx)
+    step = max(1, (w.ny * w.nz + mean_rows // 2) // mean_rows)
+    moments = 16 * M * w.nx * math.ceil(w.ny * w.nz / step)
     if npk:
         nq = 4 * (6 if nvol == 6 else 3)  # Gram bytes per pixel and energy (packed records)
         zload, zstore = zmask_fractions(w, w.energies if energies is None else energies)

@@ -1062,6 +1062,8 @@ int fft3d(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, uint32_t n
 // ---------------------------------------------------------------------------
 // Request planning
 // ---------------------------------------------------------------------------
+constexpr uint32_t kMeanPoints = 1u << 18;  // voxels per material that the field means are taken from
+
 struct Plan {
   uint32_t nx, ny, nz, nmat, ne, nk, nang;
   size_t nvox, npix;
@@ -1093,7 +1095,7 @@ struct Plan {
   uint32_t ebatch = 1;                  // energies per Ewald / rotation launch
   bool ewald_sparse = false;            // the combination coefficients keep their structural zeros
   size_t off_fcoef = 0, off_kmag = 0, off_mat = 0, off_kvec = 0, off_first = 0, off_ptrs = 0;
-  uint32_t mom_zstep = 1, mom_ystep = 1;  // z planes and rows between the moment samples
+  uint32_t mom_step = 1;                // rows of the volume per row sampled for the means
 };
 
 // Energies per Gram record: the FIELDS strategy packs 12 floats per pixel (4
@@ -1415,8 +1417,9 @@ int make_plan(const cyr_options *o, const float *optical, Plan &pl) {
     const uint32_t eb = (pl.ne + nbatches - 1) / nbatches;
     pl.ebatch = nbatches == 1 ? pl.ne : std::min(pl.ne, (eb + nep - 1) / nep * nep);
   }
-  pl.mom_zstep = std::max(1u, pl.nz / 16);  // 16 sampled planes, 256 K points in all (at least 16 rows of a plane)
-  pl.mom_ystep = std::max<uint32_t>(1, std::min<uint32_t>(pl.ny / 16, uint32_t(pl.npix * std::min(pl.nz, 16u) >> 18)));
+  // whole rows, kMeanPoints voxels of each material in all (every row up to one and a half times that)
+  const uint32_t mean_rows = std::max<uint32_t>(64, kMeanPoints / pl.nx);
+  pl.mom_step = std::max<uint32_t>(1, (pl.ny * pl.nz + mean_rows / 2) / mean_rows);
   if (pl.fields) {
     // coef[e][v][j] = (alpha, beta): Nt_v(k) = sum_j alpha Z_j(k) + beta conj Z_j(-k), where
     // Z_j = F_2j + i F_2j+1 and field g = 7 m + f of the m-th material walked (f: u_x^2 u_y^2 u_z^2 u_xu_y u_xu_z u_yu_z phi_ui), T in the place of
@@ -2112,14 +2115,14 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
     }
     mp.out = sc.moments();
     mp.conv = convert ? sc.conv.as<float4>() : nullptr;
-    // the conversion needs every voxel; the means alone need only a subsample of planes
+    // the conversion needs every voxel; the means alone need only a sample of rows
     // (with a slab upload: the planes copied first for that purpose)
-    mp.zstep = convert ? 1u : pl.mom_zstep;
-    mp.ystep = convert ? 1u : pl.mom_ystep;
+    mp.step = convert ? 1u : pl.mom_step;
+    mp.rows = (pl.ny * pl.nz + mp.step - 1) / mp.step;
     if (slabs && upload.sample) {
-      mp.zstep = upload.planes;
+      mp.chunk = pl.ny, mp.step = upload.planes * pl.ny, mp.rows = upload.count * pl.ny;
       CYR_CUDA(cudaStreamWaitEvent(st, upload.sample, 0));
-    } else if (slabs) {  // few slabs: the means wait for the whole volume, whose planes they sample as ever
+    } else if (slabs) {  // few slabs: the means wait for the whole volume, whose rows they sample as ever
       CYR_TRY(upload.issue(upload.count - 1));
       CYR_CUDA(cudaStreamWaitEvent(st, upload.events.back(), 0));
     }
@@ -2127,7 +2130,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
     const int nsm = ctx.sms;
     // about 8 samples per thread: small volumes get few blocks (each block ends in
     // kMoments double atomics on the same addresses), large ones 4 per SM
-    const size_t nsamp = size_t(pl.nx) * ((pl.ny + mp.ystep - 1) / mp.ystep) * ((pl.nz + mp.zstep - 1) / mp.zstep);
+    const size_t nsamp = size_t(pl.nx) * mp.rows;
     const dim3 grid(uint32_t(std::max<size_t>(1, std::min<size_t>((nsamp + 2047) / 2048, size_t(nsm) * 4))), pl.nmat);
     int slot = ctx.prof.begin(kMom, st);
     if (o->morphology_type == 0)
@@ -2882,7 +2885,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   float2 *spec = sc.spec.as<float2>();
   const int sms = ctx.sms;
   const float4 *const *vox_g = reinterpret_cast<const float4 *const *>(dp + off_v);
-  // moments of every request (blockIdx.z = request), over the z-plane subsample
+  // moments of every request (blockIdx.z = request), over a sample of rows
   MomentParams mp{};
   mp.vox_g = vox_g;
   mp.nx = p0.nx, mp.ny = p0.ny, mp.nz = p0.nz, mp.nmat = nmat;
@@ -2893,8 +2896,8 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     mp.hann_z = reinterpret_cast<const float *>(dp + p0.off_hz);
   }
   mp.out = sc.moments();
-  mp.zstep = p0.mom_zstep, mp.ystep = p0.mom_ystep;
-  const size_t nsamp = size_t(p0.nx) * ((p0.ny + mp.ystep - 1) / mp.ystep) * ((p0.nz + mp.zstep - 1) / mp.zstep);
+  mp.step = p0.mom_step, mp.rows = (p0.ny * p0.nz + mp.step - 1) / mp.step;
+  const size_t nsamp = size_t(p0.nx) * mp.rows;
   {
     const dim3 grid(uint32_t(std::max<size_t>(1, std::min<size_t>((nsamp + 2047) / 2048, size_t(sms) * 4))), nmat, G);
     const int slot = ctx.prof.begin(kMom, st);

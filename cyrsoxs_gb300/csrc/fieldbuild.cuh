@@ -40,8 +40,8 @@ constexpr uint32_t kMaxPacked = num_packed(kMaxMaterials);
 // Field means from the per-material moments (k_moments over nsamp voxels), T
 // last, computed by the calling block.  Any constant subtracted from a field
 // changes only bin 0, which is replaced, so the means need only be close (a
-// z-plane subsample suffices); they keep the FP32 rounding of the transform
-// proportional to the fluctuations.
+// sample of rows from all over the volume, sample_row); they keep the FP32
+// rounding of the transform proportional to the fluctuations.
 __device__ __forceinline__ uint32_t walked_material(uint32_t m, uint32_t first, uint32_t nmat) {
   return m + first < nmat ? m + first : m + first - nmat;
 }

@@ -122,10 +122,27 @@ struct MomentParams {
   double *out;      // [nmat][kMoments], accumulated
   float4 *conv;     // Euler only: (sqrt(phi_a) s, phi_ui) per material and voxel, or null
   unsigned *neg;    // set when some phi_a < 0
-  // sample every ystep-th row of every zstep-th z plane (1: all; must be 1 with conv).  The sums only have to give
-  // a constant near the mean: 16 planes of about 16 K points each leave a residual far below the strongest bins
-  uint32_t ystep, zstep;
+  // The rows sampled, `rows` of the ny nz rows of the volume (with conv: all of them, step 1).  chunk = 0: one row of
+  // every `step`, at a place drawn by a hash; chunk > 0: runs of `chunk` rows, `step` rows apart (sample_row).
+  uint32_t rows, step, chunk;
 };
+
+// The volume row (z ny + y) of sampled row r.  The sums only have to give a
+// constant near the mean, but near it for every structure: whole rows average
+// what varies along x, every plane gives about ny / step of them, so a layer
+// counts as much as it holds, and the place inside each run of `step` rows is
+// drawn by a hash (Marsaglia's xorshift of a multiplicative one), so a grating
+// along y is met at every phase, whatever its pitch.  256 K points leave a
+// residual below a tenth of the fluctuations, which the rounding of the
+// transform, proportional to the root of their squares' sum, does not show.
+__device__ __forceinline__ uint32_t sample_row(uint32_t r, uint32_t step, uint32_t chunk, uint32_t total) {
+  if (chunk) return r / chunk * step + r % chunk;
+  if (step == 1) return r;
+  uint32_t h = (r + 1u) * 0x9e3779b9u;
+  h ^= h << 13, h ^= h >> 17, h ^= h << 5;
+  const uint32_t first = r * step;
+  return first + __umulhi(h * 0x9e3779b9u, min(step, total - first));
+}
 
 template <int MORPH>
 __global__ void __launch_bounds__(256) k_moments(MomentParams p) {
@@ -140,11 +157,10 @@ __global__ void __launch_bounds__(256) k_moments(MomentParams p) {
   float acc[kMoments];
 #pragma unroll
   for (int q = 0; q < kMoments; ++q) acc[q] = 0.f;
-  // samples: the rows y = 0, ystep, 2 ystep, ... of the planes z = 0, zstep,
-  // 2 zstep, ..., whole rows, so that a warp's loads stay contiguous; the
-  // thread's (row, x) position advances by the grid stride
+  // whole rows, so that a warp's loads stay contiguous; the thread's (sampled
+  // row, x) position advances by the grid stride
   const uint32_t stride = gridDim.x * blockDim.x, srow = stride / p.nx, sx0 = stride % p.nx;
-  const uint32_t nys = (p.ny + p.ystep - 1) / p.ystep, rows = nys * ((p.nz + p.zstep - 1) / p.zstep);
+  const uint32_t total = p.ny * p.nz, rows = p.rows;
   const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t row = first / p.nx, x = first % p.nx;
   for (; row < rows; row += srow, x += sx0) {
@@ -152,8 +168,8 @@ __global__ void __launch_bounds__(256) k_moments(MomentParams p) {
       x -= p.nx;
       if (++row >= rows) break;
     }
-    const uint32_t zi = row / nys, y = (row - zi * nys) * p.ystep, z = zi * p.zstep;
-    const size_t i = (size_t(z) * p.ny + y) * p.nx + x;
+    const uint32_t at = sample_row(row, p.step, p.chunk, total);
+    const size_t i = size_t(at) * p.nx + x;
     float sx, sy, sz, pa, pui;
     director<MORPH>(__ldg(&p.vox[m * p.nvox + i]), sx, sy, sz, pa, pui);
     if (MORPH == 0 && p.conv) {
@@ -162,7 +178,7 @@ __global__ void __launch_bounds__(256) k_moments(MomentParams p) {
       p.conv[m * p.nvox + i] = make_float4(r * sx, r * sy, r * sz, pui);
     }
     float w = 1.f;
-    if (p.hann_x) w = p.hann_x[x] * p.hann_y[y] * p.hann_z[z];
+    if (p.hann_x) w = p.hann_x[x] * p.hann_y[at % p.ny] * p.hann_z[at / p.ny];
     const float wa = w * pa;
     acc[0] += wa * sx * sx;
     acc[1] += wa * sy * sy;
