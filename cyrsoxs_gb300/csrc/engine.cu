@@ -47,6 +47,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <numeric>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -371,6 +372,7 @@ struct Scratch {
   // from kMomentsAt on, the moment sums
   DeviceBuffer errors;
   DeviceBuffer zmask;              // store mask of the FIELDS z pass (k_zmask)
+  DeviceBuffer sample;             // rows of a host morphology that the means are taken from (SlabUpload)
   cudaEvent_t last_use = nullptr;  // completion of the last request that used it
   uint64_t generation = 0;         // bumped by every (re)allocation of a buffer above
   static constexpr size_t kMomentsAt = 256;
@@ -388,11 +390,11 @@ struct Scratch {
   }
   // serving slots: stream-ordered allocations on `st`
   void bind(cudaStream_t st) {
-    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &means, &errors, &conv, &zmask})
+    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &means, &errors, &conv, &zmask, &sample})
       b->stream = st, b->generation = &generation;
   }
   void release() {
-    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &means, &errors, &conv, &zmask})
+    for (DeviceBuffer *b : {&spec, &images, &avg, &params, &dc, &means, &errors, &conv, &zmask, &sample})
       b->release();
   }
 };
@@ -1576,7 +1578,9 @@ struct SlabUpload {
     CYR_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
     return CYR_OK;
   }
-  // the first plane of every slab, copied first for the means (a sample spread over the volume)
+  // Rows copied ahead of the slabs, for the means: `rows` of them, `step` apart (sample_row), packed in a buffer of
+  // their own, which the first kernel waits for instead of the volume: 1/32 of it, at least 64 K points a material.
+  uint32_t rows = 0, step = 0;
   cudaEvent_t sample = nullptr;
   const float *host = nullptr;
   float4 *dev = nullptr;
@@ -1584,26 +1588,25 @@ struct SlabUpload {
   size_t nvox = 0, npix = 0;
   size_t max_pitch = 0;  // of a 2D copy (2^31 - 1 bytes)
   cudaStream_t stream = nullptr;
-  // `rows` runs of `width` bytes, `pitch` apart on both sides: one 2D copy where the pitch allows it, else a copy each
-  int copy(float4 *to, const float *from, size_t pitch, size_t width, size_t rows) {
-    if (rows == 1 || pitch > max_pitch) {
+  // `rows` runs of `width` bytes, their starts tp bytes apart at `to` and fp at `from`: one 2D copy where the pitches
+  // allow it, else a copy each
+  int copy(float4 *to, size_t tp, const float *from, size_t fp, size_t width, size_t rows) {
+    if (rows == 1 || std::max(tp, fp) > max_pitch) {
       for (size_t r = 0; r < rows; ++r)
-        CYR_CUDA(cudaMemcpyAsync(reinterpret_cast<char *>(to) + r * pitch,
-                                 reinterpret_cast<const char *>(from) + r * pitch, width, cudaMemcpyHostToDevice, stream));
+        CYR_CUDA(cudaMemcpyAsync(reinterpret_cast<char *>(to) + r * tp, reinterpret_cast<const char *>(from) + r * fp,
+                                 width, cudaMemcpyHostToDevice, stream));
       return CYR_OK;
     }
-    CYR_CUDA(cudaMemcpy2DAsync(to, pitch, from, pitch, width, rows, cudaMemcpyHostToDevice, stream));
+    CYR_CUDA(cudaMemcpy2DAsync(to, tp, from, fp, width, rows, cudaMemcpyHostToDevice, stream));
     return CYR_OK;
   }
   // One copy per slab (the materials are the rows of a 2D copy, below 2^27 voxels): from pageable memory every copy
-  // call stages its data and waits, about 10 us beyond the transfer.  The first plane of a slab has come with the sample.
+  // call stages its data and waits, about 10 us beyond the transfer.
   int issue(uint32_t s) {  // queues the copies of slabs up to s
     for (; issued <= s && issued < count; ++issued) {
-      const uint32_t z0 = issued * planes + (sample ? 1u : 0u), z1 = std::min(nz, (issued + 1) * planes);
-      if (z1 > z0) {
-        const size_t off = size_t(z0) * npix;  // float4 elements
-        CYR_TRY(copy(dev + off, host + 4 * off, nvox * sizeof(float4), size_t(z1 - z0) * npix * sizeof(float4), nmat));
-      }
+      const uint32_t z0 = issued * planes, z1 = std::min(nz, z0 + planes);
+      const size_t off = size_t(z0) * npix, pitch = nvox * sizeof(float4);  // off: float4 elements
+      CYR_TRY(copy(dev + off, pitch, host + 4 * off, pitch, size_t(z1 - z0) * npix * sizeof(float4), nmat));
       cudaEvent_t ev = nullptr;
       CYR_TRY(next_event(&ev));
       events.push_back(ev);
@@ -1611,10 +1614,37 @@ struct SlabUpload {
     }
     return CYR_OK;
   }
-  int issue_sample() {
-    const size_t pitch = size_t(planes) * npix * sizeof(float4);
+  // The rows' distance, about total / want: every plane gets its share of them, and they must also spread along y from
+  // plane to plane.  So the step is coprime to ny, and among the first 32 such between 3/4 and 3/2 of the quotient it is
+  // the one whose multiples spread best modulo ny: the smallest partial quotients of step / ny, as far as the
+  // denominators stay below the number of rows.
+  static uint32_t row_step(uint32_t ny, uint32_t total, uint32_t want) {
+    const uint32_t top = std::max(1u, total / want), low = std::max(1u, top / 4 * 3 + top % 4 * 3 / 4);
+    uint32_t best = 0, least = 0;
+    for (uint32_t s = low; s < low + 32 && s <= top + top / 2; ++s) {
+      if (std::gcd(s, ny) != 1) continue;
+      const uint32_t count = (total - 1) / s + 1;
+      uint32_t a = s % ny, b = ny, q = 0, d0 = 0, d1 = 1;  // d1: denominator of the last convergent of (s mod ny) / ny
+      for (uint32_t i = 0; a != 0; ++i) {
+        const uint32_t p = b / a, r = b % a;
+        const uint64_t d = d0 + uint64_t(p) * d1;
+        if (i > 0 || s > ny) q = std::max(q, p);
+        if (d > count) break;
+        b = a, a = r, d0 = d1, d1 = uint32_t(d);
+      }
+      if (best == 0 || q < least) best = s, least = q;
+    }
+    return best ? best : top;
+  }
+  int issue_sample(DeviceBuffer &buf, uint32_t nx, uint32_t ny) {
+    const uint32_t total = ny * nz;
+    const uint32_t want = std::max<uint32_t>(64, std::max<uint32_t>(1u << 16, uint32_t(nvox / 32)) / nx);
+    step = row_step(ny, total, std::max(1u, std::min(want, total / 8)));
+    rows = (total - 1) / step + 1;
+    const size_t row = size_t(nx) * sizeof(float4);
+    CYR_TRY(buf.ensure(nmat * rows * row));
     for (uint32_t m = 0; m < nmat; ++m)
-      CYR_TRY(copy(dev + size_t(m) * nvox, host + 4 * size_t(m) * nvox, pitch, npix * sizeof(float4), count));
+      CYR_TRY(copy(buf.as<float4>() + size_t(m) * rows * nx, row, host + 4 * size_t(m) * nvox, step * row, row, rows));
     CYR_TRY(next_event(&sample));
     CYR_CUDA(cudaEventRecord(sample, stream));
     return CYR_OK;
@@ -2031,7 +2061,7 @@ struct RunMode {
 // exchanges hide it), 32 of 403 with other z lengths (x 90).
 constexpr size_t kConvertBuildsWarp = 64, kConvertBuilds = 6;
 constexpr size_t kSlabBytes = size_t(24) << 20;
-constexpr uint32_t kSampleSlabs = 2;  // slabs from which the means come from the planes copied first
+constexpr uint32_t kSampleSlabs = 2;  // slabs from which the means come from rows copied ahead of them
 
 int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const float *optical, const float4 *d_vox,
                 float *d_out, cudaStream_t st, const RunMode &mode = RunMode()) {
@@ -2087,7 +2117,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
     upload.planes = (pl.nz + upload.count - 1) / upload.count;
     upload.count = (pl.nz + upload.planes - 1) / upload.planes;
     if (pl.fields) {
-      if (upload.count >= kSampleSlabs) CYR_TRY(upload.issue_sample());
+      if (upload.count >= kSampleSlabs) CYR_TRY(upload.issue_sample(sc.sample, pl.nx, pl.ny));
       CYR_TRY(upload.issue(0));
     } else {
       CYR_TRY(upload.issue(upload.count - 1));
@@ -2116,11 +2146,12 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
     mp.out = sc.moments();
     mp.conv = convert ? sc.conv.as<float4>() : nullptr;
     // the conversion needs every voxel; the means alone need only a sample of rows
-    // (with a slab upload: the planes copied first for that purpose)
+    // (with a slab upload: the rows copied first for that purpose)
     mp.step = convert ? 1u : pl.mom_step;
     mp.rows = (pl.ny * pl.nz + mp.step - 1) / mp.step;
     if (slabs && upload.sample) {
-      mp.chunk = pl.ny, mp.step = upload.planes * pl.ny, mp.rows = upload.count * pl.ny;
+      mp.even = 1, mp.step = upload.step, mp.rows = upload.rows;
+      mp.packed = sc.sample.as<float4>();
       CYR_CUDA(cudaStreamWaitEvent(st, upload.sample, 0));
     } else if (slabs) {  // few slabs: the means wait for the whole volume, whose rows they sample as ever
       CYR_TRY(upload.issue(upload.count - 1));

@@ -122,9 +122,10 @@ struct MomentParams {
   double *out;      // [nmat][kMoments], accumulated
   float4 *conv;     // Euler only: (sqrt(phi_a) s, phi_ui) per material and voxel, or null
   unsigned *neg;    // set when some phi_a < 0
-  // The rows sampled, `rows` of the ny nz rows of the volume (with conv: all of them, step 1).  chunk = 0: one row of
-  // every `step`, at a place drawn by a hash; chunk > 0: runs of `chunk` rows, `step` rows apart (sample_row).
-  uint32_t rows, step, chunk;
+  // The rows sampled, `rows` of the ny nz rows of the volume (with conv: all of them, step 1): one row of every `step`,
+  // the first (even) or one drawn by a hash (sample_row).
+  uint32_t rows, step, even;
+  const float4 *packed;  // [nmat][rows][nx]: the sampled rows themselves, or null (read from vox)
 };
 
 // The volume row (z ny + y) of sampled row r.  The sums only have to give a
@@ -135,9 +136,10 @@ struct MomentParams {
 // along y is met at every phase, whatever its pitch.  256 K points leave a
 // residual below a tenth of the fluctuations, which the rounding of the
 // transform, proportional to the root of their squares' sum, does not show.
-__device__ __forceinline__ uint32_t sample_row(uint32_t r, uint32_t step, uint32_t chunk, uint32_t total) {
-  if (chunk) return r / chunk * step + r % chunk;
-  if (step == 1) return r;
+// Rows of a host morphology come in one strided copy, so they are evenly
+// spaced, `step` chosen for their spread along y (SlabUpload::row_step).
+__device__ __forceinline__ uint32_t sample_row(uint32_t r, uint32_t step, uint32_t even, uint32_t total) {
+  if (even || step == 1) return r * step;
   uint32_t h = (r + 1u) * 0x9e3779b9u;
   h ^= h << 13, h ^= h >> 17, h ^= h << 5;
   const uint32_t first = r * step;
@@ -168,10 +170,11 @@ __global__ void __launch_bounds__(256) k_moments(MomentParams p) {
       x -= p.nx;
       if (++row >= rows) break;
     }
-    const uint32_t at = sample_row(row, p.step, p.chunk, total);
+    const uint32_t at = sample_row(row, p.step, p.even, total);
     const size_t i = size_t(at) * p.nx + x;
+    const float4 *v = p.packed ? p.packed + (size_t(m) * rows + row) * p.nx + x : p.vox + m * p.nvox + i;
     float sx, sy, sz, pa, pui;
-    director<MORPH>(__ldg(&p.vox[m * p.nvox + i]), sx, sy, sz, pa, pui);
+    director<MORPH>(__ldg(v), sx, sy, sz, pa, pui);
     if (MORPH == 0 && p.conv) {
       if (pa < 0.f) atomicOr(p.neg, 1u);
       const float r = sqrtf(fmaxf(pa, 0.f));
