@@ -16,7 +16,7 @@
 //   k_build -> 3D FFT -> k_dc -> per k: k_ewald_angles ->
 //   k_rotate_gram -> k_warp_out (detector) -> projection[e][k]
 //
-// FIELDS strategy (fields.cuh): the spectra of the 7 M energy independent
+// FIELDS strategy (fields.cuh): the spectra of the 7 M + 1 energy independent
 // morphology fields are formed once per request; every energy and angle is
 // combined from them inside the Ewald kernel, batched over energies:
 //
@@ -1093,10 +1093,9 @@ struct Plan {
   // FIELDS strategy
   bool fields = false;
   uint32_t npk = 0;                     // packed field volumes
-  uint32_t first_mat = 0;               // the material whose fields come first (fields.cuh)
   uint32_t ebatch = 1;                  // energies per Ewald / rotation launch
   bool ewald_sparse = false;            // the combination coefficients keep their structural zeros
-  size_t off_fcoef = 0, off_kmag = 0, off_mat = 0, off_kvec = 0, off_first = 0, off_ptrs = 0;
+  size_t off_fcoef = 0, off_kmag = 0, off_mat = 0, off_kvec = 0, off_ptrs = 0;
   uint32_t mom_step = 1;                // rows of the volume per row sampled for the means
 };
 
@@ -1424,35 +1423,24 @@ int make_plan(const cyr_options *o, const float *optical, Plan &pl) {
   pl.mom_step = std::max<uint32_t>(1, (pl.ny * pl.nz + mean_rows / 2) / mean_rows);
   if (pl.fields) {
     // coef[e][v][j] = (alpha, beta): Nt_v(k) = sum_j alpha Z_j(k) + beta conj Z_j(-k), where
-    // Z_j = F_2j + i F_2j+1 and field g = 7 m + f of the m-th material walked (f: u_x^2 u_y^2 u_z^2 u_xu_y u_xu_z u_yu_z phi_ui), T in the place of
-    // the last phi_ui
+    // Z_j = F_2j + i F_2j+1 and field g = 7 m + f (f: u_x^2 u_y^2 u_z^2 u_xu_y u_xu_z u_yu_z phi_ui), T last
     const uint32_t nf = num_fields(pl.nmat), npk = pl.npk;
     std::vector<float4> fc(size_t(pl.ne) * 6 * npk);
     std::vector<std::complex<double>> c(size_t(6) * 2 * npk);
-    // the material walked last gives the common part R = C: the one that leaves the smallest coefficients
-    double least = 0.0;
-    for (uint32_t l = 0; l < pl.nmat; ++l) {
-      double rest = 0.0;
-      for (uint32_t e = 0; e < pl.ne; ++e)
-        for (uint32_t m = 0; m < pl.nmat; ++m) {
-          const size_t em = size_t(e) * pl.nmat + m;
-          const std::complex<double> R = cC[size_t(e) * pl.nmat + l];
-          rest += std::norm(cB[em] - R) + std::norm(cC[em] - R);
-        }
-      if (l == 0 || rest < least) least = rest, pl.first_mat = (l + 1) % pl.nmat;
-    }
     for (uint32_t e = 0; e < pl.ne; ++e) {
       std::fill(c.begin(), c.end(), std::complex<double>(0.0, 0.0));
       auto at = [&](int v, uint32_t g) -> std::complex<double> & { return c[size_t(v) * 2 * npk + g]; };
-      const std::complex<double> R = cC[size_t(e) * pl.nmat + (pl.first_mat + pl.nmat - 1) % pl.nmat];  // common part of the diagonal coefficients
+      std::complex<double> R(0.0, 0.0);  // common part of the diagonal coefficients
+      for (uint32_t m = 0; m < pl.nmat; ++m) R += cB[size_t(e) * pl.nmat + m] + cC[size_t(e) * pl.nmat + m];
+      R /= double(2 * pl.nmat);
       for (uint32_t m = 0; m < pl.nmat; ++m) {
-        const size_t em = size_t(e) * pl.nmat + (pl.first_mat + m) % pl.nmat;
+        const size_t em = size_t(e) * pl.nmat + m;
         const uint32_t g = kFieldsPerMaterial * m;
         const std::complex<double> B = cB[em] - R, C = cC[em] - R, DB = cD[em] + cB[em] - R;
         const int diag[3] = {0, 3, 5};  // xx yy zz
         for (int i = 0; i < 3; ++i) {
           for (int f = 0; f < 3; ++f) at(diag[i], g + f) = f == i ? DB : B;
-          if (m + 1 < pl.nmat) at(diag[i], g + 6) = C;
+          at(diag[i], g + 6) = C;
         }
         at(1, g + 3) = cD[em];  // xy
         at(2, g + 4) = cD[em];  // xz
@@ -1478,7 +1466,6 @@ int make_plan(const cyr_options *o, const float *optical, Plan &pl) {
             pl.ewald_sparse = false;
         }
     pl.off_fcoef = arena_put(pl.arena, fc.data(), fc.size());
-    pl.off_first = arena_put(pl.arena, &pl.first_mat, 1);
     const void *none[2] = {nullptr, nullptr};
     pl.off_ptrs = arena_put(pl.arena, none, 2);  // the morphology's and the projection's address (RunMode::indirect)
     std::vector<float> km(pl.ne);
@@ -1907,7 +1894,6 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
   fp.vox = d_vox;
   fp.vox_g = vox_g;
   fp.nx = pl.nx, fp.ny = pl.ny, fp.nz = pl.nz, fp.nmat = pl.nmat;
-  fp.first_g = reinterpret_cast<const uint32_t *>(dp + pl.off_first);
   fp.nvox = pl.nvox;
   fp.mom = sc.moments();  // each block forms the field means from the moments
   fp.nsamp = nsamp;
@@ -2876,7 +2862,6 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   std::vector<float> km;
   std::vector<const float4 *> vp;
   std::vector<float *> op;
-  std::vector<uint32_t> first;
   bool sparse = nmat <= 4 && ctx.sparse_ewald;  // every member's coefficients keep the structural zeros
   for (const auto &r : g) {
     const Plan &pl = r->plan;
@@ -2887,7 +2872,6 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     km.insert(km.end(), k, k + E);
     vp.push_back(r->d_vox);
     op.push_back(r->d_out);
-    first.push_back(pl.first_mat);
   }
   const size_t off_c = arena_put(arena, fc.data(), fc.size());
   const size_t off_k = arena_put(arena, km.data(), km.size());
@@ -2895,7 +2879,6 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   const size_t off_kv = arena_put(arena, kv0, 3);
   const size_t off_v = arena_put(arena, vp.data(), vp.size());
   const size_t off_o = arena_put(arena, op.data(), op.size());
-  const size_t off_f = arena_put(arena, first.data(), first.size());
   arena.resize((arena.size() + 255) & ~size_t(255));
   CYR_TRY(ensure_host_arena(sl, arena.size()));
   std::memcpy(sl.host_arena, arena.data(), arena.size());
@@ -2942,7 +2925,6 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   // field build + x pass (blockIdx.y = request), then y and z over all G npk volumes
   FieldParams fp{};
   fp.vox_g = vox_g;
-  fp.first_g = reinterpret_cast<const uint32_t *>(dp + off_f);
   fp.nx = p0.nx, fp.ny = p0.ny, fp.nz = p0.nz, fp.nmat = nmat;
   fp.nvox = nvox;
   fp.mom = sc.moments();

@@ -30,8 +30,8 @@ __device__ __forceinline__ void director(float4 s, float &sx, float &sy, float &
 
 constexpr int kFieldsPerMaterial = 7;
 
-// field 7 m + f of the m-th material walked; the last one (phi_ui of the last material) is T
-__host__ __device__ constexpr uint32_t num_fields(uint32_t nmat) { return kFieldsPerMaterial * nmat; }
+// field 7 m + f of material m, and T last
+__host__ __device__ constexpr uint32_t num_fields(uint32_t nmat) { return kFieldsPerMaterial * nmat + 1; }
 __host__ __device__ constexpr uint32_t num_packed(uint32_t nmat) { return (num_fields(nmat) + 1) / 2; }
 
 constexpr uint32_t kMaxFields = num_fields(kMaxMaterials);
@@ -42,17 +42,13 @@ constexpr uint32_t kMaxPacked = num_packed(kMaxMaterials);
 // changes only bin 0, which is replaced, so the means need only be close (a
 // sample of rows from all over the volume, sample_row); they keep the FP32
 // rounding of the transform proportional to the fluctuations.
-__device__ __forceinline__ uint32_t walked_material(uint32_t m, uint32_t first, uint32_t nmat) {
-  return m + first < nmat ? m + first : m + first - nmat;
-}
-
-__device__ __forceinline__ void field_means(const double *__restrict__ mom, uint32_t first, uint32_t nmat, size_t nsamp,
+__device__ __forceinline__ void field_means(const double *__restrict__ mom, uint32_t nmat, size_t nsamp,
                                             float *__restrict__ out) {
   const uint32_t nf = num_fields(nmat);
   for (uint32_t g = threadIdx.x; g < nf; g += blockDim.x) {
     double v = 0.0;
     if (g + 1 < nf) {
-      v = mom[walked_material(g / kFieldsPerMaterial, first, nmat) * kMoments + g % kFieldsPerMaterial];
+      v = mom[(g / kFieldsPerMaterial) * kMoments + g % kFieldsPerMaterial];
     } else {
       for (uint32_t m = 0; m < nmat; ++m) {
         const double *M = mom + m * kMoments;
@@ -70,9 +66,6 @@ struct FieldParams {
   const float4 *const *vox_g;
   size_t mom_stride, out_stride;
   uint32_t nx, ny, nz, nmat;
-  const uint32_t *first_g;  // [request] the material walked first: in the parameter arena, because it follows from the
-                            // optical constants, which a captured graph's replays change
-  uint32_t first;           // this request's (field_group)
   size_t nvox;
   const double *mom;     // [nmat][kMoments] moment sums over nsamp voxels
   size_t nsamp;
@@ -81,9 +74,8 @@ struct FieldParams {
   float2 *out;           // [num_packed][nvox]: field 2j in .x, field 2j+1 in .y
 };
 
-// Selects request blockIdx.y of a request group (0: the only one).
+// Selects request blockIdx.y of a request group.
 __device__ __forceinline__ void field_group(FieldParams &p) {
-  p.first = __ldg(&p.first_g[blockIdx.y]);
   if (!p.vox_g) return;
   p.vox = p.vox_g[blockIdx.y];
   p.mom += size_t(blockIdx.y) * p.mom_stride;
@@ -105,7 +97,7 @@ __device__ __forceinline__ void voxel_fields(const FieldParams &p, size_t i, flo
       pend = v;
     ++g;
   };
-  auto material = [&](float4 sv, bool last) {
+  auto material = [&](float4 sv) {
     float sx, sy, sz, pa, pui;
     director<MORPH>(sv, sx, sy, sz, pa, pui);
     const float wa = w * pa;
@@ -117,23 +109,23 @@ __device__ __forceinline__ void voxel_fields(const FieldParams &p, size_t i, flo
     emit(wa * sx * sy);
     emit(wa * sx * sz);
     emit(wa * sy * sz);
-    if (!last) emit(f6);
+    emit(f6);
   };
   if constexpr (MT > 0) {
     float4 sv[MT];
 #pragma unroll
-    for (int m = 0; m < MT; ++m) sv[m] = __ldg(&p.vox[walked_material(uint32_t(m), p.first, MT) * p.nvox + i]);
+    for (int m = 0; m < MT; ++m) sv[m] = __ldg(&p.vox[m * p.nvox + i]);
 #pragma unroll
-    for (int m = 0; m < MT; ++m) material(sv[m], m + 1 == MT);
+    for (int m = 0; m < MT; ++m) material(sv[m]);
   } else {
     for (uint32_t m0 = 0; m0 < p.nmat; m0 += 4) {
       float4 sv[4];  // the loads of up to 4 materials are issued before any is used
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (m0 + u < p.nmat) sv[u] = __ldg(&p.vox[walked_material(m0 + u, p.first, p.nmat) * p.nvox + i]);
+        if (m0 + u < p.nmat) sv[u] = __ldg(&p.vox[(m0 + u) * p.nvox + i]);
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (m0 + u < p.nmat) material(sv[u], m0 + u + 1 == p.nmat);
+        if (m0 + u < p.nmat) material(sv[u]);
     }
   }
   emit(T);

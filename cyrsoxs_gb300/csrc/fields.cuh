@@ -9,18 +9,19 @@
 // seven real fields u_x^2, u_y^2, u_z^2, u_x u_y, u_x u_z, u_y u_z, phi_ui,
 // with energy dependent complex coefficients.  The FFT is linear, hence
 //   FFT(Nt_v) = sum_g c_vg(E) FFT(F_g),
-// exactly.  The diagonal coefficients share a common part (the base optical
-// constants are alike for every material), which would cancel in the sum and
-// amplify the FP32 rounding of the field spectra; it is taken out with the
-// field T = sum_m (|u_m|^2 + phi_ui_m), constant where the volume fractions
-// sum to one:
+// exactly.  The diagonal coefficients share a common part R(E) (the base
+// optical constants are alike for every material), which would cancel in the
+// sum and amplify the FP32 rounding of the field spectra; it is taken out with
+// one more field, T = sum_m (|u_m|^2 + phi_ui_m), constant where the volume
+// fractions sum to one:
 //   Nt_xx = sum_m [(D+B-R) u_x^2 + (B-R)(u_y^2 + u_z^2) + (C-R) phi_ui] + R T.
-// With R(E) = C of one material that material's phi_ui drops out, so T takes
-// its place and 7 M fields do (R as the mean of all B and C needs 7 M + 1: one
-// packed volume more for every even M).  The planner takes the material whose C
-// lies nearest to all B and C of the request; the materials are walked from the
-// one after it, so it comes last.
-// The 7 M real fields are packed in pairs into complex volumes
+// R is the mean of all B and C.  (7 M fields would do, with R = C of one
+// material, whose phi_ui then drops out: one packed volume less for every even
+// M, 7% of a 256 x 512 x 512 request.  But the fields that hold the same
+// structure, as phi_ui of two materials that share the space, then no longer
+// average each other's rounding: the error against 64 bits grew by 23% on
+// 256 x 256 x 64 with 2 materials and on 256 x 256 x 32 with 4 and a window.)
+// The 7 M + 1 real fields are packed in pairs into complex volumes
 // Z_j = F_2j + i F_2j+1 and transformed with the engine's complex 3D FFT; the
 // Ewald kernel unpacks them with
 //   F_2j(k) = (Z_j(k) + conj Z_j(-k)) / 2,  F_2j+1(k) = (Z_j(k) - conj Z_j(-k)) / 2i.
@@ -39,7 +40,7 @@ template <int MORPH, int MT>
 __global__ void __launch_bounds__(256) k_build_fields(FieldParams p) {
   __shared__ float mean[kMaxFields];  // volume mean of each windowed field
   field_group(p);
-  field_means(p.mom, p.first, p.nmat, p.nsamp, mean);
+  field_means(p.mom, p.nmat, p.nsamp, mean);
   __syncthreads();
   const size_t stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = p.i0 + size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < p.i1; i += stride) {
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(256, V == 4 ? 5 : V == 8 ? 4 : V == 16 ? 3 : 1
   float2 *lines = fsm + N;  // [npk][N]: element x of line j at lines[j N + swz(x)]
   __shared__ float mean[kMaxFields];
   field_group(p);
-  field_means(p.mom, p.first, p.nmat, p.nsamp, mean);
+  field_means(p.mom, p.nmat, p.nsamp, mean);
   warp_twiddles<V>(tws, tw_n);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const uint32_t nrows = uint32_t((p.i1 - p.i0) / N);
@@ -148,7 +149,7 @@ struct FieldEwaldParams {
 // diagonal, which also takes T), u_x u_y (xy), u_x u_z (xz) or u_y u_z (yz)
 // (include/uniaxial.h:94-151 in the contrast form above); coef[e][v][j] can
 // be non-zero only when field 2j or 2j+1 enters entry v.  With 4 materials
-// 32 of the 70 (entry, volume) pairs of the LAB frame's five entries are used.
+// 34 of the 75 (entry, volume) pairs of the LAB frame's five entries are used.
 __host__ __device__ constexpr bool field_enters(uint32_t nmat, int v, uint32_t g) {
   return g >= num_fields(nmat)        ? false                                    // T's zero partner
          : g + 1 == num_fields(nmat)  ? (v == 0 || v == 3 || v == 5)             // T

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(kMixThreads, 3) k_build_fields_mix(const __gri
   __shared__ float mean[kMaxFields];
   FieldParams f = q.f;
   field_group(f);
-  field_means(f.mom, f.first, f.nmat, f.nsamp, mean);
+  field_means(f.mom, f.nmat, f.nsamp, mean);
   const MixParams<float2> &p = q.m;
   const uint32_t nx = p.nx, nrows = uint32_t((f.i1 - f.i0) / nx);
   BuildTile tile{q, bsm, nullptr, f.nvox, 0};

@@ -70,7 +70,7 @@ typedef struct cyr_options {
   uint32_t strategy;           /* engine only (zero-initialised = auto): how the spectra are formed.
                                   1 PER_ENERGY: tensor-entry spectra per energy (per angle in the
                                   Material frame), as the reference's pipeline does;
-                                  2 FIELDS: the 7 M energy-independent morphology fields are
+                                  2 FIELDS: the 7 M + 1 energy-independent morphology fields are
                                   transformed once per request and combined per energy and angle
                                   at the Ewald sample points (exact by linearity of the FFT);
                                   0 AUTO: FIELDS when there are enough energies x angles to
