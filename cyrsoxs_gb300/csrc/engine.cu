@@ -450,6 +450,12 @@ struct DeviceContext {
   std::map<std::pair<const void *, size_t>, int> occupancy;  // blocks per SM of a kernel at a shared-memory size
   struct Fp64Scratch {
     DeviceBuffer spec, images, avg, params, params64, vox, out;
+    cudaEvent_t last_use = nullptr;     // completion of the last request that used them, on whatever stream
+    int wait(cudaStream_t st) {         // orders st behind it
+      if (!last_use) CYR_CUDA(cudaEventCreateWithFlags(&last_use, cudaEventDisableTiming));
+      CYR_CUDA(cudaStreamWaitEvent(st, last_use, 0));
+      return CYR_OK;
+    }
   } f64;                                // the FP64 pipeline's buffers (plain entry points)
   Scratch main;
   DeviceBuffer vox_in, out_in;  // host-buffer entry points: morphology and projections
@@ -2521,6 +2527,12 @@ int run_fp64(DeviceContext &ctx, const cyr_options *o, const double *optical, co
   CYR_TRY(make_plan64(o, optical, o->algorithm == 0 && o->windowing == 1, pl, p64));
   CYR_TRY(setup_attrs(ctx));
   auto &f = ctx.f64;
+  CYR_TRY(f.wait(st));
+  struct Record {  // at every return: whatever was enqueued by then
+    cudaEvent_t ev;
+    cudaStream_t st;
+    ~Record() { cudaEventRecord(ev, st); }
+  } record{f.last_use, st};
   const uint32_t nvol = pl.material_frame ? 3u : pl.nvol;
   // Field spectra (one transform of the 7 M packed fields for every energy and
   // angle) when they are fewer volumes than the per-energy spectra and fit;
@@ -3504,6 +3516,7 @@ int cyr_cuda_main_fp64(const cyr_options *opt, const double *optical, const doub
   CYR_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   int rc = CYR_OK;
   do {
+    if ((rc = ctx->f64.wait(st)) != CYR_OK) break;
     if (cudaMemcpyAsync(ctx->f64.vox.ptr, voxels, vox_bytes, cudaMemcpyHostToDevice, st) != cudaSuccess) {
       rc = fail(CYR_ERR_CUDA, "voxel upload failed: %s", cudaGetErrorString(cudaGetLastError()));
       break;
@@ -3552,6 +3565,7 @@ int cyr_compute_polarization_fp64(const cyr_options *opt, const double *optical,
   CYR_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   int rc = CYR_OK;
   do {
+    if ((rc = f.wait(st)) != CYR_OK) break;
     cudaMemcpyAsync(f.params64.ptr, p64.arena.data(), p64.arena.size(), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(f.vox.ptr, voxels, vox_bytes, cudaMemcpyHostToDevice, st);
     const unsigned char *dq = f.params64.as<unsigned char>();
@@ -3587,6 +3601,7 @@ int cyr_compute_polarization_fp64(const cyr_options *opt, const double *optical,
     const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = fail(CYR_ERR_CUDA, "FP64 polarization failed: %s", cudaGetErrorString(e));
   } while (false);
+  cudaStreamSynchronize(st);  // an early end too leaves nothing of this call in flight
   cudaStreamDestroy(st);
   return rc;
 }
