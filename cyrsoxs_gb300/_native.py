@@ -79,6 +79,7 @@ def lib():
     L.cyr_fft3d_device.argtypes = [ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint32,
                                    ctypes.c_uint32, ctypes.c_void_p]
     L.cyr_selftest_wait_limit.argtypes = [ctypes.POINTER(ctypes.c_int)]
+    L.cyr_selftest_request_waits.argtypes = [ctypes.POINTER(ctypes.c_uint32)]
     L.cyr_fft3d_device_static.argtypes = [ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint32,
                                           ctypes.c_uint32, ctypes.c_void_p]
     L.cyr_warp_affine_device.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int,
@@ -224,6 +225,13 @@ def selftest_wait_limit() -> bool:
     flag = ctypes.c_int(0)
     check(lib().cyr_selftest_wait_limit(ctypes.byref(flag)))
     return bool(flag.value)
+
+
+def selftest_request_waits() -> int:
+    """Bits of what reported a request whose transform's waits ran out (cyr_selftest_request_waits); 15 is a pass."""
+    bits = ctypes.c_uint32(0)
+    check(lib().cyr_selftest_request_waits(ctypes.byref(bits)))
+    return int(bits.value)
 
 
 def fft3d_device(d_data: int, nx: int, ny: int, nz: int, count: int = 1, stream: int = 0) -> None:

@@ -364,19 +364,39 @@ struct ZTune {
   float ms = 0.f;
 };
 
+// The bounded waits of a column pass's tile copies: the word that is set when one runs out, and, for the self-tests, a
+// short limit and bytes that the barriers expect beyond the copies', so that every wait does (ColTmaParams).
+struct ColWaits {
+  unsigned *error = nullptr;
+  uint32_t poll_limit = 0, extra_tx = 0;
+};
+constexpr uint32_t kShortWait = 1u << 16;  // polls: far longer than a tile's copies take to land
+
+// What the words of a request (Scratch) report once it has completed: null when it is sound.
+const char *request_error(const unsigned *words, char *buf, size_t len) {
+  if (words[2] != 0) return "an FFT tile copy did not complete within its wait limit";
+  if (words[0] == 0) return nullptr;
+  std::snprintf(buf, len, "%u detector pixels needed z planes outside the kept range", words[0]);
+  return buf;
+}
+
 // Device scratch of one request in flight (grow-only).  The plain entry points
 // share the device context's; every serving slot owns one.
 struct Scratch {
   DeviceBuffer spec, images, avg, params, dc, means, conv;
-  // words that a request starts at zero, cleared by one memset: the error count, the negative-fraction flag and,
-  // from kMomentsAt on, the moment sums
+  // words that a request starts at zero, cleared by one memset: the error count, the negative-fraction flag, the tile
+  // copies' flag (ColWaits) and, from kMomentsAt on, the moment sums
   DeviceBuffer errors;
   DeviceBuffer zmask;              // store mask of the FIELDS z pass (k_zmask)
   DeviceBuffer sample;             // rows of a host morphology that the means are taken from (SlabUpload)
   cudaEvent_t last_use = nullptr;  // completion of the last request that used it
   uint64_t generation = 0;         // bumped by every (re)allocation of a buffer above
   static constexpr size_t kMomentsAt = 256;
+  static constexpr size_t kWords = 3;
   unsigned *flag() const { return errors.as<unsigned>() + 1; }
+  ColWaits waits(bool run_out = false) const {
+    return ColWaits{errors.as<unsigned>() + 2, run_out ? kShortWait : 0u, run_out ? 16u : 0u};
+  }
   double *moments() const { return reinterpret_cast<double *>(errors.as<unsigned char>() + kMomentsAt); }
   int clear(size_t nmoments, cudaStream_t st) {
     const size_t bytes = kMomentsAt + nmoments * sizeof(double);
@@ -463,9 +483,9 @@ struct DeviceContext {
   // by every call (the calls hold `mu`)
   cudaStream_t main_stream = nullptr, copy_stream = nullptr;
   std::vector<cudaEvent_t> slab_events;
-  unsigned *host_errors = nullptr;  // pinned: the error count and the tile-copy word of the last cyr_cuda_main
-  // TMA column passes: the driver's tensor-map encoder, and a word set when a
-  // tile copy did not complete within the kernel's wait limit
+  unsigned *host_errors = nullptr;  // pinned: the words of the last cyr_cuda_main (Scratch::kWords)
+  // TMA column passes: the driver's tensor-map encoder, and the word that the passes outside a request
+  // (cyr_fft3d_device, the wait self-test) set when a tile copy did not complete within the kernel's wait limit
   void *encode_tiled = nullptr;
   unsigned *tma_error = nullptr;
 };
@@ -670,7 +690,8 @@ int encode_cols_map(DeviceContext &ctx, CUtensorMap *map, void *data, uint32_t n
 // a producer warp for 128-, 256- and 512-point lines; null stores every plane.
 template <int V>
 int warp_fft_pass_v(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, int axis,
-                    cudaStream_t st, size_t nvox, uint32_t form = kFormAuto, const uint32_t *zmask = nullptr) {
+                    cudaStream_t st, size_t nvox, const ColWaits &waits, uint32_t form = kFormAuto,
+                    const uint32_t *zmask = nullptr) {
   constexpr uint32_t N = 32 * V;
   const float2 *tw = nullptr;
   CYR_TRY(get_twiddles(ctx, N, &tw));
@@ -679,7 +700,7 @@ int warp_fft_pass_v(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, 
     RowPassParams rp{data, uint32_t(size_t(ny) * nz * count), tw, ny * nz, nvox};
     const size_t smem = (N + 8 * N) * sizeof(float2);
     k_fft_rows<V><<<(rp.rows + 7) / 8, 256, smem, st>>>(rp);
-  } else if (V == 32 && nx % 8 == 0 && ctx.encode_tiled && ctx.tma_error && form != kFormCp) {
+  } else if (V == 32 && nx % 8 == 0 && ctx.encode_tiled && form != kFormCp) {
     // 1024-point lines: 8-column tiles (k_fft_cols_tma64)
     CUtensorMap map;
     CYR_TRY(encode_cols_map(ctx, &map, data, nx, ny, nz, count, nvox, axis, 256, 8));
@@ -689,13 +710,13 @@ int warp_fft_pass_v(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, 
     tp.ntiles = tp.nxt * tp.others * count;
     tp.axis = uint32_t(axis);
     tp.tw = tw;
-    tp.error = ctx.tma_error;
+    tp.error = waits.error, tp.poll_limit = waits.poll_limit, tp.extra_tx = waits.extra_tx;
     const int sms = ctx.sms;
     int per_sm = 0;
     CYR_TRY(blocks_per_sm(ctx, k_fft_cols_tma64<32>, 9 * 32, cols_tma64_smem(N), &per_sm));
     const unsigned grid = unsigned(std::min<size_t>(tp.ntiles, size_t(std::max(1, per_sm)) * sms));
     k_fft_cols_tma64<32><<<grid, 9 * 32, cols_tma64_smem(N), st>>>(map, tp);
-  } else if ((V == 4 || V == 8 || V == 16) && nx % kTmaCols == 0 && ctx.encode_tiled && ctx.tma_error &&
+  } else if ((V == 4 || V == 8 || V == 16) && nx % kTmaCols == 0 && ctx.encode_tiled &&
              form != kFormCp) {
     CUtensorMap map, smap;
     CYR_TRY(encode_cols_map(ctx, &map, data, nx, ny, nz, count, nvox, axis, N < 256 ? N : 256));
@@ -711,7 +732,7 @@ int warp_fft_pass_v(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, 
     tp.ntiles = tp.nxt * tp.others * count;
     tp.axis = uint32_t(axis);
     tp.tw = tw;
-    tp.error = ctx.tma_error;
+    tp.error = waits.error, tp.poll_limit = waits.poll_limit, tp.extra_tx = waits.extra_tx;
     const int sms = ctx.sms;
     int per_sm = 0;
     // 128-point lines: 32 columns in three stages (nx a multiple of 32) or 16 in two,
@@ -787,18 +808,19 @@ int warp_fft_pass_v(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, 
 }
 
 int warp_fft_pass(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, int axis,
-                  cudaStream_t st, size_t nvox, uint32_t form = kFormAuto, const uint32_t *zmask = nullptr) {
+                  cudaStream_t st, size_t nvox, const ColWaits &waits, uint32_t form = kFormAuto,
+                  const uint32_t *zmask = nullptr) {
   const uint32_t n = axis == 0 ? nx : axis == 1 ? ny : nz;
-  if (n == 128) return warp_fft_pass_v<4>(ctx, data, nx, ny, nz, count, axis, st, nvox, form, zmask);
-  if (n == 256) return warp_fft_pass_v<8>(ctx, data, nx, ny, nz, count, axis, st, nvox, form, zmask);
-  if (n == 512) return warp_fft_pass_v<16>(ctx, data, nx, ny, nz, count, axis, st, nvox, form, zmask);
-  return warp_fft_pass_v<32>(ctx, data, nx, ny, nz, count, axis, st, nvox, form);
+  if (n == 128) return warp_fft_pass_v<4>(ctx, data, nx, ny, nz, count, axis, st, nvox, waits, form, zmask);
+  if (n == 256) return warp_fft_pass_v<8>(ctx, data, nx, ny, nz, count, axis, st, nvox, waits, form, zmask);
+  if (n == 512) return warp_fft_pass_v<16>(ctx, data, nx, ny, nz, count, axis, st, nvox, waits, form, zmask);
+  return warp_fft_pass_v<32>(ctx, data, nx, ny, nz, count, axis, st, nvox, waits, form);
 }
 
 // The forms that apply to a column pass of n-point lines (axis 1 or 2) for this nx.
 std::vector<uint32_t> column_forms(const DeviceContext &ctx, uint32_t n, uint32_t nx) {
   std::vector<uint32_t> f;
-  const bool tma = ctx.encode_tiled && ctx.tma_error;
+  const bool tma = ctx.encode_tiled;
   if (n == 256 && tma && nx % kTmaCols == 0) {
     if (nx % (2 * kTmaCols) == 0) f.push_back(kFormTmaWs);
     if (nx % (2 * kTmaCols) == 0) f.push_back(kFormTmaWs2);
@@ -1039,7 +1061,7 @@ int mix_pass(DeviceContext &ctx, T *data, uint32_t nx, uint32_t ny, uint32_t nz,
 // Axis lengths: 128-1024 powers of two run the warp FFT, 8-64 along y and z
 // one thread per line, every other length k_mix_fft.
 int fft_axes(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, cudaStream_t st,
-             int first, int last, size_t vstride = 0, const uint32_t *forms = nullptr,
+             const ColWaits &waits, int first, int last, size_t vstride = 0, const uint32_t *forms = nullptr,
              const uint32_t *zmask = nullptr) {
   const size_t nvox = vstride ? vstride : size_t(nx) * ny * nz;
   const uint32_t dims[3] = {nx, ny, nz};
@@ -1047,7 +1069,7 @@ int fft_axes(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, uint32_
     const uint32_t n = dims[axis];
     if (n == 1) continue;
     if (n == 128 || n == 256 || n == 512 || n == 1024) {
-      CYR_TRY(warp_fft_pass(ctx, data, nx, ny, nz, count, axis, st, nvox, forms ? forms[axis] : kFormAuto,
+      CYR_TRY(warp_fft_pass(ctx, data, nx, ny, nz, count, axis, st, nvox, waits, forms ? forms[axis] : kFormAuto,
                             axis == 2 ? zmask : nullptr));
     } else if (axis > 0 && (n == 8 || n == 16 || n == 32 || n == 64) && count <= 65535) {
       CYR_TRY(thread_fft_pass(ctx, data, nx, ny, nz, count, axis, st, nvox));
@@ -1063,8 +1085,8 @@ int fft_axes(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, uint32_
 }
 
 int fft3d(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t count, cudaStream_t st,
-          bool skip_z = false) {
-  return fft_axes(ctx, data, nx, ny, nz, count, st, 0, skip_z ? 1 : 2);
+          const ColWaits &waits, bool skip_z = false) {
+  return fft_axes(ctx, data, nx, ny, nz, count, st, waits, 0, skip_z ? 1 : 2);
 }
 
 // ---------------------------------------------------------------------------
@@ -1718,7 +1740,7 @@ int launch_fused_build(DeviceContext &ctx, const FieldParams &fp, uint32_t npk, 
 
 // Fields of planes [z0, z1) and their x pass: fused or the separate build and row pass.
 int build_fields_x(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan &pl, FieldParams fp, uint32_t z0,
-                   uint32_t z1, bool fused, cudaStream_t st) {
+                   uint32_t z1, bool fused, cudaStream_t st, const ColWaits &waits) {
   const uint32_t npk = pl.npk;
   float2 *spec = sc.spec.as<float2>();
   const int sms = ctx.sms;
@@ -1732,7 +1754,7 @@ int build_fields_x(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const 
   }));
   ctx.prof.end(slot, st);
   CYR_CUDA(cudaGetLastError());
-  return fft_axes(ctx, spec + fp.i0, pl.nx, pl.ny, z1 - z0, npk, st, 0, 0, pl.nvox);
+  return fft_axes(ctx, spec + fp.i0, pl.nx, pl.ny, z1 - z0, npk, st, waits, 0, 0, pl.nvox);
 }
 
 // Ewald geometry of a FIELDS request (k_ewald_fields); kmag, kx, ky, kz are set per energy and k.
@@ -1755,7 +1777,7 @@ int field_zmask(DeviceContext &ctx, Scratch &sc, const EwaldGeom &g, const float
                 const float *d_kv, uint32_t nk, cudaStream_t st, const uint32_t **out) {
   *out = nullptr;
   if (!ctx.zmask || g.twod || !(g.nz == 128 || g.nz == 256 || g.nz == 512) || g.nx % kTmaCols != 0 ||
-      !ctx.encode_tiled || !ctx.tma_error)
+      !ctx.encode_tiled)
     return CYR_OK;
   const uint32_t mw = (g.nz / 8 + 31) / 32;
   const size_t bytes = size_t(g.ny) * (g.nx / kTmaCols) * mw * sizeof(uint32_t);
@@ -1783,7 +1805,7 @@ int field_zmask(DeviceContext &ctx, Scratch &sc, const EwaldGeom &g, const float
 // candidate computes the same numbers.
 int tune_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan &pl, const FieldParams &fp,
                 bool fused_ok, cudaStream_t st, DeviceContext::FieldTune &ft,
-                const uint32_t *zmask) {
+                const uint32_t *zmask, const ColWaits &waits) {
   struct Cand {
     int kind;  // 0 build + x, 1 y pass, 2 z pass
     uint32_t choice;
@@ -1810,9 +1832,9 @@ int tune_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Pla
     for (Cand &c : cands) {
       if (pass) CYR_CUDA(cudaEventRecord(c.a, st));
       if (c.kind == 0)
-        rc = build_fields_x(ctx, sc, o, pl, fp, 0, pl.nz, c.choice == 1, st);
+        rc = build_fields_x(ctx, sc, o, pl, fp, 0, pl.nz, c.choice == 1, st, waits);
       else
-        rc = warp_fft_pass(ctx, sc.spec.as<float2>(), pl.nx, pl.ny, pl.nz, pl.npk, c.kind, st, pl.nvox, c.choice,
+        rc = warp_fft_pass(ctx, sc.spec.as<float2>(), pl.nx, pl.ny, pl.nz, pl.npk, c.kind, st, pl.nvox, waits, c.choice,
                            c.kind == 2 ? zmask : nullptr);
       if (rc != CYR_OK) break;
       if (pass) CYR_CUDA(cudaEventRecord(c.b, st));
@@ -1886,7 +1908,7 @@ void launch_ewald_fields(const FieldEwaldParams &fe, uint32_t nb, uint32_t nmat,
 // every energy (in batches) and k from them.
 int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan &pl, const unsigned char *dp,
                const float4 *d_vox, float *d_out, cudaStream_t st, size_t nsamp, const SlabUpload *up,
-               bool capturing, bool indirect) {
+               bool capturing, bool indirect, const ColWaits &waits) {
   const uint32_t npk = pl.npk;
   // indirect: the morphology's and the projection's addresses are read from the arena
   const float4 *const *vox_g = indirect ? reinterpret_cast<const float4 *const *>(dp + pl.off_ptrs) : nullptr;
@@ -1928,11 +1950,12 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
   if (!have) {
     ft.fused = fused_ok;
     if (ctx.autotune && !up && !capturing && !ctx.prof.active) {
-      CYR_TRY(tune_fields(ctx, sc, o, pl, fp, fused_ok, st, ft, zmask));
+      CYR_TRY(tune_fields(ctx, sc, o, pl, fp, fused_ok, st, ft, zmask, waits));
       std::lock_guard<std::mutex> lk(ctx.tables_mu);
       ctx.ftune[key] = ft;
     }
   }
+  if (waits.extra_tx) ft.form[1] = ft.form[2] = kFormAuto;  // self-test: a form with tile copies, whatever was tuned
   const bool fused = fused_ok && ft.fused;
   // fields of planes [z0, z1), then their x and y passes (the axes commute; z comes last)
   const uint32_t step = up ? up->planes : pl.nz, nslab = up ? up->count : 1;
@@ -1942,12 +1965,12 @@ int run_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan
       CYR_TRY(const_cast<SlabUpload *>(up)->issue(sl));
       CYR_CUDA(cudaStreamWaitEvent(st, up->events[sl], 0));
     }
-    CYR_TRY(build_fields_x(ctx, sc, o, pl, fp, z0, z1, fused, st));
-    CYR_TRY(fft_axes(ctx, spec + size_t(z0) * pl.npix, pl.nx, pl.ny, z1 - z0, npk, st, 1, 1, pl.nvox,
+    CYR_TRY(build_fields_x(ctx, sc, o, pl, fp, z0, z1, fused, st, waits));
+    CYR_TRY(fft_axes(ctx, spec + size_t(z0) * pl.npix, pl.nx, pl.ny, z1 - z0, npk, st, waits, 1, 1, pl.nvox,
                      ft.form));
     if (up) CYR_TRY(const_cast<SlabUpload *>(up)->issue(sl + 1));  // the next slab's copy, behind this slab's kernels
   }
-  CYR_TRY(fft_axes(ctx, spec, pl.nx, pl.ny, pl.nz, npk, st, 2, 2, 0, ft.form, zmask));
+  CYR_TRY(fft_axes(ctx, spec, pl.nx, pl.ny, pl.nz, npk, st, waits, 2, 2, 0, ft.form, zmask));
   // bin 0 of each packed volume replaced by the mean of its neighbours
   CYR_TRY(sc.dc.ensure(size_t(kMaxPacked) * sizeof(float2)));
   int slot = ctx.prof.begin(kDc, st);
@@ -2044,6 +2067,7 @@ struct RunMode {
   // FIELDS requests on device buffers whose addresses the arena holds (Plan::off_ptrs): a captured graph then serves
   // every morphology and projection of its signature without staging copies
   bool indirect = false;
+  bool waits_run_out = false;  // self-test: the column passes' waits run out (ColWaits)
 };
 
 
@@ -2163,7 +2187,8 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
     ctx.prof.end(slot, st);
     CYR_CUDA(cudaGetLastError());
     if (pl.fields) {
-      CYR_TRY(run_fields(ctx, sc, o, pl, dp, d_vox, d_out, st, nsamp, slabs ? &upload : nullptr, mode.capturing, mode.indirect));
+      CYR_TRY(run_fields(ctx, sc, o, pl, dp, d_vox, d_out, st, nsamp, slabs ? &upload : nullptr, mode.capturing, mode.indirect,
+                         sc.waits(mode.waits_run_out)));
       // an event recorded inside a capture cannot be waited on outside it (slots keep order by their stream)
       if (!mode.capturing) CYR_CUDA(cudaEventRecord(sc.last_use, st));
       return CYR_OK;
@@ -2304,7 +2329,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
         ctx.prof.end(slot, st);
       }
       CYR_CUDA(cudaGetLastError());
-      CYR_TRY(fft3d(ctx, spec, pl.nx, pl.ny, pl.kz, bp.nvol, st, true));
+      CYR_TRY(fft3d(ctx, spec, pl.nx, pl.ny, pl.kz, bp.nvol, st, sc.waits(mode.waits_run_out), true));
     } else {
       slot = ctx.prof.begin(kBuild, st, convert ? 2 : 1);
       if (o->morphology_type == 0) {
@@ -2315,7 +2340,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
       }
       ctx.prof.end(slot, st);
       CYR_CUDA(cudaGetLastError());
-      CYR_TRY(fft3d(ctx, spec, pl.nx, pl.ny, pl.nz, bp.nvol, st, false));
+      CYR_TRY(fft3d(ctx, spec, pl.nx, pl.ny, pl.nz, bp.nvol, st, sc.waits(mode.waits_run_out), false));
     }
     slot = ctx.prof.begin(kDc, st);
     k_dc<<<1, 32, 0, st>>>(spec, bp.nvol, pl.vstride, pl.nx, pl.ny, pl.nz, pl.p0, pl.p1, pl.pn, dc);
@@ -2758,7 +2783,7 @@ struct Slot {
   DeviceBuffer vox, out;  // staging for host-buffer requests
   unsigned char *host_arena = nullptr;
   size_t host_arena_bytes = 0;
-  unsigned *host_errors = nullptr;  // pinned copy of the request's device error counter
+  unsigned *host_errors = nullptr;  // pinned copy of the request's words (Scratch::kWords)
   std::shared_ptr<ServerRequest> req;
   std::vector<std::shared_ptr<ServerRequest>> group;  // the other requests sharing req's launches
   std::map<std::string, GraphEntry> graphs;
@@ -2774,6 +2799,7 @@ struct Server {
   double inflight_work = 0;
   bool graphs = false;
   bool groups = false;  // same-shape queued requests share one launch per kernel
+  bool waits_run_out = false;  // self-test (RunMode)
   std::mutex mu;
   std::condition_variable cv_work, cv_done;
   std::deque<std::shared_ptr<ServerRequest>> queue;
@@ -2908,6 +2934,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
   CYR_TRY(sc.avg.ensure(size_t(vb) * npix * sizeof(float)));
   CYR_TRY(sc.dc.ensure(size_t(G) * npk * sizeof(float2)));
   CYR_TRY(sc.clear(size_t(G) * nmat * kMoments, st));
+  const ColWaits waits = sc.waits(S.waits_run_out);
   float2 *spec = sc.spec.as<float2>();
   const int sms = ctx.sms;
   const float4 *const *vox_g = reinterpret_cast<const float4 *const *>(dp + off_v);
@@ -2955,6 +2982,7 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     auto it = ctx.ftune.find(key);
     if (it != ctx.ftune.end()) ft = it->second;
   }
+  if (waits.extra_tx) ft.form[1] = ft.form[2] = kFormAuto;
   if (fused_ok && ft.fused) {
     CYR_TRY(launch_fused_build(ctx, fp, npk, o->morphology_type == 0, G, st));
   } else {
@@ -2967,14 +2995,14 @@ int run_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerReque
     }));
     ctx.prof.end(slot, st);
     CYR_CUDA(cudaGetLastError());
-    CYR_TRY(fft_axes(ctx, spec, p0.nx, p0.ny, p0.nz, npk * G, st, 0, 0, 0, ft.form));
+    CYR_TRY(fft_axes(ctx, spec, p0.nx, p0.ny, p0.nz, npk * G, st, waits, 0, 0, 0, ft.form));
   }
   // the planes the Ewald projection reads for any of the G E virtual energies
   const EwaldGeom geom = field_geometry(o, p0);
   const uint32_t *zmask = nullptr;
   CYR_TRY(field_zmask(ctx, sc, geom, reinterpret_cast<const float *>(dp + off_k), G * E,
                       reinterpret_cast<const float *>(dp + off_kv), 1, st, &zmask));
-  CYR_TRY(fft_axes(ctx, spec, p0.nx, p0.ny, p0.nz, npk * G, st, 1, 2, 0, ft.form, zmask));
+  CYR_TRY(fft_axes(ctx, spec, p0.nx, p0.ny, p0.nz, npk * G, st, waits, 1, 2, 0, ft.form, zmask));
   {
     const int slot = ctx.prof.begin(kDc, st);
     k_dc<<<1, (npk * G + 31) / 32 * 32, 0, st>>>(spec, npk * G, nvox, p0.nx, p0.ny, p0.nz, 0, 1 % p0.nz, p0.nz - 1,
@@ -3059,6 +3087,7 @@ int start_request(Server &S, Slot &sl, ServerRequest &r) {
   mode.host_arena_bytes = sl.host_arena_bytes;
   mode.plan = &r.plan;
   mode.indirect = r.indirect;
+  mode.waits_run_out = S.waits_run_out;
   auto git = S.graphs ? sl.graphs.find(r.key) : sl.graphs.end();
   if (git != sl.graphs.end() && git->second.generation == sl.generation()) {
     std::memcpy(sl.host_arena, pl.arena.data(), pl.arena.size());
@@ -3095,7 +3124,8 @@ int start_request(Server &S, Slot &sl, ServerRequest &r) {
       sl.warm[r.key] = sl.generation();
     }
   }
-  CYR_CUDA(cudaMemcpyAsync(sl.host_errors, sl.sc.errors.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+  CYR_CUDA(cudaMemcpyAsync(sl.host_errors, sl.sc.errors.ptr, Scratch::kWords * sizeof(unsigned), cudaMemcpyDeviceToHost,
+                           st));
   if (staged)
     CYR_CUDA(cudaMemcpyAsync(r.h_out ? static_cast<void *>(r.h_out) : static_cast<void *>(r.d_out), d_out, r.out_bytes,
                              r.h_out ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, st));
@@ -3106,7 +3136,8 @@ int start_request(Server &S, Slot &sl, ServerRequest &r) {
 // Enqueues a group of same-key requests on slot sl (worker thread).
 int start_group(Server &S, Slot &sl, const std::vector<std::shared_ptr<ServerRequest>> &g) {
   CYR_TRY(run_group(S, sl, g));
-  CYR_CUDA(cudaMemcpyAsync(sl.host_errors, sl.sc.errors.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, sl.stream));
+  CYR_CUDA(cudaMemcpyAsync(sl.host_errors, sl.sc.errors.ptr, Scratch::kWords * sizeof(unsigned), cudaMemcpyDeviceToHost,
+                           sl.stream));
   CYR_CUDA(cudaEventRecord(sl.done, sl.stream));
   ++S.group_runs;
   S.grouped += g.size();
@@ -3146,12 +3177,11 @@ void server_loop(Server *Sp) {
       const cudaError_t q = cudaEventQuery(sl.done);
       if (q == cudaErrorNotReady) continue;
       progress = true;
+      char msg[128];
       if (q != cudaSuccess) {
         finish_request(S, sl, CYR_ERR_CUDA, std::string("request failed on the device: ") + cudaGetErrorString(q));
-      } else if (*sl.host_errors != 0) {
-        char m[128];
-        std::snprintf(m, sizeof m, "%u detector pixels needed z planes outside the kept range", *sl.host_errors);
-        finish_request(S, sl, CYR_ERR_CUDA, m);
+      } else if (const char *what = request_error(sl.host_errors, msg, sizeof msg)) {
+        finish_request(S, sl, CYR_ERR_CUDA, what);
       } else {
         finish_request(S, sl, CYR_OK, "");
       }
@@ -3339,11 +3369,11 @@ int cyr_device_errors(uint32_t *count) {
   CYR_TRY(get_context(&ctx));
   std::lock_guard<std::mutex> lk(ctx->mu);
   *count = 0;
-  if (!ctx->main.errors.ptr) return CYR_OK;
   CYR_CUDA(cudaDeviceSynchronize());
-  unsigned h = 0;
-  CYR_CUDA(cudaMemcpy(&h, ctx->main.errors.ptr, sizeof h, cudaMemcpyDeviceToHost));
-  *count = h;
+  unsigned h[Scratch::kWords] = {}, fft = 0;
+  if (ctx->main.errors.ptr) CYR_CUDA(cudaMemcpy(h, ctx->main.errors.ptr, sizeof h, cudaMemcpyDeviceToHost));
+  if (ctx->tma_error) CYR_CUDA(cudaMemcpy(&fft, ctx->tma_error, sizeof fft, cudaMemcpyDeviceToHost));
+  *count = h[0] + (h[2] != 0 ? 1u : 0u) + (fft != 0 ? 1u : 0u);
   return CYR_OK;
 }
 
@@ -3388,7 +3418,7 @@ static int cuda_main_impl(const cyr_options *opt, const float *optical, const fl
   CYR_TRY(ctx->out_in.ensure(out_bytes));
   if (!ctx->main_stream) CYR_CUDA(cudaStreamCreateWithFlags(&ctx->main_stream, cudaStreamNonBlocking));
   if (!ctx->copy_stream) CYR_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
-  if (!ctx->host_errors) CYR_CUDA(cudaMallocHost(&ctx->host_errors, 2 * sizeof(unsigned)));
+  if (!ctx->host_errors) CYR_CUDA(cudaMallocHost(&ctx->host_errors, Scratch::kWords * sizeof(unsigned)));
   cudaStream_t st = ctx->main_stream, cs = ctx->copy_stream;
   int rc = CYR_OK;
   do {
@@ -3405,16 +3435,18 @@ static int cuda_main_impl(const cyr_options *opt, const float *optical, const fl
     }
     // the error words ride ahead of the one synchronisation
     unsigned *errs = ctx->host_errors;
-    errs[0] = errs[1] = 0;
-    cudaMemcpyAsync(&errs[0], ctx->main.errors.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
-    if (ctx->tma_error) cudaMemcpyAsync(&errs[1], ctx->tma_error, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+    if (cudaMemcpyAsync(errs, ctx->main.errors.ptr, Scratch::kWords * sizeof(unsigned), cudaMemcpyDeviceToHost, st) !=
+        cudaSuccess) {
+      rc = fail(CYR_ERR_CUDA, "error words' download failed: %s", cudaGetErrorString(cudaGetLastError()));
+      break;
+    }
     const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
       rc = fail(CYR_ERR_CUDA, "simulation failed: %s", cudaGetErrorString(e));
       break;
     }
-    if (errs[0] != 0) rc = fail(CYR_ERR_CUDA, "%u detector pixels needed z planes outside the kept range", errs[0]);
-    if (errs[1] != 0) rc = fail(CYR_ERR_CUDA, "an FFT tile copy did not complete within its wait limit");
+    char msg[128];
+    if (const char *what = request_error(errs, msg, sizeof msg)) rc = fail(CYR_ERR_CUDA, "%s", what);
   } while (false);
   if (rc != CYR_OK) {  // whatever was enqueued ends before the caller's buffers may go
     cudaStreamSynchronize(cs);
@@ -3682,7 +3714,9 @@ int cyr_fft3d_device(void *d_data, uint32_t nx, uint32_t ny, uint32_t nz, uint32
   CYR_TRY(get_context(&ctx));
   std::lock_guard<std::mutex> lk(ctx->mu);
   CYR_TRY(setup_attrs(*ctx));
-  return fft3d(*ctx, static_cast<float2 *>(d_data), nx, ny, nz, count, static_cast<cudaStream_t>(stream));
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  CYR_CUDA(cudaMemsetAsync(ctx->tma_error, 0, sizeof(unsigned), st));
+  return fft3d(*ctx, static_cast<float2 *>(d_data), nx, ny, nz, count, st, ColWaits{ctx->tma_error});
 }
 
 int cyr_selftest_wait_limit(int *timed_out) {
@@ -3707,7 +3741,7 @@ int cyr_selftest_wait_limit(int *timed_out) {
     tp.nxt = 1, tp.others = 1, tp.ntiles = 1, tp.axis = 1;
     tp.tw = tw;
     tp.error = ctx->tma_error;
-    tp.poll_limit = 1u << 16;  // far longer than the 64 KB copies take to land
+    tp.poll_limit = kShortWait;
     tp.extra_tx = 16;
     if (cudaMemset(d, 0, size_t(nx) * ny * sizeof(float2)) != cudaSuccess ||
         cudaMemset(ctx->tma_error, 0, sizeof(unsigned)) != cudaSuccess) {
@@ -3777,8 +3811,8 @@ int cyr_server_create(uint32_t slots, size_t hbm_budget, uint32_t flags, cyr_ser
     std::unique_ptr<Slot> sl(new Slot);
     CYR_CUDA(cudaStreamCreateWithFlags(&sl->stream, cudaStreamNonBlocking));
     CYR_CUDA(cudaEventCreateWithFlags(&sl->done, cudaEventDisableTiming));
-    CYR_CUDA(cudaMallocHost(&sl->host_errors, sizeof(unsigned)));
-    *sl->host_errors = 0;
+    CYR_CUDA(cudaMallocHost(&sl->host_errors, Scratch::kWords * sizeof(unsigned)));
+    std::fill_n(sl->host_errors, Scratch::kWords, 0u);
     sl->sc.bind(sl->stream);
     sl->vox.stream = sl->out.stream = sl->stream;
     sl->vox.generation = sl->out.generation = &sl->sc.generation;
@@ -3876,6 +3910,74 @@ int cyr_server_destroy(cyr_server *s) {
   if (!s) return CYR_OK;
   const int rc = server_destroy(s->impl);
   delete s;
+  return rc;
+}
+
+int cyr_selftest_request_waits(uint32_t *reported) {
+  if (!reported) return fail(CYR_ERR_ARGUMENT, "reported pointer is null");
+  *reported = 0;
+  DeviceContext *ctx = nullptr;
+  CYR_TRY(get_context(&ctx));
+  CYR_TRY(setup_attrs(*ctx));
+  if (!ctx->encode_tiled) return fail(CYR_ERR_UNSUPPORTED, "no tensor-map encoder in this driver");
+  // 64 x 256 x 8 voxels of one material: the y pass is the only one with tile copies, one tile per block
+  const float energy = 285.f, optical[4] = {1e-3f, 1e-4f, 5e-4f, 1e-4f}, kz[3] = {0.f, 0.f, 1.f};
+  cyr_options o{};
+  o.nx = 64, o.ny = 256, o.nz = 8;
+  o.num_material = 1, o.num_energies = 1, o.energies = &energy;
+  o.end_angle = 90.f, o.increment_angle = 30.f, o.phys_size = 5.f;
+  o.num_k = 1, o.k_vectors = kz, o.detector[2] = 1.f;
+  o.ewald_interpolation = 1, o.rot_mask = 1, o.reference_frame = 1, o.strategy = CYR_STRATEGY_FIELDS;
+  const size_t nvox = size_t(o.nx) * o.ny * o.nz, npix = size_t(o.nx) * o.ny;
+  DeviceBuffer vox, out;
+  int rc = CYR_OK;
+  do {
+    if ((rc = vox.ensure(nvox * sizeof(float4))) != CYR_OK || (rc = out.ensure(npix * sizeof(float))) != CYR_OK) break;
+    if (cudaMemset(vox.ptr, 0, nvox * sizeof(float4)) != cudaSuccess) {
+      rc = fail(CYR_ERR_CUDA, "self-test setup failed");
+      break;
+    }
+    auto request = [&](bool run_out) -> int {  // device-resident, on the plain entry points' scratch
+      std::lock_guard<std::mutex> lk(ctx->mu);
+      RunMode mode;
+      mode.waits_run_out = run_out;
+      CYR_TRY(run_request(*ctx, ctx->main, &o, optical, vox.as<float4>(), out.as<float>(), nullptr, mode));
+      return CYR_OK;
+    };
+    uint32_t errors = 0;
+    if ((rc = request(false)) != CYR_OK || (rc = cyr_device_errors(&errors)) != CYR_OK) break;  // tunes this shape too
+    if (errors != 0) {
+      rc = fail(CYR_ERR_CUDA, "the self-test's plain request reported errors");
+      break;
+    }
+    if ((rc = request(true)) != CYR_OK || (rc = cyr_device_errors(&errors)) != CYR_OK) break;
+    if (errors == 1) *reported |= 1u;
+    // served: alone (run, capture, replay) and as a group
+    for (uint32_t flags : {CYR_SERVER_GRAPHS, CYR_SERVER_GROUPS}) {
+      cyr_server *srv = nullptr;
+      if ((rc = cyr_server_create(1, 0, flags, &srv)) != CYR_OK) break;
+      srv->impl->waits_run_out = true;  // before its first request
+      uint32_t failed = 0;
+      const uint32_t n = 4;
+      std::vector<uint64_t> ids;
+      for (uint32_t i = 0; i < n && rc == CYR_OK; ++i) {
+        uint64_t id = 0;
+        rc = cyr_server_submit(srv, &o, optical, vox.ptr, out.as<float>(), 1, &id);
+        if (rc == CYR_OK) ids.push_back(id);
+      }
+      for (uint64_t id : ids) failed += cyr_server_wait(srv, id, nullptr, nullptr) == CYR_ERR_CUDA ? 1u : 0u;
+      const int rd = cyr_server_destroy(srv);
+      if (rc == CYR_OK) rc = rd;
+      if (rc != CYR_OK) break;
+      if (failed == n) *reported |= flags == CYR_SERVER_GRAPHS ? 2u : 4u;
+    }
+    if (rc != CYR_OK) break;
+    // and the next request is sound again
+    if ((rc = request(false)) != CYR_OK || (rc = cyr_device_errors(&errors)) != CYR_OK) break;
+    if (errors == 0) *reported |= 8u;
+  } while (false);
+  cudaDeviceSynchronize();
+  vox.release(), out.release();
   return rc;
 }
 

@@ -163,8 +163,9 @@ CYR_API int cyr_plan_info(const cyr_options *opt, uint32_t *info, uint32_t n);
 
 /*
  * Device-side consistency errors counted since the last request started on
- * this device (e.g. a detector pixel needed a z plane outside the kept
- * range).  Waits for the device; 0 means none.
+ * this device (a detector pixel needed a z plane outside the kept range; a
+ * tile copy of the request's transform, or of the last cyr_fft3d_device call,
+ * did not complete within its wait limit).  Waits for the device; 0 means none.
  */
 CYR_API int cyr_device_errors(uint32_t *count);
 
@@ -217,6 +218,16 @@ CYR_API int cyr_fft3d_device_static(void *d_data, uint32_t nx, uint32_t ny, uint
  * No counterpart in the reference.
  */
 CYR_API int cyr_selftest_wait_limit(int *timed_out);
+
+/*
+ * cyr_selftest_request_waits: checks that a request whose transform's waits run
+ * out (as in cyr_selftest_wait_limit, on a 64 x 256 x 8 volume) is reported and
+ * that the next one is sound.  Bits of *reported: 1 cyr_device_errors after a
+ * device-resident request, 2 served requests (run, captured, replayed), 4 a
+ * request group, 8 no error after the next request.  15 is a pass.
+ * Synchronises the device.  No counterpart in the reference.
+ */
+CYR_API int cyr_selftest_request_waits(uint32_t *reported);
 
 /*
  * cyr_warp_affine_device: bilinear affine warp of a float [height][width]
