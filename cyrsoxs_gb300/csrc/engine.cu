@@ -2843,8 +2843,9 @@ int plan_request(ServerRequest &r, bool graphs) {
                 double(r.opt.detector[2]), staged || r.indirect ? nullptr : static_cast<const void *>(r.d_vox),
                 staged || r.indirect ? nullptr : static_cast<void *>(r.d_out));
   r.key = head;
-  for (float e : r.energies) r.key += std::to_string(e) + ",";
-  for (float k : r.kvecs) r.key += std::to_string(k) + ",";
+  // bit by bit: the captured launches hold k vectors and detector warps
+  for (const std::vector<float> *v : {&r.energies, &r.kvecs})
+    r.key.append(reinterpret_cast<const char *>(v->data()), v->size() * sizeof(float));
   // requests that can share launches: FIELDS, LAB frame, k along z, device buffers; all but the
   // morphology, the energies and the optical constants equal
   r.group_key.clear();
