@@ -2562,7 +2562,8 @@ int run_fp64(DeviceContext &ctx, const cyr_options *o, const double *optical, co
   // Field spectra (one transform of the 7 M packed fields for every energy and
   // angle) when they are fewer volumes than the per-energy spectra and fit;
   // the transforms dominate both (256 x 256 x 32, 2 materials, 3 energies:
-  // 7 volumes against 15).
+  // 7 volumes against 15).  Whatever the strategy asked for, a request whose
+  // field volumes do not fit runs per energy.
   const uint32_t npk = fields64_packed(pl.nmat);
   const double per_energy = double(pl.ne) * (pl.material_frame ? 3.0 * pl.nk * pl.nang : double(nvol));
   bool fields = o->strategy == CYR_STRATEGY_FIELDS || (o->strategy == CYR_STRATEGY_AUTO && npk < per_energy);
@@ -2570,8 +2571,7 @@ int run_fp64(DeviceContext &ctx, const cyr_options *o, const double *optical, co
   const size_t image = size_t(pl.nang) * pl.npix * sizeof(double);
   const uint32_t most =
       uint32_t(std::max<size_t>(1, std::min<size_t>(std::min(pl.ne, 65535u), (size_t(512) << 20) / image)));
-  if (fields && o->strategy == CYR_STRATEGY_AUTO &&
-      (f.spec.bytes < size_t(npk) * pl.nvox * sizeof(double2) || f.images.bytes < most * image)) {
+  if (fields && (f.spec.bytes < size_t(npk) * pl.nvox * sizeof(double2) || f.images.bytes < most * image)) {
     size_t free_b = 0, total_b = 0;
     CYR_CUDA(cudaMemGetInfo(&free_b, &total_b));
     if (size_t(npk) * pl.nvox * sizeof(double2) + most * image + (size_t(1) << 30) >
