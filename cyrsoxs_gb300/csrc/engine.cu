@@ -1529,6 +1529,23 @@ int make_plan(const cyr_options *o, const float *optical, Plan &pl) {
   return CYR_OK;
 }
 
+// Whether per-energy spectra of an Euler morphology convert it once to the
+// trigonometry-free vector form: from the builds (energies, and angles in the
+// MATERIAL frame) on that repay the pass, a read and a write of the morphology.
+// Measured (us, per build without and with the converted form, and the pass):
+//   z lengths of the warp FFT, 256 x 256 x 128: 1 material 331/322 and 56, 2:
+//   365/338 and 116, 4: 428/372 and 194, 8: 552/461 and 373; 128 x 128 x 512, 4:
+//   551/432 and 189: repaid by 1.6 to 6.5 builds.
+//   other z lengths, 256 x 256 x 90: 1 material 451/455, never repaid; 2: 468/461
+//   and 82; 4: 507/473 and 139; 8: 597/532 and 262; x 120, x 64, x 61, x 48 alike:
+//   2 materials by 9 to 23 builds, 4 and 8 by 4 to 9.
+bool converts(const Plan &pl) {
+  if (!pl.euler || pl.fields) return false;
+  const size_t builds = pl.material_frame ? size_t(pl.ne) * pl.nk * pl.nang : pl.ne;
+  if (pl.zwarp) return builds >= 4;
+  return pl.nmat >= 4 ? builds >= 6 : pl.nmat > 1 && builds >= 12;
+}
+
 size_t request_bytes(const Plan &pl) {
   if (pl.fields) return field_bytes(pl) + pl.nmat * kMoments * sizeof(double) + 64 * sizeof(float2);
   return pl.nvol * pl.vstride * sizeof(float2) + (pl.euler ? pl.nvox * pl.nmat * sizeof(float4) : 0) + image_bytes(pl) + pl.npix * sizeof(float) +
@@ -2071,11 +2088,6 @@ struct RunMode {
 };
 
 
-// Builds from which the conversion pass (a read and a write of the morphology,
-// 235 us on 256 x 256 x 128 with 4 materials) repays the trigonometry that each
-// build of the unconverted form repeats: 4 us of 293 with the warp FFT (whose
-// exchanges hide it), 32 of 403 with other z lengths (x 90).
-constexpr size_t kConvertBuildsWarp = 64, kConvertBuilds = 6;
 constexpr size_t kSlabBytes = size_t(24) << 20;
 constexpr uint32_t kSampleSlabs = 2;  // slabs from which the means come from rows copied ahead of them
 
@@ -2143,10 +2155,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
   const bool slabs = mode.host_vox && pl.fields;
   // volume moments of the morphology -> mean of every tensor entry, per energy
   CYR_TRY(sc.means.ensure(size_t(pl.ne) * 6 * sizeof(float2)));
-  // Per-energy spectra of Euler morphologies: converted to the trigonometry-free
-  // vector form once per request when enough builds follow to repay the pass
-  const size_t builds = pl.material_frame ? size_t(pl.ne) * pl.nk * pl.nang : pl.ne;
-  const bool convert = o->morphology_type == 0 && !pl.fields && builds >= (pl.zwarp ? kConvertBuildsWarp : kConvertBuilds);
+  const bool convert = converts(pl);
   if (convert) CYR_TRY(sc.conv.ensure(pl.nvox * pl.nmat * sizeof(float4)));
   {
     MomentParams mp{};
