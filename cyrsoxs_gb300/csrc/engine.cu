@@ -1548,8 +1548,8 @@ bool converts(const Plan &pl) {
 
 size_t request_bytes(const Plan &pl) {
   if (pl.fields) return field_bytes(pl) + pl.nmat * kMoments * sizeof(double) + 64 * sizeof(float2);
-  return pl.nvol * pl.vstride * sizeof(float2) + (pl.euler ? pl.nvox * pl.nmat * sizeof(float4) : 0) + image_bytes(pl) + pl.npix * sizeof(float) +
-         pl.arena.size() + 64 * sizeof(float2);
+  return pl.nvol * pl.vstride * sizeof(float2) + (converts(pl) ? pl.nvox * pl.nmat * sizeof(float4) : 0) +
+         image_bytes(pl) + pl.npix * sizeof(float) + pl.arena.size() + 64 * sizeof(float2);
 }
 
 // Ewald-kernel parameters shared by every (energy, k).
