@@ -466,8 +466,8 @@ struct DeviceContext {
   std::map<std::array<uint32_t, 3>, MixTables> mix;  // key: length, row form, bytes per real
   int sms = 0;                                       // multiprocessors
   size_t max_pitch = 0;                              // bytes that the pitch of a 2D copy may have
-  std::map<size_t, int> mix_build_occupancy;         // blocks per SM of k_build_fields_mix at a shared-memory size
   std::map<std::pair<const void *, size_t>, int> occupancy;  // blocks per SM of a kernel at a shared-memory size
+  std::map<const void *, size_t> smem_allowed;               // dynamic shared memory a kernel may have (allow_smem)
   struct Fp64Scratch {
     DeviceBuffer spec, images, avg, params, params64, vox, out;
     cudaEvent_t last_use = nullptr;     // completion of the last request that used them, on whatever stream
@@ -555,6 +555,25 @@ int with_rows_kernel(bool euler, uint32_t nmat, uint32_t nx, F &&f) {
   });
 }
 
+// Allows a kernel `smem` bytes of dynamic shared memory, at its first launch with that much: the call also loads the
+// kernel's code, and doing so for every kernel took a process's first request 35 ms.  48 KB in all need no leave; what
+// is above 32 KB asks for it, which leaves room for the static arrays of the kernels that have both.
+constexpr size_t kFreeSmem = 32 * 1024;
+int allow_smem_locked(DeviceContext &ctx, const void *kern, size_t smem) {
+  if (smem <= kFreeSmem) return CYR_OK;
+  size_t &allowed = ctx.smem_allowed[kern];
+  if (smem <= allowed) return CYR_OK;
+  CYR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  allowed = smem;
+  return CYR_OK;
+}
+template <class K>
+int allow_smem(DeviceContext &ctx, K kern, size_t smem) {
+  if (smem <= kFreeSmem) return CYR_OK;
+  std::lock_guard<std::mutex> lk(ctx.tables_mu);
+  return allow_smem_locked(ctx, reinterpret_cast<const void *>(kern), smem);
+}
+
 // Resident blocks per SM of a kernel (a driver query of 1 to 2 us, made once per kernel and shared-memory size).
 template <class K>
 int blocks_per_sm(DeviceContext &ctx, K kern, int threads, size_t smem, int *out) {
@@ -562,8 +581,9 @@ int blocks_per_sm(DeviceContext &ctx, K kern, int threads, size_t smem, int *out
   const std::pair<const void *, size_t> key(reinterpret_cast<const void *>(kern), smem);
   auto it = ctx.occupancy.find(key);
   if (it == ctx.occupancy.end()) {
+    CYR_TRY(allow_smem_locked(ctx, key.first, smem));
     int n = 0;
-    CYR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem));
+    CYR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, key.first, threads, smem));
     it = ctx.occupancy.emplace(key, n).first;
   }
   *out = it->second;
@@ -573,51 +593,6 @@ int blocks_per_sm(DeviceContext &ctx, K kern, int threads, size_t smem, int *out
 int setup_attrs(DeviceContext &ctx) {
   std::lock_guard<std::mutex> lk(ctx.tables_mu);
   if (ctx.attrs_done) return CYR_OK;
-  const int smem = int(kFftSmemBudget);
-  CYR_CUDA(mix_attributes<float2>(smem));
-  CYR_CUDA(mix_attributes<double2>(smem));
-  CYR_CUDA(mix_build_attributes(smem));
-#define CYR_COLS_ATTR(V, T) \
-  CYR_CUDA(cudaFuncSetAttribute(k_fft_cols<V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CYR_COLS_ATTR(32, 8)
-  CYR_CUDA(cudaFuncSetAttribute(k_fft_rows<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CYR_COLS_ATTR(4, kColsTxY) CYR_COLS_ATTR(8, kColsTxY) CYR_COLS_ATTR(16, kColsTxY)
-  CYR_COLS_ATTR(4, kColsTxZ) CYR_COLS_ATTR(8, kColsTxZ) CYR_COLS_ATTR(16, kColsTxZ)
-#undef CYR_COLS_ATTR
-  CYR_CUDA(cudaFuncSetAttribute(k_build_fft_z<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CYR_CUDA(cudaFuncSetAttribute(k_build_fft_z<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CYR_CUDA(cudaFuncSetAttribute(k_build_fft_z<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-#define CYR_WARP_Z_ATTR(V, T)                                                                                     \
-  CYR_CUDA(cudaFuncSetAttribute(k_build_fft_z_warp<0, true, V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));  \
-  CYR_CUDA(cudaFuncSetAttribute(k_build_fft_z_warp<0, false, V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
-  CYR_CUDA(cudaFuncSetAttribute(k_build_fft_z_warp<1, false, V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-#define CYR_WARP_Z_ATTR_V(V) CYR_WARP_Z_ATTR(V, 2) CYR_WARP_Z_ATTR(V, 4) CYR_WARP_Z_ATTR(V, 8)
-  CYR_WARP_Z_ATTR_V(4)
-  CYR_WARP_Z_ATTR_V(8)
-  CYR_WARP_Z_ATTR_V(16)
-#undef CYR_WARP_Z_ATTR_V
-#undef CYR_WARP_Z_ATTR
-  CYR_CUDA(cudaFuncSetAttribute(k_fft_cols_tma<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cols_tma_smem(256))));
-#define CYR_WS_ATTR(V, H, S)                                                                               \
-  CYR_CUDA(cudaFuncSetAttribute(k_fft_cols_tma_ws<V, H, S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                int(cols_tma_ws_smem<V, H, S>())));                                         \
-  CYR_CUDA(cudaFuncSetAttribute(k_fft_cols_tma_ws<V, H, S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                int(cols_tma_ws_smem<V, H, S>())));
-  CYR_WS_ATTR(16, 1, 2)
-  CYR_WS_ATTR(8, 2, 3)
-  CYR_WS_ATTR(8, 2, 2)
-  CYR_WS_ATTR(4, 1, 2)
-  CYR_WS_ATTR(4, 2, 3)
-#undef CYR_WS_ATTR
-  CYR_CUDA(cudaFuncSetAttribute(k_fft_cols_tma64<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                int(cols_tma64_smem(1024))));
-  for (bool euler : {true, false})
-    for (uint32_t nmat = 0; nmat <= 4; ++nmat)
-      for (uint32_t nx : {128u, 256u, 512u, 1024u})
-        CYR_TRY(with_rows_kernel(euler, nmat, nx, [&](auto kern) -> int {
-          CYR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-          return CYR_OK;
-        }));
   {
     cudaDriverEntryPointQueryResult q{};
     void *fn = nullptr;
@@ -699,6 +674,7 @@ int warp_fft_pass_v(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, 
   if (axis == 0) {
     RowPassParams rp{data, uint32_t(size_t(ny) * nz * count), tw, ny * nz, nvox};
     const size_t smem = (N + 8 * N) * sizeof(float2);
+    CYR_TRY(allow_smem(ctx, k_fft_rows<V>, smem));
     k_fft_rows<V><<<(rp.rows + 7) / 8, 256, smem, st>>>(rp);
   } else if (V == 32 && nx % 8 == 0 && ctx.encode_tiled && form != kFormCp) {
     // 1024-point lines: 8-column tiles (k_fft_cols_tma64)
@@ -789,18 +765,20 @@ int warp_fft_pass_v(DeviceContext &ctx, float2 *data, uint32_t nx, uint32_t ny, 
       cp.others = ny, cp.ostride = nx, cp.estride = nx * ny;
     }
     cp.tw = tw;
-    auto launch = [&](auto txc) {
+    auto launch = [&](auto txc) -> int {
       constexpr uint32_t TX = decltype(txc)::value;
       const size_t smem = (N + TX * line_stride(N, TX)) * sizeof(float2);
       const dim3 grid(((nx + TX - 1) / TX) * cp.others, count);
+      CYR_TRY(allow_smem(ctx, k_fft_cols<V, TX>, smem));
       k_fft_cols<V, TX><<<grid, TX * 32, smem, st>>>(cp);
+      return CYR_OK;
     };
     if (V == 32)  // 1024-point columns: 8 per block keeps the tile at 64 KB
-      launch(std::integral_constant<uint32_t, 8>{});
+      CYR_TRY(launch(std::integral_constant<uint32_t, 8>{}));
     else if (axis == 1)
-      launch(std::integral_constant<uint32_t, kColsTxY>{});
+      CYR_TRY(launch(std::integral_constant<uint32_t, kColsTxY>{}));
     else
-      launch(std::integral_constant<uint32_t, kColsTxZ>{});
+      CYR_TRY(launch(std::integral_constant<uint32_t, kColsTxZ>{}));
   }
   ctx.prof.end(slot, st);
   CYR_CUDA(cudaGetLastError());
@@ -1049,6 +1027,7 @@ int mix_pass(DeviceContext &ctx, T *data, uint32_t nx, uint32_t ny, uint32_t nz,
   if (smem > kMixSmemMax) return fail(CYR_ERR_UNSUPPORTED, "FFT length %u too large for one block", M);
   const MixForm form = !conv ? kMixPlain : conv->in ? kMixRader : kMixBluestein;
   const int slot = ctx.prof.begin(conv ? int(kBluestein) : kFftX + axis, st);
+  CYR_TRY(allow_smem(ctx, mix_kernel<T>(form, row), smem));
   CYR_CUDA(mix_launch<T>(form, row, dim3(blocks, count), threads, smem, st, p));
   ctx.prof.end(slot, st);
   return CYR_OK;
@@ -1743,12 +1722,7 @@ int launch_fused_build(DeviceContext &ctx, const FieldParams &fp, uint32_t npk, 
   q.m.rows = rpb;
   const size_t smem = rpb * row;
   if (smem > kMixSmemMax) return fail(CYR_ERR_UNSUPPORTED, "row length %u too large for the fused build", fp.nx);
-  {
-    std::lock_guard<std::mutex> lk(ctx.tables_mu);
-    auto it = ctx.mix_build_occupancy.find(smem);
-    if (it == ctx.mix_build_occupancy.end()) it = ctx.mix_build_occupancy.emplace(smem, mix_build_blocks(smem)).first;
-    per_sm = it->second;
-  }
+  CYR_TRY(blocks_per_sm(ctx, mix_build_kernel(), kMixThreads, smem, &per_sm));
   const int slot = ctx.prof.begin(kBuildFieldsRows, st);
   CYR_CUDA(mix_build_launch(grid((rows + rpb - 1) / rpb), smem, st, q));
   ctx.prof.end(slot, st);
@@ -1816,9 +1790,11 @@ int field_zmask(DeviceContext &ctx, Scratch &sc, const EwaldGeom &g, const float
 
 // Autotuning of the FIELDS transform for one shape (the first device-resident
 // request of it on this device): the fused or separate build + x pass and the
-// launch form of the y and z passes each run twice on the packed-field buffer,
-// before the build overwrites every element of it.  The second runs are timed
-// (the first also loads the kernel's code) and the fastest kept.  Every
+// launch form of the y and z passes are each timed once on the packed-field
+// buffer, before the build overwrites every element of it, and the fastest
+// kept.  Each runs on one plane or one volume first, because a kernel's first
+// launch in a process also loads its code, which made the fused build of small
+// volumes look slower than the separate one in some processes.  Every
 // candidate computes the same numbers.
 int tune_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Plan &pl, const FieldParams &fp,
                 bool fused_ok, cudaStream_t st, DeviceContext::FieldTune &ft,
@@ -1843,18 +1819,16 @@ int tune_fields(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const Pla
     CYR_CUDA(cudaEventCreate(&c.b));
   }
   int rc = CYR_OK;
-  // each candidate runs twice and its second run is timed: a kernel's first launch in a process also loads its code,
-  // which made the fused build of small volumes look slower than the separate one in some processes
-  for (int pass = 0; pass < 2 && rc == CYR_OK; ++pass)
+  for (bool timed : {false, true})
     for (Cand &c : cands) {
-      if (pass) CYR_CUDA(cudaEventRecord(c.a, st));
-      if (c.kind == 0)
-        rc = build_fields_x(ctx, sc, o, pl, fp, 0, pl.nz, c.choice == 1, st, waits);
-      else
-        rc = warp_fft_pass(ctx, sc.spec.as<float2>(), pl.nx, pl.ny, pl.nz, pl.npk, c.kind, st, pl.nvox, waits, c.choice,
-                           c.kind == 2 ? zmask : nullptr);
       if (rc != CYR_OK) break;
-      if (pass) CYR_CUDA(cudaEventRecord(c.b, st));
+      if (timed) CYR_CUDA(cudaEventRecord(c.a, st));
+      if (c.kind == 0)
+        rc = build_fields_x(ctx, sc, o, pl, fp, 0, timed ? pl.nz : 1u, c.choice == 1, st, waits);
+      else
+        rc = warp_fft_pass(ctx, sc.spec.as<float2>(), pl.nx, pl.ny, timed || c.kind == 2 ? pl.nz : 1u,
+                           timed ? pl.npk : 1u, c.kind, st, pl.nvox, waits, c.choice, c.kind == 2 ? zmask : nullptr);
+      if (timed && rc == CYR_OK) CYR_CUDA(cudaEventRecord(c.b, st));
     }
   if (rc == CYR_OK) {
     CYR_CUDA(cudaEventSynchronize(cands.back().b));
@@ -2246,18 +2220,24 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
       zp.zlo = pl.zlo;
       zp.kz = pl.kz;
       zp.out = spec;
+      auto launch_z = [&](auto kern, dim3 g, int threads, size_t smem) -> int {
+        CYR_TRY(allow_smem(ctx, kern, smem));
+        kern<<<g, threads, smem, st>>>(zp, mce);
+        return CYR_OK;
+      };
       if (pl.zwarp) {
-        auto launch_warp = [&](const ZTune &cfg) {
+        // one_block: only to load the code (the autotuner's first round)
+        auto launch_warp = [&](const ZTune &cfg, bool one_block = false) -> int {
           zp.stage = cfg.stage ? 1u : 0u;
           zp.tx = cfg.tx;
-          const dim3 g((pl.nx + cfg.tx - 1) / cfg.tx * pl.ny);
+          const dim3 g(one_block ? 1u : (pl.nx + cfg.tx - 1) / cfg.tx * pl.ny);
           const size_t smem = zwarp_smem(pl.nz, bp.nvol, cfg.tx, pl.nmat, cfg.stage);
-#define CYR_LAUNCH_WARP_ZT(V, T)                                                   \
-  if (o->morphology_type == 0) {                                                   \
-    if (convert) k_build_fft_z_warp<0, true, V, T><<<g, 256, smem, st>>>(zp, mce); \
-    k_build_fft_z_warp<0, false, V, T><<<g, 256, smem, st>>>(zp, mce);             \
-  } else {                                                                         \
-    k_build_fft_z_warp<1, false, V, T><<<g, 256, smem, st>>>(zp, mce);             \
+#define CYR_LAUNCH_WARP_ZT(V, T)                                                         \
+  if (o->morphology_type == 0) {                                                         \
+    if (convert) CYR_TRY(launch_z(k_build_fft_z_warp<0, true, V, T>, g, 256, smem));     \
+    CYR_TRY(launch_z(k_build_fft_z_warp<0, false, V, T>, g, 256, smem));                 \
+  } else {                                                                               \
+    CYR_TRY(launch_z(k_build_fft_z_warp<1, false, V, T>, g, 256, smem));                 \
   }
 #define CYR_LAUNCH_WARP_Z(V)         \
   if (cfg.tx == 2) {                 \
@@ -2276,6 +2256,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
           }
 #undef CYR_LAUNCH_WARP_Z
 #undef CYR_LAUNCH_WARP_ZT
+          return CYR_OK;
         };
         char key[96];
         std::snprintf(key, sizeof key, "%u,%u,%u,%u,%u,%u", pl.nx, pl.ny, pl.nz, pl.nmat, bp.nvol,
@@ -2292,12 +2273,12 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
           // autotune: time every candidate on this energy
           std::vector<cudaEvent_t> ev(2 * pl.zcands.size());
           for (auto &e : ev) CYR_CUDA(cudaEventCreate(&e));
-          for (int pass = 0; pass < 2; ++pass)  // the second run is timed: the first also loads the code
-            for (size_t c = 0; c < pl.zcands.size(); ++c) {
-              if (pass) CYR_CUDA(cudaEventRecord(ev[2 * c], st));
-              launch_warp(pl.zcands[c]);
-              if (pass) CYR_CUDA(cudaEventRecord(ev[2 * c + 1], st));
-            }
+          for (const ZTune &c : pl.zcands) CYR_TRY(launch_warp(c, true));
+          for (size_t c = 0; c < pl.zcands.size(); ++c) {
+            CYR_CUDA(cudaEventRecord(ev[2 * c], st));
+            CYR_TRY(launch_warp(pl.zcands[c]));
+            CYR_CUDA(cudaEventRecord(ev[2 * c + 1], st));
+          }
           CYR_CUDA(cudaGetLastError());
           CYR_CUDA(cudaEventSynchronize(ev.back()));
           ZTune best = pl.zcands[0];
@@ -2312,7 +2293,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
             std::lock_guard<std::mutex> lk(ctx.tables_mu);
             ctx.ztune[key] = best;
           }
-          launch_warp(best);  // the kept output must come from a full, ordered launch of the chosen form
+          CYR_TRY(launch_warp(best));  // the kept output must come from a full, ordered launch of the chosen form
         } else {
           ZTune cfg;
           if (have_tuned) {
@@ -2322,7 +2303,7 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
             cfg.tx = pl.ztx;
           }
           slot = ctx.prof.begin(kBuildZ, st, convert ? 2 : 1);
-          launch_warp(cfg);
+          CYR_TRY(launch_warp(cfg));
           ctx.prof.end(slot, st);
         }
       } else {
@@ -2330,10 +2311,10 @@ int run_request(DeviceContext &ctx, Scratch &sc, const cyr_options *o, const flo
         slot = ctx.prof.begin(kBuildZ, st, convert ? 2 : 1);
         const size_t smem = (size_t(2) * bp.nvol * pl.nz * (pl.ztx + 1) + pl.nz) * sizeof(float2);
         if (o->morphology_type == 0) {
-          if (convert) k_build_fft_z<0, true><<<grid, kFftThreads, smem, st>>>(zp, mce);
-          k_build_fft_z<0, false><<<grid, kFftThreads, smem, st>>>(zp, mce);
+          if (convert) CYR_TRY(launch_z(k_build_fft_z<0, true>, grid, kFftThreads, smem));
+          CYR_TRY(launch_z(k_build_fft_z<0, false>, grid, kFftThreads, smem));
         } else {
-          k_build_fft_z<1, false><<<grid, kFftThreads, smem, st>>>(zp, mce);
+          CYR_TRY(launch_z(k_build_fft_z<1, false>, grid, kFftThreads, smem));
         }
         ctx.prof.end(slot, st);
       }
@@ -3758,7 +3739,9 @@ int cyr_selftest_wait_limit(int *timed_out) {
       rc = fail(CYR_ERR_CUDA, "self-test setup failed");
       break;
     }
-    k_fft_cols_tma_ws<8, 2, 3><<<1, 17 * 32, cols_tma_ws_smem<8, 2, 3>()>>>(map, map, tp);
+    const auto kern = k_fft_cols_tma_ws<8, 2, 3, false>;
+    if ((rc = allow_smem(*ctx, kern, cols_tma_ws_smem<8, 2, 3>())) != CYR_OK) break;
+    kern<<<1, 17 * 32, cols_tma_ws_smem<8, 2, 3>()>>>(map, map, tp);
     const cudaError_t e = cudaDeviceSynchronize();
     unsigned flag = 0;
     if (e != cudaSuccess || cudaMemcpy(&flag, ctx->tma_error, sizeof flag, cudaMemcpyDeviceToHost) != cudaSuccess) {

@@ -96,12 +96,6 @@ cudaError_t mix_build_launch(dim3 grid, size_t smem, cudaStream_t st, const MixB
   k_build_fields_mix<<<grid, kMixThreads, smem, st>>>(p);
   return cudaGetLastError();
 }
-cudaError_t mix_build_attributes(int smem) {
-  return cudaFuncSetAttribute(k_build_fields_mix, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-}
-int mix_build_blocks(size_t smem) {
-  int n = 0;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_build_fields_mix, kMixThreads, smem) == cudaSuccess ? n : 0;
-}
+const void *mix_build_kernel() { return reinterpret_cast<const void *>(k_build_fields_mix); }
 
 }  // namespace cyr

@@ -493,15 +493,13 @@ struct MixBuildParams {
   uint32_t form;             // 5 (morphology) + material count up to 4 (0: any)
 };
 cudaError_t mix_build_launch(dim3 grid, size_t smem, cudaStream_t st, const MixBuildParams &p);
-cudaError_t mix_build_attributes(int smem);
-int mix_build_blocks(size_t smem);  // resident blocks per SM
+const void *mix_build_kernel();
 
 // The kernel instances live in translation units of their own (mixfft_f32.cu, mixfft_f64.cu).
 template <class T>
 cudaError_t mix_launch(MixForm form, bool row, dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
                        const MixParams<T> &p);
-// Sets the instances' shared-memory limit on the current device.
 template <class T>
-cudaError_t mix_attributes(int smem);
+const void *mix_kernel(MixForm form, bool row);
 
 }  // namespace cyr

@@ -3,28 +3,25 @@
 
 namespace cyr {
 
+namespace {
+using Kernel = void (*)(MixParams<double2>);
+Kernel kernel(MixForm form, bool row) {
+  return form == kMixPlain   ? (row ? k_mix_fft<double2, false, kMixPlain> : k_mix_fft<double2, true, kMixPlain>)
+         : form == kMixRader ? (row ? k_mix_fft<double2, false, kMixRader> : k_mix_fft<double2, true, kMixRader>)
+                             : (row ? k_mix_fft<double2, false, kMixBluestein> : k_mix_fft<double2, true, kMixBluestein>);
+}
+}  // namespace
+
 template <>
 cudaError_t mix_launch<double2>(MixForm form, bool row, dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
                                const MixParams<double2> &p) {
-  auto kern = form == kMixPlain   ? (row ? k_mix_fft<double2, false, kMixPlain> : k_mix_fft<double2, true, kMixPlain>)
-              : form == kMixRader ? (row ? k_mix_fft<double2, false, kMixRader> : k_mix_fft<double2, true, kMixRader>)
-                                  : (row ? k_mix_fft<double2, false, kMixBluestein> : k_mix_fft<double2, true, kMixBluestein>);
-  kern<<<grid, threads, smem, st>>>(p);
+  kernel(form, row)<<<grid, threads, smem, st>>>(p);
   return cudaGetLastError();
 }
 
 template <>
-cudaError_t mix_attributes<double2>(int smem) {
-  const void *kernels[] = {
-      (const void *)k_mix_fft<double2, false, kMixPlain>,     (const void *)k_mix_fft<double2, true, kMixPlain>,
-      (const void *)k_mix_fft<double2, false, kMixRader>,     (const void *)k_mix_fft<double2, true, kMixRader>,
-      (const void *)k_mix_fft<double2, false, kMixBluestein>, (const void *)k_mix_fft<double2, true, kMixBluestein>,
-  };
-  for (const void *k : kernels) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+const void *mix_kernel<double2>(MixForm form, bool row) {
+  return reinterpret_cast<const void *>(kernel(form, row));
 }
 
 }  // namespace cyr
