@@ -120,9 +120,11 @@ bool smooth7(uint32_t n) {
   return factorize(n, r);
 }
 
-// The FP64 pipeline's padded length M >= 2N - 1 for lengths with a prime
-// factor above 7: the next power of two while that is at most 1024, else the
-// smallest 7-smooth M.  It also bounds the lengths both precisions accept.
+// The lengths with a prime factor above 7 that are accepted, in both
+// precisions: those whose padding M >= 2N - 1 (the next power of two while that
+// is at most 1024, else the smallest 7-smooth M) is at most kMaxBluesteinPad.
+// What runs them is another matter (fft_axes): 11 and 13 are radices, the rest
+// are Rader's or Bluestein's convolutions, padded by mix_bluestein_length.
 constexpr uint32_t kMaxBluesteinPad = 4096;
 uint32_t bluestein_length(uint32_t n) {
   uint32_t p2 = 128;
@@ -133,8 +135,8 @@ uint32_t bluestein_length(uint32_t n) {
   return m;
 }
 
-// An axis length the FFT handles: 7-smooth within one block's shared memory,
-// or any other length whose Bluestein length is at most kMaxBluesteinPad.
+// An axis length that is accepted: 7-smooth within one block's shared memory,
+// or any other length whose bluestein_length is at most kMaxBluesteinPad.
 bool fft_length_ok(uint32_t n, const char **why) {
   if (n <= 1) return true;
   if (smooth7(n)) {
@@ -145,7 +147,7 @@ bool fft_length_ok(uint32_t n, const char **why) {
     return true;
   }
   if (n > (kMaxBluesteinPad + 1) / 2 || bluestein_length(n) > kMaxBluesteinPad) {
-    *why = "has a prime factor above 7 and exceeds the Bluestein limit of 2048";
+    *why = "has a prime factor above 7 and exceeds the limit of 2048 points for such lengths (the Bluestein limit)";
     return false;
   }
   return true;
@@ -2466,8 +2468,8 @@ int make_plan64(const cyr_options *o, const double *optical, bool window, Plan &
   if (!optical) return fail(CYR_ERR_ARGUMENT, "optical constants pointer is null");
   for (uint32_t n : {o->nx, o->ny, o->nz})
     if (n > 1 && !smooth7(n) && (n > (kMaxBluesteinPad + 1) / 2 || bluestein_length(n) > kMaxBluesteinPad))
-      return fail(CYR_ERR_UNSUPPORTED, "FP64 path: dimension %u has a prime factor above 7 and exceeds the Bluestein "
-                  "limit of 2048", n);
+      return fail(CYR_ERR_UNSUPPORTED, "FP64 path: dimension %u has a prime factor above 7 and exceeds the limit of "
+                  "2048 points for such lengths", n);
   // geometry (k frames, E rotations, q tables, warp coefficients) from the FP32 planner
   std::vector<float> of(size_t(o->num_energies) * o->num_material * 4);
   for (size_t i = 0; i < of.size(); ++i) of[i] = float(optical[i]);
@@ -2736,8 +2738,10 @@ int run_fp64(DeviceContext &ctx, const cyr_options *o, const double *optical, co
 // (request_bytes + staging) fits in the HBM budget next to the requests in
 // flight; completion is detected with one event per slot.  Optionally a slot
 // replays a CUDA graph of a request signature it has already run (the same
-// options and input pointers; the optical constants travel in the parameter
-// arena, which each replay rewrites in the slot's pinned host copy).
+// options, bit by bit; the optical constants and, for FIELDS requests on device
+// buffers, the buffers' addresses travel in the parameter arena, which each
+// replay rewrites in the slot's pinned host copy; other requests run on the
+// slot's staging buffers).
 // ---------------------------------------------------------------------------
 using Clock = std::chrono::steady_clock;
 

@@ -118,7 +118,9 @@ CYR_API int cyr_compute_polarization(const cyr_options *opt, const float *optica
  * DC replacement, intensity, interpolation, warps, angle mean); the discrete
  * decisions (NaN pixels, Ewald planes, warp taps) are made in float exactly as
  * the FP32 path makes them, so the NaN masks equal cyr_cuda_main's.  Axis
- * lengths must be 7-smooth (2^a 3^b 5^c 7^d).
+ * lengths as for cyr_cuda_main: any up to 2048, beyond that 7-smooth
+ * (2^a 3^b 5^c 7^d) up to 6144.  `strategy` as there, except that field
+ * volumes that do not fit the device make the request run PER_ENERGY.
  */
 CYR_API int cyr_cuda_main_fp64(const cyr_options *opt, const double *optical, const double *voxels, double *projection);
 
@@ -269,8 +271,9 @@ CYR_API uint32_t cyr_num_stages(void);
  * memory at creation; a request larger than the budget runs alone).  Each
  * request computes exactly what cyr_cuda_main computes for it.  With
  * CYR_SERVER_GRAPHS a slot captures a CUDA graph of a request signature
- * (options and buffer pointers) the second time it runs it, and replays it
- * for later requests with the same signature.
+ * (the options, energies and k vectors bit by bit; not the optical constants,
+ * nor the buffers' addresses) the second time it runs it, and replays it for
+ * later requests with the same signature.
  * ------------------------------------------------------------------------ */
 typedef struct cyr_server cyr_server;
 #define CYR_SERVER_GRAPHS 1u
