@@ -2816,9 +2816,11 @@ constexpr double kMaxInflightWork = 2.0;
 int plan_request(ServerRequest &r, bool graphs) {
   Plan &pl = r.plan;
   CYR_TRY(make_plan(&r.opt, r.optical.data(), pl));
-  // (a morphology that the kernels' 16-byte loads could not read in place is staged, as before)
-  r.indirect = graphs && r.d_vox && pl.fields && reinterpret_cast<uintptr_t>(r.d_vox) % sizeof(float4) == 0;
-  r.staged = r.h_vox != nullptr || (graphs && !r.indirect);
+  // device buffers that the kernels could not address in place (16-byte loads, 4-byte stores) are staged
+  const bool aligned = reinterpret_cast<uintptr_t>(r.d_vox) % sizeof(float4) == 0 &&
+                       reinterpret_cast<uintptr_t>(r.d_out) % sizeof(float) == 0;
+  r.indirect = graphs && r.d_vox && pl.fields && aligned;
+  r.staged = r.h_vox != nullptr || !aligned || (graphs && !r.indirect);
   const bool staged = r.staged;
   if (r.indirect) {
     const void *ptrs[2] = {r.d_vox, r.d_out};
@@ -2843,7 +2845,7 @@ int plan_request(ServerRequest &r, bool graphs) {
   // requests that can share launches: FIELDS, LAB frame, k along z, device buffers; all but the
   // morphology, the energies and the optical constants equal
   r.group_key.clear();
-  if (pl.fields && !pl.material_frame && r.opt.case_type == 0 && pl.nk == 1 && pl.nbasis == 2 && r.d_vox) {
+  if (pl.fields && !pl.material_frame && r.opt.case_type == 0 && pl.nk == 1 && pl.nbasis == 2 && r.d_vox && aligned) {
     char g[256];
     std::snprintf(g, sizeof g, "%u,%u,%u,%u,%u,%a,%a,%a,%a,%u,%u,%u,%u", r.opt.nx, r.opt.ny, r.opt.nz,
                   r.opt.num_material, r.opt.num_energies, double(r.opt.start_angle), double(r.opt.end_angle),
