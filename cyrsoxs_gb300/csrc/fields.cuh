@@ -62,13 +62,12 @@ __global__ void __launch_bounds__(256) k_build_fields(FieldParams p) {
 // The packed volumes leave the chip once, already x-transformed: the build's
 // write and the row pass's read-back of 8 npk bytes per voxel are gone.
 // Shared memory: (npk + 1) N float2 (lines and twiddles).  What bounds it:
-// issue (62% active) and the load and shared-memory latencies of 32% occupancy.
+// issue (57% active) and the load and shared-memory latencies of 33% occupancy.
 // The material count at compile time took the field places, parities and index
-// products out of every voxel: 3.41 -> 2.76 ms on 256 x 512 x 512 with 4 materials (with 14
-// packed volumes for 15), 70 -> 58 us on 256 x 256 x 32 with 2.  Three blocks per SM
+// products out of every voxel: 3.41 -> 2.92 ms on 256 x 512 x 512 with 4 materials,
+// 70 -> 58 us on 256 x 256 x 32 with 2.  Three blocks per SM
 // (80 registers) measured faster than two blocks that also stage the next
-// row's voxels in shared memory with cp.async; seven warps for 7 or 14 lines
-// were slower (2.90 ms).  (A hardware sine/cosine for
+// row's voxels in shared memory with cp.async.  (A hardware sine/cosine for
 // the Euler angles saved 0.17 ms of 3.6 on the 256 x 512 x 512 request but
 // doubled the full-size error against FP64, to 3.6e-5: not kept.)
 __host__ __device__ constexpr size_t fields_rows_smem(uint32_t n, uint32_t npk, uint32_t nmat) {

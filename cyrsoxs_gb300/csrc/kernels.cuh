@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(256) k_moments(MomentParams p) {
   // each of the first three exchanges a lane keeps half of its slots and gives
   // the other half away, so 4 + 2 + 1 + 1 + 1 double additions do the work of
   // 7 x 5; the FP64 pipe (1/64 of the FP32 rate) is what this reduction waits
-  // for (37 -> 12 us on 256 x 256 x 32, 2 materials, with the rest of the kernel).
+  // for (37 -> 14 us on 256 x 256 x 32, 2 materials, with the rest of the kernel).
   const uint32_t lane = threadIdx.x & 31u;
   double v[8];
 #pragma unroll

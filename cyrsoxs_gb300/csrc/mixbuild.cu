@@ -6,8 +6,8 @@
 // its slot in the row form's padded order.
 // What bounds it: issue, as k_build_fields_rows; the morphology type and material
 // count are one uniform branch per voxel around the unrolled field code.
-// Measured, build + x, separate and fused: 240 x 240 x 90, 3 materials 276 -> 222 us;
-// 450 x 450 x 75, 3 materials 1051 -> 786 us.  The rows of a block are chosen for full rounds of its
+// Measured, build + x, separate and fused: 240 x 240 x 90, 3 materials 268 -> 216 us;
+// 450 x 450 x 75, 3 materials 1042 -> 782 us.  The rows of a block are chosen for full rounds of its
 // 256 threads (two rows of 240: 292 us, three: 222); three blocks per SM (four, with smaller tiles: 249 us).
 #include "mixfft.cuh"
 
